@@ -51,6 +51,35 @@ def test_gemm_simt_fp32(dev, M, N, K, epilogue):
     assert torch.allclose(out.double(), ref.double(), atol=2e-5, rtol=1e-5)
 
 
+@pytest.mark.parametrize("N,K", [(96, 64), (200, 132), (2048, 2048), (72, 1030), (3000, 516)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+def test_gemm_simt_rows_are_the_same_bits_in_every_form(dev, N, K, epilogue):
+    """A row's result is the same bits whichever form its batch takes: few rows (edges of the compiled row counts), tiles
+    of 64 and 128, copied 16 bytes at a time or (an operand off 16 bytes, a row stride or K off four) one by one."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(N + K + epilogue)
+    n_w = (2 if epilogue == 2 else 1) * N
+    a = torch.randn(1025, K, device=dev, generator=g)
+    w = torch.randn(n_w, K, device=dev, generator=g) / math.sqrt(K)
+    prior = torch.randn(1025, N, device=dev, generator=g)
+    whole = prior.clone()
+    ops.gemm_simt(a, w, whole, epilogue)
+    ref = _ref_gemm(a.double(), w.double(), epilogue, None, prior.double())
+    assert torch.allclose(whole.double(), ref, atol=2e-5, rtol=1e-5)
+    for first, M in ((3, 1), (0, 2), (5, 3), (0, 4), (9, 7), (0, 8), (1, 16), (0, 17), (7, 64), (0, 65), (0, 129), (0, 300)):
+        out = prior[first:first + M].clone()
+        ops.gemm_simt(a[first:first + M], w, out, epilogue)
+        assert torch.equal(out, whole[first:first + M]), (first, M)
+    shifted = torch.empty(1025 * (K + 3) + 1, device=dev)[1:].view(1025, K + 3)[:, :K]  # 4 bytes off, rows K + 3 apart
+    shifted.copy_(a)
+    w_off = torch.empty(n_w * K + 1, device=dev)[1:].view(n_w, K)
+    w_off.copy_(w)
+    for M in (1, 5, 40, 1025):
+        out = prior[:M].clone()
+        ops.gemm_simt(shifted[:M], w_off, out, epilogue)
+        assert torch.equal(out, whole[:M]), M
+
+
 @pytest.mark.parametrize("M,N,K", GEMM_SHAPES)
 @pytest.mark.parametrize("epilogue", [0, 1, 2])
 @pytest.mark.parametrize("max_splits", [1, 16])
