@@ -19,6 +19,9 @@ namespace {
 
 constexpr int NT = 1024;
 constexpr int SMEM_CAND = 1024;
+constexpr int MAX_SPLIT = 32;     // CTAs of a row at most
+constexpr int SPLIT_CAND = 2048;  // candidates that the CTAs of a row hand to the last of them at most
+constexpr int SPLIT_WORDS = MAX_SPLIT + SPLIT_CAND;  // words a row: the best word or the number of candidates of every part, then the candidates
 
 __device__ __forceinline__ unsigned ordered_key(float v) {
   // larger float -> larger key; NaN and infinities are never candidates, they map to 0
@@ -36,7 +39,7 @@ __device__ __forceinline__ unsigned long long composite(unsigned key, unsigned i
 }
 
 struct Shared {
-  unsigned long long cand[SMEM_CAND];
+  unsigned long long cand[SPLIT_CAND];
   float prob[SMEM_CAND];
   float fscan[NT];
   int iscan[NT];
@@ -124,15 +127,36 @@ __device__ __forceinline__ int argmax_id(unsigned long long best) {
 }
 __device__ int block_argmax(const float* row, int V, Shared& sh) { return argmax_id(block_argmax_word(row, 0, V, sh)); }
 
-// The m best candidates by (key desc, id asc) into sh.cand[0..m) sorted; m <= SMEM_CAND, m <= n_finite.
-__device__ void select_sorted(const float* row, int V, float temp, int m, Shared& sh) {
+// sh.cand[0..n) in descending order; n <= SPLIT_CAND (bitonic, over the next power of two).
+__device__ void sort_candidates(int n, Shared& sh) {
+  int n2 = 2;
+  while (n2 < n) n2 <<= 1;
+  for (int i = n + threadIdx.x; i < n2; i += NT) sh.cand[i] = 0ull;
+  __syncthreads();
+  const int p = threadIdx.x;  // a pair of every step; SPLIT_CAND / 2 threads at most
+  for (int size = 2; size <= n2; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      if (p < n2 >> 1) {
+        const int i = 2 * p - (p & (stride - 1)), j = i + stride;
+        const bool desc = (i & size) == 0;
+        const unsigned long long a = sh.cand[i], b = sh.cand[j];
+        if ((a < b) == desc) { sh.cand[i] = b; sh.cand[j] = a; }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// The m best candidates of row[first..V) by (key desc, id asc) into sh.cand[0..m) sorted; m <= SMEM_CAND, and there are
+// as many.
+__device__ void select_sorted(const float* row, int first, int V, float temp, int m, Shared& sh) {
   // radix select of the m-th largest key
   unsigned prefix = 0, mask = 0;
   int remaining = m;
   for (int shift = 24; shift >= 0; shift -= 8) {
     for (int i = threadIdx.x; i < 256; i += NT) sh.hist[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < V; i += NT) {
+    for (int i = first + threadIdx.x; i < V; i += NT) {
       unsigned k = ordered_key(row[i] / temp);
       if (k != 0u && (k & mask) == prefix) atomicAdd(&sh.hist[(k >> shift) & 255u], 1u);
     }
@@ -157,8 +181,8 @@ __device__ void select_sorted(const float* row, int V, float temp, int m, Shared
   if (threadIdx.x == 0) sh.misc[2] = 0;
   __syncthreads();
   // contiguous id chunks so that ties are taken in id order
-  const int chunk = (V + NT - 1) / NT;
-  const int lo = threadIdx.x * chunk, hi = min(V, lo + chunk);
+  const int chunk = (V - first + NT - 1) / NT;
+  const int lo = first + threadIdx.x * chunk, hi = min(V, lo + chunk);
   int my_ties = 0;
   for (int i = lo; i < hi; ++i) {
     unsigned k = ordered_key(row[i] / temp);
@@ -181,25 +205,57 @@ __device__ void select_sorted(const float* row, int V, float temp, int m, Shared
     }
   }
   __syncthreads();
-  // pad to a power of two and sort descending (bitonic)
-  int n2 = 1;
-  while (n2 < m) n2 <<= 1;
-  for (int i = m + threadIdx.x; i < n2; i += NT) sh.cand[i] = 0ull;
-  __syncthreads();
-  for (int size = 2; size <= n2; size <<= 1) {
+  sort_candidates(m, sh);
+}
+
+// The m-th largest of one key per thread (m <= NT): a bitonic sort, in registers up to runs of 32.
+__device__ unsigned block_mth_key(unsigned k, int m, Shared& sh) {
+  unsigned* keys = reinterpret_cast<unsigned*>(sh.iscan);
+  const int t = threadIdx.x;
+  for (int size = 2; size <= NT; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      int i = threadIdx.x;
-      if (i < n2) {
-        int j = i ^ stride;
-        if (j > i) {
-          bool desc = (i & size) == 0;
-          unsigned long long a = sh.cand[i], b = sh.cand[j];
-          if ((a < b) == desc) { sh.cand[i] = b; sh.cand[j] = a; }
-        }
+      unsigned other;
+      if (stride >= 32) {
+        keys[t] = k;
+        __syncthreads();
+        other = keys[t ^ stride];
+        __syncthreads();
+      } else {
+        other = __shfl_xor_sync(0xffffffffu, k, stride);
       }
-      __syncthreads();
+      const bool larger = ((t & size) == 0) == ((t & stride) == 0);  // this thread keeps the larger of the two
+      k = larger ? max(k, other) : min(k, other);
     }
   }
+  if (t == m - 1) keys[0] = k;
+  __syncthreads();
+  const unsigned r = keys[0];
+  __syncthreads();
+  return r;
+}
+
+// The (at most m) best candidates of row[lo..hi) into sh.cand, sorted; returns how many. m <= NT. The m-th largest of the
+// threads' best keys is a bound that at least m candidates reach, and few more where the values lie in no order.
+__device__ int part_candidates(const float* row, int lo, int hi, float temp, int m, Shared& sh) {
+  unsigned best = 0u;
+  for (int i = lo + threadIdx.x; i < hi; i += NT) best = max(best, ordered_key(row[i] / temp));
+  const unsigned bound = max(block_mth_key(best, m, sh), 1u);
+  if (threadIdx.x == 0) sh.misc[2] = 0;
+  __syncthreads();
+  if (best >= bound)
+    for (int i = lo + threadIdx.x; i < hi; i += NT) {
+      const unsigned k = ordered_key(row[i] / temp);
+      if (k >= bound) {
+        const int slot = atomicAdd(&sh.misc[2], 1);
+        if (slot < SPLIT_CAND) sh.cand[slot] = composite(k, (unsigned)i);
+      }
+    }
+  __syncthreads();
+  const int n = sh.misc[2];
+  __syncthreads();
+  if (n <= SPLIT_CAND) sort_candidates(n, sh);
+  else select_sorted(row, lo, hi, temp, m, sh);  // (many equal values)
+  return min(m, n);
 }
 
 __device__ __forceinline__ float next_uniform(unsigned long long* state) {
@@ -221,28 +277,39 @@ __device__ int finish_sorted_smem(int m, float max_v, float denom, float top_p, 
     float sum = denom;
     if (sum <= 0.f) {
       sum = 0.f;
+#pragma unroll 8
       for (int i = 0; i < m; ++i) sum += sh.prob[i];
     }
-    int kept = 0;  // candidates with probability above zero stay, in order
-    float cumulative = 0.f;
-    int keep = -1;
-    for (int i = 0; i < m; ++i) {
-      float p = sh.prob[i] / sum;
-      if (!(p > 0.f)) continue;
-      sh.prob[kept] = p;
-      sh.cand[kept] = sh.cand[i];
-      ++kept;
-      cumulative += p;
-      if (keep < 0 && cumulative >= top_p) { keep = kept; break; }
+    sh.fmisc[1] = sum;
+  }
+  __syncthreads();
+  const float by = sh.fmisc[1];
+  for (int i = threadIdx.x; i < m; i += NT) sh.prob[i] = sh.prob[i] / by;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // probabilities do not ascend: those above zero, which alone can be drawn, come first
+    int keep = 0;
+    float total = 0.f;
+    for (int i0 = 0; i0 < m; i0 += 8) {
+      float p[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) p[j] = i0 + j < m ? sh.prob[i0 + j] : 0.f;
+      bool end = false;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (end || !(p[j] > 0.f)) { end = true; continue; }
+        total += p[j];
+        ++keep;
+        if (total >= top_p) end = true;
+      }
+      if (end) break;
     }
-    if (keep < 0) keep = kept;
     int result = -1;
     if (keep > 0) {
-      float total = 0.f;
-      for (int i = 0; i < keep; ++i) total += sh.prob[i];
       float target = next_uniform(rng) * total;
       float acc = 0.f;
       result = (int)(0xFFFFFFFFu - (unsigned)(sh.cand[keep - 1] & 0xFFFFFFFFull));
+#pragma unroll 8
       for (int i = 0; i < keep; ++i) {
         acc += sh.prob[i];
         if (target < acc) { result = (int)(0xFFFFFFFFu - (unsigned)(sh.cand[i] & 0xFFFFFFFFull)); break; }
@@ -317,7 +384,7 @@ sample_kernel(const float* __restrict__ logits, size_t row_stride, int V, const 
     const int lo = part * per, hi = min(V, lo + per);
     const unsigned long long best = block_argmax_word(row, lo, hi, sh);
     if (threadIdx.x == 0) {
-      split_best[(size_t)r * n_split + part] = best;
+      split_best[(size_t)r * SPLIT_WORDS + part] = best;
       __threadfence();
       last_of_row = atomicAdd(&split_count[r], 1) == n_split - 1 ? 1 : 0;
     }
@@ -327,7 +394,7 @@ sample_kernel(const float* __restrict__ logits, size_t row_stride, int V, const 
     if (threadIdx.x < 32) {
       unsigned long long b = 0ull;
       for (int i = threadIdx.x; i < n_split; i += 32) {
-        const unsigned long long c = *reinterpret_cast<volatile unsigned long long*>(&split_best[(size_t)r * n_split + i]);
+        const unsigned long long c = *reinterpret_cast<volatile unsigned long long*>(&split_best[(size_t)r * SPLIT_WORDS + i]);
         b = c > b ? c : b;
       }
 #pragma unroll
@@ -342,10 +409,46 @@ sample_kernel(const float* __restrict__ logits, size_t row_stride, int V, const 
     }
     return;
   }
-  if (part > 0) return;  // a row that draws is one CTA's work
   const int K = top_k[slot];
   const float P = top_p[slot];
   unsigned long long* state = rng + slot;
+  const bool ranked = K > 0 && K < V;
+  if (n_split > 1 && ranked && K <= SPLIT_CAND / n_split) {
+    // A row of a large vocabulary cut to a few best, over the CTAs of the row: each leaves the best of its part, the
+    // last to arrive ranks those and draws. Words order by value, then by lowest id, so the result is the one CTA's
+    // (which walks the row seven times: 24 rows of 128,256 logits, top 64, took 380 us that way, and take 39 this way).
+    unsigned long long* words = split_best + (size_t)r * SPLIT_WORDS;
+    const int per = (V + n_split - 1) / n_split;
+    const int lo = part * per, hi = min(V, lo + per);
+    const int mine = part_candidates(row, lo, hi, temp, K, sh);
+    for (int i = threadIdx.x; i < mine; i += NT) words[MAX_SPLIT + part * K + i] = sh.cand[i];
+    if (threadIdx.x == 0) words[part] = (unsigned long long)mine;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last_of_row = atomicAdd(&split_count[r], 1) == n_split - 1 ? 1 : 0;
+    __syncthreads();
+    if (!last_of_row) return;
+    __threadfence();
+    if (threadIdx.x == 0) sh.misc[2] = 0;
+    __syncthreads();
+    const volatile unsigned long long* all = words;
+    for (int i = threadIdx.x; i < n_split * K; i += NT) {
+      const int from = i / K;
+      const bool there = i % K < (int)all[from];
+      sh.cand[i] = there ? all[MAX_SPLIT + i] : 0ull;
+      if (there) atomicAdd(&sh.misc[2], 1);
+    }
+    __syncthreads();
+    const int m = min(K, sh.misc[2]);
+    sort_candidates(n_split * K, sh);
+    if (threadIdx.x == 0) split_count[r] = 0;  // ready for the next launch
+    int result = -1;
+    if (m > 0) result = finish_sorted_smem(m, key_value((unsigned)(sh.cand[0] >> 32)), 0.f, P, state, sh);
+    if (result < 0) result = block_argmax(row, V, sh);
+    if (threadIdx.x == 0) out[r] = result;
+    return;
+  }
+  if (part > 0) return;  // other rows that draw are one CTA's work
 
   // finite candidates and their maximum
   float mx = -INFINITY;
@@ -362,12 +465,11 @@ sample_kernel(const float* __restrict__ logits, size_t row_stride, int V, const 
     if (threadIdx.x == 0) out[r] = id;
     return;
   }
-  const bool ranked = K > 0 && K < V;
   int result = -1;
 
   if (ranked && min(K, n_finite) <= SMEM_CAND) {
     int m = min(K, n_finite);
-    select_sorted(row, V, temp, m, sh);
+    select_sorted(row, 0, V, temp, m, sh);
     result = finish_sorted_smem(m, mx, 0.f, P, state, sh);
   } else if (!ranked && P >= 1.0f) {
     // whole vocabulary, in id order
@@ -408,7 +510,7 @@ sample_kernel(const float* __restrict__ logits, size_t row_stride, int V, const 
       sum = block_sum(sum, sh);
       for (int m = 256; m <= SMEM_CAND && !done; m *= 4) {
         int mm = min(m, n_finite);
-        select_sorted(row, V, temp, mm, sh);
+        select_sorted(row, 0, V, temp, mm, sh);
         float part = 0.f;
         for (int i = threadIdx.x; i < mm; i += NT) part += expf(key_value((unsigned)(sh.cand[i] >> 32)) - mx);
         float mass = block_sum(part, sh) / sum;
@@ -515,9 +617,10 @@ CUCA_API int cuca_sample_scratch_stride(int V) {
 // One token per row. temperature/top_k/top_p and rng (SplitMix64 states, advanced once per drawn token)
 // are per request slot and indexed by slot_of_row[r]. scratch: n_rows * scratch_stride 64-bit words (may be null: rows that
 // would need it then yield -1).
-// split_best / split_count (may be null): split_rows x CUCA_SAMPLE_MAX_SPLIT 64-bit words and split_rows zeroed
-// counters (left zeroed), with which the greedy rows of a large vocabulary are cut over several CTAs each.
-CUCA_API int cuca_sample_max_split() { return 32; }
+// split_best / split_count (may be null): split_rows x cuca_sample_split_words() 64-bit words and split_rows zeroed
+// counters (left zeroed), with which the greedy rows of a large vocabulary, and those cut to a few best, are spread over
+// several CTAs each.
+CUCA_API int cuca_sample_split_words() { return SPLIT_WORDS; }
 CUCA_API int cuca_sample(const float* logits, size_t row_stride, int n_rows, int V, const float* temperature,
                          const int* top_k, const float* top_p, unsigned long long* rng, const int* slot_of_row,
                          int* out, unsigned long long* scratch, int scratch_stride, unsigned long long* split_best,
@@ -530,7 +633,7 @@ CUCA_API int cuca_sample(const float* logits, size_t row_stride, int n_rows, int
   int n_split = 1;
   if (split_best && split_count && n_rows <= split_rows) {
     n_split = (V + 8191) / 8192;
-    if (n_split > cuca_sample_max_split()) n_split = cuca_sample_max_split();
+    if (n_split > MAX_SPLIT) n_split = MAX_SPLIT;
     while (n_split > 1 && n_rows * n_split > 1024) n_split /= 2;
     if (n_split < 1) n_split = 1;
   }

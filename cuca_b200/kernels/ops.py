@@ -689,13 +689,13 @@ def sample_scratch_words(vocab: int) -> int:
 
 
 class SampleSplit:
-    """Scratch with which the greedy rows of a large vocabulary are cut over several CTAs each: per row the best of
-    every part and a counter of the parts that have arrived (left zeroed by every launch). One per engine; a
-    launch with more rows than it holds runs one CTA per row."""
+    """Scratch with which the rows of a large vocabulary, greedy ones and those cut to a few best, are spread over
+    several CTAs each: per row the best of every part and a counter of the parts that have arrived (left zeroed by
+    every launch). One per engine; a launch with more rows than it holds runs one CTA per row."""
 
     def __init__(self, rows: int, device):
         self.rows = int(rows)
-        self.best = torch.zeros(self.rows * int(library.load().cuca_sample_max_split()), dtype=torch.int64, device=device)
+        self.best = torch.zeros(self.rows * int(library.load().cuca_sample_split_words()), dtype=torch.int64, device=device)
         self.count = torch.zeros(self.rows, dtype=torch.int32, device=device)
 
 

@@ -107,6 +107,45 @@ def test_greedy_rows_cut_over_several_ctas_give_the_one_ctas_token(V):
     assert outs[0][8] == int(torch.argmax(logits[8]))
 
 
+@pytest.mark.parametrize("V", [8193, 50000, 128256, 300000])
+@pytest.mark.parametrize("K", [1, 2, 64, 100, 1024])
+def test_drawing_rows_cut_over_several_ctas_give_the_one_ctas_token(V, K):
+    """Rows cut to their K best, spread over several CTAs (where the parts' bests fit) and in one: the same tokens and the
+    same generator states, for rows in random, ascending and descending order, with ties across parts, with fewer finite
+    logits than K, all equal (a part's bound then cuts nothing) and without any finite logit."""
+    import torch
+    from cuca_b200.kernels import ops
+    dev = torch.device("cuda:0")
+    rs = np.random.default_rng(V + K)
+    R = 9
+    logits = torch.tensor((rs.standard_normal((R, V)) * 3).astype(np.float32), device=dev)
+    logits[1] = torch.sort(logits[1]).values
+    logits[2] = torch.sort(logits[2], descending=True).values
+    logits[3] = torch.round(logits[3])           # ties everywhere
+    logits[4] = 1.5                              # one value: the lowest ids
+    logits[5, : V - 40] = float("-inf")          # fewer candidates than most K, in the last part
+    logits[6, :] = float("-inf")
+    logits[6, 3] = float("nan")
+    logits[7, 11] = float("inf")                 # never a candidate
+    slot_of_row = torch.tensor([0, 1, 2, 3, 4, 5, 6, 7, -1], dtype=torch.int32, device=dev)
+    split = ops.SampleSplit(16, dev)
+    for temp, P in ((0.8, 0.95), (5.0, 1.0), (0.01, 0.5)):
+        temperature = torch.full((8,), temp, dtype=torch.float32, device=dev)
+        top_k = torch.full((8,), K, dtype=torch.int32, device=dev)
+        top_p = torch.full((8,), P, dtype=torch.float32, device=dev)
+        got = []
+        for use in (None, split, split):
+            rng = torch.arange(8, dtype=torch.int64, device=dev) * 977 + 5
+            out = torch.full((R,), -7, dtype=torch.int32, device=dev)
+            for _ in range(3):
+                ops.sample(logits, temperature, top_k, top_p, rng, slot_of_row, out, None, use)
+            torch.cuda.synchronize()
+            got.append((out.tolist(), rng.tolist()))
+            assert int(split.count.abs().sum().item()) == 0
+        assert got[0] == got[1] == got[2]
+        assert got[0][0][8] == -1 and all(0 <= t < V for t in got[0][0][:8])
+
+
 def test_sampler_statistics_follow_the_distribution():
     V = 50
     logits = np.linspace(-2, 2, V, dtype=np.float32)[None, :].repeat(4, 0)
