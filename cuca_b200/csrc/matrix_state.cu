@@ -13,47 +13,20 @@
 // What does not depend on the state (unit vectors, decays, gates) is computed for all rows at once by a preparing
 // kernel, in place. A scan block then takes one (head, request, run of value columns) and walks the request's rows of
 // the step in order from the state its slot holds, leaving the new state there. A value column's state rows live in
-// the registers of NS neighbouring threads (thread s holds NR consecutive rows); a token's vectors are copied to
-// shared memory a few tokens ahead of their use. The arithmetic of a token does not depend on where the sequence was
-// cut into steps or chunks; how many threads share a column's sums (and so the order of those sums) depends on how
-// many columns the launch has.
+// the registers of NS neighbouring threads (see Split); a token's vectors are copied to shared memory a few tokens
+// ahead of their use. The arithmetic of a token depends neither on where the sequence was cut into steps or chunks
+// nor on what else is in the launch.
 #include "common.cuh"
+#include "state_rows.cuh"
 #include <math.h>
-#include <stdlib.h>
 
 namespace {
 
-constexpr int MAXR = 32;  // state rows a thread holds at most
+constexpr int MAX_DIM = 1024;  // key channels
 
 __device__ __forceinline__ float sigmoidf_(float v) { return 1.f / (1.f + expf(-v)); }
 __device__ __forceinline__ float softplusf_(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 __device__ __forceinline__ float log_sigmoidf_(float v) { return v < 0.f ? v - log1pf(expf(v)) : -log1pf(expf(-v)); }
-
-// sum over the NS neighbouring threads of a value column (NS a power of two, at most 32)
-__device__ __forceinline__ float group_sum(float v, int NS) {
-  if (NS >= 32) v += __shfl_xor_sync(0xffffffffu, v, 16);
-  if (NS >= 16) v += __shfl_xor_sync(0xffffffffu, v, 8);
-  if (NS >= 8) v += __shfl_xor_sync(0xffffffffu, v, 4);
-  if (NS >= 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
-  if (NS >= 2) v += __shfl_xor_sync(0xffffffffu, v, 1);
-  return v;
-}
-
-// An asynchronous copy of 4 or 16 bytes from global to shared memory.
-__device__ __forceinline__ void cp_async_f(float* dst, const float* src, bool wide) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Where key channel r of a staged vector lies in shared memory: thread s of a value column holds the NR consecutive
-// channels s NR .. s NR + NR - 1 and reads them 16 bytes at a time; four floats of padding after every NR keep the
-// NS threads of a column on different banks.
-// (Four channels a thread are 16 bytes a thread: contiguous, nothing to pad.)
-template <int NR> __device__ __forceinline__ constexpr int staged_stride() { return NR == 4 ? 4 : NR + 4; }
-template <int NR> __device__ __forceinline__ int staged_at(int r) { return (r / NR) * staged_stride<NR>() + r % NR; }
 
 // Per row, in place: q and k heads (G heads of d at columns 0 and G d of qkv) become unit vectors, q times d^(-1/2);
 // the decay pre-activations a_raw (rows of stride ld_a, H d values) become g = exp(-exp(A_log[h]) softplus(a + dt_bias)); the gate
@@ -85,15 +58,20 @@ delta_prepare_kernel(float* __restrict__ qkv, int ld, float* __restrict__ a_raw,
 }
 
 // qkv: 32-bit rows of stride ld, prepared: unit q heads at column 0 (G heads of d), unit k heads at column G d, v
-// heads at column 2 G d (H heads of dv). g: rows of stride ld_g, H d decays; beta: rows of stride ld_b, head h at column
+// heads at column 2 G d (H heads of dv). decay: rows of stride ld_g, H d decays; beta: rows of stride ld_b, head h at column
 // b_col + h. state: [slots, H, dv, d]. out: [rows, H dv]. Two buffers of TC tokens: the next tokens' vectors are
 // copied (cp.async) while these are worked through.
-template <int NR>
-__global__ void delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ g, int ld_g,
-                                  const float* __restrict__ beta, int ld_b, int b_col, float* __restrict__ state,
-                                  float* __restrict__ out, const int* __restrict__ req_row0,
-                                  const int* __restrict__ req_count, const int* __restrict__ slots, int H, int G,
-                                  int d, int dv, int NS, int PB, int TC, int wide) {
+// What bounds it for one prompt: the chain of a token (state times decay, dot with k, three shuffles, correction), about
+// 130 clocks; the outputs' dot products belong to the token before and run in the shadow of the shuffles.
+template <typename C>
+__global__ void __launch_bounds__(128)
+delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ decay, int ld_g,
+                  const float* __restrict__ beta, int ld_b, int b_col, float* __restrict__ state,
+                  float* __restrict__ out, const int* __restrict__ req_row0,
+                  const int* __restrict__ req_count, const int* __restrict__ slots, int H, int G,
+                  int d, int dv, int wide) {
+  constexpr int NS = C::NS, NC = C::NC, DP = C::DP, PB = C::PB, TC = C::TC, PAIRS = C::PAIRS;
+  constexpr int PER = 3 * DP + ((PB + 1 + 3) & ~3);  // a token: q, k, g, the block's values, beta
   extern __shared__ __align__(16) float sm[];
   pdl_trigger();
   pdl_wait();
@@ -101,96 +79,111 @@ __global__ void delta_scan_kernel(const float* __restrict__ qkv, int ld, const f
   const int slot = slots[rq], n = req_count[rq], r0 = req_row0[rq];
   if (slot < 0 || n <= 0) return;
   const int kvh = h / (H / G);
-  const int dpp = NS * staged_stride<NR>();     // a staged vector with its padding
-  const int per = (3 * dpp + PB + 1 + 3) & ~3;  // a token: q, k, g, the block's values, beta
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
-  const int col = blockIdx.z * PB + col_local;
-  const bool live = col_local < PB && col < dv;
-  float S[NR];
-  float* st = state + (((size_t)slot * H + h) * dv + (live ? col : 0)) * d;
-#pragma unroll
-  for (int i = 0; i < NR; ++i) S[i] = (live && s * NR + i < d) ? st[s * NR + i] : 0.f;
+  const int col0 = blockIdx.z * PB, at = col_local * NC;
+  const int cols = min(NC, dv - col0 - at);               // columns of this thread that exist (none: 0 or less)
+  const int own = s / (NS / NC), col = col0 + at + own;   // the column whose sums this thread ends up with
+  const bool writes = s % (NS / NC) == 0 && own < cols;
+  float* st = state + (((size_t)slot * H + h) * dv + (cols > 0 ? col0 + at : 0)) * d;
+  f32x2 S[NC][PAIRS];
+  load_rows<C>(S, st, s, d, cols, wide);
   // what no copy writes: channels from d on (q = k = 0, g = 1) and the values of columns from dv on
   {
-    const int spare = NS * NR - d, fill = 3 * spare + PB;
-    for (int e = threadIdx.x; e < 2 * TC * fill; e += blockDim.x) {
+    const int spare = DP - d, fill = 3 * spare + PB;
+    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
       const int t = e / fill, w = e % fill;
-      float* tok = sm + (size_t)t * per;
-      if (w < 3 * spare) tok[(w / spare) * dpp + staged_at<NR>(d + w % spare)] = w / spare == 2 ? 1.f : 0.f;
-      else tok[3 * dpp + (w - 3 * spare)] = 0.f;
+      float* tok = sm + t * PER;
+      if (w < 3 * spare) tok[(w / spare) * DP + d + w % spare] = w / spare == 2 ? 1.f : 0.f;
+      else tok[3 * DP + (w - 3 * spare)] = 0.f;
     }
   }
   __syncthreads();
   auto stage = [&](int t0, int buf) {
     const int nt = n - t0 < TC ? n - t0 : TC;
-    float* base = sm + (size_t)buf * TC * per;
-    const int step = wide ? 4 : 1, units = d / step;
-    for (int e = threadIdx.x; e < nt * 3 * units; e += blockDim.x) {
-      const int t = e / (3 * units), u = e % (3 * units), which = u / units, r = (u % units) * step;
+    float* base = sm + buf * TC * PER;
+    auto copy = [&](int t, int which, int r) {
       const size_t row = (size_t)(r0 + t0 + t);
-      const float* src = which == 0 ? qkv + row * ld + (size_t)kvh * d + r
-                       : which == 1 ? qkv + row * ld + (size_t)(G + kvh) * d + r
-                                    : g + row * ld_g + (size_t)h * d + r;
-      cp_async_f(base + (size_t)t * per + which * dpp + staged_at<NR>(r), src, wide);
+      const float* src = which == 2 ? decay + row * ld_g + (size_t)h * d + r : qkv + row * ld + (size_t)(which * G + kvh) * d + r;
+      if (r < d) cp_async_f(base + t * PER + which * DP + r, src, wide);
+    };
+    if (wide)
+      for (int e = threadIdx.x; e < nt * 3 * (DP / 4); e += 128) copy(e / (3 * (DP / 4)), e / (DP / 4) % 3, e % (DP / 4) * 4);
+    else
+      for (int e = threadIdx.x; e < nt * 3 * DP; e += 128) copy(e / (3 * DP), e / DP % 3, e % DP);
+    for (int e = threadIdx.x; e < nt * PB; e += 128) {
+      const int t = e / PB, i = e % PB;
+      if (col0 + i < dv)
+        cp_async_f(base + t * PER + 3 * DP + i, qkv + (size_t)(r0 + t0 + t) * ld + (size_t)2 * G * d + (size_t)h * dv + col0 + i, false);
     }
-    for (int e = threadIdx.x; e < nt * (PB + 1); e += blockDim.x) {
-      const int t = e / (PB + 1), i = e % (PB + 1);
-      const size_t row = (size_t)(r0 + t0 + t);
-      if (i == PB) cp_async_f(base + (size_t)t * per + 3 * dpp + PB, beta + row * ld_b + b_col + h, false);
-      else if (blockIdx.z * PB + i < dv)
-        cp_async_f(base + (size_t)t * per + 3 * dpp + i, qkv + row * ld + (size_t)2 * G * d + (size_t)h * dv + blockIdx.z * PB + i, false);
-    }
+    if (threadIdx.x < nt)
+      cp_async_f(base + threadIdx.x * PER + 3 * DP + PB, beta + (size_t)(r0 + t0 + threadIdx.x) * ld_b + b_col + h, false);
     cp_async_commit();
   };
-  const int cv = col_local < PB ? col_local : PB - 1;
   const int n_chunks = (n + TC - 1) / TC;
+  float* o_at = out + (size_t)r0 * H * dv + (size_t)h * dv + col;  // the output of the token before
+  f32x2 q[PAIRS];
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) q[i] = 0;
+  auto output = [&]() {
+    float o[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) o[c] = dot_rows(S[c], q);
+    return column_sum<C>(o, s);
+  };
   stage(0, 0);
   for (int c = 0; c < n_chunks; ++c) {
     if (c + 1 < n_chunks) { stage((c + 1) * TC, (c + 1) & 1); cp_async_wait<1>(); }
     else cp_async_wait<0>();
     __syncthreads();
     const int t0 = c * TC, nt = n - t0 < TC ? n - t0 : TC;
-    const float* base = sm + (size_t)(c & 1) * TC * per;
     // every thread of a warp takes part (the sums shuffle across whole warps); spare threads work on zeros
-    const float* tok = base;
-    float* po_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col;
-    const int mine = s * staged_stride<NR>(), extra = 3 * dpp;
+    const float* tok = sm + (c & 1) * TC * PER;
+    f32x2 k[PAIRS], g[PAIRS];
+    float v[NC], b = tok[3 * DP + PB];
+    staged_rows<C>(k, tok + DP, s);
+    staged_rows<C>(g, tok + 2 * DP, s);
+    staged_values<NC>(v, tok + 3 * DP, at);
 #pragma unroll 2
-    for (int t = 0; t < nt; ++t, tok += per, po_at += H * dv) {
-      const float4* gq = reinterpret_cast<const float4*>(tok + mine);
-      const float4* gk = reinterpret_cast<const float4*>(tok + dpp + mine);
-      const float4* gg = reinterpret_cast<const float4*>(tok + 2 * dpp + mine);
-      float kk[NR];
-      float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+    for (int t = 0; t < nt; ++t) {
+      const float* next = t + 1 < nt ? tok + PER : tok;  // (read ahead of its use)
+      f32x2 Sg[NC][PAIRS], k1[PAIRS];
+      float part[NC], v1[NC], u[NC];
 #pragma unroll
-      for (int i = 0; i < NR / 4; ++i) {
-        const float4 gv = gg[i], kv4 = gk[i];
-        kk[4 * i] = kv4.x; kk[4 * i + 1] = kv4.y; kk[4 * i + 2] = kv4.z; kk[4 * i + 3] = kv4.w;
-        S[4 * i] *= gv.x; S[4 * i + 1] *= gv.y; S[4 * i + 2] *= gv.z; S[4 * i + 3] *= gv.w;
-        p0 = fmaf(S[4 * i], kv4.x, p0); p1 = fmaf(S[4 * i + 1], kv4.y, p1);
-        p2 = fmaf(S[4 * i + 2], kv4.z, p2); p3 = fmaf(S[4 * i + 3], kv4.w, p3);
-      }
-      const float part = group_sum((p0 + p1) + (p2 + p3), NS);
-      const float u = tok[extra + PB] * (tok[extra + cv] - part);
-      p0 = p1 = p2 = p3 = 0.f;
+      for (int j = 0; j < NC; ++j) {
 #pragma unroll
-      for (int i = 0; i < NR / 4; ++i) {
-        const float4 qv = gq[i];
-        S[4 * i] = fmaf(kk[4 * i], u, S[4 * i]); S[4 * i + 1] = fmaf(kk[4 * i + 1], u, S[4 * i + 1]);
-        S[4 * i + 2] = fmaf(kk[4 * i + 2], u, S[4 * i + 2]); S[4 * i + 3] = fmaf(kk[4 * i + 3], u, S[4 * i + 3]);
-        p0 = fmaf(S[4 * i], qv.x, p0); p1 = fmaf(S[4 * i + 1], qv.y, p1);
-        p2 = fmaf(S[4 * i + 2], qv.z, p2); p3 = fmaf(S[4 * i + 3], qv.w, p3);
+        for (int i = 0; i < PAIRS; ++i) Sg[j][i] = f2_mul(S[j][i], g[i]);
+        part[j] = dot_rows(Sg[j], k);
       }
-      const float po = group_sum((p0 + p1) + (p2 + p3), NS);
-      if (s == 0 && live) *po_at = po;
+      staged_rows<C>(k1, next + DP, s);
+      staged_rows<C>(g, next + 2 * DP, s);
+      staged_values<NC>(v1, next + 3 * DP, at);
+      const float b1 = next[3 * DP + PB];
+      const float sum = column_sum<C>(part, s);
+      const float o = output();
+      column_spread<C>(u, sum, s);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        const f32x2 uu = f2_both(b * (v[j] - u[j]));
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(k[i], uu, Sg[j][i]);
+      }
+      staged_rows<C>(q, tok, s);
+      if (t0 + t > 0) {
+        if (writes) *o_at = o;
+        o_at += H * dv;
+      }
+#pragma unroll
+      for (int i = 0; i < PAIRS; ++i) k[i] = k1[i];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] = v1[j];
+      b = b1;
+      tok = next;
     }
     __syncthreads();  // the buffer is free for the copies of the chunk after next
   }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < NR; ++i)
-      if (s * NR + i < d) st[s * NR + i] = S[i];
-  }
+  const float o = output();
+  if (writes) *o_at = o;
+  store_rows<C>(S, st, s, d, cols, wide);
 }
 
 // Per row, in place, of a 32-bit projection [q | f | ...]: q (H d values at q_col) becomes silu(q); the forget gate's
@@ -337,98 +330,92 @@ lightning_step_kernel(const float* __restrict__ proj, int ld, int col0, const fl
 // correction: one shuffled sum per token and column.
 // RET (retention): the second staged vector is the key k instead of the gate, and the state decays by one number per
 // head: S <- decay[h] S + k v^T.
-template <int NR, bool RET>
-__global__ void forget_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int f_col, int v_col,
-                                   const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ out,
-                                   const int* __restrict__ req_row0, const int* __restrict__ req_count,
-                                   const int* __restrict__ slots, int H, int d, int dv, int NS, int PB, int TC, int wide) {
+template <typename C, bool RET>
+__global__ void __launch_bounds__(128)
+forget_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int f_col, int v_col,
+                   const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ out,
+                   const int* __restrict__ req_row0, const int* __restrict__ req_count,
+                   const int* __restrict__ slots, int H, int d, int dv, int wide) {
+  constexpr int NS = C::NS, NC = C::NC, DP = C::DP, PB = C::PB, TC = C::TC, PAIRS = C::PAIRS;
+  constexpr int PER = 2 * DP + ((PB + 3) & ~3);  // a token: q, f, the block's values
   extern __shared__ __align__(16) float sm[];
   pdl_trigger();
   pdl_wait();
   const int h = blockIdx.x, rq = blockIdx.y;
   const int slot = slots[rq], n = req_count[rq], r0 = req_row0[rq];
   if (slot < 0 || n <= 0) return;
-  const int dpp = NS * staged_stride<NR>();  // a staged vector with its padding
-  const int per = (2 * dpp + PB + 3) & ~3;   // a token: q, f, the block's values
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
-  const int col = blockIdx.z * PB + col_local;
-  const bool live = col_local < PB && col < dv;
-  float S[NR];
-  float* st = state + (((size_t)slot * H + h) * dv + (live ? col : 0)) * d;
-#pragma unroll
-  for (int i = 0; i < NR; ++i) S[i] = (live && s * NR + i < d) ? st[s * NR + i] : 0.f;
-  // what no copy writes: channels from d on (q = 0, f = 1) and the values of columns from dv on
+  const int col0 = blockIdx.z * PB, at = col_local * NC;
+  const int cols = min(NC, dv - col0 - at);               // columns of this thread that exist (none: 0 or less)
+  const int own = s / (NS / NC), col = col0 + at + own;   // the column whose sums this thread ends up with
+  const bool writes = s % (NS / NC) == 0 && own < cols;
+  float* st = state + (((size_t)slot * H + h) * dv + (cols > 0 ? col0 + at : 0)) * d;
+  f32x2 S[NC][PAIRS];
+  load_rows<C>(S, st, s, d, cols, wide);
+  // what no copy writes: channels from d on (q = 0, f = 1, k = 0) and the values of columns from dv on
   {
-    const int spare = NS * NR - d, fill = 2 * spare + PB;
-    for (int e = threadIdx.x; e < 2 * TC * fill; e += blockDim.x) {
+    const int spare = DP - d, fill = 2 * spare + PB;
+    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
       const int t = e / fill, w = e % fill;
-      float* tok = sm + (size_t)t * per;
-      if (w < 2 * spare) tok[(w / spare) * dpp + staged_at<NR>(d + w % spare)] = (w / spare == 1 && !RET) ? 1.f : 0.f;
-      else tok[2 * dpp + (w - 2 * spare)] = 0.f;
+      float* tok = sm + t * PER;
+      if (w < 2 * spare) tok[(w / spare) * DP + d + w % spare] = (w / spare == 1 && !RET) ? 1.f : 0.f;
+      else tok[2 * DP + (w - 2 * spare)] = 0.f;
     }
   }
   __syncthreads();
   auto stage = [&](int t0, int buf) {
     const int nt = n - t0 < TC ? n - t0 : TC;
-    float* base = sm + (size_t)buf * TC * per;
-    const int step = wide ? 4 : 1, units = d / step;
-    for (int e = threadIdx.x; e < nt * 2 * units; e += blockDim.x) {
-      const int t = e / (2 * units), u = e % (2 * units), which = u / units, r = (u % units) * step;
+    float* base = sm + buf * TC * PER;
+    auto copy = [&](int t, int which, int r) {
       const float* src = proj + (size_t)(r0 + t0 + t) * ld + (which ? f_col : q_col) + (size_t)h * d + r;
-      cp_async_f(base + (size_t)t * per + which * dpp + staged_at<NR>(r), src, wide);
-    }
-    for (int e = threadIdx.x; e < nt * PB; e += blockDim.x) {
+      if (r < d) cp_async_f(base + t * PER + which * DP + r, src, wide);
+    };
+    if (wide)
+      for (int e = threadIdx.x; e < nt * 2 * (DP / 4); e += 128) copy(e / (2 * (DP / 4)), e / (DP / 4) % 2, e % (DP / 4) * 4);
+    else
+      for (int e = threadIdx.x; e < nt * 2 * DP; e += 128) copy(e / (2 * DP), e / DP % 2, e % DP);
+    for (int e = threadIdx.x; e < nt * PB; e += 128) {
       const int t = e / PB, i = e % PB;
-      if (blockIdx.z * PB + i < dv)
-        cp_async_f(base + (size_t)t * per + 2 * dpp + i,
-                   proj + (size_t)(r0 + t0 + t) * ld + v_col + (size_t)h * dv + blockIdx.z * PB + i, false);
+      if (col0 + i < dv)
+        cp_async_f(base + t * PER + 2 * DP + i, proj + (size_t)(r0 + t0 + t) * ld + v_col + (size_t)h * dv + col0 + i, false);
     }
     cp_async_commit();
   };
-  const int cv = col_local < PB ? col_local : PB - 1;
   const int n_chunks = (n + TC - 1) / TC;
-  const float dec = RET ? decay[h] : 0.f;
+  const f32x2 dec = f2_both(RET ? decay[h] : 0.f), one = f2_both(1.f), minus = f2_both(-1.f);
   stage(0, 0);
   for (int c = 0; c < n_chunks; ++c) {
     if (c + 1 < n_chunks) { stage((c + 1) * TC, (c + 1) & 1); cp_async_wait<1>(); }
     else cp_async_wait<0>();
     __syncthreads();
     const int t0 = c * TC, nt = n - t0 < TC ? n - t0 : TC;
-    const float* tok = sm + (size_t)(c & 1) * TC * per;
-    float* po_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col;
-    const int mine = s * staged_stride<NR>();
-    // (tokens depend on each other through the state's one multiply-add alone: with four rows a thread, eight
-    // tokens in flight keep the loads and the shuffled sums of the next ones going while these wait)
-#pragma unroll(NR == 4 ? 8 : 2)
-    for (int t = 0; t < nt; ++t, tok += per, po_at += H * dv) {
-      const float4* gq = reinterpret_cast<const float4*>(tok + mine);
-      const float4* gf = reinterpret_cast<const float4*>(tok + dpp + mine);
-      const float v = tok[2 * dpp + cv];
-      float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+    const float* tok = sm + (c & 1) * TC * PER;
+    float* o_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col;
+    // (tokens depend on each other through the state's one multiply-add alone: four in flight keep the loads and the
+    // shuffled sums of the next ones going while these wait)
+#pragma unroll 4
+    for (int t = 0; t < nt; ++t, tok += PER, o_at += H * dv) {
+      f32x2 f[PAIRS], q[PAIRS], w[PAIRS];  // w: what is written, k or 1 - f
+      float v[NC], o[NC];
+      staged_rows<C>(f, tok + DP, s);
+      staged_rows<C>(q, tok, s);
+      staged_values<NC>(v, tok + 2 * DP, at);
 #pragma unroll
-      for (int i = 0; i < NR / 4; ++i) {
-        const float4 f4 = gf[i], qv = gq[i];
-        if (RET) {  // decay S + k v
-          S[4 * i] = fmaf(dec, S[4 * i], f4.x * v); S[4 * i + 1] = fmaf(dec, S[4 * i + 1], f4.y * v);
-          S[4 * i + 2] = fmaf(dec, S[4 * i + 2], f4.z * v); S[4 * i + 3] = fmaf(dec, S[4 * i + 3], f4.w * v);
-        } else {
-        // f S + (1 - f) v, each product rounded as the plain recurrence rounds it
-        S[4 * i] = fmaf(f4.x, S[4 * i], (1.f - f4.x) * v); S[4 * i + 1] = fmaf(f4.y, S[4 * i + 1], (1.f - f4.y) * v);
-        S[4 * i + 2] = fmaf(f4.z, S[4 * i + 2], (1.f - f4.z) * v); S[4 * i + 3] = fmaf(f4.w, S[4 * i + 3], (1.f - f4.w) * v);
-        }
-        p0 = fmaf(S[4 * i], qv.x, p0); p1 = fmaf(S[4 * i + 1], qv.y, p1);
-        p2 = fmaf(S[4 * i + 2], qv.z, p2); p3 = fmaf(S[4 * i + 3], qv.w, p3);
+      for (int i = 0; i < PAIRS; ++i) w[i] = RET ? f[i] : f2_fma(f[i], minus, one);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        const f32x2 vv = f2_both(v[j]);
+        // decay S + k v or f S + (1 - f) v, each product rounded
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(RET ? dec : f[i], S[j][i], f2_mul(w[i], vv));
+        o[j] = dot_rows(S[j], q);
       }
-      const float po = group_sum((p0 + p1) + (p2 + p3), NS);
-      if (s == 0 && live) *po_at = po;
+      const float mine = column_sum<C>(o, s);
+      if (writes) *o_at = mine;
     }
     __syncthreads();  // the buffer is free for the copies of the chunk after next
   }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < NR; ++i)
-      if (s * NR + i < d) st[s * NR + i] = S[i];
-  }
+  store_rows<C>(S, st, s, d, cols, wide);
 }
 
 // Per row, in place: the raw input gate of head h (column i_col + h of proj) becomes cap tanh((x + b_i) / cap), the
@@ -449,141 +436,134 @@ __global__ void mlstm_prepare_kernel(float* __restrict__ proj, int ld, int i_col
 // proj: 32-bit rows of stride ld, prepared: q heads at q_col (H heads of d), k at k_col, v at v_col (H heads of dv),
 // the log input gate of head h at i_col + h, the log forget gate at f_col + h.
 // mem: [slots, H, dv, d]; nrm: [slots, H, d]; mx: [slots, H]. out: [rows, H dv].
-// The block's columns are its PB value columns and one more that carries n (its "value" is 1), so n . q comes out
-// of the same loop; the division waits until the chunk's sums are in shared memory. q enters unscaled: the sums
-// are linear in it, so d^(-1/2) multiplies them afterwards. n and m are shared by all blocks of a (head, request):
-// this launch only reads them and leaves the new ones aside (nm_new); `mlstm_commit_kernel` moves them into the slots.
-template <int NR>
-__global__ void mlstm_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int k_col, int v_col, int i_col,
-                                  int f_col, float* __restrict__ mem, float* __restrict__ nrm, float* __restrict__ mx,
-                                  float* __restrict__ out, const int* __restrict__ req_row0,
-                                  const int* __restrict__ req_count, const int* __restrict__ slots, int H, int d,
-                                  int dv, int NS, int PB, int TC, int wide, float* __restrict__ nm_new) {
+// Every column's threads carry n too (three more multiply-adds a pair of channels, and no exchange between warps), and
+// every warp works the running maximum of a run of tokens out for itself: a chain of one add and one max per token,
+// after which a lane per token takes the exponentials. q enters unscaled: the sums are linear in it, so d^(-1/2)
+// multiplies them afterwards. n and m are shared by all blocks of a (head, request): this launch only reads them and
+// leaves the new ones aside (nm_new [requests, H, d + 1]); `mlstm_commit_kernel` moves them into the slots.
+template <typename C>
+__global__ void __launch_bounds__(128)
+mlstm_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int k_col, int v_col, int i_col,
+                  int f_col, float* __restrict__ mem, const float* __restrict__ nrm, const float* __restrict__ mx,
+                  float* __restrict__ out, const int* __restrict__ req_row0,
+                  const int* __restrict__ req_count, const int* __restrict__ slots, int H, int d,
+                  int dv, int wide, float* __restrict__ nm_new) {
+  constexpr int NS = C::NS, NC = C::NC, DP = C::DP, PB = C::PB, TC = C::TC, PAIRS = C::PAIRS;
+  constexpr int PER = 2 * DP + ((PB + 2 + 3) & ~3);  // a token: q, k, the block's values, the two gates
+  static_assert(TC <= 32, "a lane a token");
   extern __shared__ __align__(16) float sm[];
+  __shared__ float gates[4][TC][3];  // a warp's own: e^(f + m - m'), e^(i - m'), e^(-m')
   pdl_trigger();
   pdl_wait();
   const int h = blockIdx.x, rq = blockIdx.y;
   const int slot = slots[rq], n = req_count[rq], r0 = req_row0[rq];
   if (slot < 0 || n <= 0) return;
-  const int dpp = NS * staged_stride<NR>();
-  const int per = (2 * dpp + (PB + 1) + 2 + 3) & ~3;  // a token: q, k, the block's values and a 1, the two gates
-  float* so = sm + (size_t)2 * TC * per;     // [TC][PB + 1] the chunk's sums
-  float* keep = so + (size_t)TC * (PB + 1);  // [TC] e^(f + m - m')
-  float* take = keep + TC;                   // [TC] e^(i - m')
-  float* floor_ = take + TC;                 // [TC] e^(-m')
-  float* ms = floor_ + TC;                   // [TC + 1] m before each token of the chunk, and after the last
+  const int lane = threadIdx.x & 31;
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
-  const bool is_n = col_local == PB;
-  const int col = blockIdx.z * PB + col_local;
-  const bool live = is_n || (col_local < PB && col < dv);
-  float S[NR];
-  float* st = is_n ? nrm + ((size_t)slot * H + h) * d
-                   : mem + (((size_t)slot * H + h) * dv + (col < dv ? col : 0)) * d;
-#pragma unroll
-  for (int i = 0; i < NR; ++i) S[i] = (live && s * NR + i < d) ? st[s * NR + i] : 0.f;
+  const int col0 = blockIdx.z * PB, at = col_local * NC;
+  const int cols = min(NC, dv - col0 - at);               // columns of this thread that exist (none: 0 or less)
+  const int own = s / (NS / NC), col = col0 + at + own;   // the column whose sums this thread ends up with
+  const bool writes = s % (NS / NC) == 0 && own < cols;
+  float* st = mem + (((size_t)slot * H + h) * dv + (cols > 0 ? col0 + at : 0)) * d;
+  using One = Split<C::NS, C::NR, 1>;
+  f32x2 S[NC][PAIRS], Zs[1][PAIRS];
+  load_rows<C>(S, st, s, d, cols, wide);
+  load_rows<One>(Zs, nrm + ((size_t)slot * H + h) * d, s, d, 1, wide);
+  f32x2(&Z)[PAIRS] = Zs[0];
+  float m = mx[(size_t)slot * H + h];
   {
-    const int spare = NS * NR - d, fill = 2 * spare + PB + 1;
-    for (int e = threadIdx.x; e < 2 * TC * fill; e += blockDim.x) {
+    const int spare = DP - d, fill = 2 * spare + PB;
+    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
       const int t = e / fill, w = e % fill;
-      float* tok = sm + (size_t)t * per;
-      if (w < 2 * spare) tok[(w / spare) * dpp + staged_at<NR>(d + w % spare)] = 0.f;
-      else tok[2 * dpp + (w - 2 * spare)] = w - 2 * spare == PB ? 1.f : 0.f;
+      float* tok = sm + t * PER;
+      if (w < 2 * spare) tok[(w / spare) * DP + d + w % spare] = 0.f;
+      else tok[2 * DP + (w - 2 * spare)] = 0.f;
     }
   }
-  if (threadIdx.x == 0) ms[0] = mx[(size_t)slot * H + h];
   __syncthreads();
   const float qscale = rsqrtf((float)d);
   auto stage = [&](int t0, int buf) {
     const int nt = n - t0 < TC ? n - t0 : TC;
-    float* base = sm + (size_t)buf * TC * per;
-    const int step = wide ? 4 : 1, units = d / step;
-    for (int e = threadIdx.x; e < nt * 2 * units; e += blockDim.x) {
-      const int t = e / (2 * units), u = e % (2 * units), which = u / units, r = (u % units) * step;
+    float* base = sm + buf * TC * PER;
+    auto copy = [&](int t, int which, int r) {
       const float* src = proj + (size_t)(r0 + t0 + t) * ld + (which ? k_col : q_col) + (size_t)h * d + r;
-      cp_async_f(base + (size_t)t * per + which * dpp + staged_at<NR>(r), src, wide);
+      if (r < d) cp_async_f(base + t * PER + which * DP + r, src, wide);
+    };
+    if (wide)
+      for (int e = threadIdx.x; e < nt * 2 * (DP / 4); e += 128) copy(e / (2 * (DP / 4)), e / (DP / 4) % 2, e % (DP / 4) * 4);
+    else
+      for (int e = threadIdx.x; e < nt * 2 * DP; e += 128) copy(e / (2 * DP), e / DP % 2, e % DP);
+    for (int e = threadIdx.x; e < nt * PB; e += 128) {
+      const int t = e / PB, i = e % PB;
+      if (col0 + i < dv)
+        cp_async_f(base + t * PER + 2 * DP + i, proj + (size_t)(r0 + t0 + t) * ld + v_col + (size_t)h * dv + col0 + i, false);
     }
-    for (int e = threadIdx.x; e < nt * (PB + 2); e += blockDim.x) {
-      const int t = e / (PB + 2), i = e % (PB + 2);
-      const float* row = proj + (size_t)(r0 + t0 + t) * ld;
-      float* tok = base + (size_t)t * per + 2 * dpp;
-      if (i == PB) cp_async_f(tok + PB + 1, row + i_col + h, false);
-      else if (i == PB + 1) cp_async_f(tok + PB + 2, row + f_col + h, false);
-      else if (blockIdx.z * PB + i < dv) cp_async_f(tok + i, row + v_col + (size_t)h * dv + blockIdx.z * PB + i, false);
+    if (threadIdx.x < 2 * nt) {
+      const int t = threadIdx.x >> 1, which = threadIdx.x & 1;
+      cp_async_f(base + t * PER + 2 * DP + PB + which, proj + (size_t)(r0 + t0 + t) * ld + (which ? f_col : i_col) + h, false);
     }
     cp_async_commit();
   };
-  const int cv = col_local <= PB ? col_local : PB;
   const int n_chunks = (n + TC - 1) / TC;
+  float(*mine)[3] = gates[threadIdx.x >> 5];
   stage(0, 0);
   for (int c = 0; c < n_chunks; ++c) {
     if (c + 1 < n_chunks) { stage((c + 1) * TC, (c + 1) & 1); cp_async_wait<1>(); }
     else cp_async_wait<0>();
     __syncthreads();
     const int t0 = c * TC, nt = n - t0 < TC ? n - t0 : TC;
-    const float* base = sm + (size_t)(c & 1) * TC * per;
-    if (threadIdx.x == 0) {  // the running maximum is a chain of one add and one max per token
-      float m = ms[0];
-      for (int t = 0; t < nt; ++t) {
-        const float* tok = base + (size_t)t * per + 2 * dpp;
-        m = fmaxf(tok[PB + 2] + m, tok[PB + 1]);
-        ms[t + 1] = m;
+    const float* tok = sm + (c & 1) * TC * PER;
+    {
+      float before = m, after = m;  // the maximum before and after this lane's token
+#pragma unroll
+      for (int t = 0; t < TC; ++t) {
+        if (t < nt) {
+          const float next = fmaxf(tok[t * PER + 2 * DP + PB + 1] + m, tok[t * PER + 2 * DP + PB]);
+          if (t == lane) { before = m; after = next; }
+          m = next;
+        }
       }
+      if (lane < nt) {
+        const float* at = tok + lane * PER + 2 * DP + PB;
+        mine[lane][0] = expf(at[1] + before - after);
+        mine[lane][1] = expf(at[0] - after);
+        mine[lane][2] = expf(-after);
+      }
+      __syncwarp();
     }
-    __syncthreads();
-    if (threadIdx.x < nt) {
-      const int t = threadIdx.x;
-      const float* tok = base + (size_t)t * per + 2 * dpp;
-      keep[t] = expf(tok[PB + 2] + ms[t] - ms[t + 1]);
-      take[t] = expf(tok[PB + 1] - ms[t + 1]);
-      floor_[t] = expf(-ms[t + 1]);
-    }
-    __syncthreads();
-    const float* tok = base;
-    const int mine = s * staged_stride<NR>();
-    float* so_at = so + col_local;
+    float* o_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col;
 #pragma unroll 2
-    for (int t = 0; t < nt; ++t, tok += per, so_at += PB + 1) {
-      const float4* gq = reinterpret_cast<const float4*>(tok + mine);
-      const float4* gk = reinterpret_cast<const float4*>(tok + dpp + mine);
-      const float kp = keep[t], w = take[t] * tok[2 * dpp + cv];
-      float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+    for (int t = 0; t < nt; ++t, tok += PER, o_at += H * dv) {
+      f32x2 k[PAIRS], q[PAIRS];
+      float v[NC], o[NC];
+      staged_rows<C>(k, tok + DP, s);
+      staged_rows<C>(q, tok, s);
+      staged_values<NC>(v, tok + 2 * DP, at);
+      const float take = mine[t][1];
+      const f32x2 keep = f2_both(mine[t][0]), w1 = f2_both(take);
 #pragma unroll
-      for (int i = 0; i < NR / 4; ++i) {
-        const float4 kv4 = gk[i], qv = gq[i];
-        S[4 * i] = fmaf(kp, S[4 * i], w * kv4.x); S[4 * i + 1] = fmaf(kp, S[4 * i + 1], w * kv4.y);
-        S[4 * i + 2] = fmaf(kp, S[4 * i + 2], w * kv4.z); S[4 * i + 3] = fmaf(kp, S[4 * i + 3], w * kv4.w);
-        p0 = fmaf(S[4 * i], qv.x, p0); p1 = fmaf(S[4 * i + 1], qv.y, p1);
-        p2 = fmaf(S[4 * i + 2], qv.z, p2); p3 = fmaf(S[4 * i + 3], qv.w, p3);
+      for (int j = 0; j < NC; ++j) {
+        const f32x2 w = f2_both(take * v[j]);
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(keep, S[j][i], f2_mul(w, k[i]));
+        o[j] = dot_rows(S[j], q);
       }
-      const float po = group_sum((p0 + p1) + (p2 + p3), NS) * qscale;
-      if (s == 0 && col_local <= PB) *so_at = po;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nt * PB; e += blockDim.x) {
-      const int t = e / PB, i = e % PB;
-      if (blockIdx.z * PB + i < dv) {
-        const float den = fmaxf(fabsf(so[(size_t)t * (PB + 1) + PB]), floor_[t]) + 1e-6f;
-        out[(size_t)(r0 + t0 + t) * H * dv + (size_t)h * dv + blockIdx.z * PB + i] = so[(size_t)t * (PB + 1) + i] / den;
-      }
-    }
-    if (threadIdx.x == 0) ms[0] = ms[nt];
-    __syncthreads();  // the buffers and the chunk's sums are free again
-  }
-  // every block of a (head, request) starts from the same n and m, so no block of this launch may replace them:
-  // the block of the first columns leaves the new ones in nm_new [requests, H, d + 1], and a launch of its own
-  // moves them into the slots once this one is through
-  if (live && col_local < PB) {
 #pragma unroll
-    for (int i = 0; i < NR; ++i)
-      if (s * NR + i < d) st[s * NR + i] = S[i];
+      for (int i = 0; i < PAIRS; ++i) Z[i] = f2_fma(keep, Z[i], f2_mul(w1, k[i]));
+      const float num = column_sum<C>(o, s) * qscale;
+      const float z = group_sum<NS>(dot_rows(Z, q)) * qscale;
+      if (writes) *o_at = num / (fmaxf(fabsf(z), mine[t][2]) + 1e-6f);
+    }
+    __syncthreads();  // the buffer is free again
   }
-  float* nm = nm_new + ((size_t)rq * H + h) * (d + 1);
-  if (is_n && blockIdx.z == 0) {
-#pragma unroll
-    for (int i = 0; i < NR; ++i)
-      if (s * NR + i < d) nm[s * NR + i] = S[i];
+  // every block of a (head, request) starts from the same n and m, so no block of this launch may replace them: the
+  // first column's threads of the first block leave the new ones aside
+  store_rows<C>(S, st, s, d, cols, wide);
+  if (blockIdx.z == 0 && col_local == 0) {
+    float* nm = nm_new + ((size_t)rq * H + h) * (d + 1);
+    store_column<C::NS, C::PAIRS>(Z, nm, s, d, 0);
+    if (s == 0) nm[d] = m;
   }
-  if (threadIdx.x == 0 && blockIdx.z == 0) nm[d] = ms[0];
 }
 
 __global__ void mlstm_commit_kernel(const float* __restrict__ nm_new, float* __restrict__ nrm, float* __restrict__ mx,
@@ -652,39 +632,23 @@ head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w, 
   }
 }
 
-int round_nr(int nr) { return nr <= 4 ? 4 : nr <= 8 ? 8 : nr <= 16 ? 16 : 32; }
-
-// (threads per value column, state rows per thread) for d key channels and `columns` value columns in the whole
-// launch. A column's chain of arithmetic per token is serial, so a launch with few columns (one prompt) is bound by
-// latency: it gets more threads per column, down to four state rows each, until the GPU's schedulers have several
-// warps apiece; a launch with many columns (a batch of single tokens) keeps longer rows per thread.
-bool split_rows(int d, long long columns, int* ns_out, int* nr_out) {
-  int ns = 1;
-  while ((d + ns - 1) / ns > MAXR && ns < 32) ns <<= 1;
-  if ((d + ns - 1) / ns > MAXR) return false;
-  int sms = 148, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  static const int forced = getenv("CUCA_SCAN_THREADS") ? atoi(getenv("CUCA_SCAN_THREADS")) : 0;  // a measuring aid
-  while (ns < 32 && ns * 4 <= d && (forced ? ns < forced : columns * ns < (long long)sms * 2048)) ns <<= 1;
-  *ns_out = ns;
-  *nr_out = round_nr((d + ns - 1) / ns);
-  return true;
-}
-
-// threads of a block: 512 where a column has 16 threads or more (the block's staged vectors then serve more
-// columns), else 128. Measured on 2,048-token prompts, 32 threads a column: at 16 heads of 128 x 128 blocks of 128
-// threads are 5 % faster for the whole prompt step than blocks of 512 (15.9 against 16.9 ms), at 24 and 32 heads they
-// are 17 % slower (23.7 against 20.1 ms, 28.9 against 24.7): 512 stays.
-int block_threads(int ns, int nr) {
-  static const int forced = getenv("CUCA_SCAN_BLOCK") ? atoi(getenv("CUCA_SCAN_BLOCK")) : 0;  // a measuring aid
-  if (forced >= ns && forced <= 512) return forced;
-  return ns >= 16 ? (nr >= 16 ? 256 : 512) : 128;
+// Runs `go` with the split of d key channels (at most MAX_DIM). A prompt of one request has few columns (16 heads of
+// 128: 2,048) and a serial chain of one token after the other, so what counts is the time of one token in one warp: at
+// 128 channels, eight channels of two columns a thread give each of the SM's four schedulers one warp.
+template <typename F>
+int with_split(int d, F go) {
+  if (d <= 16) return go(Split<2, 8, 2>());
+  if (d <= 32) return go(Split<4, 8, 2>());
+  if (d <= 64) return go(Split<8, 8, 2>());
+  if (d <= 128) return go(Split<16, 8, 2>());
+  if (d <= 256) return go(Split<32, 8, 2>());
+  if (d <= 512) return go(Split<32, 16, 2>());
+  return go(Split<32, 32, 2>());
 }
 
 }  // namespace
 
-CUCA_API int cuca_matrix_state_max_dim() { return 32 * MAXR; }
+CUCA_API int cuca_matrix_state_max_dim() { return MAX_DIM; }
 
 // qkv, a_raw and the gate column of b_raw are rewritten in place by the preparing kernel (see there), then scanned.
 CUCA_API int cuca_delta_scan(float* qkv, int ld, float* a_raw, int ld_a, const float* dt_bias, const float* a_log,
@@ -695,33 +659,19 @@ CUCA_API int cuca_delta_scan(float* qkv, int ld, float* a_raw, int ld_a, const f
   CUCA_REQUIRE(H > 0 && G > 0 && H % G == 0 && d > 0 && dv > 0, "delta_scan: bad sizes heads=%d key heads=%d dim=%d vdim=%d",
                H, G, d, dv);
   CUCA_REQUIRE(n_seqs <= 65535 && H <= 256, "delta_scan: %d requests or %d heads exceed the launch limits", n_seqs, H);
-  int ns, nr;
-  CUCA_REQUIRE(split_rows(d, (long long)n_seqs * H * dv, &ns, &nr), "delta_scan: %d key channels exceed %d", d, 32 * MAXR);
+  CUCA_REQUIRE(d <= MAX_DIM, "delta_scan: %d key channels exceed %d", d, MAX_DIM);
   cuca_launch(delta_prepare_kernel, dim3(n_rows), dim3(256), 0, stream, true, qkv, ld, a_raw, ld_a, dt_bias, a_log, b_raw, ld_b,
               b_col, seq_of_row, H, G, d);
   CUCA_CHECK_LAUNCH("delta_prepare");
-  int pb = block_threads(ns, nr) / ns;
-  pb = pb > dv ? dv : pb;
-  const int threads = (pb * ns + 31) / 32 * 32;
-  const int per = (3 * ns * (nr == 4 ? 4 : nr + 4) + pb + 1 + 3) & ~3;
-  int tc = 46000 / (2 * per * 4);
-  tc = tc > 16 ? 16 : tc;
-  CUCA_REQUIRE(tc >= 1, "delta_scan: a token of %d key channels does not fit shared memory", d);
-  const size_t smem = (size_t)2 * tc * per * 4;
   // 16-byte copies where every source is aligned for them
-  const int wide = d % 4 == 0 && ld % 4 == 0 && ld_a % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)a_raw & 15) == 0;
-  dim3 grid(H, n_seqs, (dv + pb - 1) / pb);
-#define DS(NR)                                                                                                    \
-  cuca_launch(delta_scan_kernel<NR>, grid, dim3(threads), smem, stream, true, (const float*)qkv, ld,              \
-              (const float*)a_raw, ld_a, (const float*)b_raw, ld_b, b_col, state, out, req_row0, req_count, slots, H, G, d, \
-              dv, ns, pb, tc, wide)
-  if (nr == 4) DS(4);
-  else if (nr == 8) DS(8);
-  else if (nr == 16) DS(16);
-  else DS(32);
-#undef DS
-  CUCA_CHECK_LAUNCH("delta_scan");
-  return 0;
+  const int wide = d % 4 == 0 && ld % 4 == 0 && ld_a % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)a_raw & 15) == 0 &&
+                   ((uintptr_t)state & 15) == 0;
+  return with_split(d, [&](auto split) {
+    using C = decltype(split);
+    return launch_scan<C>("delta_scan", delta_scan_kernel<C>, 3 * C::DP + ((C::PB + 4) & ~3), H, n_seqs, dv, stream,
+                          (const float*)qkv, ld, (const float*)a_raw, ld_a, (const float*)b_raw, ld_b, b_col, state, out,
+                          req_row0, req_count, slots, H, G, d, dv, wide);
+  });
 }
 
 // The two gate columns of proj are rewritten in place by the preparing kernel (see there), then scanned.
@@ -734,30 +684,19 @@ CUCA_API int cuca_mlstm_scan(float* proj, int ld, int q_col, int k_col, int v_co
   CUCA_REQUIRE(H > 0 && d > 0 && dv > 0 && cap > 0.f, "mlstm_scan: bad sizes heads=%d dim=%d vdim=%d cap=%g", H, d, dv,
                (double)cap);
   CUCA_REQUIRE(n_seqs <= 65535, "mlstm_scan: %d requests exceed the launch limit", n_seqs);
-  int ns, nr;
-  CUCA_REQUIRE(split_rows(d, (long long)n_seqs * H * dv, &ns, &nr), "mlstm_scan: %d key channels exceed %d", d, 32 * MAXR);
+  CUCA_REQUIRE(d <= MAX_DIM, "mlstm_scan: %d key channels exceed %d", d, MAX_DIM);
   cuca_launch(mlstm_prepare_kernel, dim3((n_rows * H + 127) / 128), dim3(128), 0, stream, true, proj, ld, i_col, f_col,
               i_bias, f_bias, cap, n_rows, H);
   CUCA_CHECK_LAUNCH("mlstm_prepare");
-  int pb = block_threads(ns, nr) / ns - 1;  // one more column carries n
-  pb = pb < 1 ? 1 : (pb > dv ? dv : pb);
-  const int threads = ((pb + 1) * ns + 31) / 32 * 32;
-  const int per = (2 * ns * (nr == 4 ? 4 : nr + 4) + (pb + 1) + 2 + 3) & ~3;
-  int tc = 46000 / ((2 * per + pb + 6) * 4);
-  tc = tc > 16 ? 16 : tc;
-  CUCA_REQUIRE(tc >= 1, "mlstm_scan: a token of %d key channels does not fit shared memory", d);
-  const size_t smem = ((size_t)2 * tc * per + (size_t)tc * (pb + 1) + 4 * tc + 1) * 4;
-  const int wide = d % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && ((uintptr_t)proj & 15) == 0;
-  dim3 grid(H, n_seqs, (dv + pb - 1) / pb);
-#define MS(NR)                                                                                                      \
-  cuca_launch(mlstm_scan_kernel<NR>, grid, dim3(threads), smem, stream, true, (const float*)proj, ld, q_col, k_col,   \
-              v_col, i_col, f_col, mem, nrm, mx, out, req_row0, req_count, slots, H, d, dv, ns, pb, tc, wide, nm_new)
-  if (nr == 4) MS(4);
-  else if (nr == 8) MS(8);
-  else if (nr == 16) MS(16);
-  else MS(32);
-#undef MS
-  CUCA_CHECK_LAUNCH("mlstm_scan");
+  const int wide = d % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && ((uintptr_t)proj & 15) == 0 &&
+                   (((uintptr_t)mem | (uintptr_t)nrm) & 15) == 0;
+  const int rc = with_split(d, [&](auto split) {
+    using C = decltype(split);
+    return launch_scan<C>("mlstm_scan", mlstm_scan_kernel<C>, 2 * C::DP + ((C::PB + 5) & ~3), H, n_seqs, dv, stream,
+                          (const float*)proj, ld, q_col, k_col, v_col, i_col, f_col, mem, (const float*)nrm,
+                          (const float*)mx, out, req_row0, req_count, slots, H, d, dv, wide, nm_new);
+  });
+  if (rc) return rc;
   cuca_launch(mlstm_commit_kernel, dim3(H, n_seqs), dim3(128), 0, stream, true, (const float*)nm_new, nrm, mx, req_count,
               slots, H, d);
   CUCA_CHECK_LAUNCH("mlstm_commit");
@@ -772,8 +711,7 @@ CUCA_API int cuca_forget_scan(float* proj, int ld, int q_col, int f_col, int v_c
   if (n_seqs == 0 || n_rows == 0) return 0;
   CUCA_REQUIRE(H > 0 && d > 0 && dv > 0, "forget_scan: bad sizes heads=%d dim=%d vdim=%d", H, d, dv);
   CUCA_REQUIRE(n_seqs <= 65535, "forget_scan: %d requests exceed the launch limit", n_seqs);
-  int ns, nr;
-  CUCA_REQUIRE(split_rows(d, (long long)n_seqs * H * dv, &ns, &nr), "forget_scan: %d key channels exceed %d", d, 32 * MAXR);
+  CUCA_REQUIRE(d <= MAX_DIM, "forget_scan: %d key channels exceed %d", d, MAX_DIM);
   {
     size_t blocks = ((size_t)n_rows * H * d + 255) / 256;
     blocks = blocks > 8192 ? 8192 : blocks;
@@ -781,54 +719,28 @@ CUCA_API int cuca_forget_scan(float* proj, int ld, int q_col, int f_col, int v_c
                 lower, seq_of_row, n_rows, H * d);
     CUCA_CHECK_LAUNCH("forget_prepare");
   }
-  int pb = block_threads(ns, nr) / ns;
-  pb = pb > dv ? dv : pb;
-  const int threads = (pb * ns + 31) / 32 * 32;
-  const int per = (2 * ns * (nr == 4 ? 4 : nr + 4) + pb + 3) & ~3;
-  int tc = 46000 / (2 * per * 4);
-  tc = tc > 16 ? 16 : tc;
-  CUCA_REQUIRE(tc >= 1, "forget_scan: a token of %d key channels does not fit shared memory", d);
-  const size_t smem = (size_t)2 * tc * per * 4;
-  const int wide = d % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && f_col % 4 == 0 && ((uintptr_t)proj & 15) == 0;
-  dim3 grid(H, n_seqs, (dv + pb - 1) / pb);
-#define FS(NR)                                                                                                     \
-  cuca_launch(forget_scan_kernel<NR, false>, grid, dim3(threads), smem, stream, true, (const float*)proj, ld, q_col, \
-              f_col, v_col, (const float*)nullptr, state, out, req_row0, req_count, slots, H, d, dv, ns, pb, tc, wide)
-  if (nr == 4) FS(4);
-  else if (nr == 8) FS(8);
-  else if (nr == 16) FS(16);
-  else FS(32);
-#undef FS
-  CUCA_CHECK_LAUNCH("forget_scan");
-  return 0;
+  const int wide = d % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && f_col % 4 == 0 && ((uintptr_t)proj & 15) == 0 &&
+                   ((uintptr_t)state & 15) == 0;
+  return with_split(d, [&](auto split) {
+    using C = decltype(split);
+    return launch_scan<C>("forget_scan", forget_scan_kernel<C, false>, 2 * C::DP + ((C::PB + 3) & ~3), H, n_seqs, dv, stream,
+                          (const float*)proj, ld, q_col, f_col, v_col, (const float*)nullptr, state, out, req_row0,
+                          req_count, slots, H, d, dv, wide);
+  });
 }
 
 // S <- decay[h] S + k v^T, o = S^T q along every request's rows of a prepared 32-bit projection
 static int launch_decay_scan(const char* name, const float* proj, int ld, int q_col, int k_col, int v_col, const float* decay,
                              float* state, float* out, const int* req_row0, const int* req_count, const int* slots,
                              int n_seqs, int H, int d, int dv, cudaStream_t stream) {
-  int ns, nr;
-  CUCA_REQUIRE(split_rows(d, (long long)n_seqs * H * dv, &ns, &nr), "%s: %d key channels exceed %d", name, d, 32 * MAXR);
-  int pb = block_threads(ns, nr) / ns;
-  pb = pb > dv ? dv : pb;
-  const int threads = (pb * ns + 31) / 32 * 32;
-  const int per = (2 * ns * (nr == 4 ? 4 : nr + 4) + pb + 3) & ~3;
-  int tc = 46000 / (2 * per * 4);
-  tc = tc > 16 ? 16 : tc;
-  CUCA_REQUIRE(tc >= 1, "%s: a token of %d key channels does not fit shared memory", name, d);
-  const size_t smem = (size_t)2 * tc * per * 4;
-  const int wide = d % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && ((uintptr_t)proj & 15) == 0;
-  dim3 grid(H, n_seqs, (dv + pb - 1) / pb);
-#define RS(NR)                                                                                                     \
-  cuca_launch(forget_scan_kernel<NR, true>, grid, dim3(threads), smem, stream, true, proj, ld, q_col,  \
-              k_col, v_col, decay, state, out, req_row0, req_count, slots, H, d, dv, ns, pb, tc, wide)
-  if (nr == 4) RS(4);
-  else if (nr == 8) RS(8);
-  else if (nr == 16) RS(16);
-  else RS(32);
-#undef RS
-  CUCA_CHECK_LAUNCH(name);
-  return 0;
+  CUCA_REQUIRE(d <= MAX_DIM, "%s: %d key channels exceed %d", name, d, MAX_DIM);
+  const int wide = d % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && ((uintptr_t)proj & 15) == 0 &&
+                   ((uintptr_t)state & 15) == 0;
+  return with_split(d, [&](auto split) {
+    using C = decltype(split);
+    return launch_scan<C>(name, forget_scan_kernel<C, true>, 2 * C::DP + ((C::PB + 3) & ~3), H, n_seqs, dv, stream, proj, ld,
+                          q_col, k_col, v_col, decay, state, out, req_row0, req_count, slots, H, d, dv, wide);
+  });
 }
 
 // Retention along every request's rows. proj: 32-bit rows of stride ld holding q heads at q_col, k heads at k_col (H
@@ -882,7 +794,7 @@ CUCA_API int cuca_lightning_step(const float* proj, int ld, int col0, const floa
                                  const int* req_row0, const int* req_count, const int* slots, int n_seqs, int H, int d,
                                  int dv, cudaStream_t stream) {
   if (n_seqs == 0) return 0;
-  CUCA_REQUIRE(H > 0 && d > 0 && dv > 0 && d <= 32 * MAXR, "lightning_step: bad sizes heads=%d dim=%d vdim=%d", H, d, dv);
+  CUCA_REQUIRE(H > 0 && d > 0 && dv > 0 && d <= MAX_DIM, "lightning_step: bad sizes heads=%d dim=%d vdim=%d", H, d, dv);
   CUCA_REQUIRE(n_seqs <= 65535, "lightning_step: %d requests exceed the launch limit", n_seqs);
   const bool wide = d % 4 == 0 && ld % 4 == 0 && col0 % 4 == 0 && ((uintptr_t)proj & 15) == 0 && ((uintptr_t)state & 15) == 0;
 #define LS(V, R, COLS)                                                                                              \

@@ -7,6 +7,7 @@
 // order from the state its slot holds and leaves the new state there. The order of the arithmetic along a sequence
 // does not depend on where it was cut into steps.
 #include "common.cuh"
+#include "state_rows.cuh"
 #include <math.h>
 
 namespace {
@@ -147,120 +148,113 @@ __global__ void causal_conv_kernel(const float* __restrict__ in, int ld_in, int 
   }
 }
 
-constexpr int SSM_MAXR = 32;  // state values a thread holds
+constexpr int SSM_MAX_STATE = 1024;
 
-// an asynchronous copy of 4 or 16 bytes from global to shared memory
-__device__ __forceinline__ void cp_async_f(float* dst, const float* src, int bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-
-// One block per (head, request, run of PB value columns). Thread (p, s): value column p, state rows s, s + NS,
-// s + 2 NS, ... (neighbouring threads read neighbouring shared-memory banks). state: [slots, H, P, N]. xbc: 32-bit [rows, H P + 2 G N] after the convolution (x | B | C); dt_raw: rows of stride ld_dt,
-// head h at column dt_col + h, before bias and softplus.
-// NR: state rows a thread holds at most. NST: threads per value column when that is known at compile time and divides
-// the state evenly into NR rows each (the recurrence's loop is then free of index arithmetic and predicates: the
-// kernel is bound by how many instructions it issues); 0: the number comes at run time and rows are checked.
-template <int NR, int NST>
-__global__ void ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, int ld_dt, int dt_col,
-                                const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-                                const float* __restrict__ d_skip, float* __restrict__ state, float* __restrict__ y,
-                                const int* __restrict__ req_row0, const int* __restrict__ req_count,
-                                const int* __restrict__ slots, int H, int P, int N, int G, int NS_rt, int TC,
-                                int PB) {
-  const int NS = NST ? NST : NS_rt;
+// One block per (head, request, run of PB value columns); a column's state rows lie with NS threads (see Split).
+// state: [slots, H, P, N]. xbc: 32-bit [rows, H P + 2 G N] after the convolution (x | B | C); dt_raw: rows of stride
+// ld_dt, head h at column dt_col + h, before bias and softplus.
+// Tokens hang together through one multiply-add per state value alone, so the kernel is bound by how many instructions
+// it issues and by its reads of shared memory: eight rows of four columns a thread, pairs of rows in every instruction.
+template <typename S_>
+__global__ void __launch_bounds__(128)
+ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, int ld_dt, int dt_col,
+                const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                const float* __restrict__ d_skip, float* __restrict__ state, float* __restrict__ y,
+                const int* __restrict__ req_row0, const int* __restrict__ req_count,
+                const int* __restrict__ slots, int H, int P, int N, int G, int wide) {
+  constexpr int NS = S_::NS, NC = S_::NC, DP = S_::DP, PB = S_::PB, TC = S_::TC, PAIRS = S_::PAIRS;
+  constexpr int PER = 2 * DP + ((PB + 1 + 3) & ~3);  // a token: B, C, the block's x, the raw step size
+  static_assert(TC <= 32, "a lane a token");
   extern __shared__ __align__(16) float sm[];
+  __shared__ float steps[4][TC][2];  // a warp's own: step size, decay
   pdl_trigger();
   pdl_wait();
   const int h = blockIdx.x, q = blockIdx.y;
   const int slot = slots[q], n = req_count[q], r0 = req_row0[q];
   if (slot < 0 || n <= 0) return;
-  const int p_raw = blockIdx.z * PB + threadIdx.x / NS, s = threadIdx.x % NS;
-  const bool live = threadIdx.x / NS < PB && p_raw < P;
-  const int p = live ? p_raw : P - 1;
+  const int lane = threadIdx.x & 31;
+  const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
+  const int col0 = blockIdx.z * PB, at = col_local * NC;
+  const int cols = min(NC, P - col0 - at);              // columns of this thread that exist (none: 0 or less)
+  const int own = s / (NS / NC), p = col0 + at + own;   // the column whose sums this thread ends up with
+  const bool writes = s % (NS / NC) == 0 && own < cols;
   const int g = h / (H / G);
   const int C = H * P + 2 * G * N;
-  float S[NR];
-  float* st = state + (((size_t)slot * H + h) * P + p) * N;
-#pragma unroll
-  for (int i = 0; i < NR; ++i) S[i] = (NST || s + i * NS < N) ? st[s + i * NS] : 0.f;
+  float* st = state + (((size_t)slot * H + h) * P + (cols > 0 ? col0 + at : 0)) * N;
+  f32x2 S[NC][PAIRS];
+  load_rows<S_>(S, st, s, N, cols, wide);
   const float A = -expf(a_log[h]);
   const float bias = dt_bias[h], D = d_skip[h];
-  // A token's inputs in shared memory: B [N], C [N], x [P], step size, decay; `per` floats, a multiple of four.
+  // what no copy writes: rows from N on (B = C = 0) and the values of columns from P on
+  {
+    const int spare = DP - N, fill = 2 * spare + PB;
+    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
+      const int t = e / fill, w = e % fill;
+      float* tok = sm + t * PER;
+      if (w < 2 * spare) tok[(w / spare) * DP + N + w % spare] = 0.f;
+      else tok[2 * DP + (w - 2 * spare)] = 0.f;
+    }
+  }
+  __syncthreads();
   // Two runs of TC tokens: the next run's copies (cp.async) are in flight while this one is worked through.
-  const int span = 2 * N + P;
-  const int per = (span + 2 + 3) & ~3;
-  const bool vec4 = ((N | P | (H * P)) & 3) == 0;
   auto stage = [&](int t0, int buf) {
     const int nt = n - t0 < TC ? n - t0 : TC;
-    float* dst = sm + (size_t)buf * TC * per;
-    if (vec4) {
-      const int units = span >> 2;
-      for (int e = threadIdx.x; e < nt * units; e += blockDim.x) {
-        const int tt = e / units, i = (e - tt * units) << 2;
-        const int col = i < 2 * N ? H * P + g * N + i + (i >= N ? (G - 1) * N : 0) : h * P + (i - 2 * N);
-        cp_async_f(dst + tt * per + i, xbc + (size_t)(r0 + t0 + tt) * C + col, 16);
-      }
-    } else {
-      for (int e = threadIdx.x; e < nt * span; e += blockDim.x) {
-        const int tt = e / span, i = e - tt * span;
-        const int col = i < 2 * N ? H * P + g * N + i + (i >= N ? (G - 1) * N : 0) : h * P + (i - 2 * N);
-        cp_async_f(dst + tt * per + i, xbc + (size_t)(r0 + t0 + tt) * C + col, 4);
-      }
+    float* base = sm + buf * TC * PER;
+    auto copy = [&](int t, int which, int r) {
+      const float* src = xbc + (size_t)(r0 + t0 + t) * C + H * P + (which * G + g) * N + r;
+      if (r < N) cp_async_f(base + t * PER + which * DP + r, src, wide);
+    };
+    if (wide)
+      for (int e = threadIdx.x; e < nt * 2 * (DP / 4); e += 128) copy(e / (2 * (DP / 4)), e / (DP / 4) % 2, e % (DP / 4) * 4);
+    else
+      for (int e = threadIdx.x; e < nt * 2 * DP; e += 128) copy(e / (2 * DP), e / DP % 2, e % DP);
+    for (int e = threadIdx.x; e < nt * PB; e += 128) {
+      const int t = e / PB, i = e % PB;
+      if (col0 + i < P) cp_async_f(base + t * PER + 2 * DP + i, xbc + (size_t)(r0 + t0 + t) * C + h * P + col0 + i, false);
     }
-    for (int e = threadIdx.x; e < nt; e += blockDim.x)
-      cp_async_f(dst + e * per + span, dt_raw + (size_t)(r0 + t0 + e) * ld_dt + dt_col + h, 4);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (threadIdx.x < nt)
+      cp_async_f(base + threadIdx.x * PER + 2 * DP + PB, dt_raw + (size_t)(r0 + t0 + threadIdx.x) * ld_dt + dt_col + h, false);
+    cp_async_commit();
   };
+  float(*mine)[2] = steps[threadIdx.x >> 5];
+  const int n_chunks = (n + TC - 1) / TC;
   stage(0, 0);
-  for (int t0 = 0, run = 0; t0 < n; t0 += TC, ++run) {
-    const int nt = n - t0 < TC ? n - t0 : TC;
-    float* cur = sm + (size_t)(run & 1) * TC * per;
-    if (t0 + TC < n) {
-      stage(t0 + TC, (run & 1) ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
+  for (int c = 0; c < n_chunks; ++c) {
+    if (c + 1 < n_chunks) { stage((c + 1) * TC, (c + 1) & 1); cp_async_wait<1>(); }
+    else cp_async_wait<0>();
     __syncthreads();
-    if (threadIdx.x < nt) {  // step size and decay of every token of the run, once
-      float* in = cur + threadIdx.x * per;
-      const float raw = in[span] + bias;
+    const int t0 = c * TC, nt = n - t0 < TC ? n - t0 : TC;
+    const float* tok = sm + (c & 1) * TC * PER;
+    if (lane < nt) {  // step size and decay of every token of the run
+      const float raw = tok[lane * PER + 2 * DP + PB] + bias;
       const float dt = raw > 20.f ? raw : log1pf(expf(raw));
-      in[span] = dt;
-      in[span + 1] = expf(A * dt);
+      mine[lane][0] = dt;
+      mine[lane][1] = expf(A * dt);
     }
-    __syncthreads();
-    // (tokens only hang together through one multiply-add per state value: four of them are worked through at once)
-#pragma unroll 4
-    for (int tt = 0; tt < nt; ++tt) {
-      const float* in = cur + tt * per;
-      const float dt = in[span], decay = in[span + 1];
-      const float x = in[2 * N + p];
-      const float* Br = in + s;
-      const float* Cr = in + N + s;
-      const float dx = dt * x;
-      // four partial sums, in an order that depends on the sizes alone
-      float part[4] = {0.f, 0.f, 0.f, 0.f};
+    __syncwarp();
+    float* y_at = y + (size_t)(r0 + t0) * (H * P) + h * P + p;
+#pragma unroll 2
+    for (int t = 0; t < nt; ++t, tok += PER, y_at += H * P) {
+      f32x2 B[PAIRS], Cv[PAIRS];
+      staged_rows<S_>(B, tok, s);
+      staged_rows<S_>(Cv, tok + DP, s);
+      float x[NC], acc[NC];
+      staged_values<NC>(x, tok + 2 * DP, at);
+      const float dt = mine[t][0], x_own = tok[2 * DP + at + own];
+      const f32x2 decay = f2_both(mine[t][1]);
 #pragma unroll
-      for (int i = 0; i < NR; ++i) {
-        if (NST || s + i * NS < N) {
-          S[i] = fmaf(decay, S[i], dx * Br[i * NS]);
-          part[i & 3] = fmaf(S[i], Cr[i * NS], part[i & 3]);
-        }
+      for (int j = 0; j < NC; ++j) {
+        const f32x2 dx = f2_both(dt * x[j]);
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(decay, S[j][i], f2_mul(dx, B[i]));
+        acc[j] = dot_rows(S[j], Cv);
       }
-      float acc = (part[0] + part[1]) + (part[2] + part[3]);
-      for (int o = NS >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (live && s == 0) y[(size_t)(r0 + t0 + tt) * (H * P) + h * P + p] = acc + D * x;
+      const float sum = column_sum<S_>(acc, s);
+      if (writes) *y_at = sum + D * x_own;
     }
     __syncthreads();  // this run is read to the end before the run after next is copied over it
   }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < NR; ++i)
-      if (NST || s + i * NS < N) st[s + i * NS] = S[i];
-  }
+  store_rows<S_>(S, st, s, N, cols, wide);
 }
 
 // One block per (row, part). v = y * silu(z); out = v * rsqrt(mean over the part (v^2) + eps) * w.
@@ -382,16 +376,6 @@ CUCA_API int cuca_causal_conv(const float* in, int ld_in, int col0, const void* 
 }
 
 // How the state rows of a head are dealt to threads: (threads per value column, state rows per thread).
-CUCA_API int cuca_ssm_scan_split(int P, int N, int* ns_out, int* nr_out) {
-  int ns = 1;
-  while ((N + ns - 1) / ns > SSM_MAXR && ns < 32) ns <<= 1;
-  if ((N + ns - 1) / ns > SSM_MAXR) return 1;
-  while (ns < 16 && ns * 4 <= N) ns <<= 1;  // at least four state rows a thread, at most sixteen threads a column
-  *ns_out = ns;
-  *nr_out = (N + ns - 1) / ns;
-  return 0;
-}
-
 CUCA_API int cuca_ssm_scan(const float* xbc, const float* dt_raw, int ld_dt, int dt_col, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, float* y, const int* req_row0,
                            const int* req_count, const int* slots, int n_seqs, int H, int P, int N, int G,
@@ -400,41 +384,21 @@ CUCA_API int cuca_ssm_scan(const float* xbc, const float* dt_raw, int ld_dt, int
   CUCA_REQUIRE(H > 0 && P > 0 && N > 0 && G > 0 && H % G == 0, "ssm_scan: bad sizes heads=%d vdim=%d state=%d groups=%d",
                H, P, N, G);
   CUCA_REQUIRE(n_seqs <= 65535, "ssm_scan: %d requests exceed the launch limit", n_seqs);
-  int ns, nr;
-  CUCA_REQUIRE(cuca_ssm_scan_split(P, N, &ns, &nr) == 0, "ssm_scan: state size %d exceeds %d", N, 32 * SSM_MAXR);
-  // value columns of a block: what fills 128 threads, so that a head's columns spread over several SMs
-  int pb = 128 / ns;
-  pb = pb < 1 ? 1 : (pb > P ? P : pb);
-  const int threads = (pb * ns + 31) / 32 * 32;
-  // tokens whose inputs are staged together: two runs of as many as 44 KB of shared memory hold, 16 at most
-  const int per = (2 * N + P + 2 + 3) & ~3;
-  int tc = 45056 / (2 * per * 4);
-  tc = tc > 16 ? 16 : tc;
-  CUCA_REQUIRE(tc >= 1, "ssm_scan: state size %d and value size %d exceed a token's shared memory", N, P);
-#define SSM(NR, NST)                                                                                              \
-  cuca_launch(ssm_scan_kernel<NR, NST>, dim3(H, n_seqs, (P + pb - 1) / pb), dim3(threads), (size_t)2 * tc * per * 4, \
-              stream, true, xbc, dt_raw, ld_dt, dt_col, dt_bias, a_log, d_skip, state, y, req_row0, req_count, slots, \
-              H, P, N, G, ns, tc, pb)
-#define SSM_BY_NS(NR)                                     \
-  do {                                                    \
-    if (!exact) SSM(NR, 0);                               \
-    else if (ns == 16) SSM(NR, 16);                       \
-    else if (ns == 8) SSM(NR, 8);                         \
-    else if (ns == 4) SSM(NR, 4);                         \
-    else if (ns == 2) SSM(NR, 2);                         \
-    else SSM(NR, 1);                                      \
-  } while (0)
-  // the state divides evenly into a row count the kernels are compiled for: the form without checks
-  const bool exact = N % ns == 0 && (nr == 4 || nr == 8 || nr == 16 || nr == 32);
-  if (nr <= 4) SSM_BY_NS(4);
-  else if (nr <= 8) SSM_BY_NS(8);
-  else if (nr <= 16) SSM_BY_NS(16);
-  else SSM_BY_NS(32);
-#undef SSM_BY_NS
-#undef SSM
-  CUCA_CHECK_LAUNCH("ssm_scan");
-  return 0;
+  CUCA_REQUIRE(N <= SSM_MAX_STATE, "ssm_scan: state size %d exceeds %d", N, SSM_MAX_STATE);
+  const int wide = N % 4 == 0 && (H * P) % 4 == 0 && (((uintptr_t)xbc | (uintptr_t)state) & 15) == 0;
+  auto go = [&](auto split) {
+    using C = decltype(split);
+    return launch_scan<C>("ssm_scan", ssm_scan_kernel<C>, 2 * C::DP + ((C::PB + 4) & ~3), H, n_seqs, P, stream, xbc, dt_raw,
+                          ld_dt, dt_col, dt_bias, a_log, d_skip, state, y, req_row0, req_count, slots, H, P, N, G, wide);
+  };
+  if (N <= 32) return go(Split<4, 8, 4>());
+  if (N <= 64) return go(Split<8, 8, 4>());
+  if (N <= 128) return go(Split<16, 8, 4>());
+  if (N <= 256) return go(Split<32, 8, 4>());
+  if (N <= 512) return go(Split<32, 16, 4>());
+  return go(Split<32, 32, 2>());
 }
+
 
 CUCA_API int cuca_gated_group_norm(const float* y, const float* z, int ld_z, const void* w, int w_dtype, void* out,
                                    int out_dtype, int n_rows, int inner, int parts, float eps, cudaStream_t stream) {
