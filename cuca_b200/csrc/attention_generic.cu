@@ -1,12 +1,17 @@
 // Paged causal grouped-query attention, plain form: one warp per (row, query
 // head), keys in tiles of 32 absolute positions with an online softmax. It
-// serves the true 32-bit path and is the fall-back of the bfloat16 path for
-// head sizes its tensor-core kernels refuse. A row's arithmetic depends only
+// is the fall-back for what the 32-bit kernels (attention_f32.cu: head sizes up
+// to 128) and the bfloat16 path's tensor-core kernels refuse. A row's arithmetic depends only
 // on its own position and keys: tiles start at multiples of 32 key positions,
 // so cutting a prompt or batching it differently gives the same bits.
 #include "attention_options.cuh"
 #include "common.cuh"
 #include <math.h>
+
+bool cuca_attention_f32_takes(const void* kpool, const void* vpool, int nh, int nkv, int d, int dv, const CucaAttnOptions* opt);
+int cuca_attention_f32(const float* q, int q_stride, float* out, int out_stride, const float* kpool, const float* vpool,
+                       int n_blocks, int bs, const int* positions, const int* seq_of_row, const int* tables, int table_stride,
+                       int n_rows, int nh, int nkv, int d, int dv, const CucaAttnOptions* opt, int* err, cudaStream_t stream);
 
 namespace {
 
@@ -134,6 +139,10 @@ CUCA_API int cuca_attention_generic_o(const void* q, int q_stride, void* out, in
                2 * cuca_attention_max_head_dim());
   CUCA_REQUIRE(nkv > 0 && nh % nkv == 0, "attention: %d query heads do not group over %d key heads", nh, nkv);
   CUCA_REQUIRE(n_rows <= 65535, "attention: %d rows in one step exceed the launch limit 65535", n_rows);
+  if (dtype == CUCA_F32 && cuca_attention_f32_takes(kpool, vpool, nh, nkv, d, dv, opt))
+    return cuca_attention_f32((const float*)q, q_stride, (float*)out, out_stride, (const float*)kpool, (const float*)vpool,
+                              n_blocks, bs, positions, seq_of_row, tables, table_stride, n_rows, nh, nkv, d, dv, opt, err,
+                              stream);
   dim3 grid((nh + 3) / 4, n_rows);
   size_t smem = (size_t)4 * d * sizeof(float);
 #define AG(T, VC)                                                                                                  \

@@ -65,7 +65,7 @@ def test_gemm_simt_rows_are_the_same_bits_in_every_form(dev, N, K, epilogue):
     whole = prior.clone()
     ops.gemm_simt(a, w, whole, epilogue)
     ref = _ref_gemm(a.double(), w.double(), epilogue, None, prior.double())
-    assert torch.allclose(whole.double(), ref, atol=2e-5, rtol=1e-5)
+    assert torch.allclose(whole.double(), ref.double(), atol=2e-5, rtol=1e-5)
     for first, M in ((3, 1), (0, 2), (5, 3), (0, 4), (9, 7), (0, 8), (1, 16), (0, 17), (7, 64), (0, 65), (0, 129), (0, 300)):
         out = prior[first:first + M].clone()
         ops.gemm_simt(a[first:first + M], w, out, epilogue)
@@ -336,6 +336,70 @@ def test_attention_generic_paged(dev, dtype, nh, nkv, d, bs, window):
     ops.attention_generic(qbuf[i:i + 1], nh * d, one, kpool, vpool, positions[i:i + 1], seq[i:i + 1], bad, nh, nkv, d,
                           1.0 / math.sqrt(d), None, err)
     assert int(err.item()) == 2
+
+
+@pytest.mark.parametrize("nh,nkv,d,dv,bs", [(8, 2, 64, 64, 16), (6, 6, 36, 20, 8), (16, 2, 128, 128, 32), (12, 1, 68, 128, 16),
+                                            (20, 1, 64, 64, 16)])
+@pytest.mark.parametrize("what", ["plain", "window", "kept", "all"])
+def test_attention_f32_forms_agree(dev, nh, nkv, d, dv, bs, what):
+    """The 32-bit attention over portions of several requests beside single tokens and padding (tiles of 64 query vectors),
+    over few rows, and of a row alone: the same bits; and against 64 bits, with a window (whose start lies inside tiles and
+    chunks), kept first keys, cap, distance bias, a sink and an output gate. Keys up to several chunks of 128."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(nh * 100 + d + len(what))
+    rows = [(0, p) for p in range(300, 377)] + [(1, 5), (2, 127), (2, 128), (3, 640), (-1, 0)]
+    rows += [(4, p) for p in range(19)] + [(5, p) for p in range(250, 259)]
+    T, S, longest = len(rows), 6, 641
+    pages = -(-longest // bs)
+    tables = torch.randperm(S * pages, device=dev, generator=g).to(torch.int32).view(S, pages)
+    kpool = torch.randn(S * pages, nkv, bs, d, device=dev, generator=g)
+    vpool = torch.randn(S * pages, nkv, bs, dv, device=dev, generator=g)
+    q = torch.randn(T, nh * d + 4, device=dev, generator=g)
+    positions = torch.tensor([p for _, p in rows], dtype=torch.int32, device=dev)
+    seq = torch.tensor([s for s, _ in rows], dtype=torch.int32, device=dev)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    window = {"plain": None, "window": 75, "kept": 200, "all": 97}[what]
+    options = {}
+    if what in ("kept", "all"):
+        options["keep_first"] = 45
+    if what == "all":
+        options.update(softcap=4.0, slopes=torch.rand(nh, device=dev, generator=g) * 0.05, sink=True,
+                       sink_values=torch.randn(nh, device=dev, generator=g))
+    gate = torch.randn(T, nh * dv, device=dev, generator=g) if what == "all" else None
+    scale = d ** -0.5
+
+    def run(a, b):
+        out = torch.full((b - a, nh * dv), 7.0, device=dev)
+        ops.attention_generic_v(q[a:b], q.stride(0), out, kpool, vpool, positions[a:b], seq[a:b], tables, nh, nkv, d, dv,
+                                scale, window, err, gate=None if gate is None else gate[a:b], **options)
+        return out
+
+    whole = run(0, T)
+    assert int(err.item()) == 0
+    for i, (s, P) in enumerate(rows):
+        if s < 0:
+            assert torch.equal(whole[i], torch.full_like(whole[i], 7.0))
+            continue
+        at = torch.arange(P + 1, device=dev)
+        seen = torch.ones(P + 1, dtype=torch.bool, device=dev)
+        if window:
+            seen = (P - at < window) | (at < options.get("keep_first", 0))
+        page = tables[s][at // bs].long()
+        k, v = kpool[page, :, at % bs].double(), vpool[page, :, at % bs].double()
+        k, v = k.repeat_interleave(nh // nkv, 1), v.repeat_interleave(nh // nkv, 1)
+        sc = torch.einsum("hd,khd->hk", q[i, :nh * d].double().view(nh, d), k) * scale
+        if what == "all":
+            sc = 4.0 * torch.tanh(sc / 4.0) - options["slopes"].double()[:, None] * (P - at).double()
+        sc = sc.masked_fill(~seen, -math.inf)
+        if what == "all":
+            sc = torch.cat([sc, options["sink_values"].double()[:, None]], 1)
+        w = torch.softmax(sc, -1)[:, :P + 1]
+        want = torch.einsum("hk,khd->hd", w, v).reshape(-1)
+        if gate is not None:
+            want = want * torch.sigmoid(gate[i].double())
+        assert torch.allclose(whole[i].double(), want, atol=1e-5, rtol=1e-5), (i, s, P)
+    for a, b in ((0, 1), (76, 77), (77, 78), (79, 80), (80, 81), (82, 101), (60, 110), (40, 110), (10, 74)):
+        assert torch.equal(run(a, b), whole[a:b]), (a, b)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
