@@ -82,8 +82,6 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
   const int col0 = blockIdx.z * PB, at = col_local * NC;
   const int cols = min(NC, dv - col0 - at);               // columns of this thread that exist (none: 0 or less)
-  const int own = s / (NS / NC), col = col0 + at + own;   // the column whose sums this thread ends up with
-  const bool writes = s % (NS / NC) == 0 && own < cols;
   float* st = state + (((size_t)slot * H + h) * dv + (cols > 0 ? col0 + at : 0)) * d;
   f32x2 S[NC][PAIRS];
   load_rows<C>(S, st, s, d, cols, wide);
@@ -120,16 +118,14 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
     cp_async_commit();
   };
   const int n_chunks = (n + TC - 1) / TC;
-  float* o_at = out + (size_t)r0 * H * dv + (size_t)h * dv + col;  // the output of the token before
+  // A token's reductions over the channels (the corrections' of its own and the outputs' of the token before) go as one:
+  // thread s ends up with value s / (NS / 2 NC) of [corrections | outputs].
+  const int own = s / (NS / (2 * NC));
+  const bool writes = s % (NS / (2 * NC)) == 0 && own >= NC && own - NC < cols;
+  float* o_at = out + (size_t)r0 * H * dv + (size_t)h * dv + col0 + at + (own - NC);  // the output of the token before
   f32x2 q[PAIRS];
 #pragma unroll
   for (int i = 0; i < PAIRS; ++i) q[i] = 0;
-  auto output = [&]() {
-    float o[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) o[c] = dot_rows(S[c], q);
-    return column_sum<C>(o, s);
-  };
   stage(0, 0);
   for (int c = 0; c < n_chunks; ++c) {
     if (c + 1 < n_chunks) { stage((c + 1) * TC, (c + 1) & 1); cp_async_wait<1>(); }
@@ -147,23 +143,24 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
     for (int t = 0; t < nt; ++t) {
       const float* next = t + 1 < nt ? tok + PER : tok;  // (read ahead of its use)
       f32x2 Sg[NC][PAIRS], k1[PAIRS];
-      float part[NC], v1[NC], u[NC];
+      float v1[NC], sums[2 * NC];
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
 #pragma unroll
         for (int i = 0; i < PAIRS; ++i) Sg[j][i] = f2_mul(S[j][i], g[i]);
-        part[j] = dot_rows(Sg[j], k);
+        sums[j] = dot_rows(Sg[j], k);
       }
+#pragma unroll
+      for (int j = 0; j < NC; ++j) sums[NC + j] = dot_rows(S[j], q);
       staged_rows<C>(k1, next + DP, s);
       staged_rows<C>(g, next + 2 * DP, s);
       staged_values<NC>(v1, next + 3 * DP, at);
       const float b1 = next[3 * DP + PB];
-      const float sum = column_sum<C>(part, s);
-      const float o = output();
-      column_spread<C>(u, sum, s);
+      const float o = spread_sum<NS, 2 * NC>(sums, s);
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        const f32x2 uu = f2_both(b * (v[j] - u[j]));
+        const float sum = __shfl_sync(0xffffffffu, o, j * (NS / (2 * NC)), NS);
+        const f32x2 uu = f2_both(b * (v[j] - sum));
 #pragma unroll
         for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(k[i], uu, Sg[j][i]);
       }
@@ -181,7 +178,10 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
     }
     __syncthreads();  // the buffer is free for the copies of the chunk after next
   }
-  const float o = output();
+  float sums[2 * NC];
+#pragma unroll
+  for (int j = 0; j < NC; ++j) { sums[j] = 0.f; sums[NC + j] = dot_rows(S[j], q); }
+  const float o = spread_sum<NS, 2 * NC>(sums, s);
   if (writes) *o_at = o;
   store_rows<C>(S, st, s, d, cols, wide);
 }
@@ -347,8 +347,6 @@ forget_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int f_col,
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
   const int col0 = blockIdx.z * PB, at = col_local * NC;
   const int cols = min(NC, dv - col0 - at);               // columns of this thread that exist (none: 0 or less)
-  const int own = s / (NS / NC), col = col0 + at + own;   // the column whose sums this thread ends up with
-  const bool writes = s % (NS / NC) == 0 && own < cols;
   float* st = state + (((size_t)slot * H + h) * dv + (cols > 0 ? col0 + at : 0)) * d;
   f32x2 S[NC][PAIRS];
   load_rows<C>(S, st, s, d, cols, wide);
@@ -390,29 +388,38 @@ forget_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int f_col,
     __syncthreads();
     const int t0 = c * TC, nt = n - t0 < TC ? n - t0 : TC;
     const float* tok = sm + (c & 1) * TC * PER;
-    float* o_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col;
-    // (tokens depend on each other through the state's one multiply-add alone: four in flight keep the loads and the
-    // shuffled sums of the next ones going while these wait)
-#pragma unroll 4
-    for (int t = 0; t < nt; ++t, tok += PER, o_at += H * dv) {
-      f32x2 f[PAIRS], q[PAIRS], w[PAIRS];  // w: what is written, k or 1 - f
-      float v[NC], o[NC];
-      staged_rows<C>(f, tok + DP, s);
-      staged_rows<C>(q, tok, s);
-      staged_values<NC>(v, tok + 2 * DP, at);
+    float* o_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col0 + at;
+    // Tokens depend on each other through the state's one multiply-add alone, so several are worked through at once and
+    // their outputs summed together: thread s writes value s / (NS / (count NC)) of [tokens][columns].
+    auto walk = [&](int t, auto count) {
+      constexpr int U = decltype(count)::value;
+      float o[U * NC];
 #pragma unroll
-      for (int i = 0; i < PAIRS; ++i) w[i] = RET ? f[i] : f2_fma(f[i], minus, one);
+      for (int i = 0; i < U; ++i, tok += PER) {
+        f32x2 f[PAIRS], q[PAIRS], w[PAIRS];  // w: what is written, k or 1 - f
+        float v[NC];
+        staged_rows<C>(f, tok + DP, s);
+        staged_rows<C>(q, tok, s);
+        staged_values<NC>(v, tok + 2 * DP, at);
 #pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        const f32x2 vv = f2_both(v[j]);
-        // decay S + k v or f S + (1 - f) v, each product rounded
+        for (int e = 0; e < PAIRS; ++e) w[e] = RET ? f[e] : f2_fma(f[e], minus, one);
 #pragma unroll
-        for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(RET ? dec : f[i], S[j][i], f2_mul(w[i], vv));
-        o[j] = dot_rows(S[j], q);
+        for (int j = 0; j < NC; ++j) {
+          const f32x2 vv = f2_both(v[j]);
+          // decay S + k v or f S + (1 - f) v, each product rounded
+#pragma unroll
+          for (int e = 0; e < PAIRS; ++e) S[j][e] = f2_fma(RET ? dec : f[e], S[j][e], f2_mul(w[e], vv));
+          o[i * NC + j] = dot_rows(S[j], q);
+        }
       }
-      const float mine = column_sum<C>(o, s);
-      if (writes) *o_at = mine;
-    }
+      constexpr int LANES = NS / (U * NC);
+      const float sum = spread_sum<NS, U * NC>(o, s);
+      const int own = s / LANES;
+      if (s % LANES == 0 && own % NC < cols) o_at[(size_t)(t + own / NC) * H * dv + own % NC] = sum;
+    };
+    int t = 0;
+    for (; t + C::U <= nt; t += C::U) walk(t, Count<C::U>());
+    for (; t < nt; ++t) walk(t, Count<1>());
     __syncthreads();  // the buffer is free for the copies of the chunk after next
   }
   store_rows<C>(S, st, s, d, cols, wide);
@@ -462,8 +469,6 @@ mlstm_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int k_col, 
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
   const int col0 = blockIdx.z * PB, at = col_local * NC;
   const int cols = min(NC, dv - col0 - at);               // columns of this thread that exist (none: 0 or less)
-  const int own = s / (NS / NC), col = col0 + at + own;   // the column whose sums this thread ends up with
-  const bool writes = s % (NS / NC) == 0 && own < cols;
   float* st = mem + (((size_t)slot * H + h) * dv + (cols > 0 ? col0 + at : 0)) * d;
   using One = Split<C::NS, C::NR, 1>;
   f32x2 S[NC][PAIRS], Zs[1][PAIRS];
@@ -531,29 +536,41 @@ mlstm_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int k_col, 
       }
       __syncwarp();
     }
-    float* o_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col;
-#pragma unroll 2
-    for (int t = 0; t < nt; ++t, tok += PER, o_at += H * dv) {
-      f32x2 k[PAIRS], q[PAIRS];
-      float v[NC], o[NC];
-      staged_rows<C>(k, tok + DP, s);
-      staged_rows<C>(q, tok, s);
-      staged_values<NC>(v, tok + 2 * DP, at);
-      const float take = mine[t][1];
-      const f32x2 keep = f2_both(mine[t][0]), w1 = f2_both(take);
+    float* o_at = out + (size_t)(r0 + t0) * H * dv + (size_t)h * dv + col0 + at;
+    // (several tokens at once, as in the forget scan; a token's n . q ends up with the threads that write its outputs)
+    auto walk = [&](int t, auto count) {
+      constexpr int U = decltype(count)::value;
+      float o[U * NC], z[U];
 #pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        const f32x2 w = f2_both(take * v[j]);
+      for (int i = 0; i < U; ++i, tok += PER) {
+        f32x2 k[PAIRS], q[PAIRS];
+        float v[NC];
+        staged_rows<C>(k, tok + DP, s);
+        staged_rows<C>(q, tok, s);
+        staged_values<NC>(v, tok + 2 * DP, at);
+        const float take = mine[t + i][1];
+        const f32x2 keep = f2_both(mine[t + i][0]), w1 = f2_both(take);
 #pragma unroll
-        for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(keep, S[j][i], f2_mul(w, k[i]));
-        o[j] = dot_rows(S[j], q);
+        for (int j = 0; j < NC; ++j) {
+          const f32x2 w = f2_both(take * v[j]);
+#pragma unroll
+          for (int e = 0; e < PAIRS; ++e) S[j][e] = f2_fma(keep, S[j][e], f2_mul(w, k[e]));
+          o[i * NC + j] = dot_rows(S[j], q);
+        }
+#pragma unroll
+        for (int e = 0; e < PAIRS; ++e) Z[e] = f2_fma(keep, Z[e], f2_mul(w1, k[e]));
+        z[i] = dot_rows(Z, q);
       }
-#pragma unroll
-      for (int i = 0; i < PAIRS; ++i) Z[i] = f2_fma(keep, Z[i], f2_mul(w1, k[i]));
-      const float num = column_sum<C>(o, s) * qscale;
-      const float z = group_sum<NS>(dot_rows(Z, q)) * qscale;
-      if (writes) *o_at = num / (fmaxf(fabsf(z), mine[t][2]) + 1e-6f);
-    }
+      constexpr int LANES = NS / (U * NC);
+      const float num = spread_sum<NS, U * NC>(o, s) * qscale;
+      const float den = spread_sum<NS, U>(z, s) * qscale;
+      const int own = s / LANES;
+      if (s % LANES == 0 && own % NC < cols)
+        o_at[(size_t)(t + own / NC) * H * dv + own % NC] = num / (fmaxf(fabsf(den), mine[t + own / NC][2]) + 1e-6f);
+    };
+    int t = 0;
+    for (; t + C::U <= nt; t += C::U) walk(t, Count<C::U>());
+    for (; t < nt; ++t) walk(t, Count<1>());
     __syncthreads();  // the buffer is free again
   }
   // every block of a (head, request) starts from the same n and m, so no block of this launch may replace them: the
@@ -637,7 +654,6 @@ head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w, 
 // 128 channels, eight channels of two columns a thread give each of the SM's four schedulers one warp.
 template <typename F>
 int with_split(int d, F go) {
-  if (d <= 16) return go(Split<2, 8, 2>());
   if (d <= 32) return go(Split<4, 8, 2>());
   if (d <= 64) return go(Split<8, 8, 2>());
   if (d <= 128) return go(Split<16, 8, 2>());

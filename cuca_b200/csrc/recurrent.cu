@@ -99,10 +99,13 @@ __global__ void mingru_chunked_kernel(const float* __restrict__ zxg, float* __re
 }
 
 // in: 32-bit rows of stride ld_in, channel c at column col0 + c. kept: [slots, taps - 1, C] the inputs before the
-// request's first row of this step (zeros for a new request). Blocks y < n_rows take rows that have taps - 1 rows of
-// their own request before them in this step; blocks y >= n_rows take one request each: its first taps - 1 rows and
-// then its new kept inputs (only that block touches them).
-template <typename TW>
+// request's first row of this step (zeros for a new request). The first blocks y take CONV_ROWS rows each, those of them
+// that have taps - 1 rows of their own request before them in this step; the blocks y behind them take one request each:
+// its first taps - 1 rows and then its new kept inputs (only that block touches them).
+// TAPS: taps known at compile time (a thread then reads every input of its rows once, all of them in flight together:
+// 2,048 rows of 4,352 channels, 4 taps, 77 us with a row a thread), or 0.
+constexpr int CONV_ROWS = 16;
+template <typename TW, int TAPS>
 __global__ void causal_conv_kernel(const float* __restrict__ in, int ld_in, int col0, const TW* __restrict__ w,
                                    const TW* __restrict__ bias, float* __restrict__ kept, float* __restrict__ out,
                                    const int* __restrict__ seq_of_row, const int* __restrict__ req_row0,
@@ -112,21 +115,45 @@ __global__ void causal_conv_kernel(const float* __restrict__ in, int ld_in, int 
   pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
-  const int b = blockIdx.y;
-  const int back = taps - 1;
-  const TW* wc = w + (size_t)c * taps;
+  const int row_blocks = (n_rows + CONV_ROWS - 1) / CONV_ROWS;
+  const int back = (TAPS ? TAPS : taps) - 1;
+  const TW* wc = w + (size_t)c * (back + 1);
   const float b0 = bias ? to_f32(bias[c]) : 0.f;
-  if (b < n_rows) {
-    const int seq = seq_of_row[b];
-    if (seq < 0 || b < back || (back > 0 && seq_of_row[b - back] != seq)) return;
-    float acc = b0;
-    for (int k = 0; k < taps; ++k)
-      acc = fmaf(to_f32(wc[k]), in[(size_t)(b - back + k) * ld_in + col0 + c], acc);
-    out[(size_t)b * C + c] = siluf_(acc);
+  if ((int)blockIdx.y < row_blocks) {
+    const int r0 = blockIdx.y * CONV_ROWS, r1 = min(n_rows, r0 + CONV_ROWS);
+    auto whole = [&](int b) {  // whether row b has `back` rows of its request before it
+      const int seq = b < r1 ? seq_of_row[b] : -1;
+      return seq >= 0 && b >= back && (back == 0 || seq_of_row[b - back] == seq);
+    };
+    if (TAPS) {
+      float taps_w[TAPS ? TAPS : 1], x[CONV_ROWS + (TAPS ? TAPS : 1) - 1];
+#pragma unroll
+      for (int k = 0; k < TAPS; ++k) taps_w[k] = to_f32(wc[k]);
+#pragma unroll
+      for (int i = 0; i < CONV_ROWS + TAPS - 1; ++i) {
+        const int b = r0 - (TAPS - 1) + i;
+        x[i] = b >= 0 && b < r1 ? in[(size_t)b * ld_in + col0 + c] : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < CONV_ROWS; ++i) {
+        if (!whole(r0 + i)) continue;
+        float acc = b0;
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k) acc = fmaf(taps_w[k], x[i + k], acc);
+        out[(size_t)(r0 + i) * C + c] = siluf_(acc);
+      }
+    } else {
+      for (int b = r0; b < r1; ++b) {
+        if (!whole(b)) continue;
+        float acc = b0;
+        for (int k = 0; k <= back; ++k) acc = fmaf(to_f32(wc[k]), in[(size_t)(b - back + k) * ld_in + col0 + c], acc);
+        out[(size_t)b * C + c] = siluf_(acc);
+      }
+    }
     return;
   }
   if (back == 0) return;  // a one-tap convolution keeps nothing and every row was a plain row
-  const int q = b - n_rows;
+  const int q = blockIdx.y - row_blocks;
   const int slot = slots[q], n = req_count[q], r0 = req_row0[q];
   if (slot < 0 || n <= 0) return;
   float* keep = kept + (size_t)slot * back * C;
@@ -176,8 +203,6 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
   const int col0 = blockIdx.z * PB, at = col_local * NC;
   const int cols = min(NC, P - col0 - at);              // columns of this thread that exist (none: 0 or less)
-  const int own = s / (NS / NC), p = col0 + at + own;   // the column whose sums this thread ends up with
-  const bool writes = s % (NS / NC) == 0 && own < cols;
   const int g = h / (H / G);
   const int C = H * P + 2 * G * N;
   float* st = state + (((size_t)slot * H + h) * P + (cols > 0 ? col0 + at : 0)) * N;
@@ -232,26 +257,39 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
       mine[lane][1] = expf(A * dt);
     }
     __syncwarp();
-    float* y_at = y + (size_t)(r0 + t0) * (H * P) + h * P + p;
-#pragma unroll 2
-    for (int t = 0; t < nt; ++t, tok += PER, y_at += H * P) {
-      f32x2 B[PAIRS], Cv[PAIRS];
-      staged_rows<S_>(B, tok, s);
-      staged_rows<S_>(Cv, tok + DP, s);
-      float x[NC], acc[NC];
-      staged_values<NC>(x, tok + 2 * DP, at);
-      const float dt = mine[t][0], x_own = tok[2 * DP + at + own];
-      const f32x2 decay = f2_both(mine[t][1]);
+    float* y_at = y + (size_t)(r0 + t0) * (H * P) + h * P + col0 + at;
+    // several tokens at once, their outputs summed together: thread s writes value s / (NS / (count NC)) of
+    // [tokens][columns]
+    auto walk = [&](int t, auto count) {
+      constexpr int U = decltype(count)::value;
+      const float* first = tok;
+      float acc[U * NC];
 #pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        const f32x2 dx = f2_both(dt * x[j]);
+      for (int i = 0; i < U; ++i, tok += PER) {
+        f32x2 B[PAIRS], Cv[PAIRS];
+        float x[NC];
+        staged_rows<S_>(B, tok, s);
+        staged_rows<S_>(Cv, tok + DP, s);
+        staged_values<NC>(x, tok + 2 * DP, at);
+        const float dt = mine[t + i][0];
+        const f32x2 decay = f2_both(mine[t + i][1]);
 #pragma unroll
-        for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(decay, S[j][i], f2_mul(dx, B[i]));
-        acc[j] = dot_rows(S[j], Cv);
+        for (int j = 0; j < NC; ++j) {
+          const f32x2 dx = f2_both(dt * x[j]);
+#pragma unroll
+          for (int e = 0; e < PAIRS; ++e) S[j][e] = f2_fma(decay, S[j][e], f2_mul(dx, B[e]));
+          acc[i * NC + j] = dot_rows(S[j], Cv);
+        }
       }
-      const float sum = column_sum<S_>(acc, s);
-      if (writes) *y_at = sum + D * x_own;
-    }
+      constexpr int LANES = NS / (U * NC);
+      const float sum = spread_sum<NS, U * NC>(acc, s);
+      const int own = s / LANES;
+      if (s % LANES == 0 && own % NC < cols)
+        y_at[(size_t)(t + own / NC) * (H * P) + own % NC] = sum + D * first[(own / NC) * PER + 2 * DP + at + own % NC];
+    };
+    int t = 0;
+    for (; t + S_::U <= nt; t += S_::U) walk(t, Count<S_::U>());
+    for (; t < nt; ++t) walk(t, Count<1>());
     __syncthreads();  // this run is read to the end before the run after next is copied over it
   }
   store_rows<S_>(S, st, s, N, cols, wide);
@@ -361,21 +399,22 @@ CUCA_API int cuca_causal_conv(const float* in, int ld_in, int col0, const void* 
   if (n_rows == 0) return 0;
   CUCA_REQUIRE(C > 0 && taps >= 1, "causal_conv: bad sizes channels=%d taps=%d", C, taps);
   CUCA_REQUIRE(n_rows + n_seqs <= 65535, "causal_conv: %d rows in one step exceed the launch limit", n_rows);
-  dim3 grid((C + 127) / 128, n_rows + n_seqs);
-  if (w_dtype == CUCA_F32)
-    cuca_launch(causal_conv_kernel<float>, grid, dim3(128), 0, stream, true, in, ld_in, col0, (const float*)w,
-                (const float*)bias, kept, out, seq_of_row, req_row0, req_count, slots, n_rows, C, taps);
-  else if (w_dtype == CUCA_BF16)
-    cuca_launch(causal_conv_kernel<__nv_bfloat16>, grid, dim3(128), 0, stream, true, in, ld_in, col0,
-                (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, kept, out, seq_of_row, req_row0, req_count, slots,
-                n_rows, C, taps);
-  else
+  const dim3 grid((C + 127) / 128, (n_rows + CONV_ROWS - 1) / CONV_ROWS + n_seqs);
+#define CONV(TW, TAPS)                                                                                                \
+  cuca_launch(causal_conv_kernel<TW, TAPS>, grid, dim3(128), 0, stream, true, in, ld_in, col0, (const TW*)w,          \
+              (const TW*)bias, kept, out, seq_of_row, req_row0, req_count, slots, n_rows, C, taps)
+  if (w_dtype == CUCA_F32) {
+    if (taps == 4) CONV(float, 4); else CONV(float, 0);
+  } else if (w_dtype == CUCA_BF16) {
+    if (taps == 4) CONV(__nv_bfloat16, 4); else CONV(__nv_bfloat16, 0);
+  } else {
     CUCA_REQUIRE(false, "causal_conv: unknown dtype %d", w_dtype);
+  }
+#undef CONV
   CUCA_CHECK_LAUNCH("causal_conv");
   return 0;
 }
 
-// How the state rows of a head are dealt to threads: (threads per value column, state rows per thread).
 CUCA_API int cuca_ssm_scan(const float* xbc, const float* dt_raw, int ld_dt, int dt_col, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, float* y, const int* req_row0,
                            const int* req_count, const int* slots, int n_seqs, int H, int P, int N, int G,

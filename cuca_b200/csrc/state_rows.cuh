@@ -26,7 +26,9 @@ template <int NS_, int NR_, int NC_>
 struct Split {
   static constexpr int NS = NS_, NR = NR_, NC = NC_, DP = NS * NR, PB = NC * 128 / NS, PAIRS = NR / 2;
   static constexpr int TC = DP <= 128 ? 16 : 2048 / DP;  // tokens staged at a time
-  static_assert(NS >= NC && NC <= 4, "a column's sum ends up with a thread of its own");
+  // tokens whose outputs are summed together
+  static constexpr int U = NS / NC >= 4 ? 4 : NS / NC;
+  static_assert(NC <= 4 && U >= 1, "a column's sum ends up with a thread of its own");
 };
 
 // The state rows of a thread, as pairs, from `st` (the first of its columns, d channels each) and back. vec: 16 bytes at
@@ -104,20 +106,15 @@ __device__ __forceinline__ float dot_rows(const f32x2 (&a)[PAIRS], const f32x2 (
   }
   return f2_sum4(p, q);
 }
-// sum over the NS neighbouring threads of a run of columns
-template <int NS>
-__device__ __forceinline__ float group_sum(float v) {
+// The sums of N values (N a power of two, at most NS) over the NS threads of a run of columns: thread s gets the sum of
+// value s / (NS / N). The first steps halve the number of values a thread is busy with, so N sums take hardly more
+// shuffles, and no longer a chain of them, than one.
+template <int NS, int N>
+__device__ __forceinline__ float spread_sum(float (&v)[N], int s) {
+  static_assert(N <= NS, "a thread a value");
+  int stride = NS / 2;
 #pragma unroll
-  for (int o = NS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-// The sums of NC columns over the NS threads of their run: thread s gets column s / (NS / NC)'s. The first steps halve
-// the number of columns a thread is busy with.
-template <typename C>
-__device__ __forceinline__ float column_sum(float (&v)[C::NC], int s) {
-  int stride = C::NS / 2;
-#pragma unroll
-  for (int half = C::NC / 2; half > 0; half >>= 1, stride >>= 1) {
+  for (int half = N / 2; half > 0; half >>= 1, stride >>= 1) {
     const bool upper = s & stride;
 #pragma unroll
     for (int i = 0; i < half; ++i) {
@@ -126,34 +123,24 @@ __device__ __forceinline__ float column_sum(float (&v)[C::NC], int s) {
     }
   }
 #pragma unroll
-  for (int o = C::NS / C::NC / 2; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  for (int o = NS / N / 2; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
   return v[0];
 }
-// The other way: every thread's column's number to all threads of the run.
-template <typename C>
-__device__ __forceinline__ void column_spread(float (&v)[C::NC], float mine, int s) {
-  static_assert(C::NC <= 2, "one exchange");
-  if (C::NC == 1) {
-    v[0] = mine;
-  } else {
-    const float other = __shfl_xor_sync(0xffffffffu, mine, C::NS / 2);
-    const bool upper = s & (C::NS / 2);
-    v[0] = upper ? other : mine;
-    v[C::NC - 1] = upper ? mine : other;
-  }
-}
+
+template <int N_> struct Count { static constexpr int value = N_; };
 
 // Launches a scan with `floats_per_token` floats of shared memory a token, twice over. A prompt's few blocks are to lie on
 // an SM each: launched while the kernel before drains they would pile up on the SMs that come free first (measured on
-// 128 blocks: twice the time), so such a launch asks for as much shared memory as one (or two) blocks of an SM can have.
+// 128 blocks: twice the time), so such a launch asks for so much shared memory that no SM takes more than its share.
 template <typename C, typename... KArgs, typename... Args>
 int launch_scan(const char* name, void (*kernel)(KArgs...), int floats_per_token, int H, int n_seqs, int dv, cudaStream_t stream,
                 Args... args) {
   int smem = 2 * C::TC * floats_per_token * 4;
   const dim3 grid(H, n_seqs, (dv + C::PB - 1) / C::PB);
   const long long blocks = (long long)grid.x * grid.y * grid.z, sms = cuca_device_sms();
-  const int alone = blocks <= sms ? 116 * 1024 : blocks <= 2 * sms ? 78 * 1024 : 0;
-  if (smem < alone) smem = alone;
+  const long long per_sm = (blocks + sms - 1) / sms;
+  const int spread = per_sm <= 4 ? 228 * 1024 / ((int)per_sm + 1) + 1024 : 0;
+  if (smem < spread) smem = spread;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     CUCA_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused: %s", name, smem, cudaGetErrorString(e));
