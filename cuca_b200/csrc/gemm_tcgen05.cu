@@ -1210,7 +1210,12 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
     const double cost128 = (double)((t128 + sms - 1) / sms);
     const double cost_tall = (double)((t256 + sms - 1) / sms) * 1.95;
     const double cost_pair = (double)((t256 + pairs - 1) / pairs) * (K > 8192 ? 1.02 : 0.96);
-    pair = allow_pair == 2 || (allow_pair == 1 && t256 >= pairs && cost_pair < cost128 && cost_pair < (tall ? cost_tall : 1e30));
+    // SwiGLU over so few tokens that one round of tall tiles does: a second, partly filled round of pairs costs more
+    // (gate/up of the Llama-3.1-8B widths at 130 to 256 tokens 60.1-62.0 us tall, 63.6-64.7 in pairs; of the 1B widths at
+    // 257 to 512 tokens 44.2-44.9, 47.8-48.9)
+    const bool one_tall_round = dual && tall && t256 <= sms;
+    pair = allow_pair == 2 || (allow_pair == 1 && t256 >= pairs && cost_pair < cost128 && !one_tall_round &&
+                               cost_pair < (tall ? cost_tall : 1e30));
   }
   if (pair) {
     p.tile_rows = 2 * TILE_A;
