@@ -129,14 +129,11 @@ __device__ __forceinline__ float spread_sum(float (&v)[N], int s) {
 
 template <int N_> struct Count { static constexpr int value = N_; };
 
-// Launches a scan with `floats_per_token` floats of shared memory a token, twice over. A prompt's few blocks are to lie on
-// an SM each: launched while the kernel before drains they would pile up on the SMs that come free first (measured on
-// 128 blocks: twice the time), so such a launch asks for so much shared memory that no SM takes more than its share.
-template <typename C, typename... KArgs, typename... Args>
-int launch_scan(const char* name, void (*kernel)(KArgs...), int floats_per_token, int H, int n_seqs, int dv, cudaStream_t stream,
-                Args... args) {
-  int smem = 2 * C::TC * floats_per_token * 4;
-  const dim3 grid(H, n_seqs, (dv + C::PB - 1) / C::PB);
+// Launches a scan of `smem` bytes of shared memory a block. A prompt's few blocks are to lie spread over the SMs: launched
+// while the kernel before drains they would pile up on the SMs that come free first (measured on 128 blocks: twice the
+// time), so such a launch asks for so much shared memory that no SM takes more than its share.
+template <typename... KArgs, typename... Args>
+int launch_blocks(const char* name, void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t stream, Args... args) {
   const long long blocks = (long long)grid.x * grid.y * grid.z, sms = cuca_device_sms();
   const long long per_sm = (blocks + sms - 1) / sms;
   const int spread = per_sm <= 4 ? 228 * 1024 / ((int)per_sm + 1) + 1024 : 0;
@@ -145,9 +142,17 @@ int launch_scan(const char* name, void (*kernel)(KArgs...), int floats_per_token
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     CUCA_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused: %s", name, smem, cudaGetErrorString(e));
   }
-  cuca_launch(kernel, grid, dim3(128), smem, stream, true, args...);
+  cuca_launch(kernel, grid, dim3(threads), smem, stream, true, args...);
   CUCA_CHECK_LAUNCH(name);
   return 0;
+}
+
+// The same for a scan with `floats_per_token` floats of shared memory a token, twice over.
+template <typename C, typename... KArgs, typename... Args>
+int launch_scan(const char* name, void (*kernel)(KArgs...), int floats_per_token, int H, int n_seqs, int dv, cudaStream_t stream,
+                Args... args) {
+  return launch_blocks(name, kernel, dim3(H, n_seqs, (dv + C::PB - 1) / C::PB), 128, 2 * C::TC * floats_per_token * 4, stream,
+                       args...);
 }
 
 }  // namespace

@@ -207,7 +207,8 @@ class GatedDelta(Mixer):
         qkv = rt.empty(rows, C, dtype=torch.float32)
         ops.causal_conv(proj, 0, self.conv_w, None, cache.state["conv"], qkv, step)
         o = rt.empty(rows, H * dv, dtype=torch.float32)
-        ops.delta_scan(qkv, a_raw, self.dt_bias, self.a_log, proj, C, cache.state["delta"], o, step, H, G, d, dv)
+        ops.delta_scan(qkv, a_raw, self.dt_bias, self.a_log, proj, C, cache.state["delta"], o, step, H, G, d, dv,
+                       chunks=h.dtype == torch.bfloat16)
         out = rt.empty(rows, H * dv)
         ops.head_norm_gate(o, self.norm_w, False, gate, out, H, dv, self.eps)
         rt.stream(stream).add_linear(out, self.w_o)

@@ -1,6 +1,8 @@
 """Dupenex on the GPU against the plain implementation (`plain_dupenex.py`): every mechanism alone, whole and cut,
 then whole models through the replayer in the four work splits, pages and slots used again, long decoding past
 every window, and greedy generation through the entry point and its scheduler."""
+import types
+
 import numpy as np
 import pytest
 import torch
@@ -119,6 +121,48 @@ def test_delta_rule_alone_whole_and_cut(rt32, layer):
         got = _run_cut(dev, fwd, xs, cuts, [1, 3, 0], E)
         for a, b in zip(got, want):
             assert np.abs(a - b).max() < 3e-5 * max(1.0, np.abs(b).max())
+
+
+@pytest.mark.parametrize("H, G, d, dv", [(3, 3, 128, 128), (4, 2, 40, 8), (9, 3, 64, 150), (1, 1, 4, 17), (2, 1, 124, 33)])
+@pytest.mark.parametrize("counts", [[32], [1, 3, 45, 4, 2], [100, 0, 33], [37, 64]])
+def test_delta_rule_in_chunks_of_four(rt32, H, G, d, dv, counts):
+    """Four tokens at a time against the recurrence token by token in 64 bits, from states that are not empty: portions
+    that end anywhere in a chunk and start anywhere in the step, decays from nearly none to nearly all."""
+    from cuca_b200.kernels import ops
+    dev = rt32.device
+    rs = np.random.default_rng(sum(counts) + d)
+    rows, C = sum(counts), 2 * G * d + H * dv
+    C4 = -(-C // 4) * 4
+    qkv, a = rs.normal(0, 1, (rows, C4)), rs.normal(-1, 3, (rows, H * d))
+    b, dt, al = rs.normal(0, 1, (rows, H)), rs.normal(0, 1, H * d), rs.normal(0, 0.5, H)
+    state = rs.normal(0, 1, (len(counts) + 1, H, dv, d))
+    qkv, a, b, dt, al, state = (x.astype(np.float32).astype(np.float64) for x in (qkv, a, b, dt, al, state))
+    t32 = lambda x: torch.tensor(x, dtype=torch.float32, device=dev)  # noqa: E731
+    slots = list(range(len(counts)))[::-1]
+    step = types.SimpleNamespace(
+        host={"counts": counts}, static_max_len=None, n_seqs=len(counts), slots=torch.tensor(slots, dtype=torch.int32, device=dev),
+        seq_of_row=torch.tensor([i for i, n in enumerate(counts) for _ in range(n)], dtype=torch.int32, device=dev),
+        req_row0=torch.tensor(np.cumsum([0] + counts[:-1]), dtype=torch.int32, device=dev),
+        req_count=torch.tensor(counts, dtype=torch.int32, device=dev))
+    got = t32(state)
+    out = torch.full((rows, H * dv), 7.0, device=dev)
+    ops.delta_scan(t32(qkv)[:, :C4], t32(a), t32(dt), t32(al), t32(b), 0, got, out, step, H, G, d, dv, chunks=True)
+    want, S = np.zeros((rows, H, dv)), state.copy()
+    g = np.exp(-np.exp(al)[:, None] * np.logaddexp(0, a + dt).reshape(rows, H, d))
+    beta, r = 1 / (1 + np.exp(-b)), 0
+    for i, n in enumerate(counts):
+        for _ in range(n):
+            for h in range(H):
+                kv = h // (H // G)
+                q, k = qkv[r, kv * d:(kv + 1) * d], qkv[r, (G + kv) * d:(G + kv + 1) * d]
+                v = qkv[r, 2 * G * d + h * dv:2 * G * d + (h + 1) * dv]
+                q, k = q / np.sqrt(q @ q + 1e-6) * d ** -0.5, k / np.sqrt(k @ k + 1e-6)
+                M = S[slots[i], h] * g[r, h]
+                M = M + np.outer(beta[r, h] * (v - M @ k), k)
+                S[slots[i], h], want[r, h] = M, M @ q
+            r += 1
+    assert np.abs(out.cpu().numpy().reshape(want.shape) - want).max() < 3e-5 * max(1.0, np.abs(want).max())
+    assert np.abs(got.cpu().numpy() - S).max() < 3e-5 * max(1.0, np.abs(S).max())
 
 
 @pytest.mark.parametrize("right", [dict(r_heads=3, r_dim=12, r_vdim=20, cap=6.0), dict(r_heads=1, r_dim=96, r_vdim=40, cap=15.0),
