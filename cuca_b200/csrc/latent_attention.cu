@@ -150,6 +150,109 @@ __device__ __forceinline__ void hl_mma(float (&d)[4], const uint32_t (&a)[4], ui
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// The same in tiles of 128 rows x 128 outputs, eight warps of 32 x 64, for operands that can be read 16 bytes at a time
+// (a's row and head strides multiples of 4, K of 8): the next K step's 16-byte loads are in flight while this one is
+// multiplied. What bounds it is the traffic: 2,048 rows of 16 heads, 128 -> 512, read 17 MB and write 75. The narrow form
+// took 88 us for that (element-wise loads, none in flight during the arithmetic) and 69 us for 512 -> 128, this one 42
+// and 44.
+template <typename TO>
+__global__ void __launch_bounds__(256)
+head_linear_wide_kernel(const float* __restrict__ a, int lda, int a_head, const __nv_bfloat16* __restrict__ w,
+                        TO* __restrict__ out, int ldo, int o_head, const float* __restrict__ gate, int ldg, int T, int N,
+                        int K) {
+  constexpr int KS = 32, RSM = KS + 8;  // rows of 80 bytes: the eight rows of an ldmatrix fall into different banks
+  __shared__ __align__(16) __nv_bfloat16 As[2][128 * RSM];
+  __shared__ __align__(16) __nv_bfloat16 Ws[2][128 * RSM];
+  pdl_trigger();
+  pdl_wait();
+  const int h = blockIdx.z, t0 = blockIdx.y * 128, n0 = blockIdx.x * 128, tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31, wr = (warp >> 1) * 32, wn = (warp & 1) * 64;
+  const int g = lane >> 2, t = lane & 3;
+  const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_col = (lane >> 4) * 8;
+  const int b_row = (lane & 7) + (lane >> 4) * 8, b_col = ((lane >> 3) & 1) * 8;
+  float acc[2][8][4];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[r][i][j] = 0.f;
+  const __nv_bfloat16* wh = w + (size_t)h * N * K;
+  const float* ah = a + (size_t)h * a_head;
+  float4 av[4];
+  uint4 wv[2];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // 128 rows x 8 runs of four values
+      const int e = tid + i * 256, r = e >> 3, kk = k0 + (e & 7) * 4;
+      av[i] = t0 + r < T && kk < K ? *reinterpret_cast<const float4*>(ah + (size_t)(t0 + r) * lda + kk)
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {  // 128 rows x 4 runs of eight values
+      const int e = tid + i * 256, r = e >> 2, kk = k0 + (e & 3) * 8;
+      wv[i] = n0 + r < N && kk < K ? *reinterpret_cast<const uint4*>(wh + (size_t)(n0 + r) * K + kk)
+                                   : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  auto put = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = tid + i * 256;
+      __nv_bfloat162 lo = __floats2bfloat162_rn(av[i].x, av[i].y), hi = __floats2bfloat162_rn(av[i].z, av[i].w);
+      *reinterpret_cast<uint2*>(As[buf] + (e >> 3) * RSM + (e & 7) * 4) =
+          make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = tid + i * 256;
+      *reinterpret_cast<uint4*>(Ws[buf] + (e >> 2) * RSM + (e & 3) * 8) = wv[i];
+    }
+  };
+  fetch(0);
+  put(0);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = 0; k0 < K; k0 += KS, buf ^= 1) {
+    const bool more = k0 + KS < K;
+    if (more) fetch(k0 + KS);
+#pragma unroll
+    for (int kk = 0; kk < KS; kk += 16) {
+      uint32_t af[2][4], bf[4][4];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) hl_ldsm_x4(af[r], As[buf] + (wr + r * 16 + a_row) * RSM + kk + a_col);
+#pragma unroll
+      for (int np = 0; np < 4; ++np) hl_ldsm_x4(bf[np], Ws[buf] + (wn + np * 16 + b_row) * RSM + kk + b_col);
+#pragma unroll
+      for (int np = 0; np < 4; ++np)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          hl_mma(acc[r][2 * np], af[r], bf[np][0], bf[np][1]);
+          hl_mma(acc[r][2 * np + 1], af[r], bf[np][2], bf[np][3]);
+        }
+    }
+    if (more) put(buf ^ 1);  // (that buffer was read to the end before the last barrier)
+    __syncthreads();
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = t0 + wr + r * 16 + g + 8 * i;
+      if (row >= T) continue;
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int n = n0 + wn + nt * 8 + 2 * t + j;
+          if (n >= N) continue;
+          float v = acc[r][nt][2 * i + j];
+          if (gate) v *= 1.f / (1.f + expf(-gate[(size_t)row * ldg + (size_t)h * N + n]));
+          out[(size_t)row * ldo + (size_t)h * o_head + n] = from_f32<TO>(v);
+        }
+    }
+}
+
 template <typename TO>
 __global__ void __launch_bounds__(128)
 head_linear_mma_kernel(const float* __restrict__ a, int lda, int a_head, const __nv_bfloat16* __restrict__ w,
@@ -401,6 +504,19 @@ CUCA_API int cuca_head_linear(const float* a, int lda, int a_head, const void* w
   }
   dim3 grid((N + 63) / 64, (T + 63) / 64, H);
   CUCA_REQUIRE(grid.y <= 65535, "head_linear: %d rows exceed the launch limit", T);
+  if (w_dtype == CUCA_BF16 && lda % 4 == 0 && a_head % 4 == 0 && K % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0) {
+    const dim3 wide((N + 127) / 128, (T + 127) / 128, H);
+    if (out_dtype == CUCA_F32)
+      cuca_launch(head_linear_wide_kernel<float>, wide, dim3(256), 0, stream, true, a, lda, a_head,
+                  (const __nv_bfloat16*)w, (float*)out, ldo, o_head, gate, ldg, T, N, K);
+    else if (out_dtype == CUCA_BF16)
+      cuca_launch(head_linear_wide_kernel<__nv_bfloat16>, wide, dim3(256), 0, stream, true, a, lda, a_head,
+                  (const __nv_bfloat16*)w, (__nv_bfloat16*)out, ldo, o_head, gate, ldg, T, N, K);
+    else
+      CUCA_REQUIRE(false, "head_linear: unsupported dtypes %d/%d", w_dtype, out_dtype);
+    CUCA_CHECK_LAUNCH("head_linear");
+    return 0;
+  }
   if (w_dtype == CUCA_BF16) {
     if (out_dtype == CUCA_F32)
       cuca_launch(head_linear_mma_kernel<float>, grid, dim3(128), 0, stream, true, a, lda, a_head,

@@ -51,6 +51,44 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// S = Q K^T of 16 rows and 16 keys over Dk values (a multiple of 16). A step's two MMAs wait for the step before and for
+// their own fragments: four steps' fragments are requested together and two sums taken in turn (2,048 tokens, 16 heads, a
+// latent of 512 + 64, window 1,024: 549 -> 520 us).
+__device__ __forceinline__ void scores_of_16_keys(float (&s)[2][4], uint32_t q_addr, uint32_t k_addr, int Dk) {
+  float part[2][2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[h][i][j] = 0.f;
+  int k0 = 0;
+  for (; k0 + 64 <= Dk; k0 += 64) {
+    uint32_t a[4][4], b[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      ldsm_x4(a[u], q_addr + (uint32_t)(k0 + 16 * u) * 2);
+      ldsm_x4(b[u], k_addr + (uint32_t)(k0 + 16 * u) * 2);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      mma_bf16(part[u & 1][0], a[u], b[u][0], b[u][1]);
+      mma_bf16(part[u & 1][1], a[u], b[u][2], b[u][3]);
+    }
+  }
+  for (; k0 < Dk; k0 += 16) {
+    uint32_t a[4], b[4];
+    ldsm_x4(a, q_addr + (uint32_t)k0 * 2);
+    ldsm_x4(b, k_addr + (uint32_t)k0 * 2);
+    mma_bf16(part[0][0], a, b[0], b[1]);
+    mma_bf16(part[0][1], a, b[2], b[3]);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[i][j] = part[0][i][j] + part[1][i][j];
+}
+
 struct Params {
   const float* qk;   // [rows, H, Dk] 32-bit: per head [query carried into the latent space | rotated part]
   float* out;        // [rows, H, rank]
@@ -179,17 +217,7 @@ latent_attention_mma_kernel(Params p) {
 
     // S for this warp's 16 keys
     float s[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-    for (int k0 = 0; k0 < Dk; k0 += 16) {
-      uint32_t a[4], b[4];
-      ldsm_x4(a, qs_addr + (uint32_t)(a_row * RS + k0 + a_col) * 2);
-      ldsm_x4(b, ks_addr + (uint32_t)((warp * 16 + b_key) * RS + k0 + b_col) * 2);
-      mma_bf16(s[0], a, b[0], b[1]);
-      mma_bf16(s[1], a, b[2], b[3]);
-    }
+    scores_of_16_keys(s, qs_addr + (uint32_t)(a_row * RS + a_col) * 2, ks_addr + (uint32_t)((warp * 16 + b_key) * RS + b_col) * 2, Dk);
     // scale and mask; s[nt][0..1]: row g, keys kbase + nt * 8 + 2 t + {0, 1}; s[nt][2..3]: row g + 8
     const int kbase = kt + warp * 16 + 2 * t;
     float mx[2] = {-INFINITY, -INFINITY};
@@ -417,17 +445,7 @@ latent_attention_pair_kernel(Params p) {
     const uint32_t kb = ks_addr + (uint32_t)(buf * KT * RS) * 2;
 
     float s[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-    for (int k0 = 0; k0 < Dk; k0 += 16) {
-      uint32_t a[4], b[4];
-      ldsm_x4(a, qs_addr + (uint32_t)(a_row * RS + k0 + a_col) * 2);
-      ldsm_x4(b, kb + (uint32_t)((warp * 16 + b_key) * RS + k0 + b_col) * 2);
-      mma_bf16(s[0], a, b[0], b[1]);
-      mma_bf16(s[1], a, b[2], b[3]);
-    }
+    scores_of_16_keys(s, qs_addr + (uint32_t)(a_row * RS + a_col) * 2, kb + (uint32_t)((warp * 16 + b_key) * RS + b_col) * 2, Dk);
     const int kbase = kt + warp * 16 + 2 * t;
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
