@@ -26,8 +26,8 @@ template <int NS_, int NR_, int NC_>
 struct Split {
   static constexpr int NS = NS_, NR = NR_, NC = NC_, DP = NS * NR, PB = NC * 128 / NS, PAIRS = NR / 2;
   static constexpr int TC = DP <= 128 ? 16 : 2048 / DP;  // tokens staged at a time
-  // tokens whose outputs are summed together
-  static constexpr int U = NS / NC >= 4 ? 4 : NS / NC;
+  // tokens whose outputs are summed together: up to four, or up to eight
+  static constexpr int U = NS / NC >= 4 ? 4 : NS / NC, U8 = NS / NC >= 8 ? 8 : U;
   static_assert(NC <= 4 && U >= 1, "a column's sum ends up with a thread of its own");
 };
 
