@@ -227,18 +227,41 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
                                const int* __restrict__ rows, int E, float eps, int groups) {
   __shared__ float red[32];
   pdl_trigger();
-  pdl_wait();
   // `groups` equal consecutive parts of a row are normed apart: a block takes one part of E values (the row is
   // groups * E wide), so a part's arithmetic is that of a whole row of its width
   int orow = blockIdx.x, part = 0;
   if (groups > 1) { part = orow % groups; orow /= groups; }
+  w += (size_t)part * E;
+  // The weights are no earlier kernel's output: the first two rounds' are requested before the wait for the predecessor.
+  // (A decode step's norm is a chain of latencies; the weights, which the step's larger ones have driven out of L2, were
+  // the last of them.)
+  const bool w_vec = (E & 3) == 0 && (((size_t)w) & (4 * sizeof(TW) - 1)) == 0;
+  auto weights = [&](int i) {
+    float4 v;
+    if (sizeof(TW) == 4 && w_vec) {
+      v = reinterpret_cast<const float4*>(w)[i];
+    } else {
+      const int e = i << 2;
+      v = make_float4(to_f32(w[e]), to_f32(w[e + 1]), to_f32(w[e + 2]), to_f32(w[e + 3]));
+    }
+    return v;
+  };
+  float4 w0[VL], w1[VL];
+  if ((E & 3) == 0) {
+#pragma unroll
+    for (int k = 0; k < VL; ++k) {
+      const int i0 = threadIdx.x + blockDim.x * k, i1 = i0 + blockDim.x * VL;
+      if (i0 < E >> 2) w0[k] = weights(i0);
+      if (i1 < E >> 2) w1[k] = weights(i1);
+    }
+  }
+  pdl_wait();
   int irow = rows ? rows[orow] : orow;
   if (irow < 0) return;
   const size_t ld = (size_t)E * groups;
   float* xr = x + (size_t)irow * ld + (size_t)part * E;
   const float* pr = PARTIAL ? partial + (size_t)irow * ld + (size_t)part * E : nullptr;
   TO* o = out + (size_t)orow * ld + (size_t)part * E;
-  w += (size_t)part * E;
   float s = 0.f;
   const bool vec = (E & 3) == 0 && (((size_t)xr) & 15) == 0 && (!PARTIAL || ((((size_t)pr) | (slice_stride * 4)) & 15) == 0);
   if (vec) {
@@ -262,10 +285,8 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
       s = fmaf(v.x, v.x, s); s = fmaf(v.y, v.y, s); s = fmaf(v.z, v.z, s); s = fmaf(v.w, v.w, s);
       return v;
     };
-    auto put = [&](int i, float4 v, float r) {
-      const int e = i << 2;
-      const float w0 = to_f32(w[e]), w1 = to_f32(w[e + 1]), w2 = to_f32(w[e + 2]), w3 = to_f32(w[e + 3]);
-      store4(o + e, v.x * r * w0, v.y * r * w1, v.z * r * w2, v.w * r * w3);
+    auto put = [&](int i, float4 v, float4 wv, float r) {
+      store4(o + (i << 2), v.x * r * wv.x, v.y * r * wv.y, v.z * r * wv.z, v.w * r * wv.w);
     };
     const int VB = blockDim.x * VL;  // virtual block width
     float4 v0[VL], v1[VL];
@@ -294,9 +315,9 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
 #pragma unroll
     for (int k = 0; k < VL; ++k) {
       const int i0 = threadIdx.x + blockDim.x * k, i1 = i0 + VB;
-      if (i0 < nvec) put(i0, v0[k], r);
-      if (i1 < nvec) put(i1, v1[k], r);
-      for (int i = i1 + VB; i < nvec; i += VB) put(i, reinterpret_cast<const float4*>(xr)[i], r);
+      if (i0 < nvec) put(i0, v0[k], w0[k], r);
+      if (i1 < nvec) put(i1, v1[k], w1[k], r);
+      for (int i = i1 + VB; i < nvec; i += VB) put(i, reinterpret_cast<const float4*>(xr)[i], weights(i), r);
     }
   } else {
     for (int i = threadIdx.x; i < E; i += blockDim.x) {
