@@ -13,6 +13,7 @@ from typing import Optional
 
 import torch
 
+from ..kernels import ops
 from .pages import GroupLayout
 
 _STATE_DTYPES = {"float32": torch.float32, "bfloat16": torch.bfloat16, "int32": torch.int32}
@@ -82,6 +83,7 @@ class DeviceCache:
         def make(need):
             return torch.zeros((max_sequences, *need.shape), dtype=_STATE_DTYPES[need.dtype], device=runtime.device)
 
+        self._state_where, self._state_table = None, None  # of `clear_slot`
         self.state = {}  # cache number -> tensor, or {name: tensor} when the layer keeps several states
         for cid, needs in cache_needs.items():
             if isinstance(needs.state, dict):
@@ -108,8 +110,20 @@ class DeviceCache:
         return sum(t[0].numel() * t.element_size() for t in self._state_tensors())
 
     def clear_slot(self, slot: int) -> None:
-        for t in self._state_tensors():
-            t[slot].zero_()
+        if not 0 <= slot < self.max_sequences:
+            raise IndexError(f"slot {slot} of {self.max_sequences}")
+        arrays = list(self._state_tensors())
+        if not arrays:
+            return
+        if not arrays[0].is_cuda:
+            for t in arrays:
+                t[slot].zero_()
+            return
+        where = [(t.data_ptr(), t[0].numel() * t.element_size()) for t in arrays]
+        if where != self._state_where:  # (the first time, or an array was replaced)
+            self._state_where = where
+            self._state_table = torch.tensor(where, dtype=torch.int64).to(arrays[0].device)
+        ops.clear_slot(self._state_table, slot)
 
     def view(self, cache_id: int, step) -> CacheView:
         gi, j = self._where.get(cache_id, (None, None))

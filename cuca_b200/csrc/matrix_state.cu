@@ -15,7 +15,7 @@
 // the step in order from the state its slot holds, leaving the new state there. A value column's state rows live in
 // the registers of NS neighbouring threads (see Split); a token's vectors are copied to shared memory a few tokens
 // ahead of their use. The arithmetic of a token depends neither on where the sequence was cut into steps or chunks
-// nor on what else is in the launch.
+// nor on what else is in the launch (but for the delta rule four tokens at a time, see there).
 #include "common.cuh"
 #include "state_rows.cuh"
 #include <math.h>

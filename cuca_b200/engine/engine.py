@@ -76,11 +76,8 @@ class GpuBackend:
         """A request takes its slot: clear its state, set its sampling constants and its generator."""
         r, s = seq.request, seq.slot
         self.core.cache.clear_slot(s)
-        state = seq.rng_state()
-        self.rng[s] = state - (1 << 64) if state >= (1 << 63) else state
-        self.temperature[s] = float(r.temperature)
-        self.top_k[s] = int(r.top_k)
-        self.top_p[s] = float(r.top_p)
+        ops.set_sampling(self.rng, self.temperature, self.top_k, self.top_p, s, seq.rng_state(), r.temperature, r.top_k,
+                         r.top_p)
         ranked = 0 < r.top_k < self.vocab
         self._needs_scratch[s] = r.temperature > 0 and ((ranked and r.top_k > 1024) or (not ranked and r.top_p < 1.0))
 

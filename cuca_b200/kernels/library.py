@@ -38,6 +38,8 @@ _SIGNATURES = {
     "cuca_scatter_int": [_P, _P, _P, _I, ctypes.c_longlong, _P],
     "cuca_sample": [_P, c_size_t, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _P],
     "cuca_sample_split_words": [],
+    "cuca_clear_slot": [_P, _I, _I, _P],
+    "cuca_set_sampling": [_P, _P, _P, _P, _I, ctypes.c_uint64, _F, _I, _F, _P],
     "cuca_attention_max_head_dim": [],
     "cuca_attention_mma_supported": [_I, _I, _I, _I, _I],
     "cuca_attention_decode": [_P, _I, _P, _I, _P, _P, _I, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _F, _I, _I, _I,

@@ -712,6 +712,23 @@ def sample(logits, temperature, top_k, top_p, rng_state, slot_of_row, out, scrat
                                   0 if split is None else split.rows, _stream()), "sample")
 
 
+def set_sampling(rng_state, temperature, top_k, top_p, slot: int, state: int, t: float, k: int, p: float) -> None:
+    """A slot's generator state (0 .. 2^64 - 1) and sampling constants, in one launch."""
+    _cuda(rng_state, temperature, top_k, top_p)
+    if not 0 <= slot < rng_state.shape[0]:
+        raise IndexError(f"slot {slot} of {rng_state.shape[0]}")
+    if not -(1 << 31) <= int(k) < 1 << 31:
+        raise OverflowError(f"top_k {k} does not fit 32 bits")
+    library.check(library.load().cuca_set_sampling(_p(rng_state), _p(temperature), _p(top_k), _p(top_p), int(slot), int(state),
+                                                   float(t), int(k), float(p), _stream()), "set_sampling")
+
+
+def clear_slot(table, slot: int) -> None:
+    """Zeros in a slot of every state array; `table`: int64 [arrays, 2] on the device, (address, bytes of a slot)."""
+    _cuda(table)
+    library.check(library.load().cuca_clear_slot(_p(table), table.shape[0], int(slot), _stream()), "clear_slot")
+
+
 def decode_advance(tokens, positions, slot_of_row, sampled, history, counter, max_steps, err=None,
                    err_out=None) -> None:
     """tokens <- sampled, positions += 1 for live rows; history[counter] <- sampled; counter += 1;
