@@ -871,7 +871,7 @@ int with_split(int d, F go) {
 
 // The same for the scans without a correction, which have less to do per channel: half as many channels a thread. (One
 // prompt of 1,501 tokens, 16 heads of 128 x 128, eight tokens summed together: 208 us with eight channels, 165 with four;
-// the matrix memory, which carries n too, 212 and 224.)
+// the matrix memory, which carries n too, 212 and 224. Eight requests of one token: 5 and 6 us.)
 template <typename F>
 int with_narrow_split(int d, F go) {
   if (d <= 32) return go(Split<8, 4, 2>());
