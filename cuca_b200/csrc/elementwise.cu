@@ -235,7 +235,7 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
   // The weights are no earlier kernel's output: the first two rounds' are requested before the wait for the predecessor.
   // (A decode step's norm is a chain of latencies; the weights, which the step's larger ones have driven out of L2, were
   // the last of them: Llama-3.1-8B widths, 16 layers, batch 8, 1,957 -> 1,927 us a step. Over many rows, four groups a
-  // thread, the registers they take cost more than the latency: 2,048 rows of 4,096 15.0 us without, 20.6 with.)
+  // thread, the registers they take cost more than the latency: 2,048 rows of 4,096 14.0 us without, 20.6 with.)
   constexpr bool EARLY = VL == 1;
   const bool w_vec = (E & 3) == 0 && (((size_t)w) & (4 * sizeof(TW) - 1)) == 0;
   auto weights = [&](int i) {
