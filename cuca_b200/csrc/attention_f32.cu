@@ -114,14 +114,22 @@ __device__ __forceinline__ void score(float (&s)[TM][4], const float* qs, const 
 template <int DV>
 struct Part {
   float m, l, acc[DV / 8];
+  bool lost;  // a tile with scores that are no numbers came by before any that is one
   __device__ void clear() {
     m = -INFINITY;
     l = 0.f;
+    lost = false;
 #pragma unroll
     for (int i = 0; i < DV / 8; ++i) acc[i] = 0.f;
   }
-  // this <- this and a later chunk
-  __device__ void merge(float m2, float l2, const float (&acc2)[DV / 8]) {
+  // this <- this and a later chunk. Such a tile counts for nothing at the start of a row, and from a row's first finite
+  // score on it makes the result no number; where a row starts is known here only.
+  __device__ void merge(float m2, float l2, const float (&acc2)[DV / 8], bool lost2) {
+    if (lost2 && m != -INFINITY) {
+      l = NAN;
+#pragma unroll
+      for (int i = 0; i < DV / 8; ++i) acc[i] = NAN;
+    }
     if (m2 == -INFINITY) return;
     const float mn = fmaxf(m, m2), c1 = expf(m - mn), c2 = expf(m2 - mn);
     l = fmaf(l2, c2, l * c1);
@@ -132,12 +140,13 @@ struct Part {
 };
 
 // A tile's scores into weights, for one query vector at position P: raw products in, weights out; the chunk's maximum,
-// denominator and values move with the maximum. `seen`: which of the thread's four keys exist (bit j).
+// denominator and values move with the maximum. `there`: which of the tile's 32 keys exist. Keys that the row does not see
+// get a negative zero: unlike a weight that came out as zero, it keeps their values out of the sums whatever they are.
 template <int DV>
 __device__ __forceinline__ void weigh(float (&s)[4], Part<DV>& p, const CucaAttnOptions& o, float slope, int t0, int tx, int P,
                                       int lo, bool row_live, unsigned there) {
   const int keep = o.window > 0 ? o.keep : 0;
-  bool valid[4];
+  bool valid[4], nan = false;
   float top = -INFINITY;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -147,18 +156,23 @@ __device__ __forceinline__ void weigh(float (&s)[4], Part<DV>& p, const CucaAttn
     if (o.softcap > 0.f) v = o.softcap * tanhf(v / o.softcap);
     if (o.slopes) v -= slope * (float)(P - kp);
     s[j] = valid[j] ? v : -INFINITY;
-    top = fmaxf(top, s[j]);
+    nan |= s[j] != s[j];
+    top = fmaxf(top, s[j]);  // (of those that are numbers)
   }
+  const unsigned nans = __ballot_sync(0xffffffffu, nan) >> (threadIdx.x & 24) & 0xffu;
 #pragma unroll
   for (int x = 4; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
   const float mn = fmaxf(p.m, top);
   const bool any = mn != -INFINITY;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) s[j] = any && valid[j] ? expf(s[j] - mn) : 0.f;
+  for (int j = 0; j < 4; ++j) s[j] = any && valid[j] ? expf(s[j] - mn) : -0.f;
   float sum = (s[0] + s[1]) + (s[2] + s[3]);
 #pragma unroll
   for (int x = 4; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-  if (!any) return;
+  if (!any) {
+    p.lost |= nans != 0;
+    return;
+  }
   const float corr = expf(p.m - mn);
   p.l = fmaf(p.l, corr, sum);
 #pragma unroll
@@ -166,8 +180,7 @@ __device__ __forceinline__ void weigh(float (&s)[4], Part<DV>& p, const CucaAttn
   p.m = mn;
 }
 
-// acc += weights (TM rows of `ps`, pitch TILE + 4) times the tile's values, keys in ascending order. A weight of zero adds
-// nothing, not even zero times a value that its row does not see.
+// acc += weights (TM rows of `ps`, pitch TILE + 4) times the tile's values, keys in ascending order.
 template <int DV, int TM>
 __device__ __forceinline__ void add_values(Part<DV> (&p)[TM], const float* ps, const float* vs, int tx) {
 #pragma unroll 2
@@ -183,7 +196,7 @@ __device__ __forceinline__ void add_values(Part<DV> (&p)[TM], const float* ps, c
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
         const float wj = j == 0 ? w[i].x : j == 1 ? w[i].y : j == 2 ? w[i].z : w[i].w;
-        if (wj != 0.f) {
+        if (__float_as_uint(wj) != 0x80000000u) {  // (a negative zero: see `weigh`)
 #pragma unroll
           for (int c = 0; c < DV / 32; ++c) {
             p[i].acc[4 * c] = fmaf(wj, v[c].x, p[i].acc[4 * c]);
@@ -316,7 +329,7 @@ tile_form_kernel(const Args a) {
       if (!more || t1 / CHUNK != t0 / CHUNK) {
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
-          total[i].merge(part[i].m, part[i].l, part[i].acc);
+          total[i].merge(part[i].m, part[i].l, part[i].acc, part[i].lost);
           part[i].clear();
         }
       }
@@ -334,7 +347,7 @@ template <int D, int TM>
 struct RowsForm {
   static constexpr int WARPS = D == 64 ? 8 : 4, VECS = 4 * TM;
   static constexpr int WARP_FLOATS = TILE * (D + 4) + TILE * D + VECS * (TILE + 4);
-  static constexpr int PART = D + 2;  // a chunk's result of a query vector: values, maximum, denominator
+  static constexpr int PART = D + 3;  // a chunk's result of a query vector: values, maximum, denominator, lost or not
   static constexpr int SMEM = (VECS * (D + 4) + WARPS * WARP_FLOATS + WARPS * VECS * PART) * 4;
 };
 
@@ -426,7 +439,7 @@ rows_form_kernel(const Args a) {
       float* to = parts + (warp * VECS + v0 + i) * PART;
 #pragma unroll
       for (int e = 0; e < D / 8; ++e) to[tx * (D / 8) + e] = part[i].acc[e];
-      if (tx == 0) { to[D] = part[i].m; to[D + 1] = part[i].l; }
+      if (tx == 0) { to[D] = part[i].m; to[D + 1] = part[i].l; to[D + 2] = part[i].lost ? 1.f : 0.f; }
     }
     __syncthreads();
     if (warp == 0) {
@@ -437,7 +450,7 @@ rows_form_kernel(const Args a) {
           float acc[D / 8];
 #pragma unroll
           for (int e = 0; e < D / 8; ++e) acc[e] = of[tx * (D / 8) + e];
-          total[i].merge(of[D], of[D + 1], acc);
+          total[i].merge(of[D], of[D + 1], acc, of[D + 2] != 0.f);
         }
     }
     __syncthreads();

@@ -402,6 +402,67 @@ def test_attention_f32_forms_agree(dev, nh, nkv, d, dv, bs, what):
         assert torch.equal(run(a, b), whole[a:b]), (a, b)
 
 
+@pytest.mark.parametrize("d", [64, 100])
+@pytest.mark.parametrize("rows_at_once", [1, 30, 130])
+def test_attention_f32_infinities_and_nans(dev, d, rows_at_once):
+    """A value that is not finite counts for every row that sees its key, also where the key's weight came out as zero, and
+    for no other row. A tile of 32 keys whose scores are no numbers makes a row's result none, wherever it lies in a chunk of
+    128, unless no key before it has a finite score: then it is passed over."""
+    from cuca_b200.kernels import ops
+    nh, nkv, bs, T = 8, 2, 16, 390
+    g = torch.Generator(device=dev).manual_seed(d)
+    pages = -(-T // bs)
+    tables = torch.arange(pages, dtype=torch.int32, device=dev).flip(0).view(1, pages)
+    q = torch.randn(T, nh * d, device=dev, generator=g)
+    k, v = torch.randn(T, nkv, d, device=dev, generator=g), torch.randn(T, nkv, d, device=dev, generator=g)
+
+    def run(k, v, window):
+        kpool, vpool = torch.zeros(pages, nkv, bs, d, device=dev), torch.zeros(pages, nkv, bs, d, device=dev)
+        at = torch.arange(T, device=dev)
+        page = tables[0][at // bs].long()
+        kpool[page, :, at % bs], vpool[page, :, at % bs] = k, v
+        out, err = torch.empty(T, nh * d, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+        seq = torch.zeros(T, dtype=torch.int32, device=dev)
+        for a in range(0, T, rows_at_once):
+            b = min(T, a + rows_at_once)
+            ops.attention_generic(q[a:b], nh * d, out[a:b], kpool, vpool, at[a:b].int(), seq[a:b], tables, nh, nkv, d, d ** -0.5,
+                                  window, err)
+        assert int(err.item()) == 0
+        return out.view(T, nh, d)
+
+    # key 40 scores so low in every head that its weight is zero; one of its values is infinite
+    q[:, ::d] = 8.0
+    far, inf = k.clone(), v.clone()
+    far[40, :, 0] = -4000.0
+    inf[40, 1, 5] = math.inf
+    for window in (None, 75):
+        clean, got = run(far, v, window), run(far, inf, window)
+        sees = torch.zeros(T, dtype=torch.bool, device=dev)
+        sees[40:T if window is None else 40 + window] = True
+        hit = torch.zeros_like(got, dtype=torch.bool)
+        hit[sees, nh // 2:, 5] = True
+        assert bool(clean.isfinite().all())
+        assert bool(got[hit].isnan().all())
+        assert torch.equal(got[~hit], clean[~hit])
+    # whole tiles of keys that are no numbers
+    clean = run(k, v, None)
+    for first in (32, 128, 160, 256):
+        bad = k.clone()
+        bad[first:first + 32] = math.nan
+        got = run(bad, v, None)
+        assert torch.equal(got[:first], clean[:first]), first
+        assert bool(got[first:].isnan().all()), first
+    bad = k.clone()
+    bad[:32] = math.nan
+    got = run(bad, v, None)
+    assert bool((got[:32] == 0).all())
+    kk, vv = k[32:].repeat_interleave(nh // nkv, 1).double(), v[32:].repeat_interleave(nh // nkv, 1).double()
+    sc = torch.einsum("qhd,khd->hqk", q[32:].view(-1, nh, d).double(), kk) * d ** -0.5
+    sc = sc.masked_fill(torch.ones(T - 32, T - 32, dtype=torch.bool, device=dev).triu(1), -math.inf)
+    want = torch.einsum("hqk,khd->qhd", torch.softmax(sc, -1), vv)
+    assert torch.allclose(got[32:].double(), want, atol=1e-5, rtol=1e-5)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nh,nkv,d,rot", [(6, 2, 48, 32), (6, 2, 48, 48), (5, 5, 128, 128), (4, 1, 80, 80)])
 def test_rope_store(dev, dtype, nh, nkv, d, rot):
