@@ -5,9 +5,10 @@
 // products in ascending order, a tile's weights added eight threads apart), tiles in chunks of 128 positions, each summed
 // from nothing, and the chunks merged in ascending order. A tile or chunk without a key that a row sees changes nothing.
 // So a row is the same bits in both forms, however a prompt is cut and whatever runs beside it:
-//   rows_form   few rows: a block per (row, key head), its warps take the row's chunks side by side
-//   tile_form   many: a block per (64 query vectors: consecutive rows times the heads of a group, key head); a run of rows
-//               of one request shares its key and value tiles
+//   rows_form   single tokens, short portions, and few rows: a block per (row, key head), its warps take the row's chunks
+//               side by side
+//   tile_form   longer portions: a block per (64 query vectors: consecutive rows times the heads of a group, key head); a run
+//               of rows of one request shares its key and value tiles, and one run is walked after the other
 // In both a thread holds 4 keys of one to four query vectors while it scores and every eighth run of four value columns
 // while it weighs; the next key tile lands while this one's values are weighed, the next value tile while keys are scored.
 // What bounds it: shared memory (128 bytes a clock feed 4 x 4 products a thread at half the multiply-adds' rate) over a
@@ -39,8 +40,22 @@ struct Args {
   const int* tables;
   int* err;
   int q_stride, out_stride, n_blocks, bs, table_stride, n_rows, nh, nkv, d, dv;
+  int least;  // the tile form leaves runs of fewer rows (within a tile) to the rows form, and that one the others (0: neither does)
   CucaAttnOptions opt;
 };
+
+// The rows of a tile, and how many of them make up the run of one request around row `row` of the step: what both forms go
+// by to tell whose it is. Every lane of a warp takes part.
+__host__ __device__ __forceinline__ int tile_rows_of(int gq) { return 64 / gq; }
+__device__ __forceinline__ int run_around(const Args& a, int row, int lane) {
+  const int rt = tile_rows_of(a.nh / a.nkv), row0 = row / rt * rt, n = min(rt, a.n_rows - row0), seq = a.seq_of_row[row];
+  const unsigned lo = __ballot_sync(0xffffffffu, lane < n && a.seq_of_row[row0 + lane] == seq);
+  const unsigned hi = __ballot_sync(0xffffffffu, lane + 32 < n && a.seq_of_row[row0 + lane + 32] == seq);
+  const unsigned long long same = (unsigned long long)hi << 32 | lo;
+  const int b = row - row0;
+  const unsigned long long above = ~(same >> b), below = ~(same << (63 - b));  // the first zero bit ends the run
+  return (above ? __ffsll((long long)above) - 1 : 64) + (below ? __clzll((long long)below) : 64) - 1;
+}
 
 // the first key position in a row's window
 __device__ __forceinline__ int window_start(const CucaAttnOptions& o, int P) {
@@ -256,13 +271,23 @@ tile_form_kernel(const Args a) {
   pdl_trigger();
   pdl_wait();
   const int gq = a.nh / a.nkv, kvh = blockIdx.y, tid = threadIdx.x;
-  const int rt = VECS / gq;                                   // rows of a block
+  const int rt = tile_rows_of(gq);                            // rows of a block
   const int row0 = (gridDim.x - 1 - blockIdx.x) * rt;         // later rows see more keys: first
   const int nr = min(rt, a.n_rows - row0);
   for (int r = tid; r < nr; r += THREADS) { s_pos[r] = a.positions[row0 + r]; s_seq[r] = a.seq_of_row[row0 + r]; }
-  for (int e = tid; e < VECS * D; e += THREADS) {
-    const int v = e / D, c = e % D, r = v / gq;
-    qs[v * (D + 4) + c] = r < nr && c < a.d ? a.q[(size_t)(row0 + r) * a.q_stride + (size_t)(kvh * gq + v % gq) * a.d + c] : 0.f;
+  if (a.q_stride % 4 == 0 && ((uintptr_t)a.q & 15) == 0) {
+#pragma unroll 4
+    for (int e = tid; e < VECS * D / 4; e += THREADS) {
+      const int v = e / (D / 4), c = e % (D / 4) * 4, r = v / gq;
+      *reinterpret_cast<float4*>(qs + v * (D + 4) + c) =
+          r < nr && c < a.d ? *reinterpret_cast<const float4*>(a.q + (size_t)(row0 + r) * a.q_stride + (size_t)(kvh * gq + v % gq) * a.d + c)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  } else {
+    for (int e = tid; e < VECS * D; e += THREADS) {
+      const int v = e / D, c = e % D, r = v / gq;
+      qs[v * (D + 4) + c] = r < nr && c < a.d ? a.q[(size_t)(row0 + r) * a.q_stride + (size_t)(kvh * gq + v % gq) * a.d + c] : 0.f;
+    }
   }
   __syncthreads();
   const int tx = tid % 8, v0 = tid / 8 * TM;  // this thread's query vectors v0 .. v0 + TM - 1
@@ -279,7 +304,7 @@ tile_form_kernel(const Args a) {
     }
     const int rb = b, re = e;
     b = e;
-    if (seq < 0) continue;
+    if (seq < 0 || re - rb < a.least) continue;
     const int* table = a.tables + (size_t)seq * a.table_stride;
     const Walk walk = walk_of(a.opt, lo_min, last);
     Part<D> total[TM], part[TM];
@@ -343,18 +368,18 @@ tile_form_kernel(const Args a) {
   }
 }
 
-template <int D, int TM>
+template <int D, int TM, int WARPS_>
 struct RowsForm {
-  static constexpr int WARPS = D == 64 ? 8 : 4, VECS = 4 * TM;
+  static constexpr int WARPS = WARPS_, VECS = 4 * TM;
   static constexpr int WARP_FLOATS = TILE * (D + 4) + TILE * D + VECS * (TILE + 4);
   static constexpr int PART = D + 3;  // a chunk's result of a query vector: values, maximum, denominator, lost or not
   static constexpr int SMEM = (VECS * (D + 4) + WARPS * WARP_FLOATS + WARPS * VECS * PART) * 4;
 };
 
-template <int D, int TM>
-__global__ void __launch_bounds__((32 * RowsForm<D, TM>::WARPS))
+template <int D, int TM, int WARPS_>
+__global__ void __launch_bounds__(32 * WARPS_)
 rows_form_kernel(const Args a) {
-  using F = RowsForm<D, TM>;
+  using F = RowsForm<D, TM, WARPS_>;
   constexpr int WARPS = F::WARPS, VECS = F::VECS, PART = F::PART;
   extern __shared__ __align__(16) float sm[];
   __shared__ long long rows[WARPS][2][TILE];
@@ -368,7 +393,7 @@ rows_form_kernel(const Args a) {
   pdl_wait();
   const int gq = a.nh / a.nkv, kvh = blockIdx.x, row = blockIdx.y;
   const int seq = a.seq_of_row[row];
-  if (seq < 0) return;
+  if (seq < 0 || (a.least && run_around(a, row, lane) >= a.least)) return;
   const int P = a.positions[row], lo = window_start(a.opt, P);
   for (int e = threadIdx.x; e < VECS * D; e += 32 * WARPS) {
     const int v = e / D, c = e % D;
@@ -471,18 +496,53 @@ int launch(F* kernel, dim3 grid, int threads, int smem, cudaStream_t stream, con
   return 0;
 }
 
+// How many chunks of keys a row may have to walk, at most.
+int chunks_of(const Args& a) {
+  const int keys = a.opt.keys > 0 ? a.opt.keys : a.table_stride * a.bs, w = a.opt.window;
+  const int chunks = (keys + CHUNK - 1) / CHUNK;
+  return w > 0 ? min(chunks, (a.opt.keep + CHUNK - 1) / CHUNK + (w + CHUNK - 1) / CHUNK + 1) : chunks;
+}
+
+template <int D, int TM>
+int run_rows(const Args& a, cudaStream_t stream) {
+  // A warp per chunk: a block of eight warps fills an SM's shared memory, and over short rows seven of them idle (single
+  // tokens of up to 32 keys, 32 heads of 64 over 8: 65 rows 22 us with eight warps, 100 rows 9 with one).
+  const int chunks = chunks_of(a);
+  const dim3 grid(a.nkv, a.n_rows);
+#define ROWS(W) return launch(rows_form_kernel<D, TM, W>, grid, 32 * W, RowsForm<D, TM, W>::SMEM, stream, a)
+  if (chunks <= 1) ROWS(1);
+  if (chunks <= 2) ROWS(2);
+  if (D == 128 || chunks <= 4) ROWS(4);
+  if constexpr (D == 64) ROWS(8);
+#undef ROWS
+  return 0;
+}
+
 template <int D>
-int run(const Args& a, cudaStream_t stream) {
-  const int gq = a.nh / a.nkv;
-  // Single tokens, or so few rows that blocks of 64 query vectors would leave most SMs idle.
-  if (a.n_rows <= 64 && gq <= 16) {
-    const dim3 grid(a.nkv, a.n_rows);
-    if (gq <= 4) return launch(rows_form_kernel<D, 1>, grid, 32 * RowsForm<D, 1>::WARPS, RowsForm<D, 1>::SMEM, stream, a);
-    if (gq <= 8) return launch(rows_form_kernel<D, 2>, grid, 32 * RowsForm<D, 2>::WARPS, RowsForm<D, 2>::SMEM, stream, a);
-    return launch(rows_form_kernel<D, 4>, grid, 32 * RowsForm<D, 4>::WARPS, RowsForm<D, 4>::SMEM, stream, a);
+int run(Args a, cudaStream_t stream) {
+  const int gq = a.nh / a.nkv, rt = tile_rows_of(gq);
+  // Runs of fewer rows than this go row by row. A tile's runs are walked one after the other, so a run of one row takes the
+  // time of a whole tile (65 rows of 300 keys, 12 heads of 64: 3,452 us in tiles, 65 row by row). Both forms cost about the
+  // same at some 32 query vectors a run (40 requests with 100 keys before, 32 heads of 64 over 8, us row by row, in tiles:
+  // 8 rows 48, 75; 16 rows 91, 44; 12 heads of 64, 16 requests: 20 rows 69, 111; 32 rows 184, 78).
+  const int least = max(4, 32 / gq + 1);
+  a.least = 0;
+  bool tiles = true, rows = false;
+  if (gq <= 16) {
+    // Few rows: blocks of 64 query vectors would leave most SMs idle. Where nothing is known of the runs, one chunk of keys is
+    // too little to share, and over more of them every row finds out for itself in both launches.
+    const bool known = a.opt.run_max > 0;
+    rows = a.n_rows <= 64 || !known || a.opt.run_min < least;
+    tiles = a.n_rows > 64 && (known ? a.opt.run_max >= least : chunks_of(a) > 1);
+    if (rows && tiles) a.least = least;
   }
-  const int rt = TileForm<D>::VECS / gq;
-  return launch(tile_form_kernel<D>, dim3((a.n_rows + rt - 1) / rt, a.nkv), TileForm<D>::THREADS, TileForm<D>::SMEM, stream, a);
+  if (tiles) {
+    const int rc = launch(tile_form_kernel<D>, dim3((a.n_rows + rt - 1) / rt, a.nkv), TileForm<D>::THREADS, TileForm<D>::SMEM,
+                          stream, a);
+    if (rc) return rc;
+  }
+  if (!rows) return 0;
+  return gq <= 4 ? run_rows<D, 1>(a, stream) : gq <= 8 ? run_rows<D, 2>(a, stream) : run_rows<D, 4>(a, stream);
 }
 
 }  // namespace
@@ -498,6 +558,6 @@ int cuca_attention_f32(const float* q, int q_stride, float* out, int out_stride,
                        int n_blocks, int bs, const int* positions, const int* seq_of_row, const int* tables, int table_stride,
                        int n_rows, int nh, int nkv, int d, int dv, const CucaAttnOptions* opt, int* err, cudaStream_t stream) {
   const Args a{q, out, kpool, vpool, positions, seq_of_row, tables, err, q_stride, out_stride, n_blocks, bs, table_stride,
-               n_rows, nh, nkv, d, dv, *opt};
+               n_rows, nh, nkv, d, dv, 0, *opt};
   return d <= 64 ? run<64>(a, stream) : run<128>(a, stream);
 }

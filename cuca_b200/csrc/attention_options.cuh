@@ -19,6 +19,9 @@ struct CucaAttnOptions {
   const float* slopes;    // [nh] or null: no distance bias
   const void* gate;       // rows of the output's type, or null
   float* key_scale;       // [pages][key heads][positions of a page] or null (written only by kernels that store keys)
+  // What the caller knows of the rows, 0 for nothing; they choose between forms and never change a result.
+  int keys;               // no row sees a position from here on
+  int run_min, run_max;   // how many rows the requests bring, the least and the most
 };
 
 #define CUCA_LOG2E 1.4426950408889634f

@@ -169,7 +169,8 @@ class AttentionOptions(ctypes.Structure):
 
     _fields_ = [("scale", ctypes.c_float), ("window", ctypes.c_int), ("keep", ctypes.c_int), ("softcap", ctypes.c_float),
                 ("sink", ctypes.c_int), ("gate_stride", ctypes.c_int), ("sink_val", ctypes.c_void_p),
-                ("slopes", ctypes.c_void_p), ("gate", ctypes.c_void_p), ("key_scale", ctypes.c_void_p)]
+                ("slopes", ctypes.c_void_p), ("gate", ctypes.c_void_p), ("key_scale", ctypes.c_void_p),
+                ("keys", ctypes.c_int), ("run_min", ctypes.c_int), ("run_max", ctypes.c_int)]
 
 
 def attention_options(n_heads, scale, window=None, softcap=0.0, sink=False, sink_values=None, keep_first=0, slopes=None,
@@ -663,7 +664,7 @@ def attention(qkv, out, cache, step, plan, n_heads, n_kv_heads, head_dim, scale,
                              window, chunk, n_splits, err, **options)
         return
     attention_generic_v(qkv, qkv.stride(0), out, cache.k, cache.v, step.positions, step.seq_of_row, cache.tables,
-                        n_heads, n_kv_heads, head_dim, head_dim, scale, window, err, **options)
+                        n_heads, n_kv_heads, head_dim, head_dim, scale, window, err, step=step, **options)
 
 
 def scatter_int(dst, idx, val) -> None:
@@ -1037,12 +1038,27 @@ def rope_store_general(qkv, k_col, v_col, positions, seq_of_row, tables, cos, si
         head_dim, v_head_dim, int(v_split), int(v_row_dim), _p(err), _stream()), "rope_store_general")
 
 
+def _runs(step):
+    """(a bound on the keys of a row, the fewest and the most rows that a request of the step brings); zeros: not known."""
+    if step.static_max_len is not None:
+        return step.static_max_len, 1, 1
+    runs = step.plans.get("runs")
+    if runs is None:
+        counts, starts = step.host.get("counts"), step.host.get("starts")
+        live = [c for c in counts or () if c > 0]
+        runs = (max(s + c for s, c in zip(starts, counts)), min(live), max(live)) if live and starts is not None else (0, 0, 0)
+        step.plans["runs"] = runs
+    return runs
+
+
 def attention_generic_v(q, q_stride, out, kpool, vpool, positions, seq_of_row, tables, n_heads, n_kv_heads,
-                        head_dim, v_head_dim, scale, window, err, **options) -> None:
+                        head_dim, v_head_dim, scale, window, err, step=None, **options) -> None:
     """The plain attention kernel with value heads of their own size (`vpool`: [pages, kv heads, block, v_head_dim]);
-    `options`: see `attention_options`."""
+    `options`: see `attention_options`. `step`: whose rows these are, where that is known (the kernels' choice of a form)."""
     _cuda(q, out, kpool, vpool)
     opt = attention_options(n_heads, scale, window, gate_width=n_heads * v_head_dim, **options)
+    if step is not None:
+        opt.keys, opt.run_min, opt.run_max = _runs(step)
     library.check(library.load().cuca_attention_generic_o(
         _p(q), int(q_stride), _p(out), out.stride(0), dtype_code(out.dtype), _p(kpool), _p(vpool), kpool.shape[0],
         kpool.shape[2], _p(positions), _p(seq_of_row), _p(tables), tables.shape[1], out.shape[0], n_heads,

@@ -289,7 +289,8 @@ class PagedAttention(Mixer):
                 ops.gate_merge(parts, gate, attn, nh, dv)
         else:
             ops.attention_generic_v(proj, proj.stride(0), attn, cache.k, vpool, step.positions, step.seq_of_row,
-                                    cache.tables, nh, nkv, d, dv, scale, self.window, self.rt.err, gate=gate, **options)
+                                    cache.tables, nh, nkv, d, dv, scale, self.window, self.rt.err, gate=gate,
+                                    step=step, **options)
         if self.head_gate:
             ops.head_gate_(attn, proj[:, g_col:g_col + nh], nh, dv)
         stream.add_linear(attn, self.w_o, bias=self.b_o)

@@ -463,6 +463,46 @@ def test_attention_f32_infinities_and_nans(dev, d, rows_at_once):
     assert torch.allclose(got[32:].double(), want, atol=1e-5, rtol=1e-5)
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(6, 6, 36), (8, 2, 64), (10, 2, 80), (16, 1, 128), (20, 1, 64)])
+@pytest.mark.parametrize("counts,start", [([1] * 70, 50), ([1] * 70, 300), ([5, 70, 1, 33, 31, 32, 2], 0), ([64, 1, 7, 90], 90),
+                                          ([100, 80], 10), ([3] * 30, 200), ([20], 0), ([1, 1], 1030)])
+def test_attention_f32_is_the_same_bits_whatever_is_known_of_the_rows(dev, nh, nkv, d, counts, start):
+    """Rows whose requests' portions are known (all short, all long, or both: row by row, in tiles, or each its own way; as
+    many warps as the keys need), the same rows with nothing known, and one after the other."""
+    import types
+
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(nh + d + len(counts))
+    bs, S, longest = 16, len(counts), start + max(counts)
+    pages = -(-longest // bs) + 70  # (a table wider than the longest request)
+    tables = torch.full((S, pages), -1, dtype=torch.int32, device=dev)
+    used = -(-longest // bs)
+    tables[:, :used] = torch.randperm(S * used, device=dev, generator=g).to(torch.int32).view(S, used)
+    kpool, vpool = (torch.randn(S * used, nkv, bs, d, device=dev, generator=g) for _ in range(2))
+    rows = [(s, start + j) for s, c in enumerate(counts) for j in range(c)]
+    q = torch.randn(len(rows), nh * d, device=dev, generator=g)
+    seq = torch.tensor([s for s, _ in rows], dtype=torch.int32, device=dev)
+    positions = torch.tensor([p for _, p in rows], dtype=torch.int32, device=dev)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    known = types.SimpleNamespace(static_max_len=None, plans={}, host={"counts": counts, "starts": [start] * S})
+    captured = types.SimpleNamespace(static_max_len=longest, plans={}, host={"counts": counts})
+
+    def run(a, b, step=None, window=None):
+        out = torch.empty(b - a, nh * d, device=dev)
+        ops.attention_generic_v(q[a:b], nh * d, out, kpool, vpool, positions[a:b], seq[a:b], tables, nh, nkv, d, d, d ** -0.5,
+                                window, err, step=step)
+        return out
+
+    for window in (None, 40):
+        whole = run(0, len(rows), None, window)
+        assert torch.equal(run(0, len(rows), known, window), whole)
+        if max(counts) == 1:
+            assert torch.equal(run(0, len(rows), captured, window), whole)
+        for i in range(0, len(rows), 13):
+            assert torch.equal(run(i, i + 1, None, window)[0], whole[i]), i
+    assert int(err.item()) == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nh,nkv,d,rot", [(6, 2, 48, 32), (6, 2, 48, 48), (5, 5, 128, 128), (4, 1, 80, 80)])
 def test_rope_store(dev, dtype, nh, nkv, d, rot):
