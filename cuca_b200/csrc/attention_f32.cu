@@ -12,8 +12,8 @@
 // In both a thread holds 4 keys of one to four query vectors while it scores and every eighth run of four value columns
 // while it weighs; the next key tile lands while this one's values are weighed, the next value tile while keys are scored.
 // What bounds it: shared memory (128 bytes a clock feed 4 x 4 products a thread at half the multiply-adds' rate) over a
-// prompt, latency over single tokens. Measured on 32 heads of 64 over 8 key heads: 700 rows 174 us, 4 rows of 516 keys
-// 20 us; a warp per (row, head) whose lanes read a key each, before: 2,400 and 568 us.
+// prompt, latency over single tokens. Measured on 32 heads of 64 over 8 key heads: 700 rows 172 us, 4 rows of 516 keys
+// 17 us; a warp per (row, head) whose lanes read a key each, before: 2,390 and 283 us.
 #include "attention_options.cuh"
 #include "common.cuh"
 #include <math.h>
@@ -129,16 +129,15 @@ __device__ __forceinline__ void score(float (&s)[TM][4], const float* qs, const 
 template <int DV>
 struct Part {
   float m, l, acc[DV / 8];
-  bool lost;  // a tile with scores that are no numbers came by before any that is one
   __device__ void clear() {
     m = -INFINITY;
     l = 0.f;
-    lost = false;
 #pragma unroll
     for (int i = 0; i < DV / 8; ++i) acc[i] = 0.f;
   }
-  // this <- this and a later chunk. Such a tile counts for nothing at the start of a row, and from a row's first finite
-  // score on it makes the result no number; where a row starts is known here only.
+  // this <- this and a later chunk. lost2: in that chunk a tile with scores that are no numbers came by before any that is
+  // one. Such a tile counts for nothing at the start of a row, and from a row's first finite score on it makes the result no
+  // number; where a row starts is known here only.
   __device__ void merge(float m2, float l2, const float (&acc2)[DV / 8], bool lost2) {
     if (lost2 && m != -INFINITY) {
       l = NAN;
@@ -157,46 +156,47 @@ struct Part {
 // A tile's scores into weights, for one query vector at position P: raw products in, weights out; the chunk's maximum,
 // denominator and values move with the maximum. `there`: which of the tile's 32 keys exist. Keys that the row does not see
 // get a negative zero: unlike a weight that came out as zero, it keeps their values out of the sums whatever they are.
-template <int DV>
-__device__ __forceinline__ void weigh(float (&s)[4], Part<DV>& p, const CucaAttnOptions& o, float slope, int t0, int tx, int P,
+// FULL: the row sees all of them. Returns whether this thread has a score that is no number while no thread has one that is.
+template <int DV, bool FULL>
+__device__ __forceinline__ bool weigh(float (&s)[4], Part<DV>& p, const CucaAttnOptions& o, float slope, int t0, int tx, int P,
                                       int lo, bool row_live, unsigned there) {
   const int keep = o.window > 0 ? o.keep : 0;
-  bool valid[4], nan = false;
+  bool valid[4];
   float top = -INFINITY;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int kp = t0 + tx + 8 * j;
-    valid[j] = row_live && (there >> (tx + 8 * j) & 1u) && (kp >= lo || kp < keep) && kp <= P;
+    valid[j] = FULL || (row_live && (there >> (tx + 8 * j) & 1u) && (kp >= lo || kp < keep) && kp <= P);
     float v = s[j] * o.scale;
     if (o.softcap > 0.f) v = o.softcap * tanhf(v / o.softcap);
     if (o.slopes) v -= slope * (float)(P - kp);
     s[j] = valid[j] ? v : -INFINITY;
-    nan |= s[j] != s[j];
     top = fmaxf(top, s[j]);  // (of those that are numbers)
   }
-  const unsigned nans = __ballot_sync(0xffffffffu, nan) >> (threadIdx.x & 24) & 0xffu;
 #pragma unroll
   for (int x = 4; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
   const float mn = fmaxf(p.m, top);
   const bool any = mn != -INFINITY;
+  bool nan = false;
+  if (!any)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) nan |= s[j] != s[j];
 #pragma unroll
   for (int j = 0; j < 4; ++j) s[j] = any && valid[j] ? expf(s[j] - mn) : -0.f;
   float sum = (s[0] + s[1]) + (s[2] + s[3]);
 #pragma unroll
   for (int x = 4; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-  if (!any) {
-    p.lost |= nans != 0;
-    return;
-  }
+  if (!any) return nan;
   const float corr = expf(p.m - mn);
   p.l = fmaf(p.l, corr, sum);
 #pragma unroll
   for (int i = 0; i < DV / 8; ++i) p.acc[i] *= corr;
   p.m = mn;
+  return false;
 }
 
 // acc += weights (TM rows of `ps`, pitch TILE + 4) times the tile's values, keys in ascending order.
-template <int DV, int TM>
+template <int DV, int TM, bool FULL>
 __device__ __forceinline__ void add_values(Part<DV> (&p)[TM], const float* ps, const float* vs, int tx) {
 #pragma unroll 2
   for (int j0 = 0; j0 < TILE; j0 += 4) {
@@ -211,7 +211,7 @@ __device__ __forceinline__ void add_values(Part<DV> (&p)[TM], const float* ps, c
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
         const float wj = j == 0 ? w[i].x : j == 1 ? w[i].y : j == 2 ? w[i].z : w[i].w;
-        if (__float_as_uint(wj) != 0x80000000u) {  // (a negative zero: see `weigh`)
+        if (FULL || __float_as_uint(wj) != 0x80000000u) {  // (a negative zero: see `weigh`)
 #pragma unroll
           for (int c = 0; c < DV / 32; ++c) {
             p[i].acc[4 * c] = fmaf(wj, v[c].x, p[i].acc[4 * c]);
@@ -221,6 +221,54 @@ __device__ __forceinline__ void add_values(Part<DV> (&p)[TM], const float* ps, c
           }
         }
       }
+    }
+  }
+}
+
+// A thread's TM query vectors through a tile: weights into its rows of `ps`. Returns which of the vectors (bit i) have
+// scores and none that is a number. Every lane of a warp takes part.
+template <int DV, int TM, bool FULL>
+__device__ __forceinline__ unsigned weigh_all(float (&s)[TM][4], Part<DV> (&p)[TM], const CucaAttnOptions& o,
+                                              const float (&slope)[TM], int t0, int tx, const int (&P)[TM], const int (&lo)[TM],
+                                              const bool (&live)[TM], unsigned there, float* ps) {
+  unsigned nans = 0;
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    if (weigh<DV, FULL>(s[i], p[i], o, slope[i], t0, tx, P[i], lo[i], live[i], there)) nans |= 1u << i;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ps[i * (TILE + 4) + tx + 8 * j] = s[i][j];
+  }
+  if (__any_sync(0xffffffffu, nans != 0))  // (a vector's eight threads as one)
+#pragma unroll
+    for (int x = 4; x > 0; x >>= 1) nans |= __shfl_xor_sync(0xffffffffu, nans, x);
+  return nans;
+}
+
+// Whether every vector of the warp that counts sees all keys of a tile (the others' results go nowhere).
+template <int TM>
+__device__ __forceinline__ bool all_seen(int t0, const int (&P)[TM], const int (&lo)[TM], const bool (&live)[TM], unsigned there) {
+  bool full = there == 0xffffffffu;
+#pragma unroll
+  for (int i = 0; i < TM; ++i) full &= !live[i] || (t0 >= lo[i] && t0 + TILE - 1 <= P[i]);
+  return __all_sync(0xffffffffu, full);
+}
+
+// N query vectors into [N][D + 4], zeros behind a.d and for those that `at` has no address for.
+template <int D, int N, int THREADS, typename At>
+__device__ __forceinline__ void load_queries(const Args& a, float* qs, int tid, At at) {
+  if (a.q_stride % 4 == 0 && ((uintptr_t)a.q & 15) == 0) {
+#pragma unroll 4
+    for (int e = tid; e < N * D / 4; e += THREADS) {
+      const int v = e / (D / 4), c = e % (D / 4) * 4;
+      const float* src = at(v);
+      *reinterpret_cast<float4*>(qs + v * (D + 4) + c) =
+          src && c < a.d ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  } else {
+    for (int e = tid; e < N * D; e += THREADS) {
+      const int v = e / D, c = e % D;
+      const float* src = at(v);
+      qs[v * (D + 4) + c] = src && c < a.d ? src[c] : 0.f;
     }
   }
 }
@@ -275,20 +323,10 @@ tile_form_kernel(const Args a) {
   const int row0 = (gridDim.x - 1 - blockIdx.x) * rt;         // later rows see more keys: first
   const int nr = min(rt, a.n_rows - row0);
   for (int r = tid; r < nr; r += THREADS) { s_pos[r] = a.positions[row0 + r]; s_seq[r] = a.seq_of_row[row0 + r]; }
-  if (a.q_stride % 4 == 0 && ((uintptr_t)a.q & 15) == 0) {
-#pragma unroll 4
-    for (int e = tid; e < VECS * D / 4; e += THREADS) {
-      const int v = e / (D / 4), c = e % (D / 4) * 4, r = v / gq;
-      *reinterpret_cast<float4*>(qs + v * (D + 4) + c) =
-          r < nr && c < a.d ? *reinterpret_cast<const float4*>(a.q + (size_t)(row0 + r) * a.q_stride + (size_t)(kvh * gq + v % gq) * a.d + c)
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  } else {
-    for (int e = tid; e < VECS * D; e += THREADS) {
-      const int v = e / D, c = e % D, r = v / gq;
-      qs[v * (D + 4) + c] = r < nr && c < a.d ? a.q[(size_t)(row0 + r) * a.q_stride + (size_t)(kvh * gq + v % gq) * a.d + c] : 0.f;
-    }
-  }
+  load_queries<D, VECS, THREADS>(a, qs, tid, [&](int v) {
+    const int r = v / gq;
+    return r < nr ? a.q + (size_t)(row0 + r) * a.q_stride + (size_t)(kvh * gq + v % gq) * a.d : nullptr;
+  });
   __syncthreads();
   const int tx = tid % 8, v0 = tid / 8 * TM;  // this thread's query vectors v0 .. v0 + TM - 1
   float slope[TM];
@@ -310,6 +348,7 @@ tile_form_kernel(const Args a) {
     Part<D> total[TM], part[TM];
     int P[TM], lo[TM];
     bool live[TM];
+    unsigned lost = 0;  // which vectors' parts of this chunk started with scores that are no numbers
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       total[i].clear();
@@ -339,24 +378,24 @@ tile_form_kernel(const Args a) {
       __syncthreads();  // the keys are read
       if (more) load_tile<D, D + 4, THREADS>(ks, a.kpool, rows[buf ^ 1], a.d, tid);
       copy_commit();
-#pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        weigh<D>(s[i], part[i], a.opt, slope[i], t0, tx, P[i], lo[i], live[i], there);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) ps[(v0 + i) * (TILE + 4) + tx + 8 * j] = s[i][j];
-      }
+      const bool full = all_seen<TM>(t0, P, lo, live, there);
+      float* mine = ps + v0 * (TILE + 4);
+      lost |= full ? weigh_all<D, TM, true>(s, part, a.opt, slope, t0, tx, P, lo, live, there, mine)
+                   : weigh_all<D, TM, false>(s, part, a.opt, slope, t0, tx, P, lo, live, there, mine);
       copy_wait<1>();
       __syncthreads();  // the values have landed, the weights are written
-      add_values<D, TM>(part, ps + v0 * (TILE + 4), vs, tx);
+      if (full) add_values<D, TM, true>(part, mine, vs, tx);
+      else add_values<D, TM, false>(part, mine, vs, tx);
       __syncthreads();  // the values are read
       if (more) load_tile<D, D, THREADS>(vs, a.vpool, rows[buf ^ 1], a.dv, tid);
       copy_commit();
       if (!more || t1 / CHUNK != t0 / CHUNK) {
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
-          total[i].merge(part[i].m, part[i].l, part[i].acc, part[i].lost);
+          total[i].merge(part[i].m, part[i].l, part[i].acc, lost >> i & 1u);
           part[i].clear();
         }
+        lost = 0;
       }
       t0 = t1;
     }
@@ -394,37 +433,41 @@ rows_form_kernel(const Args a) {
   const int gq = a.nh / a.nkv, kvh = blockIdx.x, row = blockIdx.y;
   const int seq = a.seq_of_row[row];
   if (seq < 0 || (a.least && run_around(a, row, lane) >= a.least)) return;
-  const int P = a.positions[row], lo = window_start(a.opt, P);
-  for (int e = threadIdx.x; e < VECS * D; e += 32 * WARPS) {
-    const int v = e / D, c = e % D;
-    qs[v * (D + 4) + c] = v < gq && c < a.d ? a.q[(size_t)row * a.q_stride + (size_t)(kvh * gq + v) * a.d + c] : 0.f;
-  }
+  const int P0 = a.positions[row], lo0 = window_start(a.opt, P0);
+  load_queries<D, VECS, 32 * WARPS>(a, qs, threadIdx.x, [&](int v) {
+    return v < gq ? a.q + (size_t)row * a.q_stride + (size_t)(kvh * gq + v) * a.d : nullptr;
+  });
   __syncthreads();
   const int* table = a.tables + (size_t)seq * a.table_stride;
-  const Walk walk = walk_of(a.opt, lo, P);
+  const Walk walk = walk_of(a.opt, lo0, P0);
   float slope[TM];
 #pragma unroll
   for (int i = 0; i < TM; ++i) slope[i] = a.opt.slopes && v0 + i < gq ? a.opt.slopes[kvh * gq + v0 + i] : 0.f;
+  int P[TM], lo[TM];
+  bool live[TM];
+#pragma unroll
+  for (int i = 0; i < TM; ++i) { P[i] = P0; lo[i] = lo0; live[i] = v0 + i < gq; }
   Part<D> total[TM];  // (of warp 0)
 #pragma unroll
   for (int i = 0; i < TM; ++i) total[i].clear();
   // the chunks that have tiles to walk: of the kept first keys, then of the window; n of them, chunk_of(c) ascending
   const int kept = (walk.kept_end + CHUNK - 1) / CHUNK, first = walk.first / CHUNK;
   const int from = max(first, kept);  // (a chunk that holds both kinds counts as one of the kept ones)
-  const int n = kept + max(0, P / CHUNK - from + 1);
+  const int n = kept + max(0, P0 / CHUNK - from + 1);
   for (int c0 = 0; c0 < n; c0 += WARPS) {
     const int c = c0 + warp;
     Part<D> part[TM];
+    unsigned lost = 0;
 #pragma unroll
     for (int i = 0; i < TM; ++i) part[i].clear();
     if (c < n) {
       const int chunk = c < kept ? c : from + c - kept;
-      const int end = min(P + 1, (chunk + 1) * CHUNK);
+      const int end = min(P0 + 1, (chunk + 1) * CHUNK);
       // the first tile of the chunk that the walk comes by
       int t0 = chunk * CHUNK;
       if (t0 >= walk.kept_end && t0 < walk.first) t0 = walk.first;
       int buf = 0;
-      rows[warp][0][lane] = pool_row(a, table, kvh, t0 + lane, lo, P);
+      rows[warp][0][lane] = pool_row(a, table, kvh, t0 + lane, lo0, P0);
       __syncwarp();
       load_tile<D, D + 4, 32>(ks, a.kpool, rows[warp][0], a.d, lane);
       copy_commit();
@@ -434,7 +477,7 @@ rows_form_kernel(const Args a) {
         const int t1 = walk.next(t0);
         const bool more = t1 < end;
         const unsigned there = __ballot_sync(0xffffffffu, rows[warp][buf][lane] >= 0);
-        if (more) rows[warp][buf ^ 1][lane] = pool_row(a, table, kvh, t1 + lane, lo, P);
+        if (more) rows[warp][buf ^ 1][lane] = pool_row(a, table, kvh, t1 + lane, lo0, P0);
         copy_wait<1>();
         __syncwarp();  // the keys have landed
         float s[TM][4];
@@ -442,15 +485,14 @@ rows_form_kernel(const Args a) {
         __syncwarp();  // the keys are read
         if (more) load_tile<D, D + 4, 32>(ks, a.kpool, rows[warp][buf ^ 1], a.d, lane);
         copy_commit();
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          weigh<D>(s[i], part[i], a.opt, slope[i], t0, tx, P, lo, v0 + i < gq, there);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) ps[(v0 + i) * (TILE + 4) + tx + 8 * j] = s[i][j];
-        }
+        const bool full = all_seen<TM>(t0, P, lo, live, there);
+        float* mine = ps + v0 * (TILE + 4);
+        lost |= full ? weigh_all<D, TM, true>(s, part, a.opt, slope, t0, tx, P, lo, live, there, mine)
+                     : weigh_all<D, TM, false>(s, part, a.opt, slope, t0, tx, P, lo, live, there, mine);
         copy_wait<1>();
         __syncwarp();  // the values have landed, the weights are written
-        add_values<D, TM>(part, ps + v0 * (TILE + 4), vs, tx);
+        if (full) add_values<D, TM, true>(part, mine, vs, tx);
+        else add_values<D, TM, false>(part, mine, vs, tx);
         __syncwarp();  // the values are read
         if (more) load_tile<D, D, 32>(vs, a.vpool, rows[warp][buf ^ 1], a.dv, lane);
         copy_commit();
@@ -464,7 +506,7 @@ rows_form_kernel(const Args a) {
       float* to = parts + (warp * VECS + v0 + i) * PART;
 #pragma unroll
       for (int e = 0; e < D / 8; ++e) to[tx * (D / 8) + e] = part[i].acc[e];
-      if (tx == 0) { to[D] = part[i].m; to[D + 1] = part[i].l; to[D + 2] = part[i].lost ? 1.f : 0.f; }
+      if (tx == 0) { to[D] = part[i].m; to[D + 1] = part[i].l; to[D + 2] = lost >> i & 1u ? 1.f : 0.f; }
     }
     __syncthreads();
     if (warp == 0) {
@@ -522,18 +564,18 @@ template <int D>
 int run(Args a, cudaStream_t stream) {
   const int gq = a.nh / a.nkv, rt = tile_rows_of(gq);
   // Runs of fewer rows than this go row by row. A tile's runs are walked one after the other, so a run of one row takes the
-  // time of a whole tile (65 rows of 300 keys, 12 heads of 64: 3,452 us in tiles, 65 row by row). Both forms cost about the
+  // time of a whole tile (65 rows of 300 keys, 12 heads of 64: 3,524 us in tiles, 54 row by row). Both forms cost about the
   // same at some 32 query vectors a run (40 requests with 100 keys before, 32 heads of 64 over 8, us row by row, in tiles:
   // 8 rows 48, 75; 16 rows 91, 44; 12 heads of 64, 16 requests: 20 rows 69, 111; 32 rows 184, 78).
   const int least = max(4, 32 / gq + 1);
   a.least = 0;
   bool tiles = true, rows = false;
   if (gq <= 16) {
-    // Few rows: blocks of 64 query vectors would leave most SMs idle. Where nothing is known of the runs, one chunk of keys is
-    // too little to share, and over more of them every row finds out for itself in both launches.
+    // Few rows: blocks of 64 query vectors would leave most SMs idle. Where nothing is known of the runs, few rows of one
+    // chunk of keys have little to share, and of others every row finds out for itself in both launches.
     const bool known = a.opt.run_max > 0;
     rows = a.n_rows <= 64 || !known || a.opt.run_min < least;
-    tiles = a.n_rows > 64 && (known ? a.opt.run_max >= least : chunks_of(a) > 1);
+    tiles = a.n_rows > 64 && (known ? a.opt.run_max >= least : a.n_rows > 256 || chunks_of(a) > 1);
     if (rows && tiles) a.least = least;
   }
   if (tiles) {
