@@ -139,7 +139,11 @@ int launch_blocks(const char* name, void (*kernel)(KArgs...), dim3 grid, int thr
   const int spread = per_sm <= 4 ? 228 * 1024 / ((int)per_sm + 1) + 1024 : 0;
   if (smem < spread) smem = spread;
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // The limit belongs to the kernel, not to the launch: one number for all launches, so that a smaller launch of another
+    // thread cannot lower it between these two calls.
+    constexpr int MOST = 128 * 1024;
+    CUCA_REQUIRE(smem <= MOST, "%s: a block of %d bytes of shared memory is larger than %d", name, smem, MOST);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
     CUCA_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory were refused: %s", name, smem, cudaGetErrorString(e));
   }
   cuca_launch(kernel, grid, dim3(threads), smem, stream, true, args...);

@@ -165,6 +165,43 @@ def test_delta_rule_in_chunks_of_four(rt32, H, G, d, dv, counts):
     assert np.abs(got.cpu().numpy() - S).max() < 3e-5 * max(1.0, np.abs(S).max())
 
 
+def test_scans_of_two_threads_with_grids_of_their_own(rt32):
+    """A scan asks for shared memory by the size of its grid; two threads that launch the same kernel on streams and grids of
+    their own do not take each other's away."""
+    import threading
+
+    from cuca_b200.kernels import ops
+    dev, H, d, rounds = rt32.device, 8, 128, 8000
+    cases, errors = [], []
+    for S in (1, 2):  # 128 and 256 blocks: one on an SM, and two
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)  # noqa: E731
+        step = types.SimpleNamespace(n_seqs=S, slots=i32(range(S)), seq_of_row=i32(range(S)), req_row0=i32(range(S)),
+                                     req_count=i32([1] * S), all_single=lambda: False)
+        proj = torch.randn(S, 3 * H * d, device=dev)
+        cases.append((proj, torch.full((H,), 0.9, device=dev), torch.zeros(S, H, d, d, device=dev), step))
+    outs = [torch.empty(c[0].shape[0], H * d, device=dev) for c in cases]
+    torch.cuda.synchronize()
+
+    def work(i):
+        proj, decay, state, step = cases[i]
+        try:
+            torch.cuda.set_device(dev)
+            with torch.cuda.stream(torch.cuda.Stream(dev)):
+                for r in range(rounds):
+                    ops.lightning_scan(proj, decay, state, outs[i], step, H, d, d)
+                    if r % 100 == 99:
+                        torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+
+
 @pytest.mark.parametrize("right", [dict(r_heads=3, r_dim=12, r_vdim=20, cap=6.0), dict(r_heads=1, r_dim=96, r_vdim=40, cap=15.0),
                                    dict(r_heads=2, r_dim=5, r_vdim=130, cap=1.5), dict(r_heads=2, r_dim=260, r_vdim=3, cap=30.0)])
 def test_matrix_memory_alone_whole_and_cut(rt32, right):
