@@ -15,7 +15,7 @@
 // the step in order from the state its slot holds, leaving the new state there. A value column's state rows live in
 // the registers of NS neighbouring threads (see Split); a token's vectors are copied to shared memory a few tokens
 // ahead of their use. The arithmetic of a token depends neither on where the sequence was cut into steps or chunks
-// nor on what else is in the launch (but for the delta rule four tokens at a time, see there).
+// nor on what else is in the launch (but for the delta rule four tokens at a time, which depends on the cuts, see there).
 #include "common.cuh"
 #include "state_rows.cuh"
 #include <math.h>
@@ -61,15 +61,17 @@ delta_prepare_kernel(float* __restrict__ qkv, int ld, float* __restrict__ a_raw,
 // heads at column 2 G d (H heads of dv). decay: rows of stride ld_g, H d decays; beta: rows of stride ld_b, head h at column
 // b_col + h. state: [slots, H, dv, d]. out: [rows, H dv]. Two buffers of TC tokens: the next tokens' vectors are
 // copied (cp.async) while these are worked through.
-// What bounds it for one prompt: the chain of a token (state times decay, dot with k, three shuffles, correction), about
-// 130 clocks; the outputs' dot products belong to the token before and run in the shadow of the shuffles.
+// What bounds it for one prompt: the chain of a token (state times decay, dot with k, four shuffles and one more to hand the
+// sum round, correction), about 500 clocks at 128 channels; the outputs' dot products belong to the token before and run in
+// the shadow of the shuffles.
+// Requests that bring `below` tokens or more are the chunked form's.
 template <typename C>
 __global__ void __launch_bounds__(128)
 delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ decay, int ld_g,
                   const float* __restrict__ beta, int ld_b, int b_col, float* __restrict__ state,
                   float* __restrict__ out, const int* __restrict__ req_row0,
                   const int* __restrict__ req_count, const int* __restrict__ slots, int H, int G,
-                  int d, int dv, int wide) {
+                  int d, int dv, int wide, int below) {
   constexpr int NS = C::NS, NC = C::NC, DP = C::DP, PB = C::PB, TC = C::TC, PAIRS = C::PAIRS;
   constexpr int PER = 3 * DP + ((PB + 1 + 3) & ~3);  // a token: q, k, g, the block's values, beta
   extern __shared__ __align__(16) float sm[];
@@ -77,7 +79,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
   pdl_wait();
   const int h = blockIdx.x, rq = blockIdx.y;
   const int slot = slots[rq], n = req_count[rq], r0 = req_row0[rq];
-  if (slot < 0 || n <= 0) return;
+  if (slot < 0 || n <= 0 || n >= below) return;
   const int kvh = h / (H / G);
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
   const int col0 = blockIdx.z * PB, at = col_local * NC;
@@ -195,7 +197,8 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
 //   S  <- G S + sum_t (R_t k_t) u_t^T
 // so eight sums over the channels go as one, and the scaled vectors and the numbers c and e, which do not depend on the
 // state, are made by a kernel of their own over all chunks at once. All products of decays are at most 1. The rounding
-// differs from token by token and depends on where a portion starts, so the 32-bit path does not come here.
+// differs from token by token and depends on where a portion starts, so the 32-bit path does not come here; whether a
+// request does depends on its own tokens and the sizes alone (`from` tokens or more), not on the step's other requests.
 // Measured on 1,501 tokens, 16 heads of 128 x 128: 403 us token by token, 265 + 11 us
 // this way (294 with a column a thread group, whose reads of the 13 vectors fill the shared memory's 128 bytes a clock).
 constexpr int DC_T = 4, DC_D = 128;                          // tokens of a chunk; channels, zeros behind the last
@@ -210,12 +213,12 @@ __global__ void __launch_bounds__(256)
 delta_chunk_prepare_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ decay, int ld_g,
                            const float* __restrict__ beta, int ld_b, int b_col, float* __restrict__ chunks,
                            const int* __restrict__ req_row0, const int* __restrict__ req_count,
-                           const int* __restrict__ slots, int H, int G, int d) {
+                           const int* __restrict__ slots, int H, int G, int d, int from) {
   pdl_trigger();
   pdl_wait();
   const int c = blockIdx.x, rq = blockIdx.y, h = blockIdx.z * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int n = req_count[rq], r0 = req_row0[rq];
-  if (slots[rq] < 0 || c * DC_T >= n || h >= H) return;
+  if (slots[rq] < 0 || n < from || c * DC_T >= n || h >= H) return;
   const int nt = min(DC_T, n - c * DC_T), kvh = h / (H / G), i = 4 * lane;
   float q[DC_T][4], k[DC_T][4], g[DC_T][4];
 #pragma unroll
@@ -291,7 +294,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, int ld, const float* _
 __global__ void __launch_bounds__(256)
 delta_chunk_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ chunks, float* __restrict__ state,
                         float* __restrict__ out, const int* __restrict__ req_row0, const int* __restrict__ req_count,
-                        const int* __restrict__ slots, int H, int G, int d, int dv) {
+                        const int* __restrict__ slots, int H, int G, int d, int dv, int from) {
   using C = Split<32, 4, 2>;
   constexpr int NS = C::NS, NC = C::NC, PAIRS = C::PAIRS, PB = 16, RUN = 4;  // RUN: chunks staged at a time
   constexpr int PER = DC_WORDS + DC_T * PB;                      // a staged chunk, then the block's values [4][PB]
@@ -300,14 +303,14 @@ delta_chunk_scan_kernel(const float* __restrict__ qkv, int ld, const float* __re
   pdl_wait();
   const int h = blockIdx.x, rq = blockIdx.y;
   const int slot = slots[rq], n = req_count[rq], r0 = req_row0[rq];
-  if (slot < 0 || n <= 0) return;
+  if (slot < 0 || n < from) return;
   const int s = threadIdx.x % NS, col0 = blockIdx.z * PB, at = threadIdx.x / NS * NC;
   const int cols = min(NC, dv - col0 - at);  // columns of this warp that exist (none: 0 or less)
   float* st = state + (((size_t)slot * H + h) * dv + (cols > 0 ? col0 + at : 0)) * d;
   f32x2 S[NC][PAIRS];
   load_rows<C>(S, st, s, d, cols, 1);
   const int n_chunks = (n + DC_T - 1) / DC_T, runs = (n_chunks + RUN - 1) / RUN;
-  // (values of columns from dv on and of tokens from n on: zeros, which no copy writes)
+  // (values of columns from dv on: zeros, which no copy writes)
   for (int e = threadIdx.x; e < 2 * RUN * DC_T * PB; e += 256) sm[(e / (DC_T * PB)) * PER + DC_WORDS + e % (DC_T * PB)] = 0.f;
   __syncthreads();
   auto stage = [&](int run, int buf) {
@@ -343,6 +346,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qkv, int ld, const float* __re
 #pragma unroll
         for (int j = 0; j < NC; ++j) sums[t * NC + j] = dot_rows(S[j], w[t]);
       const float* next = c + 1 < nc ? ch + PER : ch;
+      const int there = n - (run * RUN + c) * DC_T;  // tokens of this chunk and behind it
 #pragma unroll
       for (int t = 0; t < 2 * DC_T; ++t) staged_rows<C>(w[t], next + t * DC_D, s);
       f32x2 r[DC_T][PAIRS], g[PAIRS];
@@ -368,6 +372,11 @@ delta_chunk_scan_kernel(const float* __restrict__ qkv, int ld, const float* __re
         float a[DC_T];
 #pragma unroll
         for (int t = 0; t < DC_T; ++t) a[t] = __shfl_sync(0xffffffffu, mine, 2 * (t * NC + j));
+        if (there < DC_T) {  // tokens that do not exist (their write gates are zeros) correct nothing, whatever was found there
+#pragma unroll
+          for (int t = 1; t < DC_T; ++t)
+            if (t >= there) a[t] = v[t][j] = 0.f;
+        }
         const float u0 = b.x * (v[0][j] - a[0]);
         const float u1 = b.y * fmaf(-c4.x, u0, v[1][j] - a[1]);
         const float u2 = b.z * fmaf(-c4.z, u1, fmaf(-c4.y, u0, v[2][j] - a[2]));
@@ -381,10 +390,13 @@ delta_chunk_scan_kernel(const float* __restrict__ qkv, int ld, const float* __re
           for (int i = 0; i < PAIRS; ++i) S[j][i] = f2_fma(r[t][i], uu, S[j][i]);
         }
       }
-      const int row = (run * RUN + c) * DC_T + own_t;
-      if (own >= DC_T * NC && (s & 1) == 0 && own_c < cols && row < n)
-        out[(size_t)(r0 + row) * H * dv + (size_t)h * dv + col0 + at + own_c] =
-            fmaf(e4.w, mine_u[3], fmaf(e4.z, mine_u[2], fmaf(e4.y, mine_u[1], fmaf(e4.x, mine_u[0], mine))));
+      // (tokens behind this lane's own are left out, not taken times zero: theirs may be no numbers)
+      float o = fmaf(e4.x, mine_u[0], mine);
+      if (own_t > 0) o = fmaf(e4.y, mine_u[1], o);
+      if (own_t > 1) o = fmaf(e4.z, mine_u[2], o);
+      if (own_t > 2) o = fmaf(e4.w, mine_u[3], o);
+      if (own >= DC_T * NC && (s & 1) == 0 && own_c < cols && own_t < there)
+        out[(size_t)(r0 + (run * RUN + c) * DC_T + own_t) * H * dv + (size_t)h * dv + col0 + at + own_c] = o;
       ch = next;
     }
     __syncthreads();  // the buffer is free again
@@ -904,7 +916,7 @@ CUCA_API int cuca_delta_scan(float* qkv, int ld, float* a_raw, int ld_a, const f
     using C = decltype(split);
     return launch_scan<C>("delta_scan", delta_scan_kernel<C>, 3 * C::DP + ((C::PB + 4) & ~3), H, n_seqs, dv, stream,
                           (const float*)qkv, ld, (const float*)a_raw, ld_a, (const float*)b_raw, ld_b, b_col, state, out,
-                          req_row0, req_count, slots, H, G, d, dv, wide);
+                          req_row0, req_count, slots, H, G, d, dv, wide, 0x7fffffff);
   });
 }
 
@@ -912,16 +924,19 @@ CUCA_API int cuca_delta_scan(float* qkv, int ld, float* a_raw, int ld_a, const f
 // n_rows / 4 + n_seqs + 1 such fours in a step.
 CUCA_API int cuca_delta_chunk_words() { return DC_WORDS; }
 
-// The same, long portions in chunks of four tokens (see there); d a multiple of 4 up to 128, everything 16-byte aligned.
-// max_count: the longest portion. chunks: scratch.
+// The same, requests that bring `from` tokens or more in chunks of four tokens (see there), the others token by token; d a
+// multiple of 4 up to 128, everything 16-byte aligned. min_count, max_count: the shortest and the longest portion (at least
+// `from`). chunks: scratch.
 CUCA_API int cuca_delta_scan_chunked(float* qkv, int ld, float* a_raw, int ld_a, const float* dt_bias, const float* a_log,
                                      float* b_raw, int ld_b, int b_col, float* state, float* out, float* chunks,
                                      const int* seq_of_row, const int* req_row0, const int* req_count, const int* slots,
-                                     int n_rows, int n_seqs, int max_count, int H, int G, int d, int dv, cudaStream_t stream) {
+                                     int n_rows, int n_seqs, int from, int min_count, int max_count, int H, int G, int d, int dv,
+                                     cudaStream_t stream) {
   if (n_seqs == 0 || n_rows == 0) return 0;
   CUCA_REQUIRE(H > 0 && G > 0 && H % G == 0 && d > 0 && dv > 0, "delta_scan: bad sizes heads=%d key heads=%d dim=%d vdim=%d",
                H, G, d, dv);
   CUCA_REQUIRE(n_seqs <= 65535 && H <= 256, "delta_scan: %d requests or %d heads exceed the launch limits", n_seqs, H);
+  CUCA_REQUIRE(from > 0 && max_count >= from, "delta_scan: no portion of %d tokens (the longest: %d)", from, max_count);
   CUCA_REQUIRE(d <= DC_D && d % 4 == 0 && ld % 4 == 0 && ld_a % 4 == 0 &&
                    (((uintptr_t)qkv | (uintptr_t)a_raw | (uintptr_t)state | (uintptr_t)chunks) & 15) == 0,
                "delta_scan: the chunked form does not take %d key channels, row strides %d and %d or an unaligned operand", d,
@@ -931,11 +946,18 @@ CUCA_API int cuca_delta_scan_chunked(float* qkv, int ld, float* a_raw, int ld_a,
   CUCA_CHECK_LAUNCH("delta_prepare");
   cuca_launch(delta_chunk_prepare_kernel, dim3((max_count + DC_T - 1) / DC_T, n_seqs, (H + 7) / 8), dim3(256), 0, stream, true,
               (const float*)qkv, ld, (const float*)a_raw, ld_a, (const float*)b_raw, ld_b, b_col, chunks, req_row0, req_count,
-              slots, H, G, d);
+              slots, H, G, d, from);
   CUCA_CHECK_LAUNCH("delta_chunk_prepare");
-  return launch_blocks("delta_chunk_scan", delta_chunk_scan_kernel, dim3(H, n_seqs, (dv + 15) / 16), 256,
-                       2 * 4 * (DC_WORDS + DC_T * 16) * 4, stream, (const float*)qkv, ld, (const float*)chunks, state, out,
-                       req_row0, req_count, slots, H, G, d, dv);
+  const int rc = launch_blocks("delta_chunk_scan", delta_chunk_scan_kernel, dim3(H, n_seqs, (dv + 15) / 16), 256,
+                               2 * 4 * (DC_WORDS + DC_T * 16) * 4, stream, (const float*)qkv, ld, (const float*)chunks, state,
+                               out, req_row0, req_count, slots, H, G, d, dv, from);
+  if (rc || min_count >= from) return rc;
+  return with_split(d, [&](auto split) {
+    using C = decltype(split);
+    return launch_scan<C>("delta_scan", delta_scan_kernel<C>, 3 * C::DP + ((C::PB + 4) & ~3), H, n_seqs, dv, stream,
+                          (const float*)qkv, ld, (const float*)a_raw, ld_a, (const float*)b_raw, ld_b, b_col, state, out,
+                          req_row0, req_count, slots, H, G, d, dv, 1, from);
+  });
 }
 
 // The two gate columns of proj are rewritten in place by the preparing kernel (see there), then scanned.

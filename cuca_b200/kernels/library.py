@@ -105,7 +105,8 @@ _SIGNATURES = {
     "cuca_matrix_state_max_dim": [],
     "cuca_delta_scan": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "cuca_delta_chunk_words": [],
-    "cuca_delta_scan_chunked": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "cuca_delta_scan_chunked": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I,
+                                _P],
     "cuca_mlstm_scan": [_P, _I, _I, _I, _I, _I, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "cuca_head_norm_gate": [_P, _P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _F, _P],
     "cuca_moe_max_experts": [],

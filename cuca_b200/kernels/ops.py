@@ -1146,26 +1146,36 @@ def pair_norm_add(x, a, b, wa, wb, c: float, eps: float, store: bool = False) ->
 MATRIX_STATE_MAX_DIM = 1024  # `cuca_matrix_state_max_dim` says the same
 
 
-DELTA_CHUNKED_FROM = 32  # tokens of a step's longest portion (below, the extra launch costs more than it saves)
+# The delta rule four tokens at a time: for requests that bring this many tokens of a step (below, the extra launch costs more
+# than it saves), where the heads have so few value columns together that a prompt is bound by one token's latency. Token by
+# token, four at a time, in us: 1,501 tokens, 16 heads of 128 x 128 421, 303; 32 heads 522, 497; 64 heads 790, 967; 16 heads
+# of 64 x 64 366, 293. (Several prompts side by side are no reason either way: a request's rounding is not its company's.)
+DELTA_CHUNKED_FROM = 64
+
+
+def delta_chunked(H: int, d: int, dv: int) -> bool:
+    return d <= 128 and d % 4 == 0 and H * dv <= (4096 if d > 64 else 2048)
 
 
 def delta_scan(qkv, a_raw, dt_bias, a_log, b_src, b_col, state, out, step, H, G, d, dv, chunks: bool = False) -> None:
     """The delta rule with a decay per key channel along every request's rows (see `parts/recurrent.py:GatedDelta`).
     `qkv`, `a_raw` and column `b_col`.. of `b_src` hold pre-activations and are rewritten in place (unit vectors,
     decays, the write gate) before the scan. Token by token in order; with `chunks` (a caller whose bits may depend on how
-    a prompt was cut) a step with a long portion takes four tokens at a time."""
+    a prompt was cut) requests with a long portion take four tokens at a time, the step's other requests do not."""
     _cuda(qkv, a_raw, dt_bias, a_log, b_src, state, out)
     counts = step.host.get("counts") if chunks and step.static_max_len is None else None
-    if (counts and max(counts) >= DELTA_CHUNKED_FROM and d <= 128 and d % 4 == 0 and qkv.stride(0) % 4 == 0
+    if (counts and max(counts) >= DELTA_CHUNKED_FROM and delta_chunked(H, d, dv) and qkv.stride(0) % 4 == 0
             and a_raw.stride(0) % 4 == 0 and not (qkv.data_ptr() | a_raw.data_ptr() | state.data_ptr()) & 15):
         rows, lib = qkv.shape[0], library.load()
+        short = min(c for c in counts if c > 0)
         scratch = torch.empty((rows // 4 + step.n_seqs + 1) * H * int(lib.cuca_delta_chunk_words()), dtype=torch.float32,
                               device=qkv.device)
         library.check(lib.cuca_delta_scan_chunked(
             _p(qkv), qkv.stride(0), _p(a_raw), a_raw.stride(0), _p(dt_bias), _p(a_log), _p(b_src), b_src.stride(0),
             int(b_col), _p(state), _p(out), _p(scratch), _p(step.seq_of_row), _p(step.req_row0), _p(step.req_count),
-            _p(step.slots), rows, step.n_seqs, max(counts), H, G, d, dv, _stream()), "delta_scan_chunked")
-        library.launches += 2
+            _p(step.slots), rows, step.n_seqs, DELTA_CHUNKED_FROM, short, max(counts), H, G, d, dv, _stream()),
+            "delta_scan_chunked")
+        library.launches += 2 if short >= DELTA_CHUNKED_FROM else 3
         return
     library.check(library.load().cuca_delta_scan(
         _p(qkv), qkv.stride(0), _p(a_raw), a_raw.stride(0), _p(dt_bias), _p(a_log), _p(b_src), b_src.stride(0), int(b_col),

@@ -202,6 +202,59 @@ def test_scans_of_two_threads_with_grids_of_their_own(rt32):
     assert not errors, errors
 
 
+@pytest.mark.parametrize("H, G, d, dv", [(3, 3, 128, 128), (4, 2, 40, 8), (9, 3, 64, 150)])
+@pytest.mark.parametrize("counts", [[64], [1, 63, 70, 4, 2], [100, 0, 65], [67, 130, 1]])
+def test_delta_rule_goes_four_tokens_at_a_time_by_request(rt32, H, G, d, dv, counts):
+    """Which requests of a step take four tokens at a time depends on their own tokens alone: the launches say that the form
+    ran, every request's outputs and state are the same bits as in a step of its own, and token by token they are close. A
+    token that is no number leaves those before it as they are, in its chunk too, and its request's company."""
+    from cuca_b200.kernels import library, ops
+    dev = rt32.device
+    g = torch.Generator(device=dev).manual_seed(sum(counts) + d)
+    rows, C4 = sum(counts), -(-(2 * G * d + H * dv) // 4) * 4
+    rand = lambda *shape: torch.randn(*shape, device=dev, generator=g)  # noqa: E731
+    qkv, a, b, dt, al, state = rand(rows, C4), rand(rows, H * d), rand(rows, H), rand(H * d), rand(H), rand(len(counts), H, dv, d)
+    first = np.cumsum([0] + counts[:-1]).tolist()
+
+    def run(take, chunks=True, spoil=None):
+        """Outputs and states of the requests `take` in a step of theirs."""
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)  # noqa: E731
+        n = [counts[i] for i in take]
+        step = types.SimpleNamespace(host={"counts": n}, static_max_len=None, n_seqs=len(n), slots=i32(take),
+                                     seq_of_row=i32([i for i in take for _ in range(counts[i])]),
+                                     req_row0=i32(np.cumsum([0] + n[:-1]).tolist()), req_count=i32(n))
+        at = torch.cat([torch.arange(first[i], first[i] + counts[i], device=dev) for i in take])
+        x = qkv.clone()
+        if spoil is not None:
+            x[spoil, 2 * G * d:] = float("nan")
+        S, out = state.clone(), torch.full((len(at), H * dv), 7.0, device=dev)
+        before = library.launches
+        ops.delta_scan(x[at], a[at], dt, al, b[at], 0, S, out, step, H, G, d, dv, chunks=chunks)
+        launched = library.launches - before
+        return dict(zip(take, out.split(n))), S, launched
+
+    order = list(range(len(counts)))
+    out, S, launched = run(order)
+    long = [c for c in counts if c >= 64]
+    assert launched == (2 if not long else 3 if min(c for c in counts if c) >= 64 else 4)
+    slow, slow_S, launched = run(order, chunks=False)
+    assert launched == 2
+    for i in order:
+        if counts[i] == 0:
+            continue
+        alone, alone_S, _ = run([i])
+        assert torch.equal(alone[i], out[i]) and torch.equal(alone_S[i], S[i]), i
+        assert torch.equal(out[i], slow[i]) == (counts[i] < 64) and torch.allclose(out[i], slow[i], atol=1e-4, rtol=1e-4), i
+    assert torch.allclose(S, slow_S, atol=1e-4, rtol=1e-4)
+    for i in order:
+        for bad in {counts[i] - 1, counts[i] // 2, counts[i] // 2 + 1} & set(range(counts[i])):
+            got, got_S, _ = run(order, spoil=first[i] + bad)
+            assert torch.equal(got[i][:bad], out[i][:bad]) and bool(got[i][bad:].isnan().all()), (i, bad)
+            for j in order:
+                if j != i:
+                    assert torch.equal(got[j], out[j]) and torch.equal(got_S[j], S[j]), (i, j)
+
+
 @pytest.mark.parametrize("right", [dict(r_heads=3, r_dim=12, r_vdim=20, cap=6.0), dict(r_heads=1, r_dim=96, r_vdim=40, cap=15.0),
                                    dict(r_heads=2, r_dim=5, r_vdim=130, cap=1.5), dict(r_heads=2, r_dim=260, r_vdim=3, cap=30.0)])
 def test_matrix_memory_alone_whole_and_cut(rt32, right):
