@@ -89,12 +89,12 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
   load_rows<C>(S, st, s, d, cols, wide);
   // what no copy writes: channels from d on (q = k = 0, g = 1) and the values of columns from dv on
   {
-    const int spare = DP - d, fill = 3 * spare + PB;
-    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
+    const int spare = DP - d, there = min(PB, dv - col0), fill = 3 * spare + PB - there;
+    for (int e = threadIdx.x; e < (n < TC ? n : 2 * TC) * fill; e += 128) {
       const int t = e / fill, w = e % fill;
       float* tok = sm + t * PER;
       if (w < 3 * spare) tok[(w / spare) * DP + d + w % spare] = w / spare == 2 ? 1.f : 0.f;
-      else tok[3 * DP + (w - 3 * spare)] = 0.f;
+      else tok[3 * DP + there + (w - 3 * spare)] = 0.f;
     }
   }
   __syncthreads();
@@ -570,12 +570,12 @@ forget_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int f_col,
   load_rows<C>(S, st, s, d, cols, wide);
   // what no copy writes: channels from d on (q = 0, f = 1, k = 0) and the values of columns from dv on
   {
-    const int spare = DP - d, fill = 2 * spare + PB;
-    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
+    const int spare = DP - d, there = min(PB, dv - col0), fill = 2 * spare + PB - there;
+    for (int e = threadIdx.x; e < (n < TC ? n : 2 * TC) * fill; e += 128) {
       const int t = e / fill, w = e % fill;
       float* tok = sm + t * PER;
       if (w < 2 * spare) tok[(w / spare) * DP + d + w % spare] = (w / spare == 1 && !RET) ? 1.f : 0.f;
-      else tok[2 * DP + (w - 2 * spare)] = 0.f;
+      else tok[2 * DP + there + (w - 2 * spare)] = 0.f;
     }
   }
   __syncthreads();
@@ -695,12 +695,12 @@ mlstm_scan_kernel(const float* __restrict__ proj, int ld, int q_col, int k_col, 
   f32x2(&Z)[PAIRS] = Zs[0];
   float m = mx[(size_t)slot * H + h];
   {
-    const int spare = DP - d, fill = 2 * spare + PB;
-    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
+    const int spare = DP - d, there = min(PB, dv - col0), fill = 2 * spare + PB - there;
+    for (int e = threadIdx.x; e < (n < TC ? n : 2 * TC) * fill; e += 128) {
       const int t = e / fill, w = e % fill;
       float* tok = sm + t * PER;
       if (w < 2 * spare) tok[(w / spare) * DP + d + w % spare] = 0.f;
-      else tok[2 * DP + (w - 2 * spare)] = 0.f;
+      else tok[2 * DP + there + (w - 2 * spare)] = 0.f;
     }
   }
   __syncthreads();

@@ -212,12 +212,12 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
   const float bias = dt_bias[h], D = d_skip[h];
   // what no copy writes: rows from N on (B = C = 0) and the values of columns from P on
   {
-    const int spare = DP - N, fill = 2 * spare + PB;
-    for (int e = threadIdx.x; e < 2 * TC * fill; e += 128) {
+    const int spare = DP - N, there = min(PB, P - col0), fill = 2 * spare + PB - there;
+    for (int e = threadIdx.x; e < (n < TC ? n : 2 * TC) * fill; e += 128) {
       const int t = e / fill, w = e % fill;
       float* tok = sm + t * PER;
       if (w < 2 * spare) tok[(w / spare) * DP + N + w % spare] = 0.f;
-      else tok[2 * DP + (w - 2 * spare)] = 0.f;
+      else tok[2 * DP + there + (w - 2 * spare)] = 0.f;
     }
   }
   __syncthreads();
@@ -430,8 +430,12 @@ CUCA_API int cuca_ssm_scan(const float* xbc, const float* dt_raw, int ld_dt, int
     return launch_scan<C>("ssm_scan", ssm_scan_kernel<C>, 2 * C::DP + ((C::PB + 4) & ~3), H, n_seqs, P, stream, xbc, dt_raw,
                           ld_dt, dt_col, dt_bias, a_log, d_skip, state, y, req_row0, req_count, slots, H, P, N, G, wide);
   };
-  if (N <= 32) return go(Split<4, 8, 4>());
-  if (N <= 64) return go(Split<8, 8, 4>());
+  // Few state values a column: threads of four rows, so that a block's columns are no more than a head has (64). Measured
+  // with eight and four rows a thread, us: 80 heads of 64 x 16, 1,501 tokens 365, 205, 256 requests of a token 77, 48; 24
+  // heads of 64 x 64, 1,501 tokens 344, 197, 64 prompts of 40 52, 58 (as at 64 x 128: 249, 296, so eight rows stay there).
+  if (N <= 16) return go(Split<4, 4, 2>());
+  if (N <= 32) return go(Split<8, 4, 4>());
+  if (N <= 64) return go(Split<16, 4, 4>());
   if (N <= 128) return go(Split<16, 8, 4>());
   if (N <= 256) return go(Split<32, 8, 4>());
   if (N <= 512) return go(Split<32, 16, 4>());

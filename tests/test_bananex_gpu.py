@@ -146,6 +146,35 @@ def _load(part, ws, dev):
     part.load(lambda n: torch.tensor(ws[n], dtype=torch.float32, device=dev))
 
 
+@pytest.mark.parametrize("P, N", [(64, 4), (64, 16), (70, 17), (64, 32), (20, 33), (64, 64), (33, 65), (8, 130), (130, 16)])
+def test_state_scan_alone(rt32, P, N):
+    """The state-space scan over every split of the state and its edges, single tokens beside portions longer than a run of
+    staged tokens, from states that are not empty, against the recurrence in 64 bits; slots of no request stay."""
+    from cuca_b200.kernels import ops
+    dev, H, G = rt32.device, 4, 2
+    g = torch.Generator(device=dev).manual_seed(P * N)
+    counts, slots = [1, 40, 5, 17, 16], [3, 0, 5, 1, 2]
+    rows = sum(counts)
+    xbc = torch.randn(rows, H * P + 2 * G * N, device=dev, generator=g)
+    proj = torch.randn(rows, H + 3, device=dev, generator=g)
+    bias, a_log, skip = (torch.randn(H, device=dev, generator=g) for _ in range(3))
+    state = torch.randn(6, H, P, N, device=dev, generator=g)
+    got, y = state.clone(), torch.full((rows, H * P), 7.0, device=dev)
+    ops.ssm_scan(xbc, proj, 2, bias, a_log, skip, got, y, _step(dev, [(0, n) for n in counts], slots), H, P, N, G)
+    S, want, r = state.double(), torch.empty(rows, H, P, device=dev, dtype=torch.float64), 0
+    for n, slot in zip(counts, slots):
+        for _ in range(n):
+            x = xbc[r, :H * P].double().view(H, P)
+            B, C = (xbc[r, H * P + i * G * N:][:G * N].double().view(G, N).repeat_interleave(H // G, 0) for i in (0, 1))
+            dt = torch.nn.functional.softplus(proj[r, 2:2 + H].double() + bias.double(), threshold=60)
+            S[slot] = torch.exp(-torch.exp(a_log.double()) * dt)[:, None, None] * S[slot] + (dt[:, None] * x)[:, :, None] * B[:, None, :]
+            want[r] = (S[slot] * C[:, None, :]).sum(-1) + skip.double()[:, None] * x
+            r += 1
+    assert (y.view_as(want).double() - want).abs().max() < 2e-5 * want.abs().max()
+    assert (got.double() - S).abs().max() < 2e-5 * S.abs().max()
+    assert torch.equal(got[4], state[4])
+
+
 @pytest.mark.parametrize("inner", [48, 130])
 def test_mingru_alone_whole_and_cut(rt32, inner):
     from cuca_b200.parts.recurrent import MinGRU
