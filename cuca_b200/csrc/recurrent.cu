@@ -99,61 +99,16 @@ __global__ void mingru_chunked_kernel(const float* __restrict__ zxg, float* __re
 }
 
 // in: 32-bit rows of stride ld_in, channel c at column col0 + c. kept: [slots, taps - 1, C] the inputs before the
-// request's first row of this step (zeros for a new request). The first blocks y take CONV_ROWS rows each, those of them
-// that have taps - 1 rows of their own request before them in this step; the blocks y behind them take one request each:
-// its first taps - 1 rows and then its new kept inputs (only that block touches them).
-// TAPS: taps known at compile time (a thread then reads every input of its rows once, all of them in flight together:
-// 2,048 rows of 4,352 channels, 4 taps, 77 us with a row a thread), or 0.
-constexpr int CONV_ROWS = 16;
-template <typename TW, int TAPS>
-__global__ void causal_conv_kernel(const float* __restrict__ in, int ld_in, int col0, const TW* __restrict__ w,
-                                   const TW* __restrict__ bias, float* __restrict__ kept, float* __restrict__ out,
-                                   const int* __restrict__ seq_of_row, const int* __restrict__ req_row0,
-                                   const int* __restrict__ req_count, const int* __restrict__ slots, int n_rows,
-                                   int C, int taps) {
-  pdl_trigger();
-  pdl_wait();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  const int row_blocks = (n_rows + CONV_ROWS - 1) / CONV_ROWS;
-  const int back = (TAPS ? TAPS : taps) - 1;
-  const TW* wc = w + (size_t)c * (back + 1);
-  const float b0 = bias ? to_f32(bias[c]) : 0.f;
-  if ((int)blockIdx.y < row_blocks) {
-    const int r0 = blockIdx.y * CONV_ROWS, r1 = min(n_rows, r0 + CONV_ROWS);
-    auto whole = [&](int b) {  // whether row b has `back` rows of its request before it
-      const int seq = b < r1 ? seq_of_row[b] : -1;
-      return seq >= 0 && b >= back && (back == 0 || seq_of_row[b - back] == seq);
-    };
-    if (TAPS) {
-      float taps_w[TAPS ? TAPS : 1], x[CONV_ROWS + (TAPS ? TAPS : 1) - 1];
-#pragma unroll
-      for (int k = 0; k < TAPS; ++k) taps_w[k] = to_f32(wc[k]);
-#pragma unroll
-      for (int i = 0; i < CONV_ROWS + TAPS - 1; ++i) {
-        const int b = r0 - (TAPS - 1) + i;
-        x[i] = b >= 0 && b < r1 ? in[(size_t)b * ld_in + col0 + c] : 0.f;
-      }
-#pragma unroll
-      for (int i = 0; i < CONV_ROWS; ++i) {
-        if (!whole(r0 + i)) continue;
-        float acc = b0;
-#pragma unroll
-        for (int k = 0; k < TAPS; ++k) acc = fmaf(taps_w[k], x[i + k], acc);
-        out[(size_t)(r0 + i) * C + c] = siluf_(acc);
-      }
-    } else {
-      for (int b = r0; b < r1; ++b) {
-        if (!whole(b)) continue;
-        float acc = b0;
-        for (int k = 0; k <= back; ++k) acc = fmaf(to_f32(wc[k]), in[(size_t)(b - back + k) * ld_in + col0 + c], acc);
-        out[(size_t)b * C + c] = siluf_(acc);
-      }
-    }
-    return;
-  }
+// request's first row of this step (zeros for a new request). Rows that have taps - 1 rows of their own request before
+// them in this step are plain rows; a request's first taps - 1 rows and then its new kept inputs are one block's work
+// (only that block touches them): channel c of request q.
+template <typename TW>
+__device__ __forceinline__ void conv_request(const float* __restrict__ in, int ld_in, int col0, const TW* __restrict__ wc, float b0,
+                                             float* __restrict__ kept, float* __restrict__ out, const int* __restrict__ req_row0,
+                                             const int* __restrict__ req_count, const int* __restrict__ slots, int C, int taps,
+                                             int c, int q) {
+  const int back = taps - 1;
   if (back == 0) return;  // a one-tap convolution keeps nothing and every row was a plain row
-  const int q = blockIdx.y - row_blocks;
   const int slot = slots[q], n = req_count[q], r0 = req_row0[q];
   if (slot < 0 || n <= 0) return;
   float* keep = kept + (size_t)slot * back * C;
@@ -172,6 +127,86 @@ __global__ void causal_conv_kernel(const float* __restrict__ in, int ld_in, int 
   for (int k = 0; k < back; ++k) {
     const float v = val(n - back + k);
     keep[(size_t)k * C + c] = v;
+  }
+}
+
+// A row a thread: blocks y < n_rows take a row each, blocks y >= n_rows a request each.
+template <typename TW>
+__global__ void causal_conv_kernel(const float* __restrict__ in, int ld_in, int col0, const TW* __restrict__ w,
+                                   const TW* __restrict__ bias, float* __restrict__ kept, float* __restrict__ out,
+                                   const int* __restrict__ seq_of_row, const int* __restrict__ req_row0,
+                                   const int* __restrict__ req_count, const int* __restrict__ slots, int n_rows,
+                                   int C, int taps) {
+  pdl_trigger();
+  pdl_wait();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= C) return;
+  const int b = blockIdx.y;
+  const int back = taps - 1;
+  const TW* wc = w + (size_t)c * taps;
+  const float b0 = bias ? to_f32(bias[c]) : 0.f;
+  if (b < n_rows) {
+    const int seq = seq_of_row[b];
+    if (seq < 0 || b < back || (back > 0 && seq_of_row[b - back] != seq)) return;
+    float acc = b0;
+    for (int k = 0; k < taps; ++k)
+      acc = fmaf(to_f32(wc[k]), in[(size_t)(b - back + k) * ld_in + col0 + c], acc);
+    out[(size_t)b * C + c] = siluf_(acc);
+    return;
+  }
+  conv_request(in, ld_in, col0, wc, b0, kept, out, req_row0, req_count, slots, C, taps, c, b - n_rows);
+}
+
+// CONV_ROWS rows a thread. TAPS: taps known at compile time (a thread then reads every input of its rows once, all of them
+// in flight together), or 0.
+constexpr int CONV_ROWS = 16;
+template <typename TW, int TAPS>
+__global__ void causal_conv_many_kernel(const float* __restrict__ in, int ld_in, int col0, const TW* __restrict__ w,
+                                        const TW* __restrict__ bias, float* __restrict__ kept, float* __restrict__ out,
+                                        const int* __restrict__ seq_of_row, const int* __restrict__ req_row0,
+                                        const int* __restrict__ req_count, const int* __restrict__ slots, int n_rows,
+                                        int C, int taps) {
+  pdl_trigger();
+  pdl_wait();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= C) return;
+  const int row_blocks = (n_rows + CONV_ROWS - 1) / CONV_ROWS;
+  const int back = (TAPS ? TAPS : taps) - 1;
+  const TW* wc = w + (size_t)c * (back + 1);
+  const float b0 = bias ? to_f32(bias[c]) : 0.f;
+  if ((int)blockIdx.y >= row_blocks) {
+    conv_request(in, ld_in, col0, wc, b0, kept, out, req_row0, req_count, slots, C, taps, c, (int)blockIdx.y - row_blocks);
+    return;
+  }
+  const int r0 = blockIdx.y * CONV_ROWS, r1 = min(n_rows, r0 + CONV_ROWS);
+  auto whole = [&](int b) {  // whether row b has `back` rows of its request before it
+    const int seq = b < r1 ? seq_of_row[b] : -1;
+    return seq >= 0 && b >= back && (back == 0 || seq_of_row[b - back] == seq);
+  };
+  if (TAPS) {
+    float taps_w[TAPS ? TAPS : 1], x[CONV_ROWS + (TAPS ? TAPS : 1) - 1];
+#pragma unroll
+    for (int k = 0; k < TAPS; ++k) taps_w[k] = to_f32(wc[k]);
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS + TAPS - 1; ++i) {
+      const int b = r0 - (TAPS - 1) + i;
+      x[i] = b >= 0 && b < r1 ? in[(size_t)b * ld_in + col0 + c] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS; ++i) {
+      if (!whole(r0 + i)) continue;
+      float acc = b0;
+#pragma unroll
+      for (int k = 0; k < TAPS; ++k) acc = fmaf(taps_w[k], x[i + k], acc);
+      out[(size_t)(r0 + i) * C + c] = siluf_(acc);
+    }
+  } else {
+    for (int b = r0; b < r1; ++b) {
+      if (!whole(b)) continue;
+      float acc = b0;
+      for (int k = 0; k <= back; ++k) acc = fmaf(to_f32(wc[k]), in[(size_t)(b - back + k) * ld_in + col0 + c], acc);
+      out[(size_t)b * C + c] = siluf_(acc);
+    }
   }
 }
 
@@ -399,17 +434,26 @@ CUCA_API int cuca_causal_conv(const float* in, int ld_in, int col0, const void* 
   if (n_rows == 0) return 0;
   CUCA_REQUIRE(C > 0 && taps >= 1, "causal_conv: bad sizes channels=%d taps=%d", C, taps);
   CUCA_REQUIRE(n_rows + n_seqs <= 65535, "causal_conv: %d rows in one step exceed the launch limit", n_rows);
-  const dim3 grid((C + 127) / 128, (n_rows + CONV_ROWS - 1) / CONV_ROWS + n_seqs);
-#define CONV(TW, TAPS)                                                                                                \
-  cuca_launch(causal_conv_kernel<TW, TAPS>, grid, dim3(128), 0, stream, true, in, ld_in, col0, (const TW*)w,          \
-              (const TW*)bias, kept, out, seq_of_row, req_row0, req_count, slots, n_rows, C, taps)
-  if (w_dtype == CUCA_F32) {
-    if (taps == 4) CONV(float, 4); else CONV(float, 0);
-  } else if (w_dtype == CUCA_BF16) {
-    if (taps == 4) CONV(__nv_bfloat16, 4); else CONV(__nv_bfloat16, 0);
-  } else {
-    CUCA_REQUIRE(false, "causal_conv: unknown dtype %d", w_dtype);
-  }
+  // 16 rows a thread read every input once, but pay only where their blocks fill the GPU: measured with four taps, us a row a
+  // thread, 16 rows: 2,048 x 4,352 (4,352 blocks) 75, 22; 200 x 4,352 (442) 8.8, 5.7; 40 x 4,352 (102) 3.7, 4.2; 1,501 x 100
+  // (94) 3.3, 4.3; other numbers of taps (a loop, one load after the other): 1,501 x 4,352, three taps 53, 26; 2,400 x 768
+  // (900) 15.8, 17.5; 200 x 4,352 7.9, 9.7.
+  const long long blocks = (long long)((C + 127) / 128) * ((n_rows + CONV_ROWS - 1) / CONV_ROWS);
+  const bool many = blocks >= (taps == 4 ? 2 : 8) * cuca_device_sms();
+  const dim3 grid((C + 127) / 128, (many ? (n_rows + CONV_ROWS - 1) / CONV_ROWS : n_rows) + n_seqs);
+#define CONV(KERNEL, TW)                                                                                              \
+  cuca_launch(KERNEL, grid, dim3(128), 0, stream, true, in, ld_in, col0, (const TW*)w, (const TW*)bias, kept, out,    \
+              seq_of_row, req_row0, req_count, slots, n_rows, C, taps)
+#define CONV_OF(TW)                                                       \
+  do {                                                                    \
+    if (!many) CONV(causal_conv_kernel<TW>, TW);                          \
+    else if (taps == 4) CONV((causal_conv_many_kernel<TW, 4>), TW);       \
+    else CONV((causal_conv_many_kernel<TW, 0>), TW);                      \
+  } while (0)
+  if (w_dtype == CUCA_F32) CONV_OF(float);
+  else if (w_dtype == CUCA_BF16) CONV_OF(__nv_bfloat16);
+  else CUCA_REQUIRE(false, "causal_conv: unknown dtype %d", w_dtype);
+#undef CONV_OF
 #undef CONV
   CUCA_CHECK_LAUNCH("causal_conv");
   return 0;
@@ -441,7 +485,6 @@ CUCA_API int cuca_ssm_scan(const float* xbc, const float* dt_raw, int ld_dt, int
   if (N <= 512) return go(Split<32, 16, 4>());
   return go(Split<32, 32, 2>());
 }
-
 
 CUCA_API int cuca_gated_group_norm(const float* y, const float* z, int ld_z, const void* w, int w_dtype, void* out,
                                    int out_dtype, int n_rows, int inner, int parts, float eps, cudaStream_t stream) {

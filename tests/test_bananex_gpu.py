@@ -67,85 +67,6 @@ CUTS = [[1000], [1, 1, 1, 1, 1, 2, 3, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 
 
 
 # ------------------------------------------------------------------------------------------ mechanisms alone
-def test_norm_and_token_shift_alone(rt32):
-    from cuca_b200.kernels import ops
-    dev, E, eps = rt32.device, 52, 1e-5
-    rs = np.random.default_rng(0)
-    mix = rs.uniform(0, 1, E)
-    gain = 1.3
-    xs = [rs.normal(0, 2, (n, E)) for n in (23, 9)]
-    want = [pb.token_shift(pb.rms(x, eps) * gain, mix) for x in xs]
-    g = torch.tensor([gain], dtype=torch.float32, device=dev)
-    m = torch.tensor(mix, dtype=torch.float32, device=dev)
-    for cuts in ([CUTS[0], CUTS[0]], [CUTS[1], CUTS[2]], [CUTS[2], CUTS[1]]):
-        kept = torch.zeros(4, E, device=dev)
-        kept[0] = 7.0  # another request's row must stay as it is
-
-        def fwd(h, step):
-            out = torch.empty_like(h)
-            ops.norm_shift(h, g, eps, m, kept, out, step)
-            return out
-        got = _run_cut(dev, fwd, xs, cuts, [2, 3], E)
-        for a, b in zip(got, want):
-            assert np.abs(a - b).max() < 1e-5
-        assert torch.equal(kept[0].cpu(), torch.full((E,), 7.0))
-    # a vector gain through the same kernel
-    gv = rs.normal(1, 0.2, E)
-    kept = torch.zeros(4, E, device=dev)
-    out = torch.empty(23, E, device=dev)
-    ops.norm_shift(torch.tensor(xs[0], dtype=torch.float32, device=dev), torch.tensor(gv, dtype=torch.float32, device=dev),
-                   eps, m, kept, out, _step(dev, [(0, 23)], [1]))
-    assert np.abs(out.cpu().numpy() - pb.token_shift(pb.rms(xs[0], eps) * gv, mix)).max() < 1e-5
-
-
-def test_post_norm_add_alone(rt32):
-    from cuca_b200.kernels import ops
-    dev, E, eps = rt32.device, 70, 1e-6
-    rs = np.random.default_rng(1)
-    x, y = rs.normal(0, 1, (11, E)), rs.normal(0, 3, (11, E))
-    xd = torch.tensor(x, dtype=torch.float32, device=dev)
-    out = torch.empty(11, E, device=dev)
-    g1, g2 = torch.tensor([0.8], device=dev), torch.tensor([1.7], device=dev)
-    ops.post_norm_add(xd, torch.tensor(y, dtype=torch.float32, device=dev), g1, eps, gain2=g2, out=out)
-    nx = x + pb.rms(y, eps) * 0.8
-    assert np.abs(xd.cpu().numpy() - nx).max() < 1e-5
-    assert np.abs(out.cpu().numpy() - pb.rms(nx, eps) * 1.7).max() < 1e-5
-
-
-def _part(kind, cls, layer, rt, E, eps, prefix="l0.mix."):
-    from cuca_b200.config.bananex_config import BananexConfig
-    from cuca_b200.models.bananex import _mixer_spec
-    cfg = BananexConfig.from_json(bu.config([layer], width=E, eps=eps))
-    spec = _mixer_spec(cfg.layers[0], E, eps, prefix)
-    assert spec.kind == kind
-    return cls(spec, rt)
-
-
-def _weights_for(part, seed):
-    rs = np.random.default_rng(seed)
-    ws = {}
-    for name, need in part.tensors().items():
-        shape = tuple(need.shape)
-        if name.endswith("A_log"):
-            v = rs.uniform(-1.5, 1.0, shape)
-        elif name.endswith("dt_bias"):
-            v = rs.uniform(-2, 1, shape)
-        elif need.init == "ones" or name.endswith(".D"):
-            v = 1 + rs.normal(0, 0.3, shape)
-        elif len(shape) == 1:
-            v = rs.normal(0, 0.3, shape)
-        elif name.endswith(".conv"):
-            v = rs.normal(0, 0.5, shape)
-        else:
-            v = rs.normal(0, 1, shape) / np.sqrt(shape[-1])
-        ws[name] = np.asarray(v, dtype=np.float32).astype(np.float64)
-    return ws
-
-
-def _load(part, ws, dev):
-    part.load(lambda n: torch.tensor(ws[n], dtype=torch.float32, device=dev))
-
-
 @pytest.mark.parametrize("P, N", [(64, 4), (64, 16), (70, 17), (64, 32), (20, 33), (64, 64), (33, 65), (8, 130), (130, 16)])
 def test_state_scan_alone(rt32, P, N):
     """The state-space scan over every split of the state and its edges, single tokens beside portions longer than a run of
@@ -173,6 +94,38 @@ def test_state_scan_alone(rt32, P, N):
     assert (y.view_as(want).double() - want).abs().max() < 2e-5 * want.abs().max()
     assert (got.double() - S).abs().max() < 2e-5 * S.abs().max()
     assert torch.equal(got[4], state[4])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps, C, rows", [(4, 4800, 130), (4, 300, 1700), (3, 4800, 530), (6, 4736, 514), (1, 4800, 530)])
+def test_convolution_rows_are_the_same_bits_in_every_form(rt32, dtype, taps, C, rows):
+    """So many rows and channels that a thread takes 16 rows, beside the same rows a few at a time (a thread a row), of
+    requests whose borders lie anywhere; and against 64 bits."""
+    from cuca_b200.kernels import ops
+    dev = rt32.device
+    g = torch.Generator(device=dev).manual_seed(C + taps)
+    counts = [1, 2, 17, rows - 60, 3, 37]
+    src = torch.randn(rows, C + 5, device=dev, generator=g)
+    w, bias = (torch.randn(*s, device=dev, generator=g).to(dtype) for s in ((C, taps), (C,)))
+    kept = torch.randn(len(counts), max(1, taps - 1), C, device=dev, generator=g)
+
+    def run(portions, a, b, kept):
+        out = torch.full((b - a, C), 7.0, device=dev)
+        ops.causal_conv(src[a:b], 5, w, bias, kept, out, _step(dev, [(0, n) for _, n in portions], [s for s, _ in portions]))
+        return out
+
+    whole_kept = kept.clone()
+    whole = run(list(enumerate(counts)), 0, rows, whole_kept)
+    few_kept, a = kept.clone(), 0
+    for i, n in enumerate(counts):
+        pad = torch.cat([kept[i, :taps - 1], src[a:a + n, 5:]]).double()
+        want = torch.nn.functional.silu(bias.double() + sum(w[:, k].double() * pad[k:k + n] for k in range(taps)))
+        assert torch.allclose(whole[a:a + n].double(), want, atol=1e-5, rtol=1e-5)
+        for b in range(0, n, 10):
+            m = min(10, n - b)
+            assert torch.equal(run([(i, m)], a + b, a + b + m, few_kept), whole[a + b:a + b + m]), (i, b)
+        a += n
+    assert torch.equal(few_kept[:, :taps - 1], whole_kept[:, :taps - 1])
 
 
 @pytest.mark.parametrize("inner", [48, 130])
