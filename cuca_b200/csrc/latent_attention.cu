@@ -12,6 +12,8 @@
 #include "common.cuh"
 #include <math.h>
 
+int cuca_device_sms();
+
 namespace {
 
 // qkg: 32-bit rows of stride ld: [H x (dn + dr) queries | rank + dr down-projection | ...]. One block per row.
@@ -152,9 +154,9 @@ __device__ __forceinline__ void hl_mma(float (&d)[4], const uint32_t (&a)[4], ui
 
 // The same in tiles of 128 rows x 128 outputs, eight warps of 32 x 64, for operands that can be read 16 bytes at a time
 // (a's row and head strides multiples of 4, K of 8): the next K step's 16-byte loads are in flight while this one is
-// multiplied. What bounds it is the traffic: 2,048 rows of 16 heads, 128 -> 512, read 17 MB and write 75. The narrow form
-// took 88 us for that (element-wise loads, none in flight during the arithmetic) and 69 us for 512 -> 128, this one 42
-// and 44.
+// multiplied. What bounds it is the traffic: 2,048 rows of 16 heads, 128 -> 512, read 19 MB and write 67. The narrow form
+// takes 65 us for that (element-wise loads, none in flight during the arithmetic) and 61 us for 512 -> 128, this one 40
+// and 28.
 template <typename TO>
 __global__ void __launch_bounds__(256)
 head_linear_wide_kernel(const float* __restrict__ a, int lda, int a_head, const __nv_bfloat16* __restrict__ w,
@@ -240,16 +242,24 @@ head_linear_wide_kernel(const float* __restrict__ a, int lda, int a_head, const 
     for (int i = 0; i < 2; ++i) {
       const int row = t0 + wr + r * 16 + g + 8 * i;
       if (row >= T) continue;
+      TO* to = out + (size_t)row * ldo + (size_t)h * o_head;
+      const bool pairs = ((uintptr_t)to & (2 * sizeof(TO) - 1)) == 0;
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < 8; ++nt) {
+        const int n = n0 + wn + nt * 8 + 2 * t;
+        float v[2] = {acc[r][nt][2 * i], acc[r][nt][2 * i + 1]};
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int n = n0 + wn + nt * 8 + 2 * t + j;
-          if (n >= N) continue;
-          float v = acc[r][nt][2 * i + j];
-          if (gate) v *= 1.f / (1.f + expf(-gate[(size_t)row * ldg + (size_t)h * N + n]));
-          out[(size_t)row * ldo + (size_t)h * o_head + n] = from_f32<TO>(v);
+        for (int j = 0; j < 2; ++j)
+          if (gate && n + j < N) v[j] *= 1.f / (1.f + expf(-gate[(size_t)row * ldg + (size_t)h * N + n + j]));
+        if (pairs && n + 1 < N) {
+          struct alignas(2 * sizeof(TO)) Two { TO v[2]; };
+          *reinterpret_cast<Two*>(to + n) = Two{{from_f32<TO>(v[0]), from_f32<TO>(v[1])}};
+        } else {
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            if (n + j < N) to[n + j] = from_f32<TO>(v[j]);
         }
+      }
     }
 }
 
@@ -504,7 +514,12 @@ CUCA_API int cuca_head_linear(const float* a, int lda, int a_head, const void* w
   }
   dim3 grid((N + 63) / 64, (T + 63) / 64, H);
   CUCA_REQUIRE(grid.y <= 65535, "head_linear: %d rows exceed the launch limit", T);
-  if (w_dtype == CUCA_BF16 && lda % 4 == 0 && a_head % 4 == 0 && K % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0) {
+  // The wide tiles want three blocks of the narrow form a SM: with fewer, half as many blocks idle SMs. Both forms, us:
+  // 512 -> 128, 32 heads, 200 rows (256 narrow tiles) 20.6, 21.3; 16 heads, 700 rows (352) 21.1, 24.3; 512 rows of 32 heads
+  // (512) 29.9, 26.0; 128 -> 512, 16 heads, 160 rows (384) 8.2, 10.6; 200 rows (512) 11.4, 10.5; 2,048 rows (4,096) 65, 40.
+  // Up to 64 rows or outputs half of a wide tile is padding: 128 heads 128 -> 512, 48 rows (1,024) 17.7, 19.5.
+  const bool many = N > 64 && T > 64 && (long long)grid.x * grid.y * grid.z >= 3 * cuca_device_sms();
+  if (many && w_dtype == CUCA_BF16 && lda % 4 == 0 && a_head % 4 == 0 && K % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0) {
     const dim3 wide((N + 127) / 128, (T + 127) / 128, H);
     if (out_dtype == CUCA_F32)
       cuca_launch(head_linear_wide_kernel<float>, wide, dim3(256), 0, stream, true, a, lda, a_head,

@@ -128,6 +128,119 @@ def test_convolution_rows_are_the_same_bits_in_every_form(rt32, dtype, taps, C, 
     assert torch.equal(few_kept[:, :taps - 1], whole_kept[:, :taps - 1])
 
 
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H, N, K, T, o_pad", [(16, 512, 128, 300, 0), (40, 129, 40, 500, 3), (128, 100, 64, 130, 1)])
+def test_head_contraction_rows_are_the_same_bits_in_every_form(rt32, out_dtype, H, N, K, T, o_pad):
+    """So many rows that tiles of 128 are taken, beside the same rows 64 at a time (tiles of 64), with and without a gate, odd
+    numbers of outputs and output strides among them; and against 64 bits."""
+    from cuca_b200.kernels import ops
+    dev = rt32.device
+    g = torch.Generator(device=dev).manual_seed(N + T)
+    a = torch.randn(T, H * (K + 4), device=dev, generator=g)
+    w = torch.randn(H, N, K, device=dev, generator=g).to(torch.bfloat16)
+    gate = torch.randn(T, H * N, device=dev, generator=g)
+
+    def run(b, e, gate):
+        out = torch.zeros(e - b, H * (N + o_pad), device=dev, dtype=out_dtype)
+        ops.head_linear(a[b:e], a.stride(0), K + 4, w, out, out.stride(0), N + o_pad, e - b,
+                        gate=None if gate is None else gate[b:e], ldg=H * N)
+        return out
+
+    for gt in (None, gate):
+        whole = run(0, T, gt)
+        for b in range(0, T, 64):
+            e = min(T, b + 64)
+            if e - b > 16:  # (16 rows and fewer are summed by warps, in another order)
+                assert torch.equal(run(b, e, gt), whole[b:e]), b
+        want = torch.einsum("thk,hnk->thn", a.view(T, H, K + 4)[:, :, :K].to(torch.bfloat16).double(), w.double())
+        if gt is not None:
+            want = want * torch.sigmoid(gt.double().view(T, H, N))
+        got = whole.view(T, H, N + o_pad)
+        tol = 1e-5 if out_dtype == torch.float32 else 2.0 ** -8
+        assert torch.allclose(got[:, :, :N].double(), want, atol=tol * K ** 0.5, rtol=tol)
+        assert bool((got[:, :, N:] == 0).all())
+
+
+
+def test_norm_and_token_shift_alone(rt32):
+    from cuca_b200.kernels import ops
+    dev, E, eps = rt32.device, 52, 1e-5
+    rs = np.random.default_rng(0)
+    mix = rs.uniform(0, 1, E)
+    gain = 1.3
+    xs = [rs.normal(0, 2, (n, E)) for n in (23, 9)]
+    want = [pb.token_shift(pb.rms(x, eps) * gain, mix) for x in xs]
+    g = torch.tensor([gain], dtype=torch.float32, device=dev)
+    m = torch.tensor(mix, dtype=torch.float32, device=dev)
+    for cuts in ([CUTS[0], CUTS[0]], [CUTS[1], CUTS[2]], [CUTS[2], CUTS[1]]):
+        kept = torch.zeros(4, E, device=dev)
+        kept[0] = 7.0  # another request's row must stay as it is
+
+        def fwd(h, step):
+            out = torch.empty_like(h)
+            ops.norm_shift(h, g, eps, m, kept, out, step)
+            return out
+        got = _run_cut(dev, fwd, xs, cuts, [2, 3], E)
+        for a, b in zip(got, want):
+            assert np.abs(a - b).max() < 1e-5
+        assert torch.equal(kept[0].cpu(), torch.full((E,), 7.0))
+    # a vector gain through the same kernel
+    gv = rs.normal(1, 0.2, E)
+    kept = torch.zeros(4, E, device=dev)
+    out = torch.empty(23, E, device=dev)
+    ops.norm_shift(torch.tensor(xs[0], dtype=torch.float32, device=dev), torch.tensor(gv, dtype=torch.float32, device=dev),
+                   eps, m, kept, out, _step(dev, [(0, 23)], [1]))
+    assert np.abs(out.cpu().numpy() - pb.token_shift(pb.rms(xs[0], eps) * gv, mix)).max() < 1e-5
+
+
+def test_post_norm_add_alone(rt32):
+    from cuca_b200.kernels import ops
+    dev, E, eps = rt32.device, 70, 1e-6
+    rs = np.random.default_rng(1)
+    x, y = rs.normal(0, 1, (11, E)), rs.normal(0, 3, (11, E))
+    xd = torch.tensor(x, dtype=torch.float32, device=dev)
+    out = torch.empty(11, E, device=dev)
+    g1, g2 = torch.tensor([0.8], device=dev), torch.tensor([1.7], device=dev)
+    ops.post_norm_add(xd, torch.tensor(y, dtype=torch.float32, device=dev), g1, eps, gain2=g2, out=out)
+    nx = x + pb.rms(y, eps) * 0.8
+    assert np.abs(xd.cpu().numpy() - nx).max() < 1e-5
+    assert np.abs(out.cpu().numpy() - pb.rms(nx, eps) * 1.7).max() < 1e-5
+
+
+def _part(kind, cls, layer, rt, E, eps, prefix="l0.mix."):
+    from cuca_b200.config.bananex_config import BananexConfig
+    from cuca_b200.models.bananex import _mixer_spec
+    cfg = BananexConfig.from_json(bu.config([layer], width=E, eps=eps))
+    spec = _mixer_spec(cfg.layers[0], E, eps, prefix)
+    assert spec.kind == kind
+    return cls(spec, rt)
+
+
+def _weights_for(part, seed):
+    rs = np.random.default_rng(seed)
+    ws = {}
+    for name, need in part.tensors().items():
+        shape = tuple(need.shape)
+        if name.endswith("A_log"):
+            v = rs.uniform(-1.5, 1.0, shape)
+        elif name.endswith("dt_bias"):
+            v = rs.uniform(-2, 1, shape)
+        elif need.init == "ones" or name.endswith(".D"):
+            v = 1 + rs.normal(0, 0.3, shape)
+        elif len(shape) == 1:
+            v = rs.normal(0, 0.3, shape)
+        elif name.endswith(".conv"):
+            v = rs.normal(0, 0.5, shape)
+        else:
+            v = rs.normal(0, 1, shape) / np.sqrt(shape[-1])
+        ws[name] = np.asarray(v, dtype=np.float32).astype(np.float64)
+    return ws
+
+
+def _load(part, ws, dev):
+    part.load(lambda n: torch.tensor(ws[n], dtype=torch.float32, device=dev))
+
+
 @pytest.mark.parametrize("inner", [48, 130])
 def test_mingru_alone_whole_and_cut(rt32, inner):
     from cuca_b200.parts.recurrent import MinGRU
