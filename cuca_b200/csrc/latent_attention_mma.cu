@@ -16,6 +16,8 @@
 #include <math.h>
 #include <stdlib.h>
 
+int cuca_device_sms();
+
 namespace {
 
 typedef __nv_bfloat16 bf16;
@@ -52,8 +54,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // S = Q K^T of 16 rows and 16 keys over Dk values (a multiple of 16). A step's two MMAs wait for the step before and for
-// their own fragments: four steps' fragments are requested together and two sums taken in turn (2,048 tokens, 16 heads, a
-// latent of 512 + 64, window 1,024: 549 -> 520 us).
+// their own fragments. FOUR: four steps' fragments are requested together and two sums taken in turn (2,048 tokens, 16
+// heads, a latent of 512 + 64, window 1,024: 549 -> 520 us).
+template <bool FOUR>
 __device__ __forceinline__ void scores_of_16_keys(float (&s)[2][4], uint32_t q_addr, uint32_t k_addr, int Dk) {
   float part[2][2][4];
 #pragma unroll
@@ -63,7 +66,7 @@ __device__ __forceinline__ void scores_of_16_keys(float (&s)[2][4], uint32_t q_a
 #pragma unroll
       for (int j = 0; j < 4; ++j) part[h][i][j] = 0.f;
   int k0 = 0;
-  for (; k0 + 64 <= Dk; k0 += 64) {
+  for (; FOUR && k0 + 64 <= Dk; k0 += 64) {
     uint32_t a[4][4], b[4][4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -86,7 +89,7 @@ __device__ __forceinline__ void scores_of_16_keys(float (&s)[2][4], uint32_t q_a
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) s[i][j] = part[0][i][j] + part[1][i][j];
+    for (int j = 0; j < 4; ++j) s[i][j] = FOUR ? part[0][i][j] + part[1][i][j] : part[0][i][j];
 }
 
 struct Params {
@@ -115,7 +118,7 @@ struct Params {
 };
 
 // NT8: most 8-column output tiles a warp owns (rank / 4 / 8 of them are used)
-template <int NT8>
+template <int NT8, bool FOUR>
 __global__ void __launch_bounds__(128)
 latent_attention_mma_kernel(Params p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -217,7 +220,7 @@ latent_attention_mma_kernel(Params p) {
 
     // S for this warp's 16 keys
     float s[2][4];
-    scores_of_16_keys(s, qs_addr + (uint32_t)(a_row * RS + a_col) * 2, ks_addr + (uint32_t)((warp * 16 + b_key) * RS + b_col) * 2, Dk);
+    scores_of_16_keys<FOUR>(s, qs_addr + (uint32_t)(a_row * RS + a_col) * 2, ks_addr + (uint32_t)((warp * 16 + b_key) * RS + b_col) * 2, Dk);
     // scale and mask; s[nt][0..1]: row g, keys kbase + nt * 8 + 2 t + {0, 1}; s[nt][2..3]: row g + 8
     const int kbase = kt + warp * 16 + 2 * t;
     float mx[2] = {-INFINITY, -INFINITY};
@@ -445,7 +448,7 @@ latent_attention_pair_kernel(Params p) {
     const uint32_t kb = ks_addr + (uint32_t)(buf * KT * RS) * 2;
 
     float s[2][4];
-    scores_of_16_keys(s, qs_addr + (uint32_t)(a_row * RS + a_col) * 2, kb + (uint32_t)((warp * 16 + b_key) * RS + b_col) * 2, Dk);
+    scores_of_16_keys<true>(s, qs_addr + (uint32_t)(a_row * RS + a_col) * 2, kb + (uint32_t)((warp * 16 + b_key) * RS + b_col) * 2, Dk);
     const int kbase = kt + warp * 16 + 2 * t;
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -597,12 +600,12 @@ size_t smem_bytes(int Dk) {
   return (size_t)(16 + KT) * (Dk + PAD) * sizeof(bf16) + (size_t)16 * PS * sizeof(bf16) + 2 * 64 * sizeof(float);
 }
 
-template <int NT8>
-int launch(const Params& p, int n_groups, int head_blocks, cudaStream_t stream) {
+template <int NT8, bool FOUR>
+int launch_one(const Params& p, int n_groups, int head_blocks, cudaStream_t stream) {
   const size_t smem = smem_bytes(p.Dk);
   static size_t configured = 0;
   if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(latent_attention_mma_kernel<NT8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute((latent_attention_mma_kernel<NT8, FOUR>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) {
       cuca_set_error("latent_attention_mma: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
@@ -610,7 +613,7 @@ int launch(const Params& p, int n_groups, int head_blocks, cudaStream_t stream) 
     }
     configured = smem;
   }
-  cuca_launch(latent_attention_mma_kernel<NT8>, dim3(n_groups, head_blocks, p.n_splits), dim3(128), smem, stream,
+  cuca_launch((latent_attention_mma_kernel<NT8, FOUR>), dim3(n_groups, head_blocks, p.n_splits), dim3(128), smem, stream,
               true, p);
   return 0;
 }
@@ -618,6 +621,16 @@ int launch(const Params& p, int n_groups, int head_blocks, cudaStream_t stream) 
 size_t pair_smem_bytes(int Dk, int hg) {
   return (size_t)(hg * 16 + 2 * KT) * (Dk + PAD) * sizeof(bf16) + (size_t)hg * 16 * PS * sizeof(bf16) +
          (size_t)hg * 128 * sizeof(float);
+}
+
+// Four steps at a time over small latents where CTAs share SMs: 64 tokens of 300 keys, 16 heads (256 CTAs), us one step, four
+// at a time: 64 + 16 12.8, 10.6; 512 + 64 28.1, 29.7 (the outputs' registers leave no room). A CTA an SM: eight tokens of
+// 1,035 keys, 64 + 16 11.7, 12.1; 96 + 32, five heads 13.1, 13.9.
+template <int NT8>
+int launch(const Params& p, int n_groups, int head_blocks, cudaStream_t stream) {
+  if (NT8 < 16 && (long long)n_groups * head_blocks * p.n_splits > cuca_device_sms())
+    return launch_one<NT8, (NT8 < 16)>(p, n_groups, head_blocks, stream);
+  return launch_one<NT8, false>(p, n_groups, head_blocks, stream);
 }
 
 template <int NT8, int HG>
