@@ -5,11 +5,12 @@
 // the rest of the batch: the K products of a run of CHUNK in ascending order with
 // fused multiply-adds from zero, and the runs' sums in ascending order.
 //
-// Two forms. Up to FEW rows, and a few more over narrow outputs (`rows_kernel`): a block takes 16 weight rows and all of K and a thread one run of one
-// row for all tokens, so that the reading of the weights is what bounds it. Above (`tile_kernel`): register tiles of
-// 8 x 8 or 4 x 8 outputs a thread, bound by the multiply-adds (128 a clock and SM).
+// Two forms. Up to FEW rows, and a few more over narrow outputs (`rows_kernel`): a block takes 16 weight rows and all of K
+// and a thread one run of one row for all tokens, so that the reading of the weights is what bounds it. Above
+// (`tile_kernel`): register tiles of 8 x 8 or 4 x 8 outputs a thread, bound by the multiply-adds (128 a clock and SM).
 // Both read 16 bytes at a time with asynchronous copies where sizes and addresses allow it (32-bit operands,
-// K and the row stride multiples of 4); otherwise element by element, with the same arithmetic.
+// K and the row stride multiples of 4); otherwise through registers (the tile form two elements at a time where K, the row
+// stride and the addresses are even), with the same arithmetic.
 //
 // Measured on the Llama-3.2-1B widths in 32-bit: 4 rows, SwiGLU of 2 x 8192 x 2048 49 us (2.7 TB/s of weights), head of
 // 32,000 rows 82 us (3.2 TB/s); 700 rows, SwiGLU 1.34 ms (35 TFLOP/s). One form with 4 x 4 outputs a thread and
@@ -24,6 +25,8 @@
 #define EPI_RESIDUAL 1
 #define EPI_SWIGLU 2
 
+int cuca_device_sms();
+
 namespace {
 
 constexpr int CHUNK = 64;  // products of one run
@@ -36,6 +39,20 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool ok
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Two neighbouring elements from `src` on, of which `left` exist (zeros behind), and their values as floats; even: `src` is
+// aligned to two elements.
+__device__ __forceinline__ float2 load_two(const float* src, int left, bool even) {
+  if (even && left >= 2) return *reinterpret_cast<const float2*>(src);
+  return make_float2(left >= 1 ? src[0] : 0.f, left >= 2 ? src[1] : 0.f);
+}
+__device__ __forceinline__ uint32_t load_two(const __nv_bfloat16* src, int left, bool even) {
+  if (even && left >= 2) return *reinterpret_cast<const uint32_t*>(src);
+  const uint16_t* u = reinterpret_cast<const uint16_t*>(src);
+  return (left >= 1 ? u[0] : 0u) | (left >= 2 ? (uint32_t)u[1] << 16 : 0u);
+}
+__device__ __forceinline__ float2 to_f32x2(float2 t) { return t; }
+__device__ __forceinline__ float2 to_f32x2(uint32_t t) { return make_float2(__uint_as_float(t << 16), __uint_as_float(t & 0xffff0000u)); }
 
 // `v` (and for SwiGLU `u`): the sums of output (m, n)
 template <typename TI, typename TO, int EPI>
@@ -196,7 +213,7 @@ rows_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __rest
 // A block: BM tokens x BN weight rows (SwiGLU: BN / 2 gate rows and their up rows), K in steps of BK. Operands stay
 // K-major in shared memory, PITCH floats a row, and a thread reads four K at a time of its rows (BM / TM apart) and
 // columns (BN / 8 apart): neighbouring lanes read neighbouring rows, which PITCH spreads over all banks.
-template <int BM, int BN, int TM>
+template <int BM, int BN, int TM, bool VEC>
 struct Tile {
   static constexpr int BK = 32, PITCH = BK + 4, TN = 8;
   static constexpr int RT = BM / TM, CT = BN / TN;  // threads along rows, columns
@@ -204,14 +221,14 @@ struct Tile {
   static constexpr int STAGES = 3;
   static constexpr int STAGE = (BM + BN) * PITCH;  // floats
   static constexpr int SMEM = STAGES * STAGE * 4;
-  static constexpr int BLOCKS = BM == 128 ? 1 : 3;  // a SM
+  static constexpr int BLOCKS = BM == 128 ? 1 : VEC ? 3 : 2;  // a SM
 };
 
 template <typename TI, typename TO, int BM, int BN, int TM, int EPI, bool VEC>
-__global__ void __launch_bounds__((Tile<BM, BN, TM>::THREADS), (Tile<BM, BN, TM>::BLOCKS))
+__global__ void __launch_bounds__((Tile<BM, BN, TM, VEC>::THREADS), (Tile<BM, BN, TM, VEC>::BLOCKS))
 tile_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __restrict__ bias, TO* __restrict__ out, int M,
             int N, int K, int lda, int ldo) {
-  using C = Tile<BM, BN, TM>;
+  using C = Tile<BM, BN, TM, VEC>;
   constexpr bool DUAL = EPI == EPI_SWIGLU;
   constexpr int TN = C::TN, P = C::PITCH, BK = C::BK, OUTS = DUAL ? BN / 2 : BN;
   extern __shared__ __align__(16) float sm[];
@@ -223,26 +240,33 @@ tile_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __rest
   auto row_ok = [&](int r) { return (DUAL ? n0 + r % OUTS : n0 + r) < N; };
   auto load = [&](int step) {
     float* dst = sm + (step % C::STAGES) * C::STAGE;
-    if (VEC) {
 #pragma unroll
-      for (int e = threadIdx.x; e < (BM + BN) * BK / 4; e += C::THREADS) {
-        const int r = e / (BK / 4), k = e % (BK / 4) * 4, gk = step * BK + k;
-        const bool is_a = r < BM;
-        const bool ok = (is_a ? m0 + r < M : row_ok(r - BM)) && gk < K;
-        const float* src = is_a ? (const float*)A + (ok ? (size_t)(m0 + r) * lda + gk : 0)
-                                : (const float*)W + (ok ? (size_t)row_of(r - BM) * K + gk : 0);
-        cp_async16(dst + r * P + k, src, ok);
-      }
-    } else {
-      for (int e = threadIdx.x; e < (BM + BN) * BK; e += C::THREADS) {
-        const int r = e / BK, k = e % BK, gk = step * BK + k;
-        float v = 0.f;
-        if (gk < K) {
-          if (r < BM) { if (m0 + r < M) v = to_f32(A[(size_t)(m0 + r) * lda + gk]); }
-          else if (row_ok(r - BM)) v = to_f32(W[(size_t)row_of(r - BM) * K + gk]);
-        }
-        dst[r * P + k] = v;
-      }
+    for (int e = threadIdx.x; e < (BM + BN) * BK / 4; e += C::THREADS) {
+      const int r = e / (BK / 4), k = e % (BK / 4) * 4, gk = step * BK + k;
+      const bool is_a = r < BM;
+      const bool ok = (is_a ? m0 + r < M : row_ok(r - BM)) && gk < K;
+      const float* src = is_a ? (const float*)A + (ok ? (size_t)(m0 + r) * lda + gk : 0)
+                              : (const float*)W + (ok ? (size_t)row_of(r - BM) * K + gk : 0);
+      cp_async16(dst + r * P + k, src, ok);
+    }
+  };
+  // through registers: the elements of a step are requested a step before they are put down
+  constexpr int TWOS = VEC ? 1 : (BM + BN) * BK / 2 / C::THREADS;
+  const bool even = !VEC && ((K | lda) & 1) == 0 && (((uintptr_t)A | (uintptr_t)W) & (2 * sizeof(TI) - 1)) == 0;
+  decltype(load_two(A, 0, false)) held[TWOS];
+  auto fetch = [&](int step) {
+#pragma unroll
+    for (int i = 0; i < TWOS; ++i) {
+      const int e = threadIdx.x + i * C::THREADS, r = e / (BK / 2), gk = step * BK + e % (BK / 2) * 2;
+      const bool is_a = r < BM, ok = is_a ? m0 + r < M : row_ok(r - BM);
+      held[i] = load_two(is_a ? A + (size_t)(m0 + r) * lda + gk : W + (size_t)row_of(r - BM) * K + gk, ok ? K - gk : 0, even);
+    }
+  };
+  auto put = [&](int step) {
+#pragma unroll
+    for (int i = 0; i < TWOS; ++i) {
+      const int e = threadIdx.x + i * C::THREADS;
+      *reinterpret_cast<float2*>(sm + (step % C::STAGES) * C::STAGE + e / (BK / 2) * P + e % (BK / 2) * 2) = to_f32x2(held[i]);
     }
   };
   pdl_trigger();
@@ -252,15 +276,26 @@ tile_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __rest
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = total[i][j] = 0.f;
-  for (int s = 0; s < C::STAGES - 1; ++s) {
-    if (s < steps) load(s);
-    if (VEC) cp_commit();
+  if constexpr (VEC) {
+    for (int s = 0; s < C::STAGES - 1; ++s) {
+      if (s < steps) load(s);
+      cp_commit();
+    }
+  } else {
+    fetch(0);
+    put(0);
+    if (steps > 1) fetch(1);
   }
   for (int step = 0; step < steps; ++step) {
-    if (VEC) cp_wait<C::STAGES - 2>();
+    if constexpr (VEC) cp_wait<C::STAGES - 2>();
     __syncthreads();  // this step's tiles have landed, and the stage of the step before is free
-    if (step + C::STAGES - 1 < steps) load(step + C::STAGES - 1);
-    if (VEC) cp_commit();
+    if constexpr (VEC) {
+      if (step + C::STAGES - 1 < steps) load(step + C::STAGES - 1);
+      cp_commit();
+    } else {
+      if (step + 1 < steps) put(step + 1);
+      if (step + 2 < steps) fetch(step + 2);
+    }
     const float* as = sm + (step % C::STAGES) * C::STAGE;
     const float* at = as + ty * P;
     const float* bt = as + (BM + tx) * P;
@@ -321,7 +356,7 @@ int launch_rows(const void* A, const void* W, const void* bias, void* out, int M
 template <typename TI, typename TO, int BM, int BN, int TM, int EPI, bool VEC>
 int launch_tile(const void* A, const void* W, const void* bias, void* out, int M, int N, int K, int lda, int ldo,
                 cudaStream_t stream) {
-  using C = Tile<BM, BN, TM>;
+  using C = Tile<BM, BN, TM, VEC>;
   constexpr int OUTS = EPI == EPI_SWIGLU ? BN / 2 : BN;
   auto kernel = tile_kernel<TI, TO, BM, BN, TM, EPI, VEC>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
@@ -352,9 +387,8 @@ int launch_form(const void* A, const void* W, const void* bias, void* out, int M
   // A SM works through a tile of 128 alone in the time of 3.3 tiles of 64 (three at once): the larger one is 10 %
   // faster where its last round is full. Measured on K = 2048, us (64, 128): N = 3072, 700 rows 272, 234; N = 2048,
   // 700 rows 211, 258; SwiGLU N = 8192, 128 rows 279, 236; 1400 rows 2481, 2250
-  const long long rounds_64 = (blocks_64 + 147) / 148, rounds_128 = (blocks_128 + 147) / 148;
-  if constexpr (VEC)
-    if (10 * rounds_128 <= 3 * rounds_64) TILE(128, 128, 8);
+  const long long sms = cuca_device_sms(), rounds_64 = (blocks_64 + sms - 1) / sms, rounds_128 = (blocks_128 + sms - 1) / sms;
+  if (10 * rounds_128 <= 3 * rounds_64) TILE(128, 128, 8);
   TILE(64, 64, 4);
 #undef ROWS
 #undef TILE

@@ -80,6 +80,34 @@ def test_gemm_simt_rows_are_the_same_bits_in_every_form(dev, N, K, epilogue):
         assert torch.equal(out, whole[:M]), M
 
 
+@pytest.mark.parametrize("K", [60, 64, 250, 1021, 2046])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+def test_gemm_simt_of_16_bit_operands_is_the_32_bit_ones_result(dev, K, epilogue):
+    """bfloat16 operands through registers, in pairs (even sizes and addresses) and one by one (odd K, a row stride or an
+    address off two), in every form: the bits that the same values give as 32-bit operands."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(K)
+    N, M = 2100, 1030
+    a = torch.randn(M, K, device=dev, generator=g).to(torch.bfloat16)
+    w = (torch.randn((2 if epilogue == 2 else 1) * N, K, device=dev, generator=g) / math.sqrt(K)).to(torch.bfloat16)
+    prior = torch.randn(M, N, device=dev, generator=g)
+    want = prior.clone()
+    ops.gemm_simt(a.float(), w.float(), want, epilogue)
+    odd_stride = torch.empty(M, K + 1 + K % 2, device=dev, dtype=torch.bfloat16)[:, :K]
+    odd_stride.copy_(a)
+    off = torch.empty(M * K + 1, device=dev, dtype=torch.bfloat16)[1:].view(M, K)
+    off.copy_(a)
+    for x in (a, odd_stride, off):
+        for m in (1, 3, 8, 16, 17, 64, 65, 300, 1030):
+            out = prior[:m].clone()
+            ops.gemm_simt(x[:m], w, out, epilogue)
+            assert torch.equal(out, want[:m]), (m, x.stride(0))
+    if epilogue != 1:
+        out = torch.empty(65, N, device=dev, dtype=torch.bfloat16)
+        ops.gemm_simt(a[:65], w, out, epilogue)
+        assert torch.equal(out, want[:65].to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("M,N,K", GEMM_SHAPES)
 @pytest.mark.parametrize("epilogue", [0, 1, 2])
 @pytest.mark.parametrize("max_splits", [1, 16])
