@@ -110,20 +110,21 @@ class DeviceCache:
         return sum(t[0].numel() * t.element_size() for t in self._state_tensors())
 
     def clear_slot(self, slot: int) -> None:
-        if not 0 <= slot < self.max_sequences:
+        if not -self.max_sequences <= slot < self.max_sequences:
             raise IndexError(f"slot {slot} of {self.max_sequences}")
         arrays = list(self._state_tensors())
         if not arrays:
             return
-        if not arrays[0].is_cuda:
+        if not all(t.is_cuda and t[0].is_contiguous() for t in arrays):
             for t in arrays:
                 t[slot].zero_()
             return
-        where = [(t.data_ptr(), t[0].numel() * t.element_size()) for t in arrays]
-        if where != self._state_where:  # (the first time, or an array was replaced)
+        # (address of slot 0, bytes between slots, bytes of a slot); made again when an array was replaced
+        where = [(t.data_ptr(), t.stride(0) * t.element_size(), t[0].numel() * t.element_size()) for t in arrays]
+        if where != self._state_where:
             self._state_where = where
             self._state_table = torch.tensor(where, dtype=torch.int64).to(arrays[0].device)
-        ops.clear_slot(self._state_table, slot)
+        ops.clear_slot(self._state_table, slot % self.max_sequences)
 
     def view(self, cache_id: int, step) -> CacheView:
         gi, j = self._where.get(cache_id, (None, None))

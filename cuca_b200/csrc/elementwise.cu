@@ -737,12 +737,13 @@ CUCA_API int cuca_scatter_int(int* dst, const int* idx, const int* val, int n, l
 }
 
 namespace {
-// table: (address, bytes of a slot) of every state array, one block row each
+// table: (address of slot 0, bytes from slot to slot, bytes of a slot) of every state array, one block row each
 __global__ void __launch_bounds__(256)
 clear_slot_kernel(const unsigned long long* __restrict__ table, int slot) {
   pdl_trigger();
   pdl_wait();
-  const unsigned long long bytes = table[2 * blockIdx.y + 1], first = table[2 * blockIdx.y] + bytes * (unsigned)slot;
+  table += 3 * blockIdx.y;
+  const unsigned long long first = table[0] + table[1] * (unsigned)slot, bytes = table[2];
   const size_t at = (size_t)blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
   if (((first | bytes) & 15) == 0) {
     for (size_t i = at; i < bytes / 16; i += stride) reinterpret_cast<uint4*>(first)[i] = make_uint4(0u, 0u, 0u, 0u);

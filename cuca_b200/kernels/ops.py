@@ -725,7 +725,8 @@ def set_sampling(rng_state, temperature, top_k, top_p, slot: int, state: int, t:
 
 
 def clear_slot(table, slot: int) -> None:
-    """Zeros in a slot of every state array; `table`: int64 [arrays, 2] on the device, (address, bytes of a slot)."""
+    """Zeros in a slot of every state array; `table`: int64 [arrays, 3] on the device, (address of slot 0, bytes from slot to
+    slot, bytes of a slot)."""
     _cuda(table)
     library.check(library.load().cuca_clear_slot(_p(table), table.shape[0], int(slot), _stream()), "clear_slot")
 
