@@ -221,7 +221,13 @@ __device__ __forceinline__ void store4(__nv_bfloat16* o, float a, float b, float
 // VL: value groups per thread and round. A block of B threads with VL groups each does exactly the arithmetic
 // of a block of B * VL threads with one group each (thread t plays the lanes t, t + B, ...: the same warp
 // shuffles, the same order across warps), so many-row launches can use narrow blocks with bit-equal results.
-template <typename TW, typename TO, bool PARTIAL, int VL>
+// WEIGHTS: where the weights are read. NORM_EARLY: the first two rounds' before the wait for the predecessor (they are no
+// earlier kernel's output), four at a time where they are aligned; NORM_LATE: where they are used, one by one;
+// NORM_LATE_WIDE: there, four at a time, aligned.
+#define NORM_EARLY 0
+#define NORM_LATE 1
+#define NORM_LATE_WIDE 2
+template <typename TW, typename TO, bool PARTIAL, int VL, int WEIGHTS>
 __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ partial, int n_slices,
                                size_t slice_stride, const TW* __restrict__ w, TO* __restrict__ out,
                                const int* __restrict__ rows, int E, float eps, int groups) {
@@ -232,21 +238,12 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
   int orow = blockIdx.x, part = 0;
   if (groups > 1) { part = orow % groups; orow /= groups; }
   w += (size_t)part * E;
-  // The weights are no earlier kernel's output: the first two rounds' are requested before the wait for the predecessor.
-  // (A decode step's norm is a chain of latencies; the weights, which the step's larger ones have driven out of L2, were
-  // the last of them: Llama-3.1-8B widths, 16 layers, batch 8, 1,957 -> 1,927 us a step. Over many rows, four groups a
-  // thread, the registers they take cost more than the latency: 2,048 rows of 4,096 14.0 us without, 20.6 with.)
-  constexpr bool EARLY = VL == 1;
-  const bool w_vec = (E & 3) == 0 && (((size_t)w) & (4 * sizeof(TW) - 1)) == 0;
+  constexpr bool EARLY = WEIGHTS == NORM_EARLY;
+  const bool w_vec = WEIGHTS == NORM_LATE_WIDE || (EARLY && (E & 3) == 0 && (((size_t)w) & 15) == 0);
   auto weights = [&](int i) {
-    float4 v;
-    if (sizeof(TW) == 4 && w_vec) {
-      v = reinterpret_cast<const float4*>(w)[i];
-    } else {
-      const int e = i << 2;
-      v = make_float4(to_f32(w[e]), to_f32(w[e + 1]), to_f32(w[e + 2]), to_f32(w[e + 3]));
-    }
-    return v;
+    if (sizeof(TW) == 4 && WEIGHTS != NORM_LATE && w_vec) return reinterpret_cast<const float4*>(w)[i];
+    const int e = i << 2;
+    return make_float4(to_f32(w[e]), to_f32(w[e + 1]), to_f32(w[e + 2]), to_f32(w[e + 3]));
   };
   float4 w0[VL], w1[VL];
   if (EARLY && (E & 3) == 0) {
@@ -347,20 +344,29 @@ CUCA_API int cuca_rmsnorm_groups(const float* x, const void* w, int w_dtype, voi
   float* xm = const_cast<float*>(x);  // not written without PARTIAL
   // many rows: a quarter of the threads per block, four value groups each (bit-equal to the wide block)
   const bool narrow = norm_block(E) == 1024 && n_rows >= 64 && (E & 3) == 0;
+  // Where the weights are read (see the kernel). A decode step's norm is a chain of latencies, and the weights, which the
+  // step's larger ones have driven out of L2, were the last of them: Llama-3.1-8B widths, 16 layers, batch 8, 1,957 us a step
+  // late, 1,927 early. Over many rows the registers cost more: in narrow blocks 2,048 rows of 4,096 14.0 us late, 20.6 early;
+  // 8,192 rows of 2,048, 16-bit weights, 43.7 and 45.8 (32-bit ones, four at a time, 47.5 and 35.4). Late and four at a time,
+  // 32-bit weights: 8,192 rows of 8,192 77, 73 us, but of 4,096 44, 51.
+  const bool early = !narrow && (w_dtype == CUCA_F32 || n_rows <= 256);
+  const bool wide = narrow && w_dtype == CUCA_F32 && E >= 8192 && ((uintptr_t)w & 15) == 0;
+#define NORM(TW, TO, VL, WEIGHTS, THREADS)                                                                       \
+  cuca_launch(rmsnorm_kernel<TW, TO, false, VL, WEIGHTS>, dim3(n_rows), dim3(THREADS), 0, stream, true, xm,      \
+              (const float*)nullptr, 0, (size_t)0, (const TW*)w, (TO*)out, rows, E, eps, groups)
 #define LAUNCH(TW, TO)                                                                                          \
   do {                                                                                                          \
-    if (narrow)                                                                                                 \
-      cuca_launch(rmsnorm_kernel<TW, TO, false, 4>, dim3(n_rows), dim3(256), 0, stream, true, xm,               \
-                  (const float*)nullptr, 0, (size_t)0, (const TW*)w, (TO*)out, rows, E, eps, groups);           \
-    else                                                                                                        \
-      cuca_launch(rmsnorm_kernel<TW, TO, false, 1>, dim3(n_rows), dim3(norm_block(E)), 0, stream, true, xm,     \
-                  (const float*)nullptr, 0, (size_t)0, (const TW*)w, (TO*)out, rows, E, eps, groups);           \
+    if (narrow && wide) NORM(TW, TO, 4, NORM_LATE_WIDE, 256);                                                   \
+    else if (narrow) NORM(TW, TO, 4, NORM_LATE, 256);                                                           \
+    else if (early) NORM(TW, TO, 1, NORM_EARLY, norm_block(E));                                                 \
+    else NORM(TW, TO, 1, NORM_LATE, norm_block(E));                                                             \
   } while (0)
   if (w_dtype == CUCA_F32 && out_dtype == CUCA_F32) LAUNCH(float, float);
   else if (w_dtype == CUCA_F32 && out_dtype == CUCA_BF16) LAUNCH(float, __nv_bfloat16);
   else if (w_dtype == CUCA_BF16 && out_dtype == CUCA_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);
   else if (w_dtype == CUCA_BF16 && out_dtype == CUCA_F32) LAUNCH(__nv_bfloat16, float);
   else CUCA_REQUIRE(false, "rmsnorm: unknown dtypes %d %d", w_dtype, out_dtype);
+#undef NORM
 #undef LAUNCH
   CUCA_CHECK_LAUNCH("rmsnorm");
   return 0;
@@ -797,10 +803,10 @@ CUCA_API int cuca_add_partials_rmsnorm_groups(float* x, const float* partial, in
   E /= groups;
   n_rows *= groups;
   if (out_dtype == CUCA_BF16)
-    cuca_launch(rmsnorm_kernel<float, __nv_bfloat16, true, 1>, dim3(n_rows), dim3(norm_block(E)), 0, stream, true, x,
+    cuca_launch(rmsnorm_kernel<float, __nv_bfloat16, true, 1, NORM_EARLY>, dim3(n_rows), dim3(norm_block(E)), 0, stream, true, x,
                 partial, n_slices, slice_stride, w, (__nv_bfloat16*)out, rows, E, eps, groups);
   else if (out_dtype == CUCA_F32)
-    cuca_launch(rmsnorm_kernel<float, float, true, 1>, dim3(n_rows), dim3(norm_block(E)), 0, stream, true, x, partial,
+    cuca_launch(rmsnorm_kernel<float, float, true, 1, NORM_EARLY>, dim3(n_rows), dim3(norm_block(E)), 0, stream, true, x, partial,
                 n_slices, slice_stride, w, (float*)out, rows, E, eps, groups);
   else
     CUCA_REQUIRE(false, "add_partials_rmsnorm: unknown dtype %d", out_dtype);

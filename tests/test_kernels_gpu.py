@@ -836,6 +836,29 @@ def test_attention_prefill_tcgen05(dev, nh, nkv, bs, window, d, two_tiles_per_ct
         assert torch.allclose(got, want, atol=2e-2, rtol=2e-2), (r, s, pos, float((got - want).abs().max()))
 
 
+@pytest.mark.parametrize("E", [1024, 2048, 4096, 8192, 9000])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rmsnorm_is_the_same_bits_wherever_it_reads_its_weights(dev, E, dtype):
+    """Early, late, one by one and four at a time (by rows, width and type), and weights off their alignment."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(E)
+    x = torch.randn(300, E, device=dev, generator=g)
+    w = torch.randn(E, device=dev, generator=g).to(dtype)
+    off = torch.empty(E + 1, device=dev, dtype=dtype)[1:]
+    off.copy_(w)
+    outs = []
+    for weight in (w, off):
+        whole, parts = torch.empty(300, E, device=dev), torch.empty(300, E, device=dev)
+        ops.rmsnorm(x, weight, whole, 1e-5)
+        for a in range(0, 300, 50):
+            ops.rmsnorm(x[a:a + 50], weight, parts[a:a + 50], 1e-5)
+        outs += [whole, parts]
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    xd = x.double()
+    want = xd * torch.rsqrt((xd * xd).mean(1, keepdim=True) + 1e-5) * w.double()
+    assert torch.allclose(outs[0].double(), want, atol=1e-6, rtol=1e-5)
+
+
 def test_rmsnorm_many_rows_equals_few_rows_to_the_bit(dev):
     """Launches with many rows use narrower blocks; a row's bits must not depend on that."""
     from cuca_b200.kernels import ops
