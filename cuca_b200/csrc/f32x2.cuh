@@ -22,11 +22,6 @@ __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // (x + y) + (z + w) of two pairs
 __device__ __forceinline__ float f2_sum4(f32x2 xy, f32x2 zw) {
   float x, y, z, w;

@@ -12,10 +12,10 @@
 // K and the row stride multiples of 4); otherwise through registers (the tile form two elements at a time where K, the row
 // stride and the addresses are even), with the same arithmetic.
 //
-// Measured on the Llama-3.2-1B widths in 32-bit: 4 rows, SwiGLU of 2 x 8192 x 2048 49 us (2.7 TB/s of weights), head of
-// 32,000 rows 82 us (3.2 TB/s); 700 rows, SwiGLU 1.34 ms (35 TFLOP/s). One form with 4 x 4 outputs a thread and
-// element-wise loads, before: a decode step of 4 rows 14.3 ms, now 2.8; 700 tokens 32.7 ms, now 20.1. The tile form's
-// limit is shared memory: 128 bytes a clock feed 8 x 8 outputs a thread just at the multiply-adds' rate.
+// Measured on the Llama-3.2-1B widths in 32-bit: 4 rows, SwiGLU of 2 x 8192 x 2048 40 us (3.4 TB/s of weights), head of
+// 32,000 rows 71 us (3.7 TB/s); 700 rows, SwiGLU 1.36 ms (35 TFLOP/s). One form with 4 x 4 outputs a thread and
+// element-wise loads, before: 647, 585 us and 2.15 ms. The tile form's limit is shared memory: 128 bytes a clock feed 8 x 8
+// outputs a thread just at the multiply-adds' rate. 16-bit operands through registers, 2,048 rows, 4,096 x 4,090: 2.02 ms.
 //
 // Epilogues: store (optional bias), add into the 32-bit residual stream, or
 // SwiGLU over a stacked [gate; up] weight (rows 0..N-1 gate, N..2N-1 up).
