@@ -1,4 +1,5 @@
-// Token selection on the device, one block of 1024 threads per row, in the
+// Token selection on the device, one block of 1024 threads per row or, over
+// large vocabularies, several (greedy rows and rows cut to a few best), in the
 // reference's order (src/provider/local/sampler.rs:159-331): temperature <= 0
 // takes the first maximum; otherwise logits are divided by the temperature,
 // cut to the top_k best by (logit descending, id ascending), soft-maxed, cut to
@@ -7,7 +8,8 @@
 // from the request's own SplitMix64 state ((next_u64 >> 40) / 2^24).
 //
 // Up to 1024 ranked candidates are selected by a radix select on an order-
-// preserving key, sorted in shared memory, and summed by one thread in sorted
+// preserving key (several blocks: each the best of its part, the last to arrive
+// the best of those), sorted in shared memory, and summed by one thread in sorted
 // order, which reproduces the reference's 32-bit arithmetic step by step. Wider
 // cuts (top_k above 1024, or a nucleus that needs more than 1024 candidates of
 // a flat distribution) sort the whole vocabulary in a scratch row of global
