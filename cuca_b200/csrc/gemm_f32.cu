@@ -1,0 +1,660 @@
+// 32-bit contraction out = A[M,K] * W[N,K]^T on the 5th-generation tensor cores: the true 32-bit path of every projection,
+// and the bfloat16 path's stand-in for shapes that its own kernel refuses.
+//
+// A 32-bit value is the sum of three bfloat16 parts, exactly: its upper 16 bits, the upper 16 of what is left, and the rest.
+// Of the nine products of two values' parts the six largest count (what the others would add is below 2^-24 of the
+// product); tcgen05.mma sums them in 32 bits over a chunk of 64 products, the smallest first, so that only the last four
+// steps round at the chunk's full magnitude. The tensor cores cut off where a 32-bit addition rounds; over those steps
+// that takes about one unit in the last place off a chunk's sum, which REGAIN gives back. Four chunks' sums are added up to
+// a block's, the blocks' in ascending order to the total. Each output is summed in this one order whatever M and the
+// kernel's form are, so a row's result never depends on the rest of the batch. Where the total is no finite number a warp
+// computes it again with plain multiply-adds (an infinite value has no parts; no result that is finite comes this way).
+// Error against 64 bits, relative 2-norm, normal values: 9.6e-8 at K = 2,048 and 1.3e-7 at 8,192; multiply-adds in runs of 64
+// gave 1.8e-7 and 2.5e-7.
+//
+// The weights are the 128-row operand, the tokens the columns. A CTA (one an SM): the copy engine streams weight chunks
+// into a ring as they are; converter warps split them, a row a lane, into tensor memory, from where the tensor cores read
+// them (shared memory would not stand their 24 reads of a part); the tokens' parts lie in shared memory, converted by two
+// warps over few tokens, or by a kernel of its own before (`split_kernel`) from 17 tokens on, since every block of weight rows
+// reads them; eight or four warps add the chunks' sums up. Few tiles: a cluster of up to eight CTAs shares a tile's K, each
+// keeps its blocks' sums, and all add them in order out of each other's shared memory. Operands that take no copies
+// (16-bit ones, K or a row stride not a multiple of 4, an address off 16 bytes) come through registers with the same results.
+//
+// Epilogues: store (optional bias), add into the 32-bit residual stream, or SwiGLU over a stacked [gate; up] weight (rows
+// 0..N-1 gate, N..2N-1 up).
+#include "tcgen05.cuh"
+#include "f32x2.cuh"
+#include <algorithm>
+
+#define EPI_STORE 0
+#define EPI_RESIDUAL 1
+#define EPI_SWIGLU 2
+
+namespace {
+
+constexpr int CHUNK = TILE_K;         // products that one accumulator sums: 64
+constexpr int BLOCK = 4;              // chunks whose sums are added up before they meet the total
+constexpr int ROWS = TILE_A;          // weight rows of a tile
+constexpr int ROW_BYTES = CHUNK * 2;  // one row of one part in shared memory: one swizzle span
+constexpr int MAX_CLUSTER = 8;
+constexpr int PRE_TOKENS = 32;        // tiles of so many tokens and more take the tokens' parts from memory
+constexpr float REGAIN = 1.f + 1.1920929e-7f;  // one unit in the last place
+
+template <typename TI> struct Parts { static constexpr int N = 3; };
+template <> struct Parts<__nv_bfloat16> { static constexpr int N = 1; };  // (the others would be zeros)
+
+struct GemmParams {
+  const void* A;
+  const void* W;
+  const void* bias;
+  void* out;
+  int* err;
+  int M, N, K, lda, ldo;
+  int epilogue, out_f32;
+  int tiles_m;  // token tiles
+  int slices;   // CTAs of a cluster that share a tile's K
+};
+
+template <typename TI, int NT>
+struct Form {
+  static constexpr int P = Parts<TI>::N;
+  static constexpr bool PRE = NT >= PRE_TOKENS;  // the tokens' parts come from memory, else from converters of this kernel
+  // warps: sums, weight converters (eight a set; two sets take chunks in turn), the tokens' (converters, or one that copies),
+  // the ring's loader, contractions
+  static constexpr int EPI_WARPS = PRE ? 8 : 4;
+  static constexpr int SETS = PRE ? 1 : 2;
+  static constexpr int A_WARPS = 8 * SETS;
+  static constexpr int B_WARPS = PRE ? 1 : 2;
+  static constexpr int A_WARP = EPI_WARPS, B_WARP = A_WARP + A_WARPS, LOAD_WARP = B_WARP + B_WARPS, MMA_WARP = LOAD_WARP + 1;
+  static constexpr int THREADS = 32 * (MMA_WARP + 1);
+  static constexpr int COLS = NT / (EPI_WARPS / 4);  // tokens of one summing thread
+  // weights as they are: a ring of chunks, filled by the copy engine
+  static constexpr int RAW = ROWS * CHUNK * 4;
+  static constexpr int RAWS = PRE ? 4 : 6;
+  // a chunk of the parts: the weights' in tensor memory, the tokens' in shared memory
+  static constexpr int STAGES = PRE ? 2 : 3;
+  static constexpr int A_COLS = P * CHUNK / 2;
+  static constexpr int B_BYTES = P * NT * ROW_BYTES;
+  static constexpr int PASS_ROWS = B_WARPS * 2;  // 16 threads a token row, 16 bytes each
+  static constexpr int PASSES = NT / PASS_ROWS;
+  static constexpr int DATA = RAWS * RAW + STAGES * B_BYTES;
+  static constexpr int SMEM = DATA + 1024 + 256;
+  // columns of tensor memory: two accumulators, the parts, then the total (with slices: the sums of this CTA's blocks)
+  static constexpr int A_AT = 2 * NT, SUM_AT = A_AT + STAGES * A_COLS;
+  static constexpr int BLOCKS_HELD = std::min((512 - SUM_AT) / NT, DATA / (NT * ROWS * 4));
+  static_assert(SUM_AT + NT <= 512 && SMEM <= 227 * 1024, "tensor or shared memory");
+};
+
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// the A operand in tensor memory: row i in lane i, two bf16 per 32-bit column
+__device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank, uint32_t offset) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a + offset) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ bool settled(float v) { return fabsf(v) <= 3.402823466e38f; }
+// One output by a warp with plain multiply-adds.
+template <typename TI>
+__device__ float dot_again(const TI* a, const TI* w, int K) {
+  const int lane = threadIdx.x & 31;
+  float s = 0.f;
+  for (int k0 = 0; k0 < K; k0 += 128) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int k = k0 + 32 * j + lane;
+      if (k < K) s = fmaf(to_f32(a[k]), to_f32(w[k]), s);
+    }
+    if (__any_sync(0xffffffffu, isnan(s))) return __int_as_float(0x7fc00000);
+  }
+  return warp_sum(s);
+}
+// `v` of this lane's output (token m, weight row w), computed again where `again`; the whole warp comes here.
+template <typename TI>
+__device__ __noinline__ float settle(const GemmParams& p, float v, bool again, int m, int w) {
+  unsigned todo = __ballot_sync(0xffffffffu, again);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int mm = __shfl_sync(0xffffffffu, m, src), ww = __shfl_sync(0xffffffffu, w, src);
+    const float r = dot_again((const TI*)p.A + (size_t)mm * p.lda, (const TI*)p.W + (size_t)ww * p.K, p.K);
+    if ((int)(threadIdx.x & 31) == src) v = r;
+  }
+  return v;
+}
+
+// `v` (and for SwiGLU `u`): the sums of output (m, n)
+template <typename TI>
+__device__ __forceinline__ void finish(const GemmParams& p, int m, int n, float v, float u) {
+  const size_t o = (size_t)m * p.ldo + n;
+  if (p.epilogue == EPI_SWIGLU) v = v / (1.f + expf(-v)) * u;
+  else if (p.bias) v += to_f32(((const TI*)p.bias)[n]);
+  if (p.out_f32) {
+    float* out = (float*)p.out + o;
+    *out = p.epilogue == EPI_RESIDUAL ? *out + v : v;
+  } else {
+    ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(v);
+  }
+}
+
+// Four neighbouring elements from `src` on: of a row of which `left` elements are there (VEC: all four).
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float* src, int left) {
+  if (VEC) return __ldg(reinterpret_cast<const float4*>(src));
+  return make_float4(left > 0 ? __ldg(src) : 0.f, left > 1 ? __ldg(src + 1) : 0.f, left > 2 ? __ldg(src + 2) : 0.f,
+                     left > 3 ? __ldg(src + 3) : 0.f);
+}
+template <bool VEC>
+__device__ __forceinline__ uint2 load4(const __nv_bfloat16* src, int left) {
+  const uint16_t* u = reinterpret_cast<const uint16_t*>(src);
+  const uint32_t a = left > 0 ? __ldg(u) : 0, b = left > 1 ? __ldg(u + 1) : 0, c = left > 2 ? __ldg(u + 2) : 0,
+                 d = left > 3 ? __ldg(u + 3) : 0;
+  return make_uint2(a | b << 16, c | d << 16);
+}
+
+__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+// a and b minus their upper halves, exactly
+__device__ __forceinline__ void lower(float& a, float& b) {
+  const f32x2 up = f2_pack(__uint_as_float(__float_as_uint(a) & 0xffff0000u), __uint_as_float(__float_as_uint(b) & 0xffff0000u));
+  f2_unpack(f2_fma(up, f2_both(-1.f), f2_pack(a, b)), a, b);
+}
+// four elements' parts
+__device__ __forceinline__ void split(uint2 (&w)[3], float4 v) {
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    w[t] = make_uint2(upper_halves(v.x, v.y), upper_halves(v.z, v.w));
+    if (t < 2) {
+      lower(v.x, v.y);
+      lower(v.z, v.w);
+    }
+  }
+}
+__device__ __forceinline__ void split(uint2 (&w)[1], uint2 v) { w[0] = v; }
+__device__ __forceinline__ void clear(float4& v) { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+__device__ __forceinline__ void clear(uint2& v) { v = make_uint2(0, 0); }
+
+// The tokens' parts, [part][token][ld] in bf16. Bound by its bytes: 700 x 8,192 values in about 10 us.
+template <typename TI, bool VEC>
+__global__ void __launch_bounds__(256) split_kernel(const TI* __restrict__ A, __nv_bfloat16* __restrict__ parts, int M, int K, int lda, int ld) {
+  constexpr int P = Parts<TI>::N;
+  pdl_trigger();
+  pdl_wait();
+  const int quads = (K + 3) / 4;
+  const long long n = (long long)M * quads;
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < n; e += (long long)gridDim.x * 256) {
+    const int m = (int)(e / quads), k = (int)(e % quads) * 4;
+    uint2 w[P];
+    split(w, load4<VEC>(A + (size_t)m * lda + k, K - k));
+#pragma unroll
+    for (int t = 0; t < P; ++t) *reinterpret_cast<uint2*>(parts + ((size_t)t * M + m) * ld + k) = w[t];
+  }
+}
+
+template <typename TI, int NT, bool VEC>
+__global__ void __launch_bounds__((Form<TI, NT>::THREADS), 1)
+gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const GemmParams p) {
+  using C = Form<TI, NT>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* tokens = smem + C::RAWS * C::RAW;
+  uint64_t* raw_full = (uint64_t*)(smem + C::DATA);
+  uint64_t* raw_empty = raw_full + C::RAWS;
+  uint64_t* full = raw_empty + C::RAWS;
+  uint64_t* done = full + C::STAGES;  // a stage's contraction: its parts are free and its accumulator complete
+  uint64_t* acc_empty = done + C::STAGES;
+  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool dual = p.epilogue == EPI_SWIGLU;
+  const int OUTS = dual ? ROWS / 2 : ROWS;
+  const int cta = blockIdx.x / p.slices, rank = blockIdx.x % p.slices;
+  const int n0 = cta / p.tiles_m * OUTS, m0 = cta % p.tiles_m * NT;  // neighbouring CTAs share weight rows
+  const int chunks = (p.K + CHUNK - 1) / CHUNK, blocks = (chunks + BLOCK - 1) / BLOCK;
+  const int first = rank * blocks / p.slices * BLOCK, last = min((rank + 1) * blocks / p.slices * BLOCK, chunks);
+
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::RAWS; ++s) {
+      mbar_init(&raw_full[s], 1);
+      mbar_init(&raw_empty[s], 8);
+    }
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(&full[s], 8 + C::B_WARPS);  // (the copying warp's arrival brings the bytes it waits for)
+      mbar_init(&done[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) mbar_init(&acc_empty[b], C::EPI_WARPS);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == C::LOAD_WARP) {
+    // ---- weights into the ring; they are no earlier kernel's output, so no predecessor is waited for
+    if (VEC && lane == 0) {
+      const uint64_t once = l2_evict_first();
+      for (int c = first, i = 0; c < last; ++c, ++i) {
+        const int s = i % C::RAWS;
+        if (!mbar_wait(&raw_empty[s], ((i / C::RAWS) & 1) ^ 1, p.err, abort_flag)) break;
+        mbar_expect_tx(&raw_full[s], C::RAW);
+        uint8_t* dst = smem + s * C::RAW;
+        // boxes of 32 elements x 64 rows; SwiGLU's tile: 64 gate rows, then their 64 up rows
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int row = b & 1 ? (dual ? p.N + n0 : n0 + 64) : n0, k = c * CHUNK + (b >> 1) * 32;
+          if (p.tiles_m == 1) tma_load_2d_hint(dst + b * (C::RAW / 4), &tmW, &raw_full[s], k, row, once);
+          else tma_load_2d(dst + b * (C::RAW / 4), &tmW, &raw_full[s], k, row);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == C::MMA_WARP) {
+    // ---- contractions (the whole warp walks the chunks, see elect_one)
+    for (int c = first, i = 0; c < last; ++c, ++i) {
+      const int st = i % C::STAGES, buf = i & 1;
+      if (!warp_wait(&acc_empty[buf], ((i >> 1) & 1) ^ 1, p.err, abort_flag)) break;
+      if (!warp_wait(&full[st], (i / C::STAGES) & 1, p.err, abort_flag)) break;
+      // The converters' writes to the async proxy: the fence stands here, on the path from the writes through the barrier to
+      // the contraction, and not in the converters, where it would wait for their loads in flight.
+      fence_proxy_async();
+      tc_fence_after();
+      const uint32_t a = tmem + C::A_AT + st * C::A_COLS, sb = smem_u32(tokens + st * C::B_BYTES), acc = tmem + buf * NT;
+      if (elect_one()) {
+        // the smallest products first
+#pragma unroll
+        for (int t = 0; t < (C::P == 3 ? 6 : 1); ++t) {
+          constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+          const uint32_t at = a + (C::P == 3 ? PA[t] : 0) * CHUNK / 2;
+          const uint64_t bd = smem_desc(sb + (C::P == 3 ? PB[t] : 0) * NT * ROW_BYTES);
+#pragma unroll
+          for (int k = 0; k < CHUNK / UMMA_K; ++k)
+            umma_bf16_tmem_a(acc, at + k * UMMA_K / 2, bd + k * UMMA_K * 2 / 16, instr_desc(NT), t > 0 || k > 0);
+        }
+        umma_commit(&done[st]);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= C::B_WARP) {
+    pdl_wait();
+    if constexpr (C::PRE) {
+      // ---- the tokens' parts, one box of NT rows each. Rows past the end are the next part's or zeros: what they give is
+      // never stored
+      if (lane == 0) {
+        for (int c = first, n = 0; c < last; ++c, ++n) {
+          const int st = n % C::STAGES;
+          if (!mbar_wait(&done[st], ((n / C::STAGES) & 1) ^ 1, p.err, abort_flag)) break;
+          mbar_expect_tx(&full[st], C::B_BYTES);
+#pragma unroll
+          for (int t = 0; t < C::P; ++t)
+            tma_load_2d(tokens + st * C::B_BYTES + t * NT * ROW_BYTES, &tmX, &full[st], c * CHUNK, t * p.M + m0);
+        }
+      }
+      __syncwarp();
+    } else {
+      // ---- the parts of the tokens: 16 threads a row, four elements each. Rows past the end are read from the last one
+      const int pt = (warp - C::B_WARP) * 32 + lane, r0 = pt / 16, kq = pt % 16 * 4;
+      const TI* rows[C::PASSES];
+#pragma unroll
+      for (int i = 0; i < C::PASSES; ++i) rows[i] = (const TI*)p.A + (size_t)min(m0 + r0 + i * C::PASS_ROWS, p.M - 1) * p.lda;
+      decltype(load4<VEC>(rows[0], 0)) held[C::PASSES];
+      // 16-byte loads stay inside their row; what they bring from before the end is cleared in the last chunk
+      auto load = [&](int i, int c) {
+        const int k = min(c, last - 1) * CHUNK + kq;
+        return load4<VEC>(rows[i] + (VEC ? min(k, p.K - 4) : k), p.K - k);
+      };
+#pragma unroll
+      for (int i = 0; i < C::PASSES; ++i) held[i] = load(i, first);
+      const uint32_t at0 = r0 * ROW_BYTES + ((kq / 8 ^ (r0 & 7)) << 4) + (kq & 4) * 2;
+      for (int c = first, n = 0; c < last; ++c, ++n) {
+        const int st = n % C::STAGES;
+        if (VEC && (c + 1) * CHUNK > p.K && c * CHUNK + kq >= p.K) {
+#pragma unroll
+          for (int i = 0; i < C::PASSES; ++i) clear(held[i]);
+        }
+        uint2 parts[C::PASSES][C::P];
+#pragma unroll
+        for (int i = 0; i < C::PASSES; ++i) {
+          split(parts[i], held[i]);
+          held[i] = load(i, c + 1);
+        }
+        if (!warp_wait(&done[st], ((n / C::STAGES) & 1) ^ 1, p.err, abort_flag)) break;
+        uint8_t* sb = tokens + st * C::B_BYTES;
+#pragma unroll
+        for (int i = 0; i < C::PASSES; ++i)
+#pragma unroll
+          for (int t = 0; t < C::P; ++t)  // (a step of 4 rows modulo 8 turns bit 2 of the swizzled unit)
+            *reinterpret_cast<uint2*>(sb + t * NT * ROW_BYTES + i * C::PASS_ROWS * ROW_BYTES + (at0 ^ (i * C::PASS_ROWS & 4) * 16)) = parts[i][t];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[st]);
+      }
+    }
+  } else if (warp >= C::A_WARP) {
+    // ---- the parts of the weights: a row a lane, half of the chunk's K a warp
+    const int cw = warp - C::A_WARP, quarter = warp & 3, half = (cw >> 2) & 1, set = cw >> 3;
+    const int l = quarter * 32 + lane;
+    const int raw_row = dual ? quarter * 16 + (lane & 15) + (lane & 16) * 4 : l;  // 16 gate rows and their 16 up rows take turns
+    const uint32_t raw_at = (half * 2 + (raw_row >> 6)) * (C::RAW / 4) + (raw_row & 63) * 128;
+    const int w_n = min(dual ? n0 + quarter * 16 + (lane & 15) : n0 + l, p.N - 1);
+    const TI* w_row = (const TI*)p.W + (size_t)(dual && (lane & 16) ? p.N + w_n : w_n) * p.K;
+    const uint32_t a_at = tmem + ((uint32_t)(quarter * 32) << 16) + C::A_AT + half * 16;
+    for (int c = first + set, n = set; c < last; c += C::SETS, n += C::SETS) {
+      const int st = n % C::STAGES, raw = n % C::RAWS;
+      uint32_t w[C::P][16];
+      if constexpr (VEC) {
+        if (!warp_wait(&raw_full[raw], (n / C::RAWS) & 1, p.err, abort_flag)) break;
+        const uint8_t* src = smem + raw * C::RAW + raw_at;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          uint2 x[C::P];
+          split(x, *reinterpret_cast<const float4*>(src + ((q ^ (raw_row & 7)) << 4)));
+#pragma unroll
+          for (int t = 0; t < C::P; ++t) w[t][2 * q] = x[t].x, w[t][2 * q + 1] = x[t].y;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&raw_empty[raw]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int k = c * CHUNK + half * 32 + 4 * q;
+          uint2 x[C::P];
+          split(x, load4<false>(w_row + k, p.K - k));
+#pragma unroll
+          for (int t = 0; t < C::P; ++t) w[t][2 * q] = x[t].x, w[t][2 * q + 1] = x[t].y;
+        }
+      }
+      if (!warp_wait(&done[st], ((n / C::STAGES) & 1) ^ 1, p.err, abort_flag)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int t = 0; t < C::P; ++t) tmem_st16(a_at + st * C::A_COLS + t * CHUNK / 2, w[t]);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[st]);
+    }
+  } else {
+    // ---- sums: thread = weight row, COLS tokens
+    const int quarter = warp & 3, col0 = (warp >> 2) * C::COLS;
+    const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + col0, total = lane_base + C::SUM_AT;
+    float sum[C::COLS];
+    bool ok = true;
+    for (int c = first, i = 0; c < last; ++c, ++i) {
+      const uint32_t acc = lane_base + (i & 1) * NT;
+      ok = warp_wait(&done[i % C::STAGES], (i / C::STAGES) & 1, p.err, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      const bool begins = i % BLOCK == 0, ends = i % BLOCK == BLOCK - 1 || c == last - 1, more = p.slices == 1 && i >= BLOCK;
+      const uint32_t at = total + (p.slices > 1 ? i / BLOCK * NT : 0);
+#pragma unroll
+      for (int j = 0; j < C::COLS; j += 16) {
+        uint32_t x[16];
+        tmem_ld16_async(acc + j, x);
+        tmem_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          sum[j + q] = begins ? __uint_as_float(x[q]) * REGAIN : fmaf(__uint_as_float(x[q]), REGAIN, sum[j + q]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[i & 1]);
+      if (ends) {
+#pragma unroll
+        for (int j = 0; j < C::COLS; j += 16) {
+          if (more) {
+            uint32_t x[16];
+            tmem_ld16_async(at + j, x);
+            tmem_wait_ld();
+#pragma unroll
+            for (int q = 0; q < 16; ++q) sum[j + q] = __uint_as_float(x[q]) + sum[j + q];
+          }
+          tmem_st16(at + j, reinterpret_cast<const uint32_t*>(sum + j));
+        }
+        tmem_wait_st();
+      }
+    }
+    if (ok) {
+      // [block][token][row]; every contraction is done, so the stages are free
+      float* sums = reinterpret_cast<float*>(smem);
+      const int mine = p.slices > 1 ? (last - first + BLOCK - 1) / BLOCK : 1;
+#pragma unroll 1
+      for (int b = 0; b < mine; ++b)
+#pragma unroll 1
+        for (int j = 0; j < C::COLS; j += 16) {
+          float v[16];
+          tmem_ld16(total + b * NT + j, v);
+#pragma unroll
+          for (int q = 0; q < 16; ++q) sums[(size_t)(b * NT + col0 + j + q) * ROWS + quarter * 32 + lane] = v[q];
+        }
+    }
+  }
+  // ---- results: every thread, in one short loop (unrolled per accumulator column its code came from L2, at 290 clocks a
+  // column); the CTAs of a cluster share the tile's outputs and read each other's sums
+  __syncwarp();
+  pdl_wait();
+  if (p.slices > 1) cluster_sync_all();
+  else __syncthreads();
+  const int items = *abort_flag ? 0 : OUTS * min(NT, p.M - m0);
+#pragma unroll 1
+  for (int e0 = rank * C::THREADS; e0 < items; e0 += p.slices * C::THREADS) {
+    const int e = e0 + threadIdx.x, o = e % OUTS, m = e / OUTS, n = n0 + o;
+    const bool live = e < items && n < p.N;
+    const int row = dual ? (o >> 4) * 32 + (o & 15) : o;
+    float v = 0.f, u = 0.f;
+    if (live && p.slices == 1) {
+      const float* sums = reinterpret_cast<const float*>(smem) + (size_t)m * ROWS + row;
+      v = sums[0];
+      if (dual) u = sums[16];
+    } else if (live) {
+      bool started = false;
+      for (int s = 0; s < p.slices; ++s) {
+        const int have = (s + 1) * blocks / p.slices - s * blocks / p.slices;
+        for (int b0 = 0; b0 < have; b0 += 4) {
+          float x[4], y[4];
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const uint32_t at = (uint32_t)((min(b0 + b, have - 1) * NT + m) * ROWS + row) * 4;
+            x[b] = ld_cluster(smem_u32(smem), s, at);
+            if (dual) y[b] = ld_cluster(smem_u32(smem), s, at + 64);
+          }
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+            if (b0 + b < have) {
+              v = started ? v + x[b] : x[b];
+              if (dual) u = started ? u + y[b] : y[b];
+              started = true;
+            }
+        }
+      }
+    }
+    if (__any_sync(0xffffffffu, live && !(settled(v) && settled(u)))) {
+      v = settle<TI>(p, v, live && !settled(v), m0 + m, n);
+      if (dual) u = settle<TI>(p, u, live && !settled(u), m0 + m, p.N + n);
+    }
+    if (live) finish<TI>(p, m0 + m, n, v, u);
+  }
+  if (p.slices > 1) cluster_sync_all();  // no CTA leaves while another reads its sums
+  if (*abort_flag) {
+    // contractions and copies in flight end before their memory is given back
+    const unsigned long long t0 = global_ns();
+    while (global_ns() - t0 < 2000000ull) { }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+int scratch_ld(int K) { return (K + 7) / 8 * 8; }
+
+template <typename TI, int NT, bool VEC>
+int prepare() {
+  using C = Form<TI, NT>;
+  static const cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<TI, NT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  CUCA_REQUIRE(e == cudaSuccess, "gemm: %d bytes of shared memory were refused: %s", C::SMEM, cudaGetErrorString(e));
+  return 0;
+}
+
+template <typename TI, int NT, bool VEC>
+int launch(GemmParams p, int slices, void* scratch, cudaStream_t stream) {
+  using C = Form<TI, NT>;
+  auto kernel = gemm_f32_kernel<TI, NT, VEC>;
+  if (int rc = prepare<TI, NT, VEC>()) return rc;
+  const bool dual = p.epilogue == EPI_SWIGLU;
+  const int outs = dual ? ROWS / 2 : ROWS;
+  p.tiles_m = (p.M + NT - 1) / NT;
+  p.slices = slices;
+  const long long ctas = (long long)p.tiles_m * ((p.N + outs - 1) / outs) * slices;
+  CUCA_REQUIRE(ctas < (1ll << 31), "gemm: %d x %d outputs are too many", p.M, p.N);
+  CUtensorMap tmW = {}, tmX = {};
+  CUCA_REQUIRE(!VEC || cuca_tensor_map_2d(p.W, 4, (uint64_t)p.N * (dual ? 2 : 1), p.K, p.K, 64, &tmW), "gemm: weight tensor map failed");
+  if (C::PRE) {
+    const int ld = scratch_ld(p.K);
+    CUCA_REQUIRE(scratch && ((uintptr_t)scratch & 15) == 0, "gemm: %d tokens need scratch", p.M);
+    CUCA_REQUIRE(cuca_tensor_map_2d(scratch, 2, (uint64_t)C::P * p.M, p.K, ld, NT, &tmX), "gemm: tensor map of the tokens failed");
+    const long long quads = (long long)p.M * ((p.K + 3) / 4);
+    const unsigned grid = (unsigned)std::min<long long>((quads + 255) / 256, 8ll * cuca_device_sms());
+    cuca_launch(split_kernel<TI, VEC>, dim3(grid), dim3(256), 0, stream, true, (const TI*)p.A, (__nv_bfloat16*)scratch, p.M, p.K, p.lda, ld);
+  }
+  if (slices > 1) cuca_launch_cluster(kernel, dim3((unsigned)ctas), dim3(C::THREADS), C::SMEM, stream, true, (unsigned)slices, tmW, tmX, p);
+  else cuca_launch(kernel, dim3((unsigned)ctas), dim3(C::THREADS), C::SMEM, stream, true, tmW, tmX, p);
+  return 0;
+}
+
+// How many clusters of `s` CTAs the device holds at once: a GPC's SMs rarely divide by 8.
+template <typename TI, int NT, bool VEC>
+int clusters_held(int s) {
+  static int held[MAX_CLUSTER + 1] = {};  // (the same answer whoever asks first)
+  if (!held[s]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s * cuca_device_sms());
+    cfg.blockDim = dim3(Form<TI, NT>::THREADS);
+    cfg.dynamicSmemBytes = Form<TI, NT>::SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = s;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (prepare<TI, NT, VEC>() || cudaOccupancyMaxActiveClusters(&n, gemm_f32_kernel<TI, NT, VEC>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = cuca_device_sms() / s / 2 + 1;
+    }
+    held[s] = n;
+  }
+  return held[s];
+}
+
+// Whether a cluster of `slices` CTAs can share K: each has blocks, and its tensor memory holds their sums.
+template <typename TI, int NT>
+bool holds(int K, int slices) {
+  const int blocks = (K + CHUNK * BLOCK - 1) / (CHUNK * BLOCK);
+  return slices == 1 || (slices > 1 && slices <= std::min(MAX_CLUSTER, blocks) && (blocks + slices - 1) / slices <= Form<TI, NT>::BLOCKS_HELD);
+}
+
+// The form with the least estimated time: rounds of CTAs times a CTA's chunks, whose cost in us (`chunk_us`) was measured as
+// the slope over K; 4 us a launch, one more for a cluster's two barriers and reads, 3 for the tokens' split. Measured, us:
+// K = 8,192, 2,048 rows, 4 tokens: 1, 4, 8 CTAs a tile 88, 37, 50 (128 CTAs in clusters of eight do not fit at once).
+struct Choice { int nt, slices; double cost; };
+template <typename TI, int NT, bool VEC>
+void consider(Choice& best, int M, int N, int K, bool dual, double chunk_us) {
+  const int outs = dual ? ROWS / 2 : ROWS, blocks = (K + CHUNK * BLOCK - 1) / (CHUNK * BLOCK);
+  const long long tiles = (long long)((M + NT - 1) / NT) * ((N + outs - 1) / outs);
+  for (int s = 1; s <= MAX_CLUSTER; ++s) {
+    const int per = (blocks + s - 1) / s;
+    if (!holds<TI, NT>(K, s) || (s > 1 && (per == (blocks + s - 2) / (s - 1) || tiles * (s - 1) >= cuca_device_sms()))) continue;
+    const int held = s > 1 ? clusters_held<TI, NT, VEC>(s) : cuca_device_sms();
+    const double cost = (double)((tiles + held - 1) / held) * (per * BLOCK * chunk_us + (s > 1 ? 5. : 4.)) + (Form<TI, NT>::PRE ? 3. : 0.);
+    if (cost < best.cost) best = {NT, s, cost};
+  }
+}
+template <typename TI, bool VEC>
+Choice choose(int M, int N, int K, bool dual) {
+  Choice best = {0, 1, 1e30};
+  consider<TI, 16, VEC>(best, M, N, K, dual, 0.52);
+  if (M > 16) consider<TI, 32, VEC>(best, M, N, K, dual, 0.68);
+  if (M > 32) consider<TI, 64, VEC>(best, M, N, K, dual, 0.76);
+  if (M > 64) consider<TI, 96, VEC>(best, M, N, K, dual, 1.1);
+  return best;
+}
+
+template <typename TI, bool VEC>
+int go(const GemmParams& p, void* scratch, int form_tokens, int form_slices, cudaStream_t stream) {
+  Choice f = {form_tokens, form_slices, 0.};
+  if (!f.nt) f = choose<TI, VEC>(p.M, p.N, p.K, p.epilogue == EPI_SWIGLU);
+#define FORM(NT)                                                                                           \
+  if (f.nt == NT) {                                                                                        \
+    CUCA_REQUIRE((holds<TI, NT>(p.K, f.slices)), "gemm: K = %d is not cut in %d this way", p.K, f.slices); \
+    return launch<TI, NT, VEC>(p, f.slices, scratch, stream);                                              \
+  }
+  FORM(16)
+  FORM(32)
+  FORM(64)
+  FORM(96)
+#undef FORM
+  CUCA_REQUIRE(false, "gemm: no tiles of %d tokens", f.nt);
+}
+
+}  // namespace
+
+// Most tokens for which cuca_gemm_f32 needs no scratch. Beyond: parts x M x K' 16-bit values, three parts of 32-bit operands and
+// one of 16-bit ones, K' = K rounded up to a multiple of 8; 16-byte aligned.
+CUCA_API int cuca_gemm_f32_few_tokens() { return 16; }
+
+// out = epilogue(A[M,K] W[N,K]^T). in_dtype: A, W and bias; out_dtype: out.
+// epilogue 0 store, 1 out (32-bit) += result, 2 SwiGLU (W has 2N rows).
+// form_tokens, form_slices: tokens of a tile (16, 32, 64, 96) and CTAs that share its K (1 to 8), 0: the library's choice.
+CUCA_API int cuca_gemm_f32(const void* A, const void* W, const void* bias, void* out, int in_dtype, int out_dtype, int M,
+                           int N, int K, int lda, int ldo, int epilogue, int* err, void* scratch, int form_tokens,
+                           int form_slices, cudaStream_t stream) {
+  if (M == 0 || N == 0) return 0;
+  CUCA_REQUIRE(K > 0 && lda >= K && ldo >= N, "gemm: bad sizes M=%d N=%d K=%d lda=%d ldo=%d", M, N, K, lda, ldo);
+  CUCA_REQUIRE(epilogue != EPI_RESIDUAL || out_dtype == CUCA_F32, "gemm: the residual stream is 32-bit");
+  CUCA_REQUIRE(epilogue != EPI_SWIGLU || bias == nullptr, "gemm: SwiGLU takes no bias");
+  CUCA_REQUIRE(epilogue >= EPI_STORE && epilogue <= EPI_SWIGLU, "gemm: unknown epilogue %d", epilogue);
+  CUCA_REQUIRE((in_dtype == CUCA_F32 && out_dtype == CUCA_F32) || (in_dtype == CUCA_BF16 && (out_dtype == CUCA_F32 || out_dtype == CUCA_BF16)),
+               "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
+  GemmParams p = {A, W, bias, out, err, M, N, K, lda, ldo, epilogue, out_dtype == CUCA_F32, 0, 0};
+  const bool vec = in_dtype == CUCA_F32 && K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+  int rc;
+  if (in_dtype == CUCA_BF16) rc = go<__nv_bfloat16, false>(p, scratch, form_tokens, form_slices, stream);
+  else if (vec) rc = go<float, true>(p, scratch, form_tokens, form_slices, stream);
+  else rc = go<float, false>(p, scratch, form_tokens, form_slices, stream);
+  if (rc) return rc;
+  CUCA_CHECK_LAUNCH("gemm_f32");
+  return 0;
+}

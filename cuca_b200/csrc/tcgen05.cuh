@@ -57,6 +57,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   }
   return true;
 }
+// A warp's wait: one lane asks and tells the others (the shuffle alone would not order their reads behind it).
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, volatile int* abort) {
+  int ok = 0;
+  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, err, abort);
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+// One lane of a converged warp. Where a whole warp walks a loop of contractions together and elects the lane for each batch,
+// the compiler keeps descriptors in uniform registers: a tcgen05.mma takes 20 to 50 clocks to issue, against 100 in a branch
+// that only one thread has entered.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t mine;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(mine));
+  return mine != 0;
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

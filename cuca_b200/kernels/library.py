@@ -31,7 +31,8 @@ _SIGNATURES = {
     "cuca_rope_store": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "cuca_swiglu": [_P, _P, _I, _I, _I, _P],
     "cuca_add_to_stream": [_P, _P, _I, c_size_t, _P],
-    "cuca_gemm_simt": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+    "cuca_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _I, _P],
+    "cuca_gemm_f32_few_tokens": [],
     "cuca_attention_generic": [_P, _I, _P, _I, _I, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "cuca_argmax": [_P, c_size_t, _I, _I, _P, _P],
     "cuca_suppress_tokens": [_P, c_size_t, _I, _I, _P, _I, _P],

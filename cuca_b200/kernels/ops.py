@@ -154,14 +154,25 @@ def add_to_stream(x, delta) -> None:
                   "add_to_stream")
 
 
-def gemm_simt(a, w, out, epilogue=EPI_STORE, bias=None) -> None:
-    """out = epilogue(a @ w.T) on CUDA cores; a: [M, K] (row stride >= K), w: [N or 2N, K]."""
+_gemm_few: list = []  # most tokens that `gemm_simt` takes without scratch
+
+
+def gemm_simt(a, w, out, epilogue=EPI_STORE, bias=None, err=None, form=(0, 0)) -> None:
+    """out = epilogue(a @ w.T) with 32-bit accuracy; a: [M, K] (row stride >= K), w: [N or 2N, K], both 32-bit or both
+    16-bit, of any size and alignment. A row's result is the same bits whatever M is. `form`: tokens of a tile and CTAs that
+    share its K (tests; 0: the library's choice)."""
     _cuda(a, w, out)
     lib = library.load()
     M, K = a.shape
     N = out.shape[1]
-    library.check(lib.cuca_gemm_simt(_p(a), _p(w), _p(bias), _p(out), dtype_code(a.dtype), dtype_code(out.dtype),
-                                     M, N, K, a.stride(0), out.stride(0), epilogue, _stream()), "gemm_simt")
+    if not _gemm_few:
+        _gemm_few.append(int(lib.cuca_gemm_f32_few_tokens()))
+    scratch = None
+    if M > _gemm_few[0] or form[0] > _gemm_few[0]:  # the tokens as bfloat16 parts
+        scratch = torch.empty((3 if a.dtype == torch.float32 else 1) * M * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=a.device)
+    library.check(lib.cuca_gemm_f32(_p(a), _p(w), _p(bias), _p(out), dtype_code(a.dtype), dtype_code(out.dtype),
+                                    M, N, K, a.stride(0), out.stride(0), epilogue, _p(err), _p(scratch), int(form[0]),
+                                    int(form[1]), _stream()), "gemm_simt")
 
 
 class AttentionOptions(ctypes.Structure):
@@ -326,13 +337,13 @@ def gemm_pair_mode(mode: int) -> None:
 
 
 def gemm(a, w, out, epilogue=EPI_STORE, bias=None, err=None) -> None:
-    """out = epilogue(a @ w.T), on the kernel that fits dtype and shape: tensor cores for bfloat16
-    (rows of 16-byte multiples), CUDA cores for the 32-bit path and for shapes the former refuses."""
+    """out = epilogue(a @ w.T), on the kernel that fits dtype and shape: `gemm_tc` for bfloat16 (rows of 16-byte
+    multiples), `gemm_simt` for the 32-bit path and for shapes the former refuses."""
     if a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16) \
             and gemm_tc_supported(a, w):
         gemm_tc(a, w, out, epilogue, bias, err)
     else:
-        gemm_simt(a, w, out, epilogue, bias)
+        gemm_simt(a, w, out, epilogue, bias, err)
 
 
 class AttentionPlan:

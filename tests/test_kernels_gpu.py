@@ -80,6 +80,55 @@ def test_gemm_simt_rows_are_the_same_bits_in_every_form(dev, N, K, epilogue):
         assert torch.equal(out, whole[:M]), M
 
 
+# (tokens, weight rows, K): edges of the tiles of 16, 32, 64 and 96 tokens and of 128 weight rows, K below a chunk of 64, with
+# a ragged end, in one block of 256 and in 8 and 33 of them
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (16, 128, 64), (17, 129, 260), (33, 65, 2048), (65, 200, 2044), (96, 300, 8196),
+                                   (97, 64, 1030), (193, 257, 512)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+def test_gemm_f32_every_form_gives_the_same_bits(dev, M, N, K, epilogue):
+    """Tiles of every width, K shared by one to eight CTAs: against 64 bits, the same bits in every form, and infinities and
+    NaN where multiply-adds have them. The bound: a product lacks 2^-24 of itself at most, a chunk's sum is off by some 4 of
+    the last of 24 places, and up to 3 + 33 additions round; all against the sum of the products' sizes."""
+    from cuca_b200.kernels import library, ops
+    g = torch.Generator(device=dev).manual_seed(M * 7 + N + K)
+    a = torch.randn(M, K, device=dev, generator=g) * torch.exp(torch.randn(M, K, device=dev, generator=g))
+    w = torch.randn((2 if epilogue == 2 else 1) * N, K, device=dev, generator=g) / math.sqrt(K)
+    bias = torch.randn(N, device=dev, generator=g) if epilogue == 0 else None
+    prior = torch.randn(M, N, device=dev, generator=g)
+    want = prior.clone()
+    ops.gemm_simt(a, w, want, epilogue, bias)
+    ref = _ref_gemm(a.double(), w.double(), epilogue, None if bias is None else bias.double(), prior.double())
+    sizes = a.double().abs() @ w.double().abs().T
+    if epilogue == 2:  # silu has a slope below 1.1 and is at most its argument's size
+        y = a.double() @ w.double().T
+        sizes = 1.1 * sizes[:, :N] * y[:, N:].abs() + sizes[:, N:] * y[:, :N].abs() + sizes[:, :N] * 1e-6 * sizes[:, N:]
+    places = 1 + 4 + 3 + 33 + 8  # (and bias, stream, exponent and division)
+    assert bool(((want.double() - ref).abs() <= places * 2.0 ** -24 * (sizes + prior.double().abs() + 4)).all())
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    ran = 0
+    for tokens in (16, 32, 64, 96):
+        for slices in range(1, 9):
+            out = prior.clone()
+            try:
+                ops.gemm_simt(a, w, out, epilogue, bias, err, form=(tokens, slices))
+            except library.KernelError:
+                assert slices > 1  # (K has too few blocks for so many, or too many for what each can hold)
+                continue
+            ran += 1
+            assert torch.equal(out, want), (tokens, slices)
+    assert ran >= 4 and int(err.item()) == 0
+    a[M // 2, K // 3] = float("inf")
+    w[N // 2, K // 2] = float("nan")
+    if M > 1:
+        a[0, K // 2] = float("-inf")
+    y = a @ w.T
+    for tokens, slices in ((16, 1), (64, 1), (0, 0)):
+        out = torch.empty(M, N, device=dev)
+        ops.gemm_simt(a, w, out, 0 if epilogue == 1 else epilogue, None, form=(tokens, slices))
+        if epilogue != 2:
+            assert torch.equal(out.isnan(), y.isnan()) and torch.equal(out.isinf() & (out > 0), y.isinf() & (y > 0)), (tokens, slices)
+
+
 @pytest.mark.parametrize("K", [60, 64, 250, 1021, 2046])
 @pytest.mark.parametrize("epilogue", [0, 1, 2])
 def test_gemm_simt_of_16_bit_operands_is_the_32_bit_ones_result(dev, K, epilogue):
