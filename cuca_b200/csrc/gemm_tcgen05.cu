@@ -6,7 +6,9 @@
 // step reads each weight once and far more of them than L2 holds; one thread issues tcgen05.mma (kind::f16, 32-bit accumulate) into one of two TMEM
 // accumulators, and four warps drain the other accumulator with tcgen05.ld and run the epilogue (store, bias,
 // add into the 32-bit residual stream, or SwiGLU), so the epilogue of one tile overlaps the main loop of the
-// next. tcgen05.commit hands stages back to the producer and accumulators to the epilogue.
+// next. tcgen05.commit hands stages back to the producer and accumulators to the epilogue. The issuing thread is elected anew
+// for each K step by a warp that walks the loop together (see elect_one); with one thread in a branch of its own the steps
+// of 256 x 256 tiles were bound by their issue (gate/up of 2,048 tokens 326 us, 303 now; a decode step of one request 2 % less).
 //
 // Two orientations share the code. Up to 256 tokens (decode, short portions; SwiGLU up to 64), the weight is the 128-row
 // MMA operand and the tokens are the N dimension (16..256): D[feature, token], one TMEM lane per output feature. Above, the tokens
@@ -494,8 +496,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         load_activations(sp, &full[st], s, ks * TILE_K);
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ------------------------------------------------ MMA issuer
+  } else if (warp == 1) {
+    // ------------------------------------------------ MMA issuer (the warp together, see elect_one)
     pdl_wait();
     SegmentWalk walk(p, C::OUT_COLS);
     Segment s;
@@ -505,28 +507,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int buf = seg % C::ACC_BUFS;
       // a column piece is narrower than a tile (never with SwiGLU, whose tile is 128 gate and 128 up columns)
       const uint32_t idesc = instr_desc((SWAP || DUAL) ? C::MMA_N : s.w);
-      if (!mbar_wait(&tmem_empty[buf], ((seg / C::ACC_BUFS) & 1) ^ 1, p.err, abort_flag)) break;
+      if (!warp_wait(&tmem_empty[buf], ((seg / C::ACC_BUFS) & 1) ^ 1, p.err, abort_flag)) break;
       tc_fence_after();
       const uint32_t acc = tmem_base + buf * C::NCOLS;
       for (int ks = s.ks0; ks < s.ks1; ++ks, ++it) {
         const int st = it % C::STAGES;
-        if (!mbar_wait(&full[st], (it / C::STAGES) & 1, p.err, abort_flag)) { ok = false; break; }
+        if (!warp_wait(&full[st], (it / C::STAGES) & 1, p.err, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sa = smem_u32(smem + st * C::STAGE_BYTES);
         const uint64_t adesc = smem_desc(sa);
         const uint64_t adesc2 = smem_desc(sa + TILE_A * TILE_K * 2);
         const uint64_t bdesc = smem_desc(sa + C::A_BYTES);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < TILE_K / UMMA_K; ++k) {
-          const uint32_t accumulate = (ks > s.ks0 || k > 0) ? 1u : 0u;
-          const uint64_t koff = (uint64_t)(k * UMMA_K * 2 >> 4);
-          umma_bf16(acc, adesc + koff, bdesc + koff, idesc, accumulate);
-          if (SWAP && DUAL) umma_bf16(acc + BN, adesc2 + koff, bdesc + koff, idesc, accumulate);
-          if (TALL) umma_bf16(acc + BN, adesc2 + koff, bdesc + koff, idesc, accumulate);  // the second row block
+          for (int k = 0; k < TILE_K / UMMA_K; ++k) {
+            const uint32_t accumulate = (ks > s.ks0 || k > 0) ? 1u : 0u;
+            const uint64_t koff = (uint64_t)(k * UMMA_K * 2 >> 4);
+            umma_bf16(acc, adesc + koff, bdesc + koff, idesc, accumulate);
+            if (SWAP && DUAL) umma_bf16(acc + BN, adesc2 + koff, bdesc + koff, idesc, accumulate);
+            if (TALL) umma_bf16(acc + BN, adesc2 + koff, bdesc + koff, idesc, accumulate);  // the second row block
+          }
+          umma_commit(&empty[st]);
         }
-        umma_commit(&empty[st]);
+        __syncwarp();
       }
-      if (ok) umma_commit(&tmem_full[buf]);
+      if (ok && elect_one()) umma_commit(&tmem_full[buf]);
+      __syncwarp();
       ++seg;
     }
   } else if (warp >= 2 && warp < 2 + C::EPI_WARPS) {
@@ -858,32 +864,36 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         pair_tma_load_2d(sp, &tmA, full_first[st], ks * TILE_K, a0);  // rows past M read as zeros
       }
     }
-  } else if (warp == 1 && lane == 0 && first) {
-    // ------------------------------------------------ MMA issuer of the pair
+  } else if (warp == 1 && first) {
+    // ------------------------------------------------ MMA issuer of the pair (the warp together, see elect_one)
     pdl_wait();
     constexpr uint32_t idesc = pair_instr_desc();
     int it = 0, seg = 0;
     bool ok = true;
     for (int u = pair; ok && u < units; u += n_pairs, ++seg) {
       const int buf = seg & 1;
-      if (!mbar_wait(&tmem_empty[buf], ((seg >> 1) & 1) ^ 1, p.err, abort_flag)) break;
+      if (!warp_wait(&tmem_empty[buf], ((seg >> 1) & 1) ^ 1, p.err, abort_flag)) break;
       tc_fence_after();
       const uint32_t acc = tmem_base + buf * C::NCOLS;
       const int ks0 = ks_first(u);
       for (int ks = ks0; ks < ks_end(u); ++ks, ++it) {
         const int st = it % C::STAGES;
-        if (!mbar_wait(&full[st], (it / C::STAGES) & 1, p.err, abort_flag)) { ok = false; break; }
+        if (!warp_wait(&full[st], (it / C::STAGES) & 1, p.err, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sa = smem_u32(smem + st * C::STAGE_BYTES);
         const uint64_t adesc = smem_desc(sa), bdesc = smem_desc(sa + C::A_BYTES);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < TILE_K / UMMA_K; ++k) {
-          const uint64_t koff = (uint64_t)(k * UMMA_K * 2 >> 4);
-          pair_umma_bf16(acc, adesc + koff, bdesc + koff, idesc, (ks > ks0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < TILE_K / UMMA_K; ++k) {
+            const uint64_t koff = (uint64_t)(k * UMMA_K * 2 >> 4);
+            pair_umma_bf16(acc, adesc + koff, bdesc + koff, idesc, (ks > ks0 || k > 0) ? 1u : 0u);
+          }
+          pair_umma_commit(&empty[st]);
         }
-        pair_umma_commit(&empty[st]);
+        __syncwarp();
       }
-      if (ok) pair_umma_commit(&tmem_full[buf]);
+      if (ok && elect_one()) pair_umma_commit(&tmem_full[buf]);
+      __syncwarp();
     }
   } else if (warp >= 2 && warp < 2 + C::EPI_WARPS) {
     // ------------------------------------------------ epilogue of this CTA's 128 rows

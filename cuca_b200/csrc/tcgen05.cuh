@@ -57,12 +57,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   }
   return true;
 }
-// A warp's wait: one lane asks and tells the others (the shuffle alone would not order their reads behind it).
+// A warp's wait. Every lane asks: one lane that tells the others adds some 60 clocks to each turn of a ring.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, volatile int* abort) {
-  int ok = 0;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, err, abort);
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, abort));
 }
 // One lane of a converged warp. Where a whole warp walks a loop of contractions together and elects the lane for each batch,
 // the compiler keeps descriptors in uniform registers: a tcgen05.mma takes 20 to 50 clocks to issue, against 100 in a branch
