@@ -102,14 +102,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
       "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// the A operand in tensor memory: row i in lane i, two bf16 per 32-bit column
-__device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -402,7 +394,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       tc_fence_after();
 #pragma unroll
       for (int t = 0; t < C::P; ++t) tmem_st16(a_at + st * C::A_COLS + t * CHUNK / 2, w[t]);
-      tmem_wait_st();
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[st]);
@@ -424,7 +416,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       for (int j = 0; j < C::COLS; j += 16) {
         uint32_t x[16];
         tmem_ld16_async(acc + j, x);
-        tmem_wait_ld();
+        tmem_ld_wait();
 #pragma unroll
         for (int q = 0; q < 16; ++q)
           sum[j + q] = begins ? __uint_as_float(x[q]) * REGAIN : fmaf(__uint_as_float(x[q]), REGAIN, sum[j + q]);
@@ -438,13 +430,13 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           if (more) {
             uint32_t x[16];
             tmem_ld16_async(at + j, x);
-            tmem_wait_ld();
+            tmem_ld_wait();
 #pragma unroll
             for (int q = 0; q < 16; ++q) sum[j + q] = __uint_as_float(x[q]) + sum[j + q];
           }
           tmem_st16(at + j, reinterpret_cast<const uint32_t*>(sum + j));
         }
-        tmem_wait_st();
+        tmem_st_wait();
       }
     }
     if (ok) {

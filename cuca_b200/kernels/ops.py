@@ -986,6 +986,7 @@ def head_linear(a, lda, a_head, w, out, ldo, o_head, T, gate=None, ldg=0) -> Non
 USE_MMA_LATENT = True  # bfloat16 caches through the tensor-core form where the sizes allow
 LATENT_TILE_ROWS = 16  # tokens of a portion that one CTA of the tensor-core form takes
 _latent_mma_ok: dict = {}
+_latent_tc_tokens: dict = {}
 
 
 def latent_attention_mma_supported(rank: int, Dk: int) -> bool:
@@ -995,10 +996,18 @@ def latent_attention_mma_supported(rank: int, Dk: int) -> bool:
     return _latent_mma_ok[key]
 
 
+def latent_attention_tc_tokens(H: int, rank: int, Dk: int, scale: float) -> int:
+    """Tokens of a portion that a group of the tcgen05 form takes (0: it refuses the sizes)."""
+    key = (H, rank, Dk)
+    if key not in _latent_tc_tokens:
+        _latent_tc_tokens[key] = int(library.load().cuca_latent_attention_tc_tokens(H, rank, Dk))
+    return _latent_tc_tokens[key] if scale > 0 else 0
+
+
 def latent_attention(qk, out, cache, step, H, rank, Dk, scale, window, err, sink_values=None) -> None:
-    """Every row's heads attend over the cached rows of the row's request. A bfloat16 cache goes through the
-    tensor-core form, portions of prompts in groups of 16 tokens per head and single tokens with their heads as the
-    group (the step's attention plan names both); the 32-bit path and other sizes go through the plain kernel.
+    """Every row's heads attend over the cached rows of the row's request. A bfloat16 cache goes through a
+    tensor-core form, portions of prompts in groups of tokens and heads (tcgen05 where it takes the sizes, else 16 tokens per
+    head) and single tokens with their heads as the group (the step's attention plan names both); the 32-bit path and other sizes go through the plain kernel.
     `sink_values` (32-bit, one number per head): every denominator holds one more term exp(sink_values[head])."""
     pool = cache.k
     sink = _sink_values(sink_values, H)
@@ -1012,8 +1021,15 @@ def latent_attention(qk, out, cache, step, H, rank, Dk, scale, window, err, sink
                 _p(cache.tables), cache.tables.shape[1], _p(row0), _p(nrows), _p(rows), n, H, rank, Dk, float(scale),
                 int(window or 0), sink, splits, _p(acc), _p(ml), _p(err), _stream()), "latent_attention_mma")
         if plan.n_portions:
-            row0, nrows, n = plan.tiles(LATENT_TILE_ROWS)
-            launch(row0, nrows, None, n)
+            tokens = latent_attention_tc_tokens(H, rank, Dk, scale)
+            row0, nrows, n = plan.tiles(tokens or LATENT_TILE_ROWS)
+            if tokens:
+                library.check(lib.cuca_latent_attention_tc(
+                    _p(qk), _p(out), _p(pool), pool.shape[0], pool.shape[2], _p(step.positions), _p(step.seq_of_row),
+                    _p(cache.tables), cache.tables.shape[1], _p(row0), _p(nrows), n, H, rank, Dk, float(scale),
+                    int(window or 0), sink, _p(err), _stream()), "latent_attention_tc")
+            else:
+                launch(row0, nrows, None, n)
         if plan.n_decode:
             # single tokens: few groups (one per token and 16 heads), so a group's key tiles are dealt to several
             # CTAs where that fills more of the GPU, and a second launch merges what they leave

@@ -400,6 +400,21 @@ def test_latent_attention_on_tensor_cores(layer):
     assert int(rt.err.item()) == 0
 
 
+@pytest.mark.parametrize("layer,tokens", [
+    (bu.latent(heads=16, dim=8, rot_dim=64, vdim=8, kv_rank=512, window=130, scale=1.0), 8),  # two halves of the columns
+    (bu.latent(heads=16, dim=16, rot_dim=0, vdim=8, kv_rank=64, window=None, scale=1.0), 8),  # one chunk of values
+    (bu.latent(heads=8, dim=24, rot_dim=64, vdim=12, kv_rank=320, window=70, scale=0.9), 16),  # unequal parts of the columns
+    (bu.latent(heads=24, dim=8, rot_dim=0, vdim=8, kv_rank=256, window=1, scale=0.8), 16),  # all queries in tensor memory
+    (bu.latent(heads=32, dim=8, rot_dim=128, vdim=8, kv_rank=448, window=64, scale=1.0), 8)])  # two groups of heads
+def test_latent_attention_in_groups_of_tokens_and_heads(layer, tokens):
+    """The tcgen05 form's sizes through the test above: portions that end inside a group and inside a key tile, windows over
+    several key tiles, pages that hold NaN where nothing was written."""
+    from cuca_b200.kernels import ops
+    m = layer["mixer"]
+    assert ops.latent_attention_tc_tokens(m["heads"], m["kv_rank"], m["kv_rank"] + m["rot_dim"], m["scale"]) == tokens
+    test_latent_attention_on_tensor_cores(layer)
+
+
 def test_dense_feed_forward_and_loop_entry_alone(rt32):
     from cuca_b200.parts.base import PartSpec
     from cuca_b200.parts.mlp import DenseActivation
