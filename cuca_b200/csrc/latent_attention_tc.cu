@@ -27,8 +27,9 @@ constexpr int Q_CHUNK = ROWS * 128, K_CHUNK = KEYS * 128;  // 64 values of every
 constexpr int Q_COLS = 128;                                // tensor memory for the first 256 values of Q
 constexpr int MAX_DK = 576;
 constexpr int O_AT = 0, S_AT = 256, Q_AT = 384;            // columns of tensor memory
-constexpr int SOFT_WARPS = 4, LOAD_WARPS = 4, MMA_WARP = SOFT_WARPS + LOAD_WARPS;
+constexpr int SOFT_WARPS = 8, LOAD_WARPS = 4, MMA_WARP = SOFT_WARPS + LOAD_WARPS;
 constexpr int NTHREADS = 32 * (MMA_WARP + 1);
+constexpr int HALVES = ROWS * 2 * 4;                       // a float of both halves of every row
 constexpr int OUT_PITCH = 36;                              // floats a row of 32 output columns on its way out
 
 struct Params {
@@ -47,13 +48,23 @@ struct Params {
   int window;
   const float* sink;
   int parts;        // CTAs that share a group's output columns
+  int tma;          // whole key tiles come through the copy engine
   int* err;
 };
 
+constexpr int OUT_BYTES = SOFT_WARPS * 32 * OUT_PITCH * 4;  // all results on their way out lie in the two key tiles' memory
+// A key tile's memory: the tile, the first 256 values of the queries on their way, or half of the results, whatever is larger.
+__host__ __device__ constexpr int tile_bytes_of(int Dk) {
+  int bytes = Dk / 64 * K_CHUNK;
+  const int queries = (Dk < 256 ? Dk / 64 : 4) * Q_CHUNK, results = OUT_BYTES / 2;
+  if (queries > bytes) bytes = queries;
+  if (results > bytes) bytes = results;
+  return bytes;
+}
+static_assert(OUT_BYTES / 2 % 1024 == 0, "tiles start at multiples of 1024 bytes");
 int smem_bytes(int Dk) {
   const int q_chunks = Dk / 64 > 4 ? Dk / 64 - 4 : 0;
-  const int tiles = 2 * (Dk / 64) * K_CHUNK, out = SOFT_WARPS * 32 * OUT_PITCH * 4;
-  return q_chunks * Q_CHUNK + (tiles > out ? tiles : out) + 1024 + 256;
+  return q_chunks * Q_CHUNK + 2 * tile_bytes_of(Dk) + HALVES + 1024 + 128;
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
@@ -63,18 +74,30 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {  // when this thread's copies so far have landed
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// the two warps that hold the halves of 32 rows
+__device__ __forceinline__ void soft_sync(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(4 + quarter) : "memory"); }
+__device__ __forceinline__ void tmem_st16_raw(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-__global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const Params p) {
+__global__ void __launch_bounds__(NTHREADS, 1)
+latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* q_s = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int chunks = p.Dk / 64, q_chunks = max(chunks - 4, 0);
   uint8_t* kv_s = q_s + q_chunks * Q_CHUNK;
-  const int tile_bytes = chunks * K_CHUNK;
-  uint64_t* q_full = (uint64_t*)(kv_s + max(2 * tile_bytes, SOFT_WARPS * 32 * OUT_PITCH * 4));
+  const int tile_bytes = tile_bytes_of(p.Dk);
+  float* halves = (float*)(kv_s + 2 * tile_bytes);  // [2][ROWS]
+  uint64_t* q_full = (uint64_t*)(halves + 2 * ROWS);
   uint64_t* kv_full = q_full + 1;   // [2]
   uint64_t* kv_empty = kv_full + 2; // [2]
   uint64_t* s_full = kv_empty + 2;  // [2]
@@ -100,7 +123,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
   const int cols = (c_last - c_first) * 64;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 32 * (SOFT_WARPS + LOAD_WARPS));
+    mbar_init(q_full, 32 * SOFT_WARPS);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&kv_full[s], 32 * LOAD_WARPS);
       mbar_init(&kv_empty[s], 1);
@@ -119,56 +142,125 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // row r of the group: token r / HB, head head0 + r % HB
-  auto q_row = [&](int r) { return p.qk + ((size_t)(row0 + r / p.HB) * p.H + head0 + r % p.HB) * p.Dk; };
+  // The queries as bfloat16, by all but the contracting warp: row r of the group is token r / HB, head head0 + r % HB. The first
+  // 256 values are staged in the second key tile's memory for the threads that put them into tensor memory.
+  uint8_t* staged = kv_s + tile_bytes;
+  auto stage_queries = [&]() {
+    const int quads = p.Dk / 4;
+    for (int r0 = warp; r0 < ROWS; r0 += 4 * (SOFT_WARPS + LOAD_WARPS)) {
+      // four rows at a time, so that a warp has 20 loads in flight
+      float4 v[4][5];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + i * (SOFT_WARPS + LOAD_WARPS), tok = r / p.HB;
+        const float4* q = reinterpret_cast<const float4*>(p.qk + ((size_t)(row0 + tok) * p.H + head0 + r % p.HB) * p.Dk);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+          v[i][n] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (r < ROWS && tok < nrows && lane + 32 * n < quads) v[i][n] = __ldg(q + lane + 32 * n);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + i * (SOFT_WARPS + LOAD_WARPS);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+          const int e = lane + 32 * n, c = e >> 4, unit = (e >> 1) & 7;  // 16 quads a chunk, two a 16-byte unit
+          if (r < ROWS && e < quads)
+            *reinterpret_cast<uint2*>((c < 4 ? staged + c * Q_CHUNK : q_s + (c - 4) * Q_CHUNK) + r * 128 + ((unit ^ (r & 7)) << 4) + (e & 1) * 8) =
+                make_uint2(pack_bf16(v[i][n].x, v[i][n].y), pack_bf16(v[i][n].z, v[i][n].w));
+        }
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * (SOFT_WARPS + LOAD_WARPS)) : "memory");
+  };
 
   if (warp == MMA_WARP) {
     // ---- contractions (the whole warp walks the tiles, see elect_one)
     const uint32_t idesc_pv = instr_desc_b(true, cols);
-    auto scores = [&](int t) {
-      if (!warp_wait(&kv_full[t & 1], (t >> 1) & 1, p.err, abort_flag)) return false;
-      fence_proxy_async();  // the copies' writes (and the queries') to the tensor cores
-      tc_fence_after();
-      const uint32_t acc = tmem + S_AT + (t & 1) * KEYS;
-      const uint64_t kd = smem_desc(smem_u32(kv_s + (t & 1) * tile_bytes)), qd = smem_desc(smem_u32(q_s));
-      if (elect_one()) {
-        for (int c = 0; c < chunks; ++c) {
+    const uint64_t qd = smem_desc(smem_u32(q_s));
+    auto ready = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)); };
+    bool ok = warp_wait(q_full, 0, p.err, abort_flag);
+    int next_sc = 0, next_pv = 0;
+    unsigned spins = 0;
+    unsigned long long idle_since = 0;
+    // whatever is ready: the scores of tile t need its keys, and P of tile t - 2 to have left their buffer
+    while (ok && next_pv < n_tiles) {
+      bool progressed = false;
+      if (next_sc < n_tiles && next_sc <= next_pv + 1 && ready(&kv_full[next_sc & 1], (next_sc >> 1) & 1)) {
+        const int t = next_sc;
+        fence_proxy_async();  // the copies' writes (and the queries') to the tensor cores
+        tc_fence_after();
+        const uint32_t acc = tmem + S_AT + (t & 1) * KEYS;
+        const uint64_t kd = smem_desc(smem_u32(kv_s + (t & 1) * tile_bytes));
+        if (elect_one()) {
+          for (int c = 0; c < chunks; ++c) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint64_t b = kd + (uint64_t)((c * K_CHUNK + k * 32) >> 4);
-            if (c < 4) umma_bf16_tmem_a(acc, tmem + Q_AT + c * 32 + k * 8, b, instr_desc(KEYS), c > 0 || k > 0);
-            else umma_bf16(acc, qd + (uint64_t)(((c - 4) * Q_CHUNK + k * 32) >> 4), b, instr_desc(KEYS), 1);
+            for (int k = 0; k < 4; ++k) {
+              const uint64_t b = kd + (uint64_t)((c * K_CHUNK + k * 32) >> 4);
+              if (c < 4) umma_bf16_tmem_a(acc, tmem + Q_AT + c * 32 + k * 8, b, instr_desc(KEYS), c > 0 || k > 0);
+              else umma_bf16(acc, qd + (uint64_t)(((c - 4) * Q_CHUNK + k * 32) >> 4), b, instr_desc(KEYS), 1);
+            }
           }
+          umma_commit(&s_full[t & 1]);
         }
-        umma_commit(&s_full[t & 1]);
+        __syncwarp();
+        ++next_sc;
+        progressed = true;
       }
-      __syncwarp();
-      return true;
-    };
-    bool ok = warp_wait(q_full, 0, p.err, abort_flag) && scores(0);
-    for (int j = 0; ok && j < n_tiles; ++j) {
-      // (the buffer of tile j + 1 held P of tile j - 1, whose contraction was issued before)
-      if (j + 1 < n_tiles && !scores(j + 1)) break;
-      if (!warp_wait(p_full, j & 1, p.err, abort_flag)) break;
-      tc_fence_after();
-      const uint64_t vd = desc_mnmajor(smem_u32(kv_s + (j & 1) * tile_bytes + c_first * K_CHUNK), K_CHUNK, 1024);
-      if (elect_one()) {
+      if (next_pv < next_sc && ready(p_full, next_pv & 1)) {
+        const int j = next_pv;
+        tc_fence_after();
+        const uint64_t vd = desc_mnmajor(smem_u32(kv_s + (j & 1) * tile_bytes + c_first * K_CHUNK), K_CHUNK, 1024);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < KEYS / 16; ++k)
-          umma_bf16_tmem_a(tmem + O_AT, tmem + S_AT + (j & 1) * KEYS + k * 8, vd + (uint64_t)((k * 2048) >> 4), idesc_pv, j > 0 || k > 0);
-        umma_commit(&kv_empty[j & 1]);
-        umma_commit(pv_done);
+          for (int k = 0; k < KEYS / 16; ++k)
+            umma_bf16_tmem_a(tmem + O_AT, tmem + S_AT + (j & 1) * KEYS + k * 8, vd + (uint64_t)((k * 2048) >> 4), idesc_pv, j > 0 || k > 0);
+          umma_commit(&kv_empty[j & 1]);
+          umma_commit(pv_done);
+        }
+        __syncwarp();
+        ++next_pv;
+        progressed = true;
       }
-      __syncwarp();
+      if (progressed) {
+        idle_since = 0;
+      } else if ((++spins & 63u) == 0) {
+        if (__any_sync(0xffffffffu, *abort_flag)) break;
+        const unsigned long long now = __shfl_sync(0xffffffffu, global_ns(), 0);
+        if (idle_since == 0) {
+          idle_since = now;
+        } else if (now - idle_since > WAIT_LIMIT_NS) {
+          if (p.err && lane == 0) atomicExch(p.err, CUCA_ERR_WAIT_TIMEOUT);
+          *abort_flag = 1;
+          break;
+        }
+      }
     }
   } else if (warp >= SOFT_WARPS) {
-    // ---- key tiles: eight threads a key, 16 bytes each; then, after the first two, this CTA's queries in shared memory
+    // ---- key tiles: page by page through the copy engine; a tile with keys outside the group's by these threads, eight a key,
+    // 16 bytes each, with zeros there
     const int tid = threadIdx.x - 32 * SOFT_WARPS, piece = tid & 7;
     auto load_tile = [&](int t) {
-      const uint32_t dst = smem_u32(kv_s + (t & 1) * tile_bytes);
+      uint8_t* tile = kv_s + (t & 1) * tile_bytes;
+      const int key0 = first_key + t * KEYS;
+      if (p.tma && key0 >= lo && key0 + KEYS - 1 <= Pmax) {
+        if (tid == 0) mbar_expect_tx(&kv_full[t & 1], chunks * K_CHUNK);
+        const int c = tid % chunks, page = tid / chunks;
+        if (page * p.bs < KEYS) {
+          int blk = table[(key0 + page * p.bs) / p.bs];
+          if (blk < 0 || blk >= p.n_blocks) {
+            if (p.err) atomicExch(p.err, CUCA_ERR_BLOCK_RANGE);
+            blk = 0;
+          }
+          tma_load_2d(tile + c * K_CHUNK + page * p.bs * 128, &tmK, &kv_full[t & 1], c * 64, blk * p.bs);
+        }
+        if (tid != 0) mbar_arrive(&kv_full[t & 1]);
+        return;
+      }
 #pragma unroll
       for (int i = 0; i < KEYS / 16; ++i) {
-        const int j = tid / 8 + 16 * i, kp = first_key + t * KEYS + j;
+        const int j = tid / 8 + 16 * i, kp = key0 + j;
         bool valid = kp >= lo && kp <= Pmax;
         const bf16* src = p.pool;
         if (valid) {
@@ -180,50 +272,44 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
             src += ((size_t)blk * p.bs + kp % p.bs) * p.Dk;
           }
         }
-        const uint32_t at = dst + j * 128 + ((piece ^ (j & 7)) << 4);
+        const uint32_t at = smem_u32(tile) + j * 128 + ((piece ^ (j & 7)) << 4);
         for (int c = 0; c < chunks; ++c) cp_async16(at + c * K_CHUNK, valid ? src + c * 64 + piece * 8 : p.pool, valid);
       }
       cp_async_arrive(&kv_full[t & 1]);
     };
     load_tile(0);
-    if (n_tiles > 1) load_tile(1);
-    const int quads = (p.Dk - 256) / 4;  // of a row, behind its first 256 values
-    if (q_chunks) {
-#pragma unroll 4
-      for (int e = tid; e < ROWS * quads; e += 32 * LOAD_WARPS) {
-        const int r = e / quads, k = (e - r * quads) * 4, unit = (k >> 3) & 7;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r / p.HB < nrows) v = __ldg(reinterpret_cast<const float4*>(q_row(r) + 256 + k));
-        *reinterpret_cast<uint2*>(q_s + (k >> 6) * Q_CHUNK + r * 128 + ((unit ^ (r & 7)) << 4) + (k & 4) * 2) =
-            make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
-      }
+    stage_queries();
+    if (n_tiles > 1) {
+      // (the queries' staging lay in the second tile's memory: read by all before, and written by generic stores)
+      asm volatile("bar.sync 2, %0;" ::"n"(32 * (SOFT_WARPS + LOAD_WARPS)) : "memory");
+      fence_proxy_async();
+      load_tile(1);
+    } else {
+      asm volatile("bar.sync 2, %0;" ::"n"(32 * (SOFT_WARPS + LOAD_WARPS)) : "memory");
     }
-    mbar_arrive(q_full);
     for (int t = 2; t < n_tiles; ++t) {
       if (!warp_wait(&kv_empty[t & 1], ((t >> 1) & 1) ^ 1, p.err, abort_flag)) break;
       load_tile(t);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
-    // ---- a row a thread: its queries into tensor memory, then the softmax
-    const int r = warp * 32 + lane, tok = r / p.HB;
-    const uint32_t lane_bits = (uint32_t)(warp * 32) << 16;
+    // ---- two threads a row, 32 keys of a tile and half of the output columns each: first the queries into tensor memory
+    const int quarter = warp & 3, half = warp >> 2;
+    const int r = quarter * 32 + lane, tok = r / p.HB;
+    const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
     const bool row_ok = tok < nrows;
     const int row_pos = P0 + tok;
     const int row_lo = (p.window > 0 && row_pos - (p.window - 1) > 0) ? row_pos - (p.window - 1) : 0;
-    const float* q = q_row(row_ok ? r : 0);
+    stage_queries();
 #pragma unroll 1
-    for (int c = 0; c < min(chunks, 4); ++c) {
+    for (int c = half; c < min(chunks, 4); c += 2) {
       uint32_t w[32];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float4 v = __ldg(reinterpret_cast<const float4*>(q + c * 64) + i);
-        if (!row_ok) v = make_float4(0.f, 0.f, 0.f, 0.f);
-        w[2 * i] = pack_bf16(v.x, v.y);
-        w[2 * i + 1] = pack_bf16(v.z, v.w);
-      }
+      for (int u = 0; u < 8; ++u)
+        *reinterpret_cast<uint4*>(w + 4 * u) = *reinterpret_cast<const uint4*>(staged + c * Q_CHUNK + r * 128 + ((u ^ (r & 7)) << 4));
       tmem_st32_raw(tmem + lane_bits + Q_AT + c * 32, w);
     }
+    asm volatile("bar.sync 2, %0;" ::"n"(32 * (SOFT_WARPS + LOAD_WARPS)) : "memory");  // the staging memory is free
     tmem_st_wait();
     tc_fence_before();
     mbar_arrive(q_full);
@@ -235,24 +321,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
       if (!ok) break;
       tc_fence_after();
       const int key0 = first_key + j * KEYS;
-      uint32_t raw[2][32];
-      tmem_ld32_nowait(s_at, raw[0]);
-      tmem_ld32_nowait(s_at + 32, raw[1]);
+      uint32_t raw[32];
+      tmem_ld32_nowait(s_at + half * 32, raw);
       tmem_ld_wait();
       // scores that every row of the group sees go without tests
       const bool whole = nrows == TQ && key0 + KEYS - 1 <= P0 && (p.window <= 0 || key0 >= Pmax - (p.window - 1));
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          if (!whole) {
-            const int kp = key0 + c * 32 + i;
-            if (!(row_ok && kp <= row_pos && kp >= row_lo)) raw[c][i] = 0xff800000u;  // -inf
-          }
-          mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(raw[c][i]));
+      for (int i = 0; i < 32; ++i) {
+        if (!whole) {
+          const int kp = key0 + half * 32 + i;
+          if (!(row_ok && kp <= row_pos && kp >= row_lo)) raw[i] = 0xff800000u;  // -inf
         }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+        mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(raw[i]));
+      }
+      // the other half's maximum; behind the barrier both halves have read their scores, so P may take their place
+      halves[half * ROWS + r] = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      soft_sync(quarter);
+      const float mx = fmaxf(halves[r], halves[ROWS + r]) * p.scale_log2;
+      soft_sync(quarter);  // (both have read before either writes the next tile's)
       // The reference only moves when the maximum exceeds it by more than 8 (in log2 units): values up to 2^8 above it are
       // as exact in 32-bit sums and in bfloat16, and O is rescaled far less often.
       float m_new = m;
@@ -261,17 +348,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
       const float m_use = m_new == -INFINITY ? 0.f : m_new;
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), neg_m2 = make_float2(-m_use, -m_use);
-      uint32_t pw[32];
+      uint32_t pw[16];
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const float2 x2 = __ffma2_rn(make_float2(__uint_as_float(raw[c][2 * e]), __uint_as_float(raw[c][2 * e + 1])), scale2, neg_m2);
-          const float2 p2 = make_float2(fast_exp2(x2.x), fast_exp2(x2.y));
-          sum2[e & 1] = __fadd2_rn(sum2[e & 1], p2);
-          pw[c * 16 + e] = pack_bf16(p2.x, p2.y);
-        }
-      tmem_st32_raw(s_at, pw);
+      for (int e = 0; e < 16; ++e) {
+        const float2 x2 = __ffma2_rn(make_float2(__uint_as_float(raw[2 * e]), __uint_as_float(raw[2 * e + 1])), scale2, neg_m2);
+        const float2 p2 = make_float2(fast_exp2(x2.x), fast_exp2(x2.y));
+        sum2[e & 1] = __fadd2_rn(sum2[e & 1], p2);
+        pw[e] = pack_bf16(p2.x, p2.y);
+      }
+      tmem_st16_raw(s_at + half * 16, pw);
       l = l * corr + (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
       m = m_new;
       // the P V before this one has finished before O is rescaled (its phase is awaited every time, so that the barrier never
@@ -282,7 +367,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
         tc_fence_after();
         if (__any_sync(0xffffffffu, corr != 1.f)) {
 #pragma unroll 1
-          for (int c = 0; c < cols; c += 32) {
+          for (int c = half * 32; c < cols; c += 64) {
             float o[32];
             tmem_ld32(tmem + lane_bits + O_AT + c, o);
 #pragma unroll
@@ -297,13 +382,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
     }
     if (ok && warp_wait(pv_done, (n_tiles - 1) & 1, p.err, abort_flag)) {
       tc_fence_after();
+      halves[half * ROWS + r] = l;
+      soft_sync(quarter);
+      l = halves[r] + halves[ROWS + r];
       if (p.sink && m != -INFINITY) l += fast_exp2(p.sink[head0 + r % p.HB] * 1.4426950408889634f - m);
       const float inv = l > 0.f ? 1.f / l : 0.f;
       // every contraction is done, so the key tiles' memory is free: 32 columns at a time through this warp's share of it, so
       // that eight lanes store 128 bytes of a row
       float* mine = reinterpret_cast<float*>(kv_s) + warp * 32 * OUT_PITCH;
 #pragma unroll 1
-      for (int c = 0; c < cols; c += 32) {
+      for (int c = half * 32; c < cols; c += 64) {
         float o[32];
         tmem_ld32(tmem + lane_bits + O_AT + c, o);
 #pragma unroll
@@ -313,7 +401,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) latent_attention_tc_kernel(const 
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int rr = i * 4 + lane / 8, row = warp * 32 + rr, tk = row / p.HB;
+          const int rr = i * 4 + lane / 8, row = quarter * 32 + rr, tk = row / p.HB;
           if (tk < nrows)
             *reinterpret_cast<float4*>(p.out + ((size_t)(row0 + tk) * p.H + head0 + row % p.HB) * p.rank + c_first * 64 + c + lane % 8 * 4) =
                 *reinterpret_cast<const float4*>(mine + rr * OUT_PITCH + lane % 8 * 4);
@@ -357,9 +445,11 @@ CUCA_API int cuca_latent_attention_tc(const float* qk, float* out, const void* p
   p.seq_of_row = seq_of_row; p.tables = tables; p.table_stride = table_stride; p.tile_row0 = tile_row0;
   p.tile_nrows = tile_nrows; p.H = H; p.HB = ROWS / tokens; p.rank = rank; p.Dk = Dk;
   p.scale_log2 = scale * 1.4426950408889634f; p.window = window; p.sink = sink; p.parts = rank > 256 ? 2 : 1; p.err = err;
+  CUtensorMap tmK = {};
+  p.tma = bs >= 8 && bs <= KEYS && (bs & (bs - 1)) == 0 && cuca_tensor_map_bf16(pool, (uint64_t)n_blocks * bs, Dk, Dk, bs, &tmK);
   static const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(MAX_DK));
   CUCA_REQUIRE(e == cudaSuccess, "latent_attention_tc: %d bytes of shared memory were refused: %s", smem_bytes(MAX_DK), cudaGetErrorString(e));
-  cuca_launch(latent_attention_tc_kernel, dim3(n_groups, H / p.HB, p.parts), dim3(NTHREADS), smem_bytes(Dk), stream, true, p);
+  cuca_launch(latent_attention_tc_kernel, dim3(n_groups, H / p.HB, p.parts), dim3(NTHREADS), smem_bytes(Dk), stream, true, tmK, p);
   CUCA_CHECK_LAUNCH("latent_attention_tc");
   return 0;
 }
