@@ -77,15 +77,6 @@ struct Params {
   int* err;
 };
 
-// test_wait never suspends the thread (try_wait may, for a time the hardware chooses): for loops that watch
-// several barriers at once
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-  return ok != 0;
-}
 // cap tanh(s / cap) in log2 units from the raw score: tanh(y) = 1 - 2 / (e^(2 y) + 1), exact at both ends
 // (e^(2 y) = inf gives 1, 0 gives -1); `arg` = 2 scale log2(e) / cap, `cap_l2` = cap log2(e)
 __device__ __forceinline__ float capped_log2(float raw, float arg, float cap_l2) {

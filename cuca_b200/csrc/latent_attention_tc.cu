@@ -8,7 +8,7 @@
 //   S[128, 64]       = Q K^T     over Dk values; two score buffers, the scores one tile ahead of the softmax
 //   O[128, columns] += P V       V the same tile in shared memory, P written as bf16 over the scores it came from
 //
-// The 512 columns of tensor memory do not hold 512 columns of O beside the scores, so a CTA takes half of them (blockIdx.z) and
+// The 512 columns of tensor memory do not hold 512 columns of O beside the scores, so a CTA takes half of them and
 // makes the scores again: 1.3 times the arithmetic, no exchange between CTAs. The first 256 values of Q lie in tensor memory
 // too, the rest in shared memory beside two key tiles (64 x 576 values: 72 KB each, 227 KB in all).
 //
@@ -25,7 +25,7 @@ typedef __nv_bfloat16 bf16;
 constexpr int ROWS = 128, KEYS = 64;
 constexpr int Q_CHUNK = ROWS * 128, K_CHUNK = KEYS * 128;  // 64 values of every row
 constexpr int Q_COLS = 128;                                // tensor memory for the first 256 values of Q
-constexpr int MAX_DK = 576;
+constexpr int MAX_DK = 576;  // (two tiles of it and the queries' rest fill shared memory)
 constexpr int O_AT = 0, S_AT = 256, Q_AT = 384;            // columns of tensor memory
 constexpr int SOFT_WARPS = 8, LOAD_WARPS = 4, MMA_WARP = SOFT_WARPS + LOAD_WARPS;
 constexpr int NTHREADS = 32 * (MMA_WARP + 1);
@@ -43,7 +43,7 @@ struct Params {
   int table_stride;
   const int* tile_row0;
   const int* tile_nrows;
-  int H, HB, rank, Dk;
+  int H, HB, rank;
   float scale_log2;
   int window;
   const float* sink;
@@ -62,7 +62,7 @@ __host__ __device__ constexpr int tile_bytes_of(int Dk) {
   return bytes;
 }
 static_assert(OUT_BYTES / 2 % 1024 == 0, "tiles start at multiples of 1024 bytes");
-int smem_bytes(int Dk) {
+constexpr int smem_bytes(int Dk) {
   const int q_chunks = Dk / 64 > 4 ? Dk / 64 - 4 : 0;
   return q_chunks * Q_CHUNK + 2 * tile_bytes_of(Dk) + HALVES + 1024 + 128;
 }
@@ -89,13 +89,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+template <int CHUNKS>  // Dk / 64
 __global__ void __launch_bounds__(NTHREADS, 1)
 latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* q_s = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int chunks = p.Dk / 64, q_chunks = max(chunks - 4, 0);
+  constexpr int chunks = CHUNKS, Dk = 64 * CHUNKS, q_chunks = chunks > 4 ? chunks - 4 : 0;
   uint8_t* kv_s = q_s + q_chunks * Q_CHUNK;
-  const int tile_bytes = tile_bytes_of(p.Dk);
+  constexpr int tile_bytes = tile_bytes_of(Dk);
   float* halves = (float*)(kv_s + 2 * tile_bytes);  // [2][ROWS]
   uint64_t* q_full = (uint64_t*)(halves + 2 * ROWS);
   uint64_t* kv_full = q_full + 1;   // [2]
@@ -109,8 +110,9 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
 
   pdl_trigger();
   pdl_wait();
-  const int row0 = p.tile_row0[blockIdx.x], TQ = ROWS / p.HB;
-  const int nrows = min(p.tile_nrows[blockIdx.x], TQ);
+  const int tile = blockIdx.x, part = blockIdx.z;
+  const int row0 = p.tile_row0[tile], TQ = ROWS / p.HB;
+  const int nrows = min(p.tile_nrows[tile], TQ);
   const int seq = p.seq_of_row[row0];
   if (seq < 0 || nrows <= 0) return;  // (the same for every thread of the block)
   const int head0 = blockIdx.y * p.HB;
@@ -119,7 +121,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
   const int first_key = lo / KEYS * KEYS, n_tiles = Pmax / KEYS - lo / KEYS + 1;
   const int* table = p.tables + (size_t)seq * p.table_stride;
   // this CTA's output columns: whole chunks of 64
-  const int v_chunks = p.rank / 64, c_first = blockIdx.z * v_chunks / p.parts, c_last = (blockIdx.z + 1) * v_chunks / p.parts;
+  const int v_chunks = p.rank / 64, c_first = part * v_chunks / p.parts, c_last = (part + 1) * v_chunks / p.parts;
   const int cols = (c_last - c_first) * 64;
 
   if (threadIdx.x == 0) {
@@ -146,16 +148,16 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
   // 256 values are staged in the second key tile's memory for the threads that put them into tensor memory.
   uint8_t* staged = kv_s + tile_bytes;
   auto stage_queries = [&]() {
-    const int quads = p.Dk / 4;
+    constexpr int quads = Dk / 4, PER = (quads + 31) / 32;
     for (int r0 = warp; r0 < ROWS; r0 += 4 * (SOFT_WARPS + LOAD_WARPS)) {
       // four rows at a time, so that a warp has 20 loads in flight
-      float4 v[4][5];
+      float4 v[4][PER];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = r0 + i * (SOFT_WARPS + LOAD_WARPS), tok = r / p.HB;
-        const float4* q = reinterpret_cast<const float4*>(p.qk + ((size_t)(row0 + tok) * p.H + head0 + r % p.HB) * p.Dk);
+        const float4* q = reinterpret_cast<const float4*>(p.qk + ((size_t)(row0 + tok) * p.H + head0 + r % p.HB) * Dk);
 #pragma unroll
-        for (int n = 0; n < 5; ++n) {
+        for (int n = 0; n < PER; ++n) {
           v[i][n] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (r < ROWS && tok < nrows && lane + 32 * n < quads) v[i][n] = __ldg(q + lane + 32 * n);
         }
@@ -164,7 +166,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
       for (int i = 0; i < 4; ++i) {
         const int r = r0 + i * (SOFT_WARPS + LOAD_WARPS);
 #pragma unroll
-        for (int n = 0; n < 5; ++n) {
+        for (int n = 0; n < PER; ++n) {
           const int e = lane + 32 * n, c = e >> 4, unit = (e >> 1) & 7;  // 16 quads a chunk, two a 16-byte unit
           if (r < ROWS && e < quads)
             *reinterpret_cast<uint2*>((c < 4 ? staged + c * Q_CHUNK : q_s + (c - 4) * Q_CHUNK) + r * 128 + ((unit ^ (r & 7)) << 4) + (e & 1) * 8) =
@@ -179,7 +181,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
     // ---- contractions (the whole warp walks the tiles, see elect_one)
     const uint32_t idesc_pv = instr_desc_b(true, cols);
     const uint64_t qd = smem_desc(smem_u32(q_s));
-    auto ready = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)); };
+    auto ready = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)); };
     bool ok = warp_wait(q_full, 0, p.err, abort_flag);
     int next_sc = 0, next_pv = 0;
     unsigned spins = 0;
@@ -194,6 +196,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
         const uint32_t acc = tmem + S_AT + (t & 1) * KEYS;
         const uint64_t kd = smem_desc(smem_u32(kv_s + (t & 1) * tile_bytes));
         if (elect_one()) {
+#pragma unroll
           for (int c = 0; c < chunks; ++c) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -246,7 +249,8 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
       const int key0 = first_key + t * KEYS;
       if (p.tma && key0 >= lo && key0 + KEYS - 1 <= Pmax) {
         if (tid == 0) mbar_expect_tx(&kv_full[t & 1], chunks * K_CHUNK);
-        const int c = tid % chunks, page = tid / chunks;
+        // one copy a thread, dealt to the warps in turn: a lane's copy takes 70 clocks to issue
+        const int copy = lane * LOAD_WARPS + warp - SOFT_WARPS, c = copy % chunks, page = copy / chunks;
         if (page * p.bs < KEYS) {
           int blk = table[(key0 + page * p.bs) / p.bs];
           if (blk < 0 || blk >= p.n_blocks) {
@@ -269,10 +273,11 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
             if (p.err) atomicExch(p.err, CUCA_ERR_BLOCK_RANGE);
             valid = false;
           } else {
-            src += ((size_t)blk * p.bs + kp % p.bs) * p.Dk;
+            src += ((size_t)blk * p.bs + kp % p.bs) * Dk;
           }
         }
         const uint32_t at = smem_u32(tile) + j * 128 + ((piece ^ (j & 7)) << 4);
+#pragma unroll
         for (int c = 0; c < chunks; ++c) cp_async16(at + c * K_CHUNK, valid ? src + c * 64 + piece * 8 : p.pool, valid);
       }
       cp_async_arrive(&kv_full[t & 1]);
@@ -302,7 +307,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
     const int row_lo = (p.window > 0 && row_pos - (p.window - 1) > 0) ? row_pos - (p.window - 1) : 0;
     stage_queries();
 #pragma unroll 1
-    for (int c = half; c < min(chunks, 4); c += 2) {
+    for (int c = half; c < (chunks < 4 ? chunks : 4); c += 2) {
       uint32_t w[32];
 #pragma unroll
       for (int u = 0; u < 8; ++u)
@@ -421,6 +426,17 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
+template <int CHUNKS>
+int launch(const CUtensorMap& tmK, const Params& p, int n_groups, cudaStream_t stream) {
+  constexpr int smem = smem_bytes(64 * CHUNKS);
+  static_assert(smem <= 227 * 1024, "shared memory");
+  static const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel<CHUNKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  CUCA_REQUIRE(e == cudaSuccess, "latent_attention_tc: %d bytes of shared memory were refused: %s", smem, cudaGetErrorString(e));
+  cuca_launch(latent_attention_tc_kernel<CHUNKS>, dim3(n_groups, p.H / p.HB, p.parts), dim3(NTHREADS), smem, stream, true, tmK, p);
+  CUCA_CHECK_LAUNCH("latent_attention_tc");
+  return 0;
+}
+
 }  // namespace
 
 // Tokens of a portion that one group of the tcgen05 form takes, 0 if it refuses the sizes: Dk and rank multiples of 64, Dk up
@@ -439,17 +455,24 @@ CUCA_API int cuca_latent_attention_tc(const float* qk, float* out, const void* p
   const int tokens = cuca_latent_attention_tc_tokens(H, rank, Dk);
   CUCA_REQUIRE(tokens > 0, "latent_attention_tc: sizes H=%d rank=%d Dk=%d are not taken", H, rank, Dk);
   CUCA_REQUIRE((((uintptr_t)qk | (uintptr_t)out | (uintptr_t)pool) & 15) == 0, "latent_attention_tc: operands off 16 bytes");
+  CUCA_REQUIRE(n_groups < (1 << 30) && H / (ROWS / tokens) <= 65535, "latent_attention_tc: too many groups or heads");
   CUCA_REQUIRE(scale > 0.f, "latent_attention_tc: scale %g", scale);
   Params p;
   p.qk = qk; p.out = out; p.pool = (const bf16*)pool; p.n_blocks = n_blocks; p.bs = bs; p.positions = positions;
   p.seq_of_row = seq_of_row; p.tables = tables; p.table_stride = table_stride; p.tile_row0 = tile_row0;
-  p.tile_nrows = tile_nrows; p.H = H; p.HB = ROWS / tokens; p.rank = rank; p.Dk = Dk;
+  p.tile_nrows = tile_nrows; p.H = H; p.HB = ROWS / tokens; p.rank = rank;
   p.scale_log2 = scale * 1.4426950408889634f; p.window = window; p.sink = sink; p.parts = rank > 256 ? 2 : 1; p.err = err;
   CUtensorMap tmK = {};
   p.tma = bs >= 8 && bs <= KEYS && (bs & (bs - 1)) == 0 && cuca_tensor_map_bf16(pool, (uint64_t)n_blocks * bs, Dk, Dk, bs, &tmK);
-  static const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(MAX_DK));
-  CUCA_REQUIRE(e == cudaSuccess, "latent_attention_tc: %d bytes of shared memory were refused: %s", smem_bytes(MAX_DK), cudaGetErrorString(e));
-  cuca_launch(latent_attention_tc_kernel, dim3(n_groups, H / p.HB, p.parts), dim3(NTHREADS), smem_bytes(Dk), stream, true, tmK, p);
-  CUCA_CHECK_LAUNCH("latent_attention_tc");
-  return 0;
+  switch (Dk / 64) {
+    case 1: return launch<1>(tmK, p, n_groups, stream);
+    case 2: return launch<2>(tmK, p, n_groups, stream);
+    case 3: return launch<3>(tmK, p, n_groups, stream);
+    case 4: return launch<4>(tmK, p, n_groups, stream);
+    case 5: return launch<5>(tmK, p, n_groups, stream);
+    case 6: return launch<6>(tmK, p, n_groups, stream);
+    case 7: return launch<7>(tmK, p, n_groups, stream);
+    case 8: return launch<8>(tmK, p, n_groups, stream);
+    default: return launch<9>(tmK, p, n_groups, stream);
+  }
 }

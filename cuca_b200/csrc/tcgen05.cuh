@@ -57,6 +57,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   }
   return true;
 }
+// test_wait never suspends the thread (try_wait may, for a time the hardware chooses): for loops that watch
+// several barriers at once
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
 // A warp's wait. Every lane asks: one lane that tells the others adds some 60 clocks to each turn of a ring.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, volatile int* abort) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, abort));
