@@ -10,7 +10,7 @@
 // for each K step by a warp that walks the loop together (see elect_one); with one thread in a branch of its own the steps
 // of 256 x 256 tiles were bound by their issue (gate/up of 2,048 tokens 326 us, 303 now; a decode step of one request 2 % less).
 //
-// Two orientations share the code. Up to 256 tokens (decode, short portions; SwiGLU up to 64), the weight is the 128-row
+// Two orientations share the code. Over few tokens (decode, short portions: see `swapped`), the weight is the 128-row
 // MMA operand and the tokens are the N dimension (16..256): D[feature, token], one TMEM lane per output feature. Above, the tokens
 // are the 128-row operand and 256 weight rows the N dimension: D[token, feature], so a thread owns a run of
 // consecutive features of one token and stores vectors. For SwiGLU the gate and up tiles accumulate side by
@@ -40,7 +40,7 @@
 
 namespace {
 
-constexpr int SWAP_MAX_TOKENS = 256;  // up to here the weights are the 128-row operand and the tokens the columns
+constexpr int SWAP_MAX_TOKENS = 256;  // most tokens as columns of the form with the weights as the 128-row operand
 // SwiGLU: up to here. Beyond, its two accumulators leave no room in the tensor memory for a second tile's, and the
 // token-row forms are as fast or faster (measured on the Llama-3.1-8B widths, us: 65..128 tokens 46.0-46.5 against
 // 46.4-49.4 this way; 129..256 tokens 55.4-59.3 in the tall form against 56.7-65.7).
@@ -1126,6 +1126,19 @@ static bool pair_partial_takes(int M, int N) {
 // -1 as the environment variable CUCA_GEMM_PAIR says (1 without it).
 CUCA_API void cuca_gemm_pair_mode(int mode) { allow_pair = mode; }
 
+// Whether the weights are the 128-row operand. A result stored (or added into the stream) at once is better off with the
+// tokens as rows from few tokens on: its column pieces take all of K each and add nothing up. Measured, us (weights as rows,
+// tokens as rows): K = 2,048, N = 2,048, 32 tokens 18.5, 16.4; 64 tokens 25.6, 16.4; 128 tokens 38.0, 16.4; 256 tokens 67.6,
+// 16.4; N = 20,480, 32 tokens 31.6, 30.7; 64 tokens 33.8, 30.7. K = 4,096, N = 6,144, 32 tokens 24.6, 26.6; 64 tokens 28.6,
+// 26.6; 90 tokens 34.8, 26.7. K = 8,192, N = 2,048, 64 tokens 30.7, 38.9; 90 tokens 43.0, 38.9; 256 tokens 71.7, 38.9.
+// K = 14,336 into the stream, 128 tokens 45.1, 69.7; 256 tokens 63.5, 55.3. Up to 32 tokens they differ by a few us either way.
+static bool swapped(int M, int K, int epilogue, bool rows_of_16_bytes) {
+  if (epilogue == EPI_SWIGLU) return M <= SWAP_MAX_TOKENS_SWIGLU;
+  if (epilogue == EPI_PARTIAL || !rows_of_16_bytes) return M <= SWAP_MAX_TOKENS;
+  if (K > 8192) return M <= (epilogue == EPI_RESIDUAL ? 128 : SWAP_MAX_TOKENS);
+  return M <= (K > 2048 ? 64 : 32);
+}
+
 // out = epilogue(A[M,K] W[N,K]^T), bf16 operands. workspace/counters: scratch for tiles split along K
 // (ws_bytes of 32-bit partials; n_counters zeroed ints, left zeroed). max_splits <= 1: whole tiles only.
 static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* out, int out_dtype, int M, int N,
@@ -1164,7 +1177,9 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
     const int pairs = units < sms_pairs() ? (int)units : sms_pairs();
     return launch_pair<false>(tmA, tmB, tmO, p, 2 * pairs, stream);
   }
-  const bool swap = M <= (epilogue == EPI_SWIGLU ? SWAP_MAX_TOKENS_SWIGLU : SWAP_MAX_TOKENS);
+  const int out_bytes = out_dtype == CUCA_F32 ? 4 : 2;
+  const bool rows_of_16_bytes = ((uintptr_t)out & 15) == 0 && ((size_t)ldo * out_bytes) % 16 == 0;
+  const bool swap = swapped(M, K, epilogue, rows_of_16_bytes);
   const int bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
   const uint64_t w_rows = (uint64_t)N * (dual ? 2 : 1);
   CUtensorMap tmA, tmB, tmO;
@@ -1176,9 +1191,7 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
     CUCA_REQUIRE(cuca_tensor_map_bf16(A, M, K, lda, TILE_A, &tmA), "gemm_tc: activation tensor map failed");
     CUCA_REQUIRE(cuca_tensor_map_bf16(W, w_rows, K, K, 128, &tmB), "gemm_tc: weight tensor map failed");
     // whole tiles leave through the copy engine where the output's rows are 16-byte multiples
-    const int esize = out_dtype == CUCA_F32 ? 4 : 2;
-    if (((uintptr_t)out & 15) == 0 && ((size_t)ldo * esize) % 16 == 0)
-      tma_out = cuca_tensor_map_2d(out, esize, M, N, ldo, 32, &tmO) ? 1 : 0;
+    if (rows_of_16_bytes) tma_out = cuca_tensor_map_2d(out, out_bytes, M, N, ldo, 32, &tmO) ? 1 : 0;
   }
   if (!tma_out) tmO = tmA;  // unused
   Params p;
@@ -1252,11 +1265,13 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
   p.pieces = p.piece_w = 0;
   p.per_tile = 1;
   p.max_parts = 1;
-  // Tokens as rows (more than 256 of them), fewer tiles than SMs, K not long: column pieces as narrow as it takes for about one per SM,
-  // each over all of K, so nothing is added up afterwards. (Measured at 256 tokens, K = 4096: 31 us against 57 us
-  // with K slices; with K = 14336 no gain. A piece's main loop runs at the pace of its loads, 4 stages deep, not
-  // of its MMAs, so a piece takes as long as a whole tile: cutting the last round of many tiles this way gains
-  // nothing and is not done.)
+  // Tokens as rows, fewer tiles than SMs, K not long: column pieces as narrow as it takes for about one per SM, each over all
+  // of K, so nothing is added up afterwards; where even the narrowest are few, those, or whole tiles where a tile is as
+  // narrow. A piece's main loop runs at the pace of its loads, 330 ns a K step whatever its width, so few pieces cost idle
+  // SMs but no time, while K slices added up by the last to arrive cost 40 us more than their share of K. Measured, us
+  // (slices, pieces): K = 2,048, 256 tokens, N = 2,048 53, 16.4; N = 256 63, 16.4; 1,000 tokens, N = 256 55, 16.4; K = 8,192, N =
+  // 2,048, 256 tokens 58, 38.9; into the stream, K = 4,096, N = 1,024 109, 23.6. At K = 14,336 pieces gain nothing. Cutting the
+  // last round of many tiles this way gains nothing either and is not done.
   bool pieced = false;
   if (tall) {
     // whole tiles in turn, nothing split
@@ -1265,14 +1280,15 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
     for (int w = unit; w < out_cols && !pieced; w += unit) {
       const int pieces = p.tiles_a * ((N + w - 1) / w);
       if (pieces > sms) continue;
-      if (pieces * 2 < sms || pieces <= p.tiles) break;  // too few even at the narrowest: K is shared out below instead
+      if (pieces <= p.tiles) break;
       pieced = true;
       p.pieces = pieces;
       p.piece_w = w;
       grid = pieces;
     }
   }
-  if (pieced || tall) {
+  if (pieced || tall || (!swap && p.tiles < sms && p.ksteps <= 128)) {
+    // nothing is split along K
   } else if (epilogue == EPI_PARTIAL) {
     CUCA_REQUIRE(swap && out_dtype == CUCA_F32 && bias == nullptr && n_slices_out != nullptr,
                  "gemm_tc: partial sums are for up to %d tokens, 32-bit, without bias", SWAP_MAX_TOKENS);

@@ -157,6 +157,31 @@ def test_gemm_simt_of_16_bit_operands_is_the_32_bit_ones_result(dev, K, epilogue
         assert torch.equal(out, want[:65].to(torch.bfloat16))
 
 
+# where the operands change places (32, 64, 128, 256 tokens; K of 2,048, 8,192 and more), few column pieces, tiles narrower
+# than a piece, output rows that take no 16-byte copies
+@pytest.mark.parametrize("M,N,K", [(32, 192, 2048), (33, 192, 2048), (64, 64, 2056), (65, 256, 4096), (128, 576, 8192), (128, 200, 8200),
+                                   (129, 576, 8200), (256, 42, 136), (257, 264, 72), (700, 64, 1024), (1000, 256, 320)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+def test_gemm_tcgen05_where_its_form_changes(dev, M, N, K, epilogue):
+    """Against 32-bit math on the same bf16 inputs, the same bits again; the bounds are those of the test below."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(M + N * 5 + K)
+    a = torch.randn(M, K, device=dev, generator=g).bfloat16()
+    w = (torch.randn((2 if epilogue == 2 else 1) * N, K, device=dev, generator=g) / math.sqrt(K)).bfloat16()
+    bias = torch.randn(N, device=dev, generator=g).bfloat16() if epilogue != 2 else None
+    prior = torch.randn(M, N, device=dev, generator=g).to(torch.float32 if epilogue == 1 else torch.bfloat16)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    outs = []
+    for _ in range(2):
+        out = prior.clone()
+        ops.gemm_tc(a, w, out, epilogue, bias, err)
+        outs.append(out)
+    ref = _ref_gemm(a, w, epilogue, bias, prior.float())
+    assert int(err.item()) == 0 and torch.equal(outs[0], outs[1])
+    tol = 1e-3 if epilogue == 1 else 2e-2
+    assert torch.allclose(outs[0].float(), ref, atol=tol, rtol=tol)
+
+
 @pytest.mark.parametrize("M,N,K", GEMM_SHAPES)
 @pytest.mark.parametrize("epilogue", [0, 1, 2])
 @pytest.mark.parametrize("max_splits", [1, 16])
