@@ -1308,7 +1308,12 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
     // If a whole number of CTAs per tile fills most of the GPU, every CTA gets one even K slice of one tile (one
     // accumulator drain each); else the K steps are dealt out evenly across tile borders.
     const int per_tile = sms / p.tiles;
-    if (per_tile >= 1 && (long long)per_tile * p.tiles * 4 >= 3LL * sms && p.ksteps >= 2 * per_tile) {
+    if (swap && bn > 16 && 20 * p.tiles >= 8 * sms && p.tiles < sms) {
+      // Tiles for 40 % of the SMs and more over 17 to 64 tokens: one whole tile per CTA. What the last to arrive has to add grows
+      // with the tokens (measured in a chain of launches, us, K shared out and whole: SwiGLU of 2 x 11,008 x 4,096, 86 tiles, 24
+      // tokens 38.1, 34.5; 64 tokens 51.8, 39.7; 2 x 8,192 x 2,048, 64 tiles, 18.8, 17.7 and 25.5, 23.0; up to 16 tokens equal).
+      grid = p.tiles;
+    } else if (per_tile >= 1 && (long long)per_tile * p.tiles * 4 >= 3LL * sms && p.ksteps >= 2 * per_tile) {
       size_t need = (size_t)p.tiles * per_tile * ncols * TILE_A * sizeof(float);
       if (per_tile == 1) {
         grid = p.tiles;  // one CTA per tile, nothing to add up
