@@ -860,6 +860,34 @@ def test_rope_store_from_partial_sums(dev):
         assert torch.allclose(vpool[page, :, off].float(), heads[nh + nkv:], atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("d,n_slices", [(128, 3), (64, 1), (8, 5), (72, 4)])
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_rope_store_partial_sixteen_bytes_at_a_time(dev, d, n_slices, with_bias):
+    """The form of 16-byte pieces gives the bits of the form of single values (which a table off 16 bytes makes the library
+    take); heads that end inside a block, rows of padding, a position behind the table, which both report."""
+    from cuca_b200.kernels import ops
+    nh, nkv, bs, T = 5, 3, 16, 37
+    g = torch.Generator(device=dev).manual_seed(d + n_slices)
+    width = (nh + 2 * nkv) * d
+    slices = torch.randn(n_slices, T, width, device=dev, generator=g)
+    bias = torch.randn(width, device=dev, generator=g).to(torch.bfloat16) if with_bias else None
+    seq = torch.tensor([(-1 if i % 7 == 3 else i % 2) for i in range(T)], dtype=torch.int32, device=dev)
+    positions = torch.arange(T, device=dev, dtype=torch.int32)
+    tables = torch.tensor([[4, 1, 0], [2, 5, 3]], dtype=torch.int32, device=dev)
+    angle = torch.rand(T - 1, d // 2, device=dev, generator=g) * 6
+    got = []
+    for off in (0, 1):
+        cos, sin = (torch.empty(angle.numel() + off, device=dev)[off:].view(angle.shape).copy_(f(angle)) for f in (torch.cos, torch.sin))
+        kpool = torch.zeros(6, nkv, bs, d, device=dev, dtype=torch.bfloat16)
+        vpool, q = torch.zeros_like(kpool), torch.zeros(T, nh * d, device=dev, dtype=torch.bfloat16)
+        err = torch.zeros(1, dtype=torch.int32, device=dev)
+        ops.rope_store_partial(ops.PartialSums(slices, n_slices), bias, q, positions, seq, tables, cos, sin, d, kpool, vpool, bs,
+                               nh, nkv, d, err)
+        assert int(err.item()) != 0
+        got.append((q, kpool, vpool))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and all(bool(t.any()) for t in got[0])
+
+
 @pytest.mark.parametrize("nh,nkv,bs,window", [(4, 2, 16, None), (8, 8, 32, None), (8, 2, 16, 150), (2, 1, 8, None),
                                               (3, 1, 64, 40)])
 @pytest.mark.parametrize("d", [128, 64])
