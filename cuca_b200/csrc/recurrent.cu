@@ -211,6 +211,7 @@ __global__ void causal_conv_many_kernel(const float* __restrict__ in, int ld_in,
 }
 
 constexpr int SSM_MAX_STATE = 1024;
+constexpr int SSM_SEGMENT = 512;  // tokens of a segment (below)
 
 // One block per (head, request, run of PB value columns); a column's state rows lie with NS threads (see Split).
 // state: [slots, H, P, N]. xbc: 32-bit [rows, H P + 2 G N] after the convolution (x | B | C); dt_raw: rows of stride
@@ -223,7 +224,8 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
                 const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                 const float* __restrict__ d_skip, float* __restrict__ state, float* __restrict__ y,
                 const int* __restrict__ req_row0, const int* __restrict__ req_count,
-                const int* __restrict__ slots, int H, int P, int N, int G, int wide) {
+                const int* __restrict__ slots, int H, int P, int N, int G, int wide, float* __restrict__ ends,
+                float* __restrict__ decays) {
   constexpr int NS = S_::NS, NC = S_::NC, DP = S_::DP, PB = S_::PB, TC = S_::TC, PAIRS = S_::PAIRS;
   constexpr int PER = 2 * DP + ((PB + 1 + 3) & ~3);  // a token: B, C, the block's x, the raw step size
   static_assert(TC <= 32, "a lane a token");
@@ -231,8 +233,10 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
   __shared__ float steps[4][TC][2];  // a warp's own: step size, decay
   pdl_trigger();
   pdl_wait();
-  const int h = blockIdx.x, q = blockIdx.y;
-  const int slot = slots[q], n = req_count[q], r0 = req_row0[q];
+  // with `ends`, a segment of the request: from no state but the first, and its state goes there (see ssm_join_kernel)
+  const int h = blockIdx.x % H, seg = blockIdx.x / H, q = blockIdx.y;
+  const int slot = slots[q], whole = req_count[q], n = ends ? min(SSM_SEGMENT, whole - seg * SSM_SEGMENT) : whole;
+  const int r0 = req_row0[q] + seg * SSM_SEGMENT;
   if (slot < 0 || n <= 0) return;
   const int lane = threadIdx.x & 31;
   const int col_local = threadIdx.x / NS, s = threadIdx.x % NS;
@@ -242,7 +246,10 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
   const int C = H * P + 2 * G * N;
   float* st = state + (((size_t)slot * H + h) * P + (cols > 0 ? col0 + at : 0)) * N;
   f32x2 S[NC][PAIRS];
-  load_rows<S_>(S, st, s, N, cols, wide);
+  load_rows<S_>(S, st, s, N, seg > 0 ? 0 : cols, wide);
+  const size_t cell = ((size_t)seg * gridDim.y + q) * H + h;
+  if (ends && whole > SSM_SEGMENT) st = ends + (cell * P + (cols > 0 ? col0 + at : 0)) * N;
+  float product = 1.f;  // of the decays
   const float A = -expf(a_log[h]);
   const float bias = dt_bias[h], D = d_skip[h];
   // what no copy writes: rows from N on (B = C = 0) and the values of columns from P on
@@ -308,6 +315,7 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
         staged_values<NC>(x, tok + 2 * DP, at);
         const float dt = mine[t + i][0];
         const f32x2 decay = f2_both(mine[t + i][1]);
+        product *= mine[t + i][1];
 #pragma unroll
         for (int j = 0; j < NC; ++j) {
           const f32x2 dx = f2_both(dt * x[j]);
@@ -328,6 +336,115 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
     __syncthreads();  // this run is read to the end before the run after next is copied over it
   }
   store_rows<S_>(S, st, s, N, cols, wide);
+  if (ends && threadIdx.x == 0 && blockIdx.z == 0) decays[cell] = product;
+}
+
+// What a segment's tokens owe to the segments before it. A prompt's scan is 2,048 steps one behind the other in a warp a
+// scheduler, so it is cut into segments that run side by side, each from no state; with S the state a segment should have
+// begun with, its outputs lack C_t S times the decays since, and the state behind it lacks S times all of its decays.
+// One block per (head, request, JOIN tokens of a segment behind the first): S from the segments' ends in turn, then 64
+// tokens x 64 columns at a time as a contraction in 32 bits, 4 x 4 outputs a thread, bound by shared memory. 64 heads of
+// 64 x 128, 2,048 tokens in four segments: scan 340 -> 218 us and 80 for this. Requests of one segment are scanned as before.
+constexpr int JOIN = 256, JOIN_P = 64, JOIN_PITCH = JOIN_P + 4;
+// a state's share behind a decay that may have come out as zero: what is no number stays so, as it does token by token
+__device__ __forceinline__ float decayed(float d, float v) { return d > 0.f ? d * v : (fabsf(v) <= 3.402823466e38f ? 0.f : v); }
+__global__ void __launch_bounds__(256)
+ssm_join_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, int ld_dt, int dt_col,
+                const float* __restrict__ dt_bias, const float* __restrict__ a_log, float* __restrict__ state,
+                float* __restrict__ y, const int* __restrict__ req_row0, const int* __restrict__ req_count,
+                const int* __restrict__ slots, int H, int P, int N, int G, const float* __restrict__ ends,
+                const float* __restrict__ decays) {
+  extern __shared__ __align__(16) float sm[];
+  float* S = sm;                        // [N][JOIN_PITCH]
+  float* Cs = S + N * JOIN_PITCH;       // [64][N + 4]
+  float* since = Cs + 64 * (N + 4);     // [SSM_SEGMENT]: the decays of the segment up to and with each token
+  pdl_trigger();
+  pdl_wait();
+  const int h = blockIdx.x, q = blockIdx.y, tid = threadIdx.x;
+  const int seg = 1 + blockIdx.z / (SSM_SEGMENT / JOIN), part0 = blockIdx.z % (SSM_SEGMENT / JOIN) * JOIN;
+  const int slot = slots[q], whole = req_count[q], n = min(SSM_SEGMENT, whole - seg * SSM_SEGMENT);
+  if (slot < 0 || n <= part0) return;
+  const int g = h / (H / G), C = H * P + 2 * G * N, row0 = req_row0[q] + seg * SSM_SEGMENT;
+  const bool last = part0 == 0 && (seg + 1) * SSM_SEGMENT >= whole;  // this block leaves the request's state behind
+  auto cell = [&](int k) { return ((size_t)k * gridDim.y + q) * H + h; };
+  for (int e = tid; e < P * N; e += 256) {
+    float v = ends[cell(0) * P * N + e];
+    for (int k = 1; k < seg; ++k) v = decayed(decays[cell(k)], v) + ends[cell(k) * P * N + e];
+    S[e % N * JOIN_PITCH + e / N] = v;
+    if (last) state[((size_t)slot * H + h) * P * N + e] = decayed(decays[cell(seg)], v) + ends[cell(seg) * P * N + e];
+  }
+  for (int e = tid; e < N * (JOIN_P - P); e += 256) S[e / (JOIN_P - P) * JOIN_PITCH + P + e % (JOIN_P - P)] = 0.f;
+  const int end = min(n, part0 + JOIN);
+  const float A = -expf(a_log[h]), bias = dt_bias[h];
+  for (int t = tid; t < end; t += 256) {
+    const float raw = dt_raw[(size_t)(row0 + t) * ld_dt + dt_col + h] + bias;
+    since[t] = expf(A * (raw > 20.f ? raw : log1pf(expf(raw))));
+  }
+  __syncthreads();
+  if (tid < 32) {  // products up to each token: a run of 16 a lane, then over the lanes
+    constexpr int RUN = SSM_SEGMENT / 32;
+    float p = 1.f;
+    for (int i = 0; i < RUN; ++i) {
+      const int t = tid * RUN + i;
+      if (t < end) since[t] = p *= since[t];
+    }
+    float before = p;
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, before, o);
+      if (tid >= o) before *= v;
+    }
+    before = __shfl_up_sync(0xffffffffu, before, 1);
+    if (tid > 0)
+      for (int i = 0; i < RUN; ++i)
+        if (tid * RUN + i < end) since[tid * RUN + i] *= before;
+  }
+  const int tx = tid % 16, ty = tid / 16;
+  for (int t0 = part0; t0 < end; t0 += 64) {
+    __syncthreads();  // (the products are there; the tile before is read)
+    for (int e = tid; e < 64 * (N / 4); e += 256) {
+      const int t = e / (N / 4), k = e % (N / 4) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t0 + t < end) v = *reinterpret_cast<const float4*>(xbc + (size_t)(row0 + t0 + t) * C + H * P + (G + g) * N + k);
+      *reinterpret_cast<float4*>(Cs + t * (N + 4) + k) = v;
+    }
+    __syncthreads();
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < N; k += 4) {
+      float4 c[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) c[i] = *reinterpret_cast<const float4*>(Cs + (ty + 16 * i) * (N + 4) + k);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 b = *reinterpret_cast<const float4*>(S + (k + u) * JOIN_PITCH + 4 * tx);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float cu = u == 0 ? c[i].x : u == 1 ? c[i].y : u == 2 ? c[i].z : c[i].w;
+          acc[i][0] = fmaf(cu, b.x, acc[i][0]);
+          acc[i][1] = fmaf(cu, b.y, acc[i][1]);
+          acc[i][2] = fmaf(cu, b.z, acc[i][2]);
+          acc[i][3] = fmaf(cu, b.w, acc[i][3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = t0 + ty + 16 * i;
+      if (t >= end || 4 * tx >= P) continue;
+      float4* at = reinterpret_cast<float4*>(y + (size_t)(row0 + t) * (H * P) + h * P + 4 * tx);
+      float4 v = *at;
+      const float d = since[t];
+      v.x += decayed(d, acc[i][0]);
+      v.y += decayed(d, acc[i][1]);
+      v.z += decayed(d, acc[i][2]);
+      v.w += decayed(d, acc[i][3]);
+      *at = v;
+    }
+  }
 }
 
 // One block per (row, part). v = y * silu(z); out = v * rsqrt(mean over the part (v^2) + eps) * w.
@@ -459,31 +576,53 @@ CUCA_API int cuca_causal_conv(const float* in, int ld_in, int col0, const void* 
   return 0;
 }
 
+// Tokens of a segment, and whether the sizes allow segments.
+CUCA_API int cuca_ssm_segment() { return SSM_SEGMENT; }
+CUCA_API int cuca_ssm_segments_allowed(int P, int N) { return P > 0 && P <= JOIN_P && P % 4 == 0 && N > 0 && N <= 128 && N % 4 == 0; }
+
+// n_segments > 1: no request brings more than n_segments runs of cuca_ssm_segment() tokens, and one with more than one run has
+// them walked side by side (another rounding); scratch: n_segments n_seqs H (P N + 1) floats, 16-byte aligned.
 CUCA_API int cuca_ssm_scan(const float* xbc, const float* dt_raw, int ld_dt, int dt_col, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, float* y, const int* req_row0,
-                           const int* req_count, const int* slots, int n_seqs, int H, int P, int N, int G,
-                           cudaStream_t stream) {
+                           const int* req_count, const int* slots, int n_seqs, int H, int P, int N, int G, int n_segments,
+                           float* scratch, cudaStream_t stream) {
   if (n_seqs == 0) return 0;
   CUCA_REQUIRE(H > 0 && P > 0 && N > 0 && G > 0 && H % G == 0, "ssm_scan: bad sizes heads=%d vdim=%d state=%d groups=%d",
                H, P, N, G);
   CUCA_REQUIRE(n_seqs <= 65535, "ssm_scan: %d requests exceed the launch limit", n_seqs);
   CUCA_REQUIRE(N <= SSM_MAX_STATE, "ssm_scan: state size %d exceeds %d", N, SSM_MAX_STATE);
   const int wide = N % 4 == 0 && (H * P) % 4 == 0 && (((uintptr_t)xbc | (uintptr_t)state) & 15) == 0;
+  const bool cut = n_segments > 1 && scratch;
+  CUCA_REQUIRE(!cut || (cuca_ssm_segments_allowed(P, N) && (((uintptr_t)xbc | (uintptr_t)state | (uintptr_t)y | (uintptr_t)scratch) & 15) == 0 &&
+                        (long long)H * n_segments < (1ll << 31) && n_segments <= 16384), "ssm_scan: %d segments of %d x %d", n_segments, P, N);
+  float* ends = cut ? scratch : nullptr;
+  float* decays = cut ? scratch + (size_t)n_segments * n_seqs * H * P * N : nullptr;
   auto go = [&](auto split) {
     using C = decltype(split);
-    return launch_scan<C>("ssm_scan", ssm_scan_kernel<C>, 2 * C::DP + ((C::PB + 4) & ~3), H, n_seqs, P, stream, xbc, dt_raw,
-                          ld_dt, dt_col, dt_bias, a_log, d_skip, state, y, req_row0, req_count, slots, H, P, N, G, wide);
+    return launch_scan<C>("ssm_scan", ssm_scan_kernel<C>, 2 * C::DP + ((C::PB + 4) & ~3), cut ? H * n_segments : H, n_seqs, P, stream,
+                          xbc, dt_raw, ld_dt, dt_col, dt_bias, a_log, d_skip, state, y, req_row0, req_count, slots, H, P, N, G, wide,
+                          ends, decays);
   };
   // Few state values a column: threads of four rows, so that a block's columns are no more than a head has (64). Measured
   // with eight and four rows a thread, us: 80 heads of 64 x 16, 1,501 tokens 365, 205, 256 requests of a token 77, 48; 24
   // heads of 64 x 64, 1,501 tokens 344, 197, 64 prompts of 40 52, 58 (as at 64 x 128: 249, 296, so eight rows stay there).
-  if (N <= 16) return go(Split<4, 4, 2>());
-  if (N <= 32) return go(Split<8, 4, 4>());
-  if (N <= 64) return go(Split<16, 4, 4>());
-  if (N <= 128) return go(Split<16, 8, 4>());
-  if (N <= 256) return go(Split<32, 8, 4>());
-  if (N <= 512) return go(Split<32, 16, 4>());
-  return go(Split<32, 32, 2>());
+  int rc;
+  if (N <= 16) rc = go(Split<4, 4, 2>());
+  else if (N <= 32) rc = go(Split<8, 4, 4>());
+  else if (N <= 64) rc = go(Split<16, 4, 4>());
+  else if (N <= 128) rc = go(Split<16, 8, 4>());
+  else if (N <= 256) rc = go(Split<32, 8, 4>());
+  else if (N <= 512) rc = go(Split<32, 16, 4>());
+  else rc = go(Split<32, 32, 2>());
+  if (rc || !cut) return rc;
+  const int smem = (N * JOIN_PITCH + 64 * (N + 4) + SSM_SEGMENT) * 4;
+  static const cudaError_t e = cudaFuncSetAttribute(ssm_join_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (128 * JOIN_PITCH + 64 * 132 + SSM_SEGMENT) * 4);
+  CUCA_REQUIRE(e == cudaSuccess, "ssm_scan: %d bytes of shared memory were refused: %s", smem, cudaGetErrorString(e));
+  cuca_launch(ssm_join_kernel, dim3(H, n_seqs, (n_segments - 1) * (SSM_SEGMENT / JOIN)), dim3(256), smem, stream, true, xbc, dt_raw,
+              ld_dt, dt_col, dt_bias, a_log, state, y, req_row0, req_count, slots, H, P, N, G, (const float*)ends, (const float*)decays);
+  CUCA_CHECK_LAUNCH("ssm_join");
+  return 0;
 }
 
 CUCA_API int cuca_gated_group_norm(const float* y, const float* z, int ld_z, const void* w, int w_dtype, void* out,

@@ -96,6 +96,54 @@ def test_state_scan_alone(rt32, P, N):
     assert torch.equal(got[4], state[4])
 
 
+@pytest.mark.parametrize("P, N", [(64, 128), (20, 40), (64, 4)])
+def test_state_scan_in_segments(rt32, P, N):
+    """Long portions cut into runs that are walked side by side: against the recurrence in 64 bits, portions that end at,
+    before and behind a run's end, in steps of several; portions of one run have the bits of the scan that cuts nothing, and
+    a value that is no number stays with its request's later tokens."""
+    from cuca_b200.kernels import ops
+    dev, H, G = rt32.device, 4, 2
+    run = int(__import__("cuca_b200.kernels.library", fromlist=["load"]).load().cuca_ssm_segment())
+    g = torch.Generator(device=dev).manual_seed(P * N + 1)
+    counts, slots = [1, run, run + 1, 2 * run, 2 * run + 301, 40], [3, 0, 5, 1, 2, 6]
+    rows = sum(counts)
+    xbc = torch.randn(rows, H * P + 2 * G * N, device=dev, generator=g)
+    proj = torch.randn(rows, H + 3, device=dev, generator=g) - 2.0
+    bias, a_log, skip = (torch.randn(H, device=dev, generator=g) for _ in range(3))
+    state = torch.randn(7, H, P, N, device=dev, generator=g)
+    step = _step(dev, [(0, n) for n in counts], slots)
+
+    def scan(segments, x=xbc):
+        st, y = state.clone(), torch.full((rows, H * P), 7.0, device=dev)
+        ops.ssm_scan(x, proj, 2, bias, a_log, skip, st, y, step, H, P, N, G, segments=segments)
+        return y, st
+    y, got = scan(True)
+    plain_y, plain = scan(False)
+    r0 = 0
+    for n, slot in zip(counts, slots):
+        same = torch.equal(y[r0:r0 + n], plain_y[r0:r0 + n]) and torch.equal(got[slot], plain[slot])
+        assert same == (n <= run), n
+        S, r = state[slot].double(), r0
+        xr = xbc[r:r + n, :H * P].double().view(n, H, P)
+        B, C = (xbc[r:r + n, H * P + i * G * N:][:, :G * N].double().view(n, G, N).repeat_interleave(H // G, 1) for i in (0, 1))
+        dt = torch.nn.functional.softplus(proj[r:r + n, 2:2 + H].double() + bias.double(), threshold=60)
+        decay = torch.exp(-torch.exp(a_log.double()) * dt)
+        want = torch.empty(n, H, P, device=dev, dtype=torch.float64)
+        for t in range(n):
+            S = decay[t][:, None, None] * S + (dt[t][:, None] * xr[t])[:, :, None] * B[t][:, None, :]
+            want[t] = (S * C[t][:, None, :]).sum(-1) + skip.double()[:, None] * xr[t]
+        assert (y[r0:r0 + n].view_as(want).double() - want).abs().max() < 2e-5 * want.abs().max(), n
+        assert (got[slot].double() - S).abs().max() < 2e-5 * S.abs().max(), n
+        r0 += n
+    assert torch.equal(got[4], state[4])
+    bad, at = xbc.clone(), sum(counts[:4]) + 100  # token 100 of the longest portion, the first head's first value
+    bad[at, 0] = float("inf")
+    z, zs = scan(True, bad)
+    keep = torch.ones(rows, dtype=torch.bool, device=dev)
+    keep[at:at + counts[4] - 100] = False
+    assert torch.equal(z[keep], y[keep]) and not bool(z[~keep][:, 0].isfinite().any()) and not bool(zs[2, 0, 0].isfinite().all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps, C, rows", [(4, 4800, 130), (4, 300, 1700), (3, 4800, 530), (6, 4736, 514), (1, 4800, 530)])
 def test_convolution_rows_are_the_same_bits_in_every_form(rt32, dtype, taps, C, rows):
