@@ -568,7 +568,9 @@ CUCA_API int cuca_attention_prefill_tc_o(const void* q, int q_stride, int n_rows
   p.cap_arg = softcap > 0.f ? 2.f * scale * 1.4426950408889634f / softcap : 0.f;
   p.sink = opt->sink ? 1 : 0;
   p.sink_val = opt->sink ? opt->sink_val : nullptr;
-  p.heads_per_cta = ((nh / nkv) % NQ == 0) ? NQ : 1;
+  // A head a CTA where those are all resident at once: alone a tile is done sooner (32 heads of 128 over 8, us, two heads and
+  // one: 203 tokens 13.9, 11.7; 512 tokens 18.3, 15.4). Beyond, two heads a CTA overlap each other's softmax and contractions.
+  p.heads_per_cta = (nh / nkv) % NQ == 0 && (long long)n_tiles * nh > cuca_device_sms() ? NQ : 1;
   p.n_tiles = n_tiles;
   // Two tiles per CTA, a heavy and a light one, where that makes one round of CTAs out of more than one
   // (CUCA_ATTN_PAIR_TILES=0 never, =2 whenever there are two tiles).

@@ -12,10 +12,11 @@
 // makes the scores again: 1.3 times the arithmetic, no exchange between CTAs. The first 256 values of Q lie in tensor memory
 // too, the rest in shared memory beside two key tiles (64 x 576 values: 72 KB each, 227 KB in all).
 //
-// Four warps copy key tiles (16-byte cp.async through the page table, zeros outside the group's keys, in the 128-byte swizzle
-// the tensor cores read), one issues contractions, four own a row a thread. Bound by the tensor pipe: 1,500 clocks of scores,
-// of which the steps with Q in shared memory run at its bandwidth, and 512 of P V a tile. 2,048 tokens, 16 heads, 512 + 64,
-// window 1,024: see the figures at cuca_latent_attention_tc.
+// Key tiles come page by page through the copy engine, those with keys outside the group's by 16-byte cp.async with zeros there;
+// one warp issues contractions, whatever is ready first; eight warps own the rows, two threads a row. A tile takes 4,150
+// clocks: 1,550 of scores and 520 of P V on the tensor pipe, and with two tiles' memory a tile's copies (2,500) start when the
+// P V two tiles before is done. A CTA's start, 288 KB of 32-bit queries, is 15 us of some 40. 2,048 tokens, 16 heads, 512 + 64,
+// window 1,024: 140 us (391 TFLOP/s); 16 tokens of a head a group on mma.sync 521.
 #include "tcgen05.cuh"
 #include <math.h>
 

@@ -938,6 +938,13 @@ def test_attention_prefill_tcgen05(dev, nh, nkv, bs, window, d, two_tiles_per_ct
         assert torch.allclose(got, want, atol=2e-2, rtol=2e-2), (r, s, pos, float((got - want).abs().max()))
 
 
+@pytest.mark.parametrize("d", [128, 64])
+@pytest.mark.parametrize("two_tiles_per_cta", [False, True])
+def test_attention_prefill_tcgen05_two_heads_a_cta(dev, d, two_tiles_per_cta):
+    """The test above with more heads than CTAs are resident at once: two heads of a group share a CTA."""
+    test_attention_prefill_tcgen05(dev, 32, 8, 16, 150, d, two_tiles_per_cta)
+
+
 @pytest.mark.parametrize("E", [1024, 2048, 4096, 8192, 9000])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_rmsnorm_is_the_same_bits_wherever_it_reads_its_weights(dev, E, dtype):
