@@ -117,6 +117,9 @@ def test_gemm_f32_every_form_gives_the_same_bits(dev, M, N, K, epilogue):
             ran += 1
             assert torch.equal(out, want), (tokens, slices)
     assert ran >= 4 and int(err.item()) == 0
+    tiny, got = a * 1e-37, torch.empty(M, N, device=dev)  # lower parts that bfloat16 does not hold: within 2^-20 of the sizes
+    ops.gemm_simt(tiny, w[:N], got, 0)
+    assert bool(((got.double() - tiny.double() @ w[:N].double().T).abs() <= tiny.double().abs() @ w[:N].double().abs().T * 2.0 ** -20 + 2.0 ** -148).all())
     a[M // 2, K // 3] = float("inf")
     w[N // 2, K // 2] = float("nan")
     if M > 1:
