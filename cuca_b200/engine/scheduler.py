@@ -219,9 +219,9 @@ class Scheduler:
         self._events()  # preemptions and failures found while planning
         if n == 0:
             return 0
-        buf, plans = self._plan_buf, []
-        for i in range(n):
-            sid, offset, cnt, want_last, _slot, _blocks, start, token = buf[8 * i:8 * i + 8]
+        buf, plans = self._plan_buf[:8 * n], []
+        for i in range(0, 8 * n, 8):
+            sid, offset, cnt, want_last, _slot, _blocks, start, token = buf[i:i + 8]
             seq = self._seqs[sid]
             plans.append(Plan(seq, [token] if token >= 0 else seq.prompt[offset:offset + cnt], bool(want_last), start))
         t0 = time.perf_counter()
@@ -266,9 +266,9 @@ class Scheduler:
                 self._event_buf = buf = (ctypes.c_int * (4 * -n))()
                 continue
             break
-        now = None
-        for i in range(n):
-            kind, sid, value, extra = buf[4 * i:4 * i + 4]
+        buf = buf[:4 * n]
+        for i in range(0, 4 * n, 4):
+            kind, sid, value, extra = buf[i:i + 4]
             seq = self._seqs[sid]
             if kind == _EV_TOKEN:
                 if not seq.completion:

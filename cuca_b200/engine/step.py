@@ -18,7 +18,9 @@ step function does not plan for any kernel: mixers do that from `StepBatch`.
 from __future__ import annotations
 
 import ctypes
+from array import array
 from dataclasses import dataclass, field
+from itertools import chain
 from typing import Optional, Sequence
 
 import numpy as np
@@ -149,14 +151,18 @@ class Stepper:
         lib, pools = host.load(), self.pools
         n = len(entries)
         counts = [len(e.tokens) for e in entries]
-        flat_tokens = [int(t) for e in entries for t in e.tokens]
+        try:
+            packed = array("i", chain.from_iterable(e.tokens for e in entries))
+            flat_tokens = packed.tolist()
+        except (TypeError, OverflowError):  # (numbers that are no ints, or too large for one)
+            packed = flat_tokens = [int(t) for e in entries for t in e.tokens]
         n_want = [len(e.want) for e in entries]
         flat_want = [int(w) for e in entries for w in e.want]
         seqs = host.ints(e.blocks.handle for e in entries)
         slots_c = host.ints(e.slot for e in entries)
         sizes = (ctypes.c_int * (N_FIXED_SECTIONS + 2 * pools.n_groups))()
         meta = (ctypes.c_int * 4)()
-        args = (pools._h, n, seqs, slots_c, host.ints(counts), host.ints(flat_tokens), host.ints(n_want),
+        args = (pools._h, n, seqs, slots_c, host.ints(counts), host.ints(packed), host.ints(n_want),
                 host.ints(flat_want), self.context_length, self.vocab, self.cache.max_sequences, self.cache.table_width)
         buf = self._staging.take()
         code = lib.cuca_host_step_pack(*args, buf.data_ptr(), buf.shape[0], sizes, meta)
