@@ -77,6 +77,15 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {  // when this t
 }
 // the two warps that hold the halves of 32 rows
 __device__ __forceinline__ void soft_sync(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(4 + quarter) : "memory"); }
+// The same, and whether both are well: a wait can run out in one of them alone, so they leave only by this vote, together.
+// A warp that left on its own would leave the other at the barrier, which has no limit.
+__device__ __forceinline__ bool soft_vote(int quarter, bool ok) {
+  uint32_t both;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.b32 p, %2, 0;\nbar.red.and.pred q, %1, 64, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+      : "=r"(both) : "r"(4 + quarter), "r"((uint32_t)ok) : "memory");
+  return both != 0;
+}
 __device__ __forceinline__ void tmem_st16_raw(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -323,8 +332,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
       const uint32_t s_at = tmem + lane_bits + S_AT + (j & 1) * KEYS;
-      ok = warp_wait(&s_full[j & 1], (j >> 1) & 1, p.err, abort_flag);
-      if (!ok) break;
+      ok = ok && warp_wait(&s_full[j & 1], (j >> 1) & 1, p.err, abort_flag);
       tc_fence_after();
       const int key0 = first_key + j * KEYS;
       uint32_t raw[32];
@@ -343,7 +351,8 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
       }
       // the other half's maximum; behind the barrier both halves have read their scores, so P may take their place
       halves[half * ROWS + r] = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      soft_sync(quarter);
+      ok = soft_vote(quarter, ok);
+      if (!ok) break;
       const float mx = fmaxf(halves[r], halves[ROWS + r]) * p.scale_log2;
       soft_sync(quarter);  // (both have read before either writes the next tile's)
       // The reference only moves when the maximum exceeds it by more than 8 (in log2 units): values up to 2^8 above it are
@@ -369,7 +378,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
       // runs two phases ahead of its waiters)
       if (j > 0) {
         ok = warp_wait(pv_done, (j - 1) & 1, p.err, abort_flag);
-        if (!ok) break;
+        if (!ok) continue;  // (to the next vote)
         tc_fence_after();
         if (__any_sync(0xffffffffu, corr != 1.f)) {
 #pragma unroll 1
@@ -386,10 +395,11 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
       tc_fence_before();
       mbar_arrive(p_full);
     }
-    if (ok && warp_wait(pv_done, (n_tiles - 1) & 1, p.err, abort_flag)) {
+    ok = ok && warp_wait(pv_done, (n_tiles - 1) & 1, p.err, abort_flag);
+    halves[half * ROWS + r] = l;
+    ok = soft_vote(quarter, ok);
+    if (ok) {
       tc_fence_after();
-      halves[half * ROWS + r] = l;
-      soft_sync(quarter);
       l = halves[r] + halves[ROWS + r];
       if (p.sink && m != -INFINITY) l += fast_exp2(p.sink[head0 + r % p.HB] * 1.4426950408889634f - m);
       const float inv = l > 0.f ? 1.f / l : 0.f;
