@@ -1,6 +1,7 @@
 """The host core's step packer (csrc/host/step_pack.cpp) without a GPU: what goes into the one buffer a step
 uploads, and what is refused before anything changes."""
 import ctypes
+from array import array
 
 import numpy as np
 import pytest
@@ -140,3 +141,25 @@ def test_validation_alone_for_steps_that_live_on_the_device():
     assert check([5], context=8) == host.INVALID and "context length 8" in host.last_error()
     a.length = 16
     assert check([5]) == host.INVALID and "pages for 16 positions" in host.last_error()
+
+
+@pytest.mark.parametrize("values, want", [
+    ([1, -2, 3], [1, -2, 3]), ((np.int64(5), True), [5, 1]), (np.arange(3), [0, 1, 2]), (iter([7, 8]), [7, 8]), ([], [0]),
+    (array("i", [4, 5]), [4, 5]), (array("q", [4, 5, -6]), [4, 5, -6]), (array("h", [9, 10]), [9, 10]),
+    ([2 ** 31, 2 ** 40 + 5], [-2 ** 31, 5]), (array("q", [2 ** 40 + 5]), [5]), (array("q"), [0])])
+def test_ints_are_the_numbers_that_were_given(values, want):
+    assert list(host.ints(values)) == want
+
+
+@pytest.mark.parametrize("values", [[1.0], ["1"], [None], array("d", [1.0])])
+def test_ints_refuses_what_is_no_whole_number(values):
+    with pytest.raises(TypeError):
+        host.ints(values)
+
+
+def test_ints_have_memory_of_their_own():
+    given = array("i", [1, 2])
+    taken = host.ints(given)
+    given.append(3)
+    given[0] = 9
+    assert list(taken) == [1, 2]
