@@ -1,16 +1,20 @@
 // 32-bit contraction out = A[M,K] * W[N,K]^T on the 5th-generation tensor cores: the true 32-bit path of every projection,
 // and the bfloat16 path's stand-in for shapes that its own kernel refuses.
 //
-// A 32-bit value is the sum of three bfloat16 parts, exactly: its upper 16 bits, the upper 16 of what is left, and the rest.
-// Of the nine products of two values' parts the six largest count (what the others would add is below 2^-24 of the
-// product); tcgen05.mma sums them in 32 bits over a chunk of 64 products, the smallest first, so that only the last four
-// steps round at the chunk's full magnitude. The tensor cores cut off where a 32-bit addition rounds; over those steps
-// that takes about one unit in the last place off a chunk's sum, which REGAIN gives back. Four chunks' sums are added up to
-// a block's, the blocks' in ascending order to the total. Each output is summed in this one order whatever M and the
-// kernel's form are, so a row's result never depends on the rest of the batch. Where the total is no finite number (an infinite
-// value has no parts) or a tiny one a warp computes it again with plain multiply-adds.
-// Error against 64 bits, relative 2-norm, normal values: 9.6e-8 at K = 2,048 and 1.3e-7 at 8,192; multiply-adds in runs of 64
-// gave 1.8e-7 and 2.5e-7.
+// A 32-bit value from 2^-110 on is the sum of three bfloat16 parts, exactly: the nearest bfloat16 number, the nearest to what
+// is left, and the rest, at most 2^-8 and 2^-16 of the value's power of two. Of the nine products of two values' parts the six
+// largest count; the others come to at most 2^-23 of the product, 2^-28 on average, of either sign. tcgen05.mma sums
+// them in 32 bits, and the tensor cores cut off where a 32-bit addition rounds. So the largest products, which take 16 bits
+// each, have an accumulator of their own over a chunk of 64 products, where little is left to cut off, and the five others,
+// a 2^-8th as large, one over a block of four chunks. Everything else is added with rounding: the chunks' sums of a block and its small
+// products, and the blocks' in ascending order. What 32 bits hold exactly (whole numbers, one product with a power of
+// two) comes out exactly. Each output is summed in this one order whatever M and the kernel's form are, so a row's result never depends
+// on the rest of the batch. Where the total is no finite number (an infinite value has no parts) or a tiny one a warp computes it
+// again with plain multiply-adds.
+// Error against 64 bits, relative 2-norm, normal values (multiply-adds in runs of 64 in brackets): K = 1 2.6e-8 (2.5e-8), 16
+// 3.6e-8 (7.4e-8), 2,048 9.8e-8 (1.8e-7), 8,192 1.3e-7 (2.5e-7); values of one sign, K = 64 7.9e-8 (1.2e-7), 256 8.1e-8
+// (7.0e-8), 2,048 8.2e-8 (8.1e-8), 8,192 1.0e-7 (1.5e-7). With one accumulator for all products and a unit in the last place given
+// back to every chunk for what is cut off, sums that are exact came out wrong (1 x 1) and K = 1 had 6.5e-8.
 //
 // The weights are the 128-row operand, the tokens the columns. A CTA (one an SM): the copy engine streams weight chunks
 // into a ring as they are; converter warps split them, a row a lane, into tensor memory, from where the tensor cores read
@@ -38,7 +42,6 @@ constexpr int ROWS = TILE_A;          // weight rows of a tile
 constexpr int ROW_BYTES = CHUNK * 2;  // one row of one part in shared memory: one swizzle span
 constexpr int MAX_CLUSTER = 8;
 constexpr int PRE_TOKENS = 32;        // tiles of so many tokens and more take the tokens' parts from memory
-constexpr float REGAIN = 1.f + 1.1920929e-7f;  // one unit in the last place
 
 template <typename TI> struct Parts { static constexpr int N = 3; };
 template <> struct Parts<__nv_bfloat16> { static constexpr int N = 1; };  // (the others would be zeros)
@@ -70,19 +73,23 @@ struct Form {
   static constexpr int COLS = NT / (EPI_WARPS / 4);  // tokens of one summing thread
   // weights as they are: a ring of chunks, filled by the copy engine
   static constexpr int RAW = ROWS * CHUNK * 4;
-  static constexpr int RAWS = PRE ? 4 : 6;
+  static constexpr int RAWS = NT > 64 ? 3 : PRE ? 4 : 6;
   // a chunk of the parts: the weights' in tensor memory, the tokens' in shared memory
   static constexpr int STAGES = PRE ? 2 : 3;
   static constexpr int A_COLS = P * CHUNK / 2;
   static constexpr int B_BYTES = P * NT * ROW_BYTES;
   static constexpr int PASS_ROWS = B_WARPS * 2;  // 16 threads a token row, 16 bytes each
   static constexpr int PASSES = NT / PASS_ROWS;
+  // columns of tensor memory: two accumulators of the largest products, one of the small ones, the parts, then the total (with
+  // slices: the sums of this CTA's blocks but for the last, which stays in registers), which lies in shared memory where
+  // there is no room left
+  static constexpr int SMALL_AT = 2 * NT, A_AT = (P == 3 ? 3 : 2) * NT, SUM_AT = A_AT + STAGES * A_COLS;
+  static constexpr bool SUM_IN_SMEM = SUM_AT + NT > 512;
   static constexpr int DATA = RAWS * RAW + STAGES * B_BYTES;
-  static constexpr int SMEM = DATA + 1024 + 256;
-  // columns of tensor memory: two accumulators, the parts, then the total (with slices: the sums of this CTA's blocks)
-  static constexpr int A_AT = 2 * NT, SUM_AT = A_AT + STAGES * A_COLS;
-  static constexpr int BLOCKS_HELD = std::min((512 - SUM_AT) / NT, DATA / (NT * ROWS * 4));
-  static_assert(SUM_AT + NT <= 512 && SMEM <= 227 * 1024, "tensor or shared memory");
+  static constexpr int SUM_BYTES = SUM_IN_SMEM ? NT * ROWS * 4 : 0;
+  static constexpr int SMEM = DATA + SUM_BYTES + 1024 + 256;
+  static constexpr int BLOCKS_HELD = SUM_IN_SMEM ? 0 : std::min((512 - SUM_AT) / NT + 1, DATA / (NT * ROWS * 4));
+  static_assert(SUM_AT <= 512 && SMEM <= 227 * 1024, "tensor or shared memory");
 };
 
 __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
@@ -176,23 +183,20 @@ __device__ __forceinline__ uint2 load4(const __nv_bfloat16* src, int left) {
   return make_uint2(a | b << 16, c | d << 16);
 }
 
-__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
-  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-}
-// a and b minus their upper halves, exactly
-__device__ __forceinline__ void lower(float& a, float& b) {
-  const f32x2 up = f2_pack(__uint_as_float(__float_as_uint(a) & 0xffff0000u), __uint_as_float(__float_as_uint(b) & 0xffff0000u));
+// The bfloat16 numbers nearest to a and to b; a and b become what is left, exactly.
+__device__ __forceinline__ uint32_t take_part(float& a, float& b) {
+  const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+  const uint32_t part = *reinterpret_cast<const uint32_t*>(&t);
+  const f32x2 up = f2_pack(__uint_as_float(part << 16), __uint_as_float(part & 0xffff0000u));
   f2_unpack(f2_fma(up, f2_both(-1.f), f2_pack(a, b)), a, b);
+  return part;
 }
 // four elements' parts
 __device__ __forceinline__ void split(uint2 (&w)[3], float4 v) {
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
-    w[t] = make_uint2(upper_halves(v.x, v.y), upper_halves(v.z, v.w));
-    if (t < 2) {
-      lower(v.x, v.y);
-      lower(v.z, v.w);
-    }
+    w[t].x = take_part(v.x, v.y);
+    w[t].y = take_part(v.z, v.w);
   }
 }
 __device__ __forceinline__ void split(uint2 (&w)[1], uint2 v) { w[0] = v; }
@@ -223,12 +227,15 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tokens = smem + C::RAWS * C::RAW;
-  uint64_t* raw_full = (uint64_t*)(smem + C::DATA);
+  float* total_s = (float*)(smem + C::DATA);  // (with SUM_IN_SMEM: [token][row])
+  uint64_t* raw_full = (uint64_t*)(smem + C::DATA + C::SUM_BYTES);
   uint64_t* raw_empty = raw_full + C::RAWS;
   uint64_t* full = raw_empty + C::RAWS;
   uint64_t* done = full + C::STAGES;  // a stage's contraction: its parts are free and its accumulator complete
   uint64_t* acc_empty = done + C::STAGES;
-  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  uint64_t* small_full = acc_empty + 2;  // a block's small products are complete
+  uint64_t* small_empty = small_full + 1;
+  uint32_t* tmem_slot = (uint32_t*)(small_empty + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool dual = p.epilogue == EPI_SWIGLU;
@@ -249,6 +256,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       mbar_init(&done[s], 1);
     }
     for (int b = 0; b < 2; ++b) mbar_init(&acc_empty[b], C::EPI_WARPS);
+    mbar_init(small_full, 1);
+    mbar_init(small_empty, C::EPI_WARPS);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -290,18 +299,31 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       // the contraction, and not in the converters, where it would wait for their loads in flight.
       fence_proxy_async();
       tc_fence_after();
-      const uint32_t a = tmem + C::A_AT + st * C::A_COLS, sb = smem_u32(tokens + st * C::B_BYTES), acc = tmem + buf * NT;
+      const uint32_t a = tmem + C::A_AT + st * C::A_COLS, sb = smem_u32(tokens + st * C::B_BYTES);
+      // products of the weights' part pa and the tokens' part pb
+      auto contract = [&](uint32_t acc, int pa, int pb, bool add) {
+        const uint32_t at = a + pa * CHUNK / 2;
+        const uint64_t bd = smem_desc(sb + pb * NT * ROW_BYTES);
+#pragma unroll
+        for (int k = 0; k < CHUNK / UMMA_K; ++k)
+          umma_bf16_tmem_a(acc, at + k * UMMA_K / 2, bd + k * UMMA_K * 2 / 16, instr_desc(NT), add || k > 0);
+      };
+      // The small products' one accumulator is drained while largest products are contracted: those of a block's last chunk
+      // come behind its small ones, those of its first chunk before them.
+      const bool begins = i % BLOCK == 0, ends = i % BLOCK == BLOCK - 1 || c == last - 1, ahead = C::P == 3 && begins && !ends;
+      if (ahead && elect_one()) contract(tmem + buf * NT, 0, 0, false);
+      __syncwarp();
+      if (C::P == 3 && begins && !warp_wait(small_empty, ((i / BLOCK) & 1) ^ 1, p.err, abort_flag)) break;
       if (elect_one()) {
-        // the smallest products first
-#pragma unroll
-        for (int t = 0; t < (C::P == 3 ? 6 : 1); ++t) {
-          constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
-          const uint32_t at = a + (C::P == 3 ? PA[t] : 0) * CHUNK / 2;
-          const uint64_t bd = smem_desc(sb + (C::P == 3 ? PB[t] : 0) * NT * ROW_BYTES);
-#pragma unroll
-          for (int k = 0; k < CHUNK / UMMA_K; ++k)
-            umma_bf16_tmem_a(acc, at + k * UMMA_K / 2, bd + k * UMMA_K * 2 / 16, instr_desc(NT), t > 0 || k > 0);
+        if (C::P == 3) {  // the smallest first
+          contract(tmem + C::SMALL_AT, 2, 0, !begins);
+          contract(tmem + C::SMALL_AT, 0, 2, true);
+          contract(tmem + C::SMALL_AT, 1, 1, true);
+          contract(tmem + C::SMALL_AT, 1, 0, true);
+          contract(tmem + C::SMALL_AT, 0, 1, true);
+          if (ends) umma_commit(small_full);
         }
+        if (!ahead) contract(tmem + buf * NT, 0, 0, false);
         umma_commit(&done[st]);
       }
       __syncwarp();
@@ -409,26 +431,38 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + col0, total = lane_base + C::SUM_AT;
     float sum[C::COLS];
     bool ok = true;
-    for (int c = first, i = 0; c < last; ++c, ++i) {
-      const uint32_t acc = lane_base + (i & 1) * NT;
-      ok = warp_wait(&done[i % C::STAGES], (i / C::STAGES) & 1, p.err, abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      const bool begins = i % BLOCK == 0, ends = i % BLOCK == BLOCK - 1 || c == last - 1, more = p.slices == 1 && i >= BLOCK;
-      const uint32_t at = total + (p.slices > 1 ? i / BLOCK * NT : 0);
+    auto add_up = [&](uint32_t at, bool starts) {
 #pragma unroll
       for (int j = 0; j < C::COLS; j += 16) {
         uint32_t x[16];
-        tmem_ld16_async(acc + j, x);
+        tmem_ld16_async(at + j, x);
         tmem_ld_wait();
 #pragma unroll
-        for (int q = 0; q < 16; ++q)
-          sum[j + q] = begins ? __uint_as_float(x[q]) * REGAIN : fmaf(__uint_as_float(x[q]), REGAIN, sum[j + q]);
+        for (int q = 0; q < 16; ++q) sum[j + q] = starts ? __uint_as_float(x[q]) : sum[j + q] + __uint_as_float(x[q]);
       }
       tc_fence_before();
       __syncwarp();
+    };
+    for (int c = first, i = 0; c < last; ++c, ++i) {
+      const bool begins = i % BLOCK == 0, ends = i % BLOCK == BLOCK - 1 || c == last - 1, more = p.slices == 1 && i >= BLOCK;
+      if (C::P == 3 && ends) {
+        ok = warp_wait(small_full, (i / BLOCK) & 1, p.err, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        add_up(lane_base + C::SMALL_AT, begins);
+        if (lane == 0) mbar_arrive(small_empty);
+      }
+      ok = warp_wait(&done[i % C::STAGES], (i / C::STAGES) & 1, p.err, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      add_up(lane_base + (i & 1) * NT, begins && !(C::P == 3 && ends));
       if (lane == 0) mbar_arrive(&acc_empty[i & 1]);
-      if (ends) {
+      if (ends && C::SUM_IN_SMEM) {
+        float* mine = total_s + col0 * ROWS + quarter * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < C::COLS; ++j) mine[j * ROWS] = more ? mine[j * ROWS] + sum[j] : sum[j];
+      } else if (ends) {
+        const uint32_t at = total + (p.slices > 1 ? i / BLOCK * NT : 0);
 #pragma unroll
         for (int j = 0; j < C::COLS; j += 16) {
           if (more) {
@@ -438,24 +472,26 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
             for (int q = 0; q < 16; ++q) sum[j + q] = __uint_as_float(x[q]) + sum[j + q];
           }
-          tmem_st16(at + j, reinterpret_cast<const uint32_t*>(sum + j));
+          if (c < last - 1) tmem_st16(at + j, reinterpret_cast<const uint32_t*>(sum + j));
         }
         tmem_st_wait();
       }
     }
-    if (ok) {
+    if (ok && !C::SUM_IN_SMEM) {
       // [block][token][row]; every contraction is done, so the stages are free
-      float* sums = reinterpret_cast<float*>(smem);
-      const int mine = p.slices > 1 ? (last - first + BLOCK - 1) / BLOCK : 1;
+      float* mine = reinterpret_cast<float*>(smem) + col0 * ROWS + quarter * 32 + lane;
+      const int held = p.slices > 1 ? (last - first - 1) / BLOCK : 0;
 #pragma unroll 1
-      for (int b = 0; b < mine; ++b)
+      for (int b = 0; b < held; ++b)
 #pragma unroll 1
         for (int j = 0; j < C::COLS; j += 16) {
           float v[16];
           tmem_ld16(total + b * NT + j, v);
 #pragma unroll
-          for (int q = 0; q < 16; ++q) sums[(size_t)(b * NT + col0 + j + q) * ROWS + quarter * 32 + lane] = v[q];
+          for (int q = 0; q < 16; ++q) mine[(size_t)(b * NT + j + q) * ROWS] = v[q];
         }
+#pragma unroll
+      for (int j = 0; j < C::COLS; ++j) mine[(size_t)(held * NT + j) * ROWS] = sum[j];
     }
   }
   // ---- results: every thread, in one short loop (unrolled per accumulator column its code came from L2, at 290 clocks a
@@ -472,7 +508,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const int row = dual ? (o >> 4) * 32 + (o & 15) : o;
     float v = 0.f, u = 0.f;
     if (live && p.slices == 1) {
-      const float* sums = reinterpret_cast<const float*>(smem) + (size_t)m * ROWS + row;
+      const float* sums = (C::SUM_IN_SMEM ? total_s : reinterpret_cast<const float*>(smem)) + (size_t)m * ROWS + row;
       v = sums[0];
       if (dual) u = sums[16];
     } else if (live) {

@@ -87,7 +87,7 @@ def test_gemm_simt_rows_are_the_same_bits_in_every_form(dev, N, K, epilogue):
 @pytest.mark.parametrize("epilogue", [0, 1, 2])
 def test_gemm_f32_every_form_gives_the_same_bits(dev, M, N, K, epilogue):
     """Tiles of every width, K shared by one to eight CTAs: against 64 bits, the same bits in every form, and infinities and
-    NaN where multiply-adds have them. The bound: a product lacks 2^-24 of itself at most, a chunk's sum is off by some 4 of
+    NaN where multiply-adds have them. The bound: a product lacks 2^-23 of itself at most, a chunk's sum is off by some 4 of
     the last of 24 places, and up to 3 + 33 additions round; all against the sum of the products' sizes."""
     from cuca_b200.kernels import library, ops
     g = torch.Generator(device=dev).manual_seed(M * 7 + N + K)
@@ -102,7 +102,7 @@ def test_gemm_f32_every_form_gives_the_same_bits(dev, M, N, K, epilogue):
     if epilogue == 2:  # silu has a slope below 1.1 and is at most its argument's size
         y = a.double() @ w.double().T
         sizes = 1.1 * sizes[:, :N] * y[:, N:].abs() + sizes[:, N:] * y[:, :N].abs() + sizes[:, :N] * 1e-6 * sizes[:, N:]
-    places = 1 + 4 + 3 + 33 + 8  # (and bias, stream, exponent and division)
+    places = 2 + 4 + 3 + 33 + 8  # (and bias, stream, exponent and division)
     assert bool(((want.double() - ref).abs() <= places * 2.0 ** -24 * (sizes + prior.double().abs() + 4)).all())
     err = torch.zeros(1, dtype=torch.int32, device=dev)
     ran = 0
@@ -130,6 +130,42 @@ def test_gemm_f32_every_form_gives_the_same_bits(dev, M, N, K, epilogue):
         ops.gemm_simt(a, w, out, 0 if epilogue == 1 else epilogue, None, form=(tokens, slices))
         if epilogue != 2:
             assert torch.equal(out.isnan(), y.isnan()) and torch.equal(out.isinf() & (out > 0), y.isinf() & (y > 0)), (tokens, slices)
+
+
+@pytest.mark.parametrize("K", [4, 64, 300, 1030, 2048])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gemm_f32_is_exact_where_32_bits_are(dev, K, dtype):
+    """An identity returns its input, whole numbers add up to whole numbers, in tiles of every width; mantissas full of ones
+    and one below a power of two are among the inputs."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(K)
+    a = torch.randn(97, K, device=dev, generator=g)
+    a[0], a[1], a[2] = 2 - 2.0 ** -23, 1 + 2.0 ** -7 - 2.0 ** -23, 1 + 2.0 ** -8 - 2.0 ** -16 - 2.0 ** -23
+    a = a.to(dtype)
+    one = torch.eye(K, device=dev).to(dtype)
+    i = torch.randint(-9, 10, (97, K), device=dev, generator=g).to(dtype)
+    j = torch.randint(-9, 10, (130, K), device=dev, generator=g).to(dtype)
+    sums = (i.double() @ j.double().T).float()
+    for tokens in (16, 32, 64, 96):
+        out, whole = torch.empty(97, K, device=dev), torch.empty(97, 130, device=dev)
+        ops.gemm_simt(a, one, out, 0, form=(tokens, 1))
+        ops.gemm_simt(i, j, whole, 0, form=(tokens, 1))
+        assert torch.equal(out, a.float()) and torch.equal(whole, sums), tokens
+
+
+@pytest.mark.parametrize("K", [1, 2, 4, 16])
+def test_gemm_f32_of_few_products(dev, K):
+    """A product lacks 2^-23 of itself at most. Of one product nothing else is lost but its own rounding; in sums of up to 16
+    the tensor cores cut one 2^-23th off, and the small products are added with rounding."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(K)
+    a, w = torch.randn(700, K, device=dev, generator=g), torch.randn(520, K, device=dev, generator=g)
+    a[:5], w[:5] = 1 + 2.0 ** -8 - 2.0 ** -16 - 2.0 ** -23, 1 + 2.0 ** -7 - 2.0 ** -23  # what is left of them is largest
+    want, sizes = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    for M in (7, 700):
+        out = torch.empty(M, 520, device=dev)
+        ops.gemm_simt(a[:M], w, out, 0)
+        assert bool(((out.double() - want[:M]).abs() <= (1.5 if K == 1 else 2.5) * 2.0 ** -23 * sizes[:M]).all())
 
 
 @pytest.mark.parametrize("K", [60, 64, 250, 1021, 2046])
