@@ -9,8 +9,9 @@
 // a 2^-8th as large, one over a block of four chunks. Everything else is added with rounding: the chunks' sums of a block and its small
 // products, and the blocks' in ascending order. What 32 bits hold exactly (whole numbers, one product with a power of
 // two) comes out exactly. Each output is summed in this one order whatever M and the kernel's form are, so a row's result never depends
-// on the rest of the batch. Where the total is no finite number (an infinite value has no parts) or a tiny one a warp computes it
-// again with plain multiply-adds.
+// on the rest of the batch. A warp computes an output again with plain multiply-adds where the total is no finite number (an infinite
+// value has no parts) or a tiny one, and where values below 2^-110 that lost something in their parts (the converters note whose
+// rows have any) may matter beside it: see `settled`.
 // Error against 64 bits, relative 2-norm, normal values (multiply-adds in runs of 64 in brackets): K = 1 2.6e-8 (2.5e-8), 16
 // 3.6e-8 (7.4e-8), 2,048 9.8e-8 (1.8e-7), 8,192 1.3e-7 (2.5e-7); values of one sign, K = 64 7.9e-8 (1.2e-7), 256 8.1e-8
 // (7.0e-8), 2,048 8.2e-8 (8.1e-8), 8,192 1.0e-7 (1.5e-7). With one accumulator for all products and a unit in the last place given
@@ -42,6 +43,7 @@ constexpr int ROWS = TILE_A;          // weight rows of a tile
 constexpr int ROW_BYTES = CHUNK * 2;  // one row of one part in shared memory: one swizzle span
 constexpr int MAX_CLUSTER = 8;
 constexpr int PRE_TOKENS = 32;        // tiles of so many tokens and more take the tokens' parts from memory
+constexpr int SPLIT_RUN = 2048;       // elements of a row that one block of `split_kernel` takes
 
 template <typename TI> struct Parts { static constexpr int N = 3; };
 template <> struct Parts<__nv_bfloat16> { static constexpr int N = 1; };  // (the others would be zeros)
@@ -54,6 +56,7 @@ struct GemmParams {
   int* err;
   int M, N, K, lda, ldo;
   int epilogue, out_f32;
+  const uint16_t* marks;  // of the tokens, [M][runs of SPLIT_RUN], where their parts come from memory
   int tiles_m;  // token tiles
   int slices;   // CTAs of a cluster that share a tile's K
 };
@@ -87,7 +90,7 @@ struct Form {
   static constexpr bool SUM_IN_SMEM = SUM_AT + NT > 512;
   static constexpr int DATA = RAWS * RAW + STAGES * B_BYTES;
   static constexpr int SUM_BYTES = SUM_IN_SMEM ? NT * ROWS * 4 : 0;
-  static constexpr int SMEM = DATA + SUM_BYTES + 1024 + 256;
+  static constexpr int SMEM = DATA + SUM_BYTES + 1024 + 256 + (ROWS + NT + 4) * 4;
   static constexpr int BLOCKS_HELD = SUM_IN_SMEM ? 0 : std::min((512 - SUM_AT) / NT + 1, DATA / (NT * ROWS * 4));
   static_assert(SUM_AT <= 512 && SMEM <= 227 * 1024, "tensor or shared memory");
 };
@@ -112,18 +115,31 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank, uint32_t offset) {
-  uint32_t a;
-  float v;
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t local, uint32_t rank, uint32_t offset) {
+  uint32_t a, v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a + offset) : "memory");
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a + offset) : "memory");
   return v;
 }
+__device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank, uint32_t offset) {
+  return __uint_as_float(ld_cluster_u32(local, rank, offset));
+}
 
-// Whether a total stands: finite, and not so small (2^-100) that parts of its operands may lie below what bfloat16 holds.
-__device__ __forceinline__ bool settled(float v) {
+// What is noted of a row (of weights or of a token): a value whose three parts are not all of it (one below 2^-110, whose lower
+// bits bfloat16 does not hold; up to 2^-133 of it is lost), one of at least 2^40.
+constexpr uint32_t LOSSY = 1, LARGE = 2;
+struct Marks {
+  uint32_t lost = 0;  // the third parts' bits, of which bfloat16 holds the upper half
+  float most = 0.f;
+  __device__ __forceinline__ uint32_t word() const { return (lost << 16 ? LOSSY : 0) | (most >= 1.09951163e12f ? LARGE : 0); }
+};
+// Whether a total stands. Finite, and not so small (2^-100) that products of small parts may have been lost; and where a row lost
+// something of its values, they met none of 2^40 or more and the total is no less than 2^-50, beside which K times 2^-93 is nothing.
+__device__ __forceinline__ bool settled(float v, uint32_t token, uint32_t weight) {
   const float a = fabsf(v);
-  return a <= 3.402823466e38f && (a >= 7.888609e-31f || a == 0.f);
+  if (!(a <= 3.402823466e38f && (a >= 7.888609e-31f || a == 0.f))) return false;
+  if (!((token | weight) & LOSSY)) return true;
+  return a >= 8.8817842e-16f && !((token & LOSSY) && (weight & LARGE)) && !((weight & LOSSY) && (token & LARGE));
 }
 // One output by a warp with plain multiply-adds.
 template <typename TI>
@@ -191,32 +207,53 @@ __device__ __forceinline__ uint32_t take_part(float& a, float& b) {
   f2_unpack(f2_fma(up, f2_both(-1.f), f2_pack(a, b)), a, b);
   return part;
 }
+__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
 // four elements' parts
-__device__ __forceinline__ void split(uint2 (&w)[3], float4 v) {
+__device__ __forceinline__ void split(uint2 (&w)[3], float4 v, Marks& marks) {
+  marks.most = fmaxf(marks.most, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
 #pragma unroll
-  for (int t = 0; t < 3; ++t) {
+  for (int t = 0; t < 2; ++t) {
     w[t].x = take_part(v.x, v.y);
     w[t].y = take_part(v.z, v.w);
   }
+  marks.lost |= __float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w);
+  w[2] = make_uint2(upper_halves(v.x, v.y), upper_halves(v.z, v.w));
 }
-__device__ __forceinline__ void split(uint2 (&w)[1], uint2 v) { w[0] = v; }
+__device__ __forceinline__ void split(uint2 (&w)[1], uint2 v, Marks&) { w[0] = v; }
 __device__ __forceinline__ void clear(float4& v) { v = make_float4(0.f, 0.f, 0.f, 0.f); }
 __device__ __forceinline__ void clear(uint2& v) { v = make_uint2(0, 0); }
 
-// The tokens' parts, [part][token][ld] in bf16. Bound by its bytes: 700 x 8,192 values in about 10 us.
+// The tokens' parts, [part][token][ld] in bf16, and their marks: a block takes SPLIT_RUN elements of a row. Bound by its bytes.
 template <typename TI, bool VEC>
-__global__ void __launch_bounds__(256) split_kernel(const TI* __restrict__ A, __nv_bfloat16* __restrict__ parts, int M, int K, int lda, int ld) {
-  constexpr int P = Parts<TI>::N;
+__global__ void __launch_bounds__(256)
+split_kernel(const TI* __restrict__ A, __nv_bfloat16* __restrict__ parts, uint16_t* __restrict__ out_marks, int m0, int M, int K, int lda, int ld) {
+  constexpr int P = Parts<TI>::N, QUADS = SPLIT_RUN / 4 / 256;
   pdl_trigger();
   pdl_wait();
-  const int quads = (K + 3) / 4;
-  const long long n = (long long)M * quads;
-  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < n; e += (long long)gridDim.x * 256) {
-    const int m = (int)(e / quads), k = (int)(e % quads) * 4;
-    uint2 w[P];
-    split(w, load4<VEC>(A + (size_t)m * lda + k, K - k));
+  const int m = m0 + blockIdx.y, k0 = blockIdx.x * SPLIT_RUN + threadIdx.x * 4;
+  decltype(load4<VEC>(A, 0)) v[QUADS];
 #pragma unroll
-    for (int t = 0; t < P; ++t) *reinterpret_cast<uint2*>(parts + ((size_t)t * M + m) * ld + k) = w[t];
+  for (int i = 0; i < QUADS; ++i) {
+    const int k = k0 + i * 1024;
+    if (k < K) v[i] = load4<VEC>(A + (size_t)m * lda + k, K - k);
+    else clear(v[i]);
+  }
+  Marks marks;
+#pragma unroll
+  for (int i = 0; i < QUADS; ++i) {
+    const int k = k0 + i * 1024;
+    uint2 w[P];
+    split(w, v[i], marks);
+    if (k < K)
+#pragma unroll
+      for (int t = 0; t < P; ++t) *reinterpret_cast<uint2*>(parts + ((size_t)t * M + m) * ld + k) = w[t];
+  }
+  if (P == 3) {
+    const uint32_t word = marks.word();
+    const int lossy = __syncthreads_or(word & LOSSY), large = __syncthreads_or(word & LARGE);
+    if (threadIdx.x == 0) out_marks[(size_t)m * gridDim.x + blockIdx.x] = (lossy ? LOSSY : 0) | (large ? LARGE : 0);
   }
 }
 
@@ -237,6 +274,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   uint64_t* small_empty = small_full + 1;
   uint32_t* tmem_slot = (uint32_t*)(small_empty + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  // marks of what this CTA has split: its weight rows, the tile's tokens, whether any row is lossy
+  uint32_t* row_marks = tmem_slot + 2;
+  uint32_t* token_marks = row_marks + ROWS;
+  uint32_t* any_lossy = token_marks + NT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool dual = p.epilogue == EPI_SWIGLU;
   const int OUTS = dual ? ROWS / 2 : ROWS;
@@ -261,6 +302,12 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (C::P == 3)
+    for (int e = threadIdx.x; e < ROWS + NT + 1; e += C::THREADS) row_marks[e] = 0;
+  auto note = [&](uint32_t* at, uint32_t word) {
+    if (word) atomicOr(at, word);
+    if (word & LOSSY) *any_lossy = 1;
+  };
   if (warp == 0) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -344,6 +391,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
       }
       __syncwarp();
+      if (C::P == 3) {
+        const int runs = (p.K + SPLIT_RUN - 1) / SPLIT_RUN, items = min(NT, p.M - m0) * runs;
+        for (int e = lane; e < items; e += 32) note(&token_marks[e / runs], p.marks[(size_t)m0 * runs + e]);
+      }
     } else {
       // ---- the parts of the tokens: 16 threads a row, four elements each. Rows past the end are read from the last one
       const int pt = (warp - C::B_WARP) * 32 + lane, r0 = pt / 16, kq = pt % 16 * 4;
@@ -359,6 +410,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
       for (int i = 0; i < C::PASSES; ++i) held[i] = load(i, first);
       const uint32_t at0 = r0 * ROW_BYTES + ((kq / 8 ^ (r0 & 7)) << 4) + (kq & 4) * 2;
+      Marks marks[C::PASSES];
       for (int c = first, n = 0; c < last; ++c, ++n) {
         const int st = n % C::STAGES;
         if (VEC && (c + 1) * CHUNK > p.K && c * CHUNK + kq >= p.K) {
@@ -368,7 +420,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         uint2 parts[C::PASSES][C::P];
 #pragma unroll
         for (int i = 0; i < C::PASSES; ++i) {
-          split(parts[i], held[i]);
+          split(parts[i], held[i], marks[i]);
           held[i] = load(i, c + 1);
         }
         if (!warp_wait(&done[st], ((n / C::STAGES) & 1) ^ 1, p.err, abort_flag)) break;
@@ -381,6 +433,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[st]);
       }
+      if (C::P == 3)
+#pragma unroll
+        for (int i = 0; i < C::PASSES; ++i) note(&token_marks[r0 + i * C::PASS_ROWS], marks[i].word());
     }
   } else if (warp >= C::A_WARP) {
     // ---- the parts of the weights: a row a lane, half of the chunk's K a warp
@@ -391,6 +446,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const int w_n = min(dual ? n0 + quarter * 16 + (lane & 15) : n0 + l, p.N - 1);
     const TI* w_row = (const TI*)p.W + (size_t)(dual && (lane & 16) ? p.N + w_n : w_n) * p.K;
     const uint32_t a_at = tmem + ((uint32_t)(quarter * 32) << 16) + C::A_AT + half * 16;
+    Marks marks;
     for (int c = first + set, n = set; c < last; c += C::SETS, n += C::SETS) {
       const int st = n % C::STAGES, raw = n % C::RAWS;
       uint32_t w[C::P][16];
@@ -400,7 +456,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           uint2 x[C::P];
-          split(x, *reinterpret_cast<const float4*>(src + ((q ^ (raw_row & 7)) << 4)));
+          split(x, *reinterpret_cast<const float4*>(src + ((q ^ (raw_row & 7)) << 4)), marks);
 #pragma unroll
           for (int t = 0; t < C::P; ++t) w[t][2 * q] = x[t].x, w[t][2 * q + 1] = x[t].y;
         }
@@ -411,7 +467,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         for (int q = 0; q < 8; ++q) {
           const int k = c * CHUNK + half * 32 + 4 * q;
           uint2 x[C::P];
-          split(x, load4<false>(w_row + k, p.K - k));
+          split(x, load4<false>(w_row + k, p.K - k), marks);
 #pragma unroll
           for (int t = 0; t < C::P; ++t) w[t][2 * q] = x[t].x, w[t][2 * q + 1] = x[t].y;
         }
@@ -425,6 +481,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[st]);
     }
+    if (C::P == 3) note(&row_marks[l], marks.word());
   } else {
     // ---- sums: thread = weight row, COLS tokens
     const int quarter = warp & 3, col0 = (warp >> 2) * C::COLS;
@@ -501,6 +558,18 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   if (p.slices > 1) cluster_sync_all();
   else __syncthreads();
   const int items = *abort_flag ? 0 : OUTS * min(NT, p.M - m0);
+  bool lossy = false;
+  if (C::P == 3) {
+    if (p.slices == 1) lossy = *any_lossy;
+    else lossy = __any_sync(0xffffffffu, ld_cluster_u32(smem_u32(any_lossy), lane % p.slices, 0));
+  }
+  // a row's marks in all of K
+  auto marks_of = [&](const uint32_t* at) {
+    uint32_t word = *at;
+    if (p.slices > 1)
+      for (int s = 0; s < p.slices; ++s) word |= ld_cluster_u32(smem_u32(at), s, 0);
+    return word;
+  };
 #pragma unroll 1
   for (int e0 = rank * C::THREADS; e0 < items; e0 += p.slices * C::THREADS) {
     const int e = e0 + threadIdx.x, o = e % OUTS, m = e / OUTS, n = n0 + o;
@@ -533,9 +602,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
       }
     }
-    if (__any_sync(0xffffffffu, live && !(settled(v) && settled(u)))) {
-      v = settle<TI>(p, v, live && !settled(v), m0 + m, n);
-      if (dual) u = settle<TI>(p, u, live && !settled(u), m0 + m, p.N + n);
+    uint32_t token = 0, weight = 0, up_weight = 0;
+    if (lossy && live) {
+      token = marks_of(&token_marks[m]);
+      weight = marks_of(&row_marks[row]);
+      if (dual) up_weight = marks_of(&row_marks[row + 16]);
+    }
+    const bool again = live && !settled(v, token, weight), again_u = live && dual && !settled(u, token, up_weight);
+    if (__any_sync(0xffffffffu, again || again_u)) {
+      v = settle<TI>(p, v, again, m0 + m, n);
+      if (dual) u = settle<TI>(p, u, again_u, m0 + m, p.N + n);
     }
     if (live) finish<TI>(p, m0 + m, n, v, u);
   }
@@ -577,9 +653,11 @@ int launch(GemmParams p, int slices, void* scratch, cudaStream_t stream) {
     const int ld = scratch_ld(p.K);
     CUCA_REQUIRE(scratch && ((uintptr_t)scratch & 15) == 0, "gemm: %d tokens need scratch", p.M);
     CUCA_REQUIRE(cuca_tensor_map_2d(scratch, 2, (uint64_t)C::P * p.M, p.K, ld, NT, &tmX), "gemm: tensor map of the tokens failed");
-    const long long quads = (long long)p.M * ((p.K + 3) / 4);
-    const unsigned grid = (unsigned)std::min<long long>((quads + 255) / 256, 8ll * cuca_device_sms());
-    cuca_launch(split_kernel<TI, VEC>, dim3(grid), dim3(256), 0, stream, true, (const TI*)p.A, (__nv_bfloat16*)scratch, p.M, p.K, p.lda, ld);
+    uint16_t* marks = (uint16_t*)scratch + (size_t)C::P * p.M * ld;
+    p.marks = marks;
+    for (int m = 0; m < p.M; m += 65535)  // (the most rows of a launch)
+      cuca_launch(split_kernel<TI, VEC>, dim3((p.K + SPLIT_RUN - 1) / SPLIT_RUN, std::min(p.M - m, 65535)), dim3(256), 0, stream, true,
+                  (const TI*)p.A, (__nv_bfloat16*)scratch, marks, m, p.M, p.K, p.lda, ld);
   }
   if (slices > 1) cuca_launch_cluster(kernel, dim3((unsigned)ctas), dim3(C::THREADS), C::SMEM, stream, true, (unsigned)slices, tmW, tmX, p);
   else cuca_launch(kernel, dim3((unsigned)ctas), dim3(C::THREADS), C::SMEM, stream, true, tmW, tmX, p);
@@ -663,9 +741,12 @@ int go(const GemmParams& p, void* scratch, int form_tokens, int form_slices, cud
 
 }  // namespace
 
-// Most tokens for which cuca_gemm_f32 needs no scratch. Beyond: parts x M x K' 16-bit values, three parts of 32-bit operands and
-// one of 16-bit ones, K' = K rounded up to a multiple of 8; 16-byte aligned.
+// Most tokens for which cuca_gemm_f32 needs no scratch. Beyond, for each token so many 16-bit values, the whole 16-byte aligned:
+// its parts, three of 32-bit operands and one of 16-bit ones, each K rounded up to a multiple of 8, and its marks.
 CUCA_API int cuca_gemm_f32_few_tokens() { return 16; }
+CUCA_API int cuca_gemm_f32_scratch_per_token(int in_dtype, int K) {
+  return (in_dtype == CUCA_F32 ? 3 : 1) * scratch_ld(K) + (K + SPLIT_RUN - 1) / SPLIT_RUN;
+}
 
 // out = epilogue(A[M,K] W[N,K]^T). in_dtype: A, W and bias; out_dtype: out.
 // epilogue 0 store, 1 out (32-bit) += result, 2 SwiGLU (W has 2N rows).
@@ -680,7 +761,7 @@ CUCA_API int cuca_gemm_f32(const void* A, const void* W, const void* bias, void*
   CUCA_REQUIRE(epilogue >= EPI_STORE && epilogue <= EPI_SWIGLU, "gemm: unknown epilogue %d", epilogue);
   CUCA_REQUIRE((in_dtype == CUCA_F32 && out_dtype == CUCA_F32) || (in_dtype == CUCA_BF16 && (out_dtype == CUCA_F32 || out_dtype == CUCA_BF16)),
                "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
-  GemmParams p = {A, W, bias, out, err, M, N, K, lda, ldo, epilogue, out_dtype == CUCA_F32, 0, 0};
+  GemmParams p = {A, W, bias, out, err, M, N, K, lda, ldo, epilogue, out_dtype == CUCA_F32, nullptr, 0, 0};
   const bool vec = in_dtype == CUCA_F32 && K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
   int rc;
   if (in_dtype == CUCA_BF16) rc = go<__nv_bfloat16, false>(p, scratch, form_tokens, form_slices, stream);

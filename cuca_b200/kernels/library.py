@@ -33,6 +33,7 @@ _SIGNATURES = {
     "cuca_add_to_stream": [_P, _P, _I, c_size_t, _P],
     "cuca_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _I, _P],
     "cuca_gemm_f32_few_tokens": [],
+    "cuca_gemm_f32_scratch_per_token": [_I, _I],
     "cuca_latent_attention_tc_tokens": [_I, _I, _I],
     "cuca_latent_attention_tc": [_P, _P, _P, _I, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _P],
     "cuca_attention_generic": [_P, _I, _P, _I, _I, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P],

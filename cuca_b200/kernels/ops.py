@@ -169,7 +169,7 @@ def gemm_simt(a, w, out, epilogue=EPI_STORE, bias=None, err=None, form=(0, 0)) -
         _gemm_few.append(int(lib.cuca_gemm_f32_few_tokens()))
     scratch = None
     if M > _gemm_few[0] or form[0] > _gemm_few[0]:  # the tokens as bfloat16 parts
-        scratch = torch.empty((3 if a.dtype == torch.float32 else 1) * M * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=a.device)
+        scratch = torch.empty(M * int(lib.cuca_gemm_f32_scratch_per_token(dtype_code(a.dtype), K)), dtype=torch.bfloat16, device=a.device)
     library.check(lib.cuca_gemm_f32(_p(a), _p(w), _p(bias), _p(out), dtype_code(a.dtype), dtype_code(out.dtype),
                                     M, N, K, a.stride(0), out.stride(0), epilogue, _p(err), _p(scratch), int(form[0]),
                                     int(form[1]), _stream()), "gemm_simt")

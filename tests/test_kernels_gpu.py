@@ -168,6 +168,45 @@ def test_gemm_f32_of_few_products(dev, K):
         assert bool(((out.double() - want[:M]).abs() <= (1.5 if K == 1 else 2.5) * 2.0 ** -23 * sizes[:M]).all())
 
 
+@pytest.mark.parametrize("K", [8, 1030, 4100])
+@pytest.mark.parametrize("tiny,large", [(1e-41, 1.0), (1e-36, 1e30), (1.2345e-40, 1e37), (3e-39, 2.0 ** 45), (2.0 ** -70, 2.0 ** -65),
+                                        (1e-43, 3e4)])
+@pytest.mark.parametrize("epilogue", [0, 2])
+def test_gemm_f32_of_tiny_and_large_values(dev, K, tiny, large, epilogue):
+    """Values of which bfloat16 parts hold too little, among tokens and among weights, with ones that lift them up again, in
+    rows of their own and among ordinary ones: as good as ordinary values, or as 32-bit products of that size are."""
+    from cuca_b200.kernels import library, ops
+    M, N = 70, 140
+    g = torch.Generator(device=dev).manual_seed(K)
+    a, w = torch.randn(M, K, device=dev, generator=g), torch.randn((epilogue == 2) * N + N, K, device=dev, generator=g)
+    a[3], w[5], w[-7] = a[3] * tiny, w[5] * large, w[-7] * large   # a tiny token, large weights
+    a[66], w[9], w[-20] = a[66] * large, w[9] * tiny, w[-20] * tiny   # and the other way round
+    a[8], a[8, K - 3], w[11], w[11, K - 3], w[130], w[130, K - 3] = 0, tiny, 0, large, 0, tiny  # one value of a row
+    y, sizes = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    bound = 50 * 2.0 ** -24 * sizes + K * 2.0 ** -149
+    if epilogue == 2:  # silu has a slope below 1.1 and is at most its argument's size
+        gate, up = y[:, :N], y[:, N:]
+        y = gate * torch.sigmoid(gate) * up
+        bound = 1.1 * bound[:, :N] * up.abs() + bound[:, N:] * gate.abs() + bound[:, :N] * bound[:, N:] + 8 * 2.0 ** -24 * y.abs() + 2.0 ** -148
+    fits = sizes < 1e38  # (partial sums of others may overflow)
+    if epilogue == 2:
+        fits = fits[:, :N] & fits[:, N:] & (y.abs() < 1e38)
+    ran = 0
+    for form in ((0, 0), (16, 1), (16, 4), (32, 1), (32, 3), (64, 1), (64, 2), (96, 1)):
+        out = torch.empty(M, N, device=dev)
+        try:
+            ops.gemm_simt(a, w, out, epilogue, form=form)
+        except library.KernelError:
+            assert form[1] > 1
+            continue
+        ran += 1
+        assert bool(((out.double() - y).abs() <= bound)[fits].all()), form
+        few = torch.empty(9, N, device=dev)  # (the tiny token among few)
+        ops.gemm_simt(a[:9], w, few, epilogue)
+        assert torch.equal(few, out[:9]) or torch.equal(few.nan_to_num(1.0), out[:9].nan_to_num(1.0))
+    assert ran >= 5
+
+
 @pytest.mark.parametrize("K", [60, 64, 250, 1021, 2046])
 @pytest.mark.parametrize("epilogue", [0, 1, 2])
 def test_gemm_simt_of_16_bit_operands_is_the_32_bit_ones_result(dev, K, epilogue):
