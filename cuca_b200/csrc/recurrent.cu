@@ -5,7 +5,7 @@
 //   gated_group_norm   y * silu(z), RMS-normed in equal parts, times a weight
 // A step brings each request a run of consecutive rows (req_row0, req_count); a kernel walks a request's rows in
 // order from the state its slot holds and leaves the new state there. The order of the arithmetic along a sequence
-// does not depend on where it was cut into steps.
+// does not depend on where it was cut into steps, but for the state-space scan's long portions in segments (16-bit models).
 #include "common.cuh"
 #include "state_rows.cuh"
 #include <math.h>
@@ -212,20 +212,29 @@ __global__ void causal_conv_many_kernel(const float* __restrict__ in, int ld_in,
 
 constexpr int SSM_MAX_STATE = 1024;
 constexpr int SSM_SEGMENT = 512;  // tokens of a segment (below)
+constexpr int SSM_MAX_CUT = 64;
+
+// The requests of a step whose portions are cut: request q[i], ascending, has the cells first[i] .. first[i + 1] - 1, one a segment.
+struct Cut {
+  int n;
+  int q[SSM_MAX_CUT], first[SSM_MAX_CUT + 1];
+};
 
 // One block per (head, request, run of PB value columns); a column's state rows lie with NS threads (see Split).
 // state: [slots, H, P, N]. xbc: 32-bit [rows, H P + 2 G N] after the convolution (x | B | C); dt_raw: rows of stride
 // ld_dt, head h at column dt_col + h, before bias and softplus.
 // Tokens hang together through one multiply-add per state value alone, so the kernel is bound by how many instructions
 // it issues and by its reads of shared memory: eight rows of four columns a thread, pairs of rows in every instruction.
-template <typename S_>
+// CUT: blocks of segments come first, each from no state but the request's first, whose state goes to its cell (see
+// ssm_join_kernel), then those of the requests that are walked whole.
+template <typename S_, bool CUT>
 __global__ void __launch_bounds__(128)
 ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, int ld_dt, int dt_col,
                 const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                 const float* __restrict__ d_skip, float* __restrict__ state, float* __restrict__ y,
                 const int* __restrict__ req_row0, const int* __restrict__ req_count,
                 const int* __restrict__ slots, int H, int P, int N, int G, int wide, float* __restrict__ ends,
-                float* __restrict__ decays) {
+                float* __restrict__ decays, const __grid_constant__ Cut cut) {
   constexpr int NS = S_::NS, NC = S_::NC, DP = S_::DP, PB = S_::PB, TC = S_::TC, PAIRS = S_::PAIRS;
   constexpr int PER = 2 * DP + ((PB + 1 + 3) & ~3);  // a token: B, C, the block's x, the raw step size
   static_assert(TC <= 32, "a lane a token");
@@ -233,9 +242,23 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
   __shared__ float steps[4][TC][2];  // a warp's own: step size, decay
   pdl_trigger();
   pdl_wait();
-  // with `ends`, a segment of the request: from no state but the first, and its state goes there (see ssm_join_kernel)
-  const int h = blockIdx.x % H, seg = blockIdx.x / H, q = blockIdx.y;
-  const int slot = slots[q], whole = req_count[q], n = ends ? min(SSM_SEGMENT, whole - seg * SSM_SEGMENT) : whole;
+  int h = blockIdx.x, q = blockIdx.y, seg = 0, unit = 0;
+  bool segment = false;
+  if (CUT) {
+    h = blockIdx.x % H;
+    unit = blockIdx.x / H;
+    segment = unit < cut.first[cut.n];
+    int i = 0;
+    if (segment) {
+      while (unit >= cut.first[i + 1]) ++i;
+      q = cut.q[i];
+      seg = unit - cut.first[i];
+    } else {
+      q = unit - cut.first[cut.n];
+      while (i < cut.n && cut.q[i] <= q) ++i, ++q;
+    }
+  }
+  const int slot = slots[q], whole = req_count[q], n = segment ? min(SSM_SEGMENT, whole - seg * SSM_SEGMENT) : whole;
   const int r0 = req_row0[q] + seg * SSM_SEGMENT;
   if (slot < 0 || n <= 0) return;
   const int lane = threadIdx.x & 31;
@@ -247,8 +270,8 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
   float* st = state + (((size_t)slot * H + h) * P + (cols > 0 ? col0 + at : 0)) * N;
   f32x2 S[NC][PAIRS];
   load_rows<S_>(S, st, s, N, seg > 0 ? 0 : cols, wide);
-  const size_t cell = ((size_t)seg * gridDim.y + q) * H + h;
-  if (ends && whole > SSM_SEGMENT) st = ends + (cell * P + (cols > 0 ? col0 + at : 0)) * N;
+  const size_t cell = (size_t)unit * H + h;
+  if (segment) st = ends + (cell * P + (cols > 0 ? col0 + at : 0)) * N;
   float product = 1.f;  // of the decays
   const float A = -expf(a_log[h]);
   const float bias = dt_bias[h], D = d_skip[h];
@@ -315,7 +338,7 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
         staged_values<NC>(x, tok + 2 * DP, at);
         const float dt = mine[t + i][0];
         const f32x2 decay = f2_both(mine[t + i][1]);
-        product *= mine[t + i][1];
+        if (CUT) product *= mine[t + i][1];
 #pragma unroll
         for (int j = 0; j < NC; ++j) {
           const f32x2 dx = f2_both(dt * x[j]);
@@ -336,13 +359,13 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
     __syncthreads();  // this run is read to the end before the run after next is copied over it
   }
   store_rows<S_>(S, st, s, N, cols, wide);
-  if (ends && threadIdx.x == 0 && blockIdx.z == 0) decays[cell] = product;
+  if (segment && threadIdx.x == 0 && blockIdx.z == 0) decays[cell] = product;
 }
 
 // What a segment's tokens owe to the segments before it. A prompt's scan is 2,048 steps one behind the other in a warp a
 // scheduler, so it is cut into segments that run side by side, each from no state; with S the state a segment should have
 // begun with, its outputs lack C_t S times the decays since, and the state behind it lacks S times all of its decays.
-// One block per (head, request, JOIN tokens of a segment behind the first): S from the segments' ends in turn, then 64
+// One block per (head, segment behind a request's first, JOIN of its tokens): S from the segments' ends in turn, then 64
 // tokens x 64 columns at a time as a contraction in 32 bits, 4 x 4 outputs a thread, bound by shared memory. 64 heads of
 // 64 x 128, 2,048 tokens in four segments: scan 340 -> 218 us and 80 for this. Requests of one segment are scanned as before.
 constexpr int JOIN = 256, JOIN_P = 64, JOIN_PITCH = JOIN_P + 4;
@@ -353,20 +376,22 @@ ssm_join_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw,
                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, float* __restrict__ state,
                 float* __restrict__ y, const int* __restrict__ req_row0, const int* __restrict__ req_count,
                 const int* __restrict__ slots, int H, int P, int N, int G, const float* __restrict__ ends,
-                const float* __restrict__ decays) {
+                const float* __restrict__ decays, const __grid_constant__ Cut cut) {
   extern __shared__ __align__(16) float sm[];
   float* S = sm;                        // [N][JOIN_PITCH]
   float* Cs = S + N * JOIN_PITCH;       // [64][N + 4]
   float* since = Cs + 64 * (N + 4);     // [SSM_SEGMENT]: the decays of the segment up to and with each token
   pdl_trigger();
   pdl_wait();
-  const int h = blockIdx.x, q = blockIdx.y, tid = threadIdx.x;
-  const int seg = 1 + blockIdx.z / (SSM_SEGMENT / JOIN), part0 = blockIdx.z % (SSM_SEGMENT / JOIN) * JOIN;
+  const int h = blockIdx.x, tid = threadIdx.x, part0 = blockIdx.z * JOIN;
+  int i = 0;
+  while ((int)blockIdx.y >= cut.first[i + 1] - (i + 1)) ++i;  // (each request before has a first segment that is not joined)
+  const int q = cut.q[i], seg = 1 + blockIdx.y - (cut.first[i] - i), cell0 = cut.first[i];
   const int slot = slots[q], whole = req_count[q], n = min(SSM_SEGMENT, whole - seg * SSM_SEGMENT);
   if (slot < 0 || n <= part0) return;
   const int g = h / (H / G), C = H * P + 2 * G * N, row0 = req_row0[q] + seg * SSM_SEGMENT;
   const bool last = part0 == 0 && (seg + 1) * SSM_SEGMENT >= whole;  // this block leaves the request's state behind
-  auto cell = [&](int k) { return ((size_t)k * gridDim.y + q) * H + h; };
+  auto cell = [&](int k) { return (size_t)(cell0 + k) * H + h; };
   for (int e = tid; e < P * N; e += 256) {
     float v = ends[cell(0) * P * N + e];
     for (int k = 1; k < seg; ++k) v = decayed(decays[cell(k)], v) + ends[cell(k) * P * N + e];
@@ -580,47 +605,75 @@ CUCA_API int cuca_causal_conv(const float* in, int ld_in, int col0, const void* 
 CUCA_API int cuca_ssm_segment() { return SSM_SEGMENT; }
 CUCA_API int cuca_ssm_segments_allowed(int P, int N) { return P > 0 && P <= JOIN_P && P % 4 == 0 && N > 0 && N <= 128 && N % 4 == 0; }
 
-// n_segments > 1: no request brings more than n_segments runs of cuca_ssm_segment() tokens, and one with more than one run has
-// them walked side by side (another rounding); scratch: n_segments n_seqs H (P N + 1) floats, 16-byte aligned.
+// Calls `go` with the split of the state that its size takes.
+template <typename F>
+static int with_split(int N, F go) {
+  // Few state values a column: threads of four rows, so that a block's columns are no more than a head has (64). Measured
+  // with eight and four rows a thread, us: 80 heads of 64 x 16, 1,501 tokens 365, 205, 256 requests of a token 77, 48; 24
+  // heads of 64 x 64, 1,501 tokens 344, 197, 64 prompts of 40 52, 58 (as at 64 x 128: 249, 296, so eight rows stay there).
+  if (N <= 16) return go(Split<4, 4, 2>());
+  if (N <= 32) return go(Split<8, 4, 4>());
+  if (N <= 64) return go(Split<16, 4, 4>());
+  if (N <= 128) return go(Split<16, 8, 4>());
+  if (N <= 256) return go(Split<32, 8, 4>());
+  if (N <= 512) return go(Split<32, 16, 4>());
+  return go(Split<32, 32, 2>());
+}
+
+// The portions that are cut where one of at least `cut_from` tokens is: requests of counts[0 .. n_seqs - 1] tokens.
+static Cut cut_of(const int* counts, int n_seqs, int cut_from) {
+  Cut cut = {};
+  for (int q = 0; q < n_seqs && cut.n < SSM_MAX_CUT; ++q) {
+    if (counts[q] < cut_from || counts[q] <= SSM_SEGMENT) continue;
+    cut.q[cut.n] = q;
+    cut.first[cut.n + 1] = cut.first[cut.n] + (counts[q] + SSM_SEGMENT - 1) / SSM_SEGMENT;
+    ++cut.n;
+  }
+  return cut;
+}
+
+// Cells that cuca_ssm_scan's scratch has to hold: one a segment, whatever other requests the step has.
+CUCA_API int cuca_ssm_cells(const int* counts, int n_seqs, int cut_from) {
+  const Cut cut = cut_of(counts, n_seqs, cut_from);
+  return cut.first[cut.n];
+}
+
+// cut_from > 0: portions of at least so many tokens and more than cuca_ssm_segment() (the first 64 of them) have their segments
+// walked side by side (another rounding). counts: the requests' tokens, as in req_count, on the host; scratch: cuca_ssm_cells
+// times H (P N + 1) floats, 16-byte aligned.
 CUCA_API int cuca_ssm_scan(const float* xbc, const float* dt_raw, int ld_dt, int dt_col, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, float* y, const int* req_row0,
-                           const int* req_count, const int* slots, int n_seqs, int H, int P, int N, int G, int n_segments,
-                           float* scratch, cudaStream_t stream) {
+                           const int* req_count, const int* slots, int n_seqs, int H, int P, int N, int G, int cut_from,
+                           const int* counts, float* scratch, cudaStream_t stream) {
   if (n_seqs == 0) return 0;
   CUCA_REQUIRE(H > 0 && P > 0 && N > 0 && G > 0 && H % G == 0, "ssm_scan: bad sizes heads=%d vdim=%d state=%d groups=%d",
                H, P, N, G);
   CUCA_REQUIRE(n_seqs <= 65535, "ssm_scan: %d requests exceed the launch limit", n_seqs);
   CUCA_REQUIRE(N <= SSM_MAX_STATE, "ssm_scan: state size %d exceeds %d", N, SSM_MAX_STATE);
   const int wide = N % 4 == 0 && (H * P) % 4 == 0 && (((uintptr_t)xbc | (uintptr_t)state) & 15) == 0;
-  const bool cut = n_segments > 1 && scratch;
-  CUCA_REQUIRE(!cut || (cuca_ssm_segments_allowed(P, N) && (((uintptr_t)xbc | (uintptr_t)state | (uintptr_t)y | (uintptr_t)scratch) & 15) == 0 &&
-                        (long long)H * n_segments < (1ll << 31) && n_segments <= 16384), "ssm_scan: %d segments of %d x %d", n_segments, P, N);
-  float* ends = cut ? scratch : nullptr;
-  float* decays = cut ? scratch + (size_t)n_segments * n_seqs * H * P * N : nullptr;
-  auto go = [&](auto split) {
+  const Cut cut = cut_from > 0 && counts ? cut_of(counts, n_seqs, cut_from) : Cut{};
+  const int cells = cut.first[cut.n], units = cells + n_seqs - cut.n;
+  CUCA_REQUIRE(!cut.n || (cuca_ssm_segments_allowed(P, N) && scratch &&
+                          (((uintptr_t)xbc | (uintptr_t)state | (uintptr_t)y | (uintptr_t)scratch) & 15) == 0 && (H * P + 2 * G * N) % 4 == 0 &&
+                          cells <= 65535 && (long long)H * units < (1ll << 31)), "ssm_scan: %d segments of %d x %d", cells, P, N);
+  float* ends = scratch;
+  float* decays = scratch + (size_t)cells * H * P * N;
+  const int rc = with_split(N, [&](auto split) {
     using C = decltype(split);
-    return launch_scan<C>("ssm_scan", ssm_scan_kernel<C>, 2 * C::DP + ((C::PB + 4) & ~3), cut ? H * n_segments : H, n_seqs, P, stream,
-                          xbc, dt_raw, ld_dt, dt_col, dt_bias, a_log, d_skip, state, y, req_row0, req_count, slots, H, P, N, G, wide,
-                          ends, decays);
-  };
-  // Few state values a column: threads of four rows, so that a block's columns are no more than a head has (64). Measured
-  // with eight and four rows a thread, us: 80 heads of 64 x 16, 1,501 tokens 365, 205, 256 requests of a token 77, 48; 24
-  // heads of 64 x 64, 1,501 tokens 344, 197, 64 prompts of 40 52, 58 (as at 64 x 128: 249, 296, so eight rows stay there).
-  int rc;
-  if (N <= 16) rc = go(Split<4, 4, 2>());
-  else if (N <= 32) rc = go(Split<8, 4, 4>());
-  else if (N <= 64) rc = go(Split<16, 4, 4>());
-  else if (N <= 128) rc = go(Split<16, 8, 4>());
-  else if (N <= 256) rc = go(Split<32, 8, 4>());
-  else if (N <= 512) rc = go(Split<32, 16, 4>());
-  else rc = go(Split<32, 32, 2>());
-  if (rc || !cut) return rc;
+    const int per_token = 2 * C::DP + ((C::PB + 4) & ~3);
+    if (cut.n)
+      return launch_scan<C>("ssm_scan", ssm_scan_kernel<C, true>, per_token, H * units, 1, P, stream, xbc, dt_raw, ld_dt, dt_col, dt_bias,
+                            a_log, d_skip, state, y, req_row0, req_count, slots, H, P, N, G, wide, ends, decays, cut);
+    return launch_scan<C>("ssm_scan", ssm_scan_kernel<C, false>, per_token, H, n_seqs, P, stream, xbc, dt_raw, ld_dt, dt_col, dt_bias,
+                          a_log, d_skip, state, y, req_row0, req_count, slots, H, P, N, G, wide, ends, decays, cut);
+  });
+  if (rc || !cut.n) return rc;
   const int smem = (N * JOIN_PITCH + 64 * (N + 4) + SSM_SEGMENT) * 4;
   static const cudaError_t e = cudaFuncSetAttribute(ssm_join_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     (128 * JOIN_PITCH + 64 * 132 + SSM_SEGMENT) * 4);
   CUCA_REQUIRE(e == cudaSuccess, "ssm_scan: %d bytes of shared memory were refused: %s", smem, cudaGetErrorString(e));
-  cuca_launch(ssm_join_kernel, dim3(H, n_seqs, (n_segments - 1) * (SSM_SEGMENT / JOIN)), dim3(256), smem, stream, true, xbc, dt_raw,
-              ld_dt, dt_col, dt_bias, a_log, state, y, req_row0, req_count, slots, H, P, N, G, (const float*)ends, (const float*)decays);
+  cuca_launch(ssm_join_kernel, dim3(H, cells - cut.n, SSM_SEGMENT / JOIN), dim3(256), smem, stream, true, xbc, dt_raw, ld_dt, dt_col,
+              dt_bias, a_log, state, y, req_row0, req_count, slots, H, P, N, G, (const float*)ends, (const float*)decays, cut);
   CUCA_CHECK_LAUNCH("ssm_join");
   return 0;
 }

@@ -11,6 +11,7 @@ import os
 
 import torch
 
+from ..native import host
 from . import library
 
 F32, BF16 = 0, 1
@@ -944,22 +945,33 @@ def causal_conv(src, col0, weight, bias, kept, out, step) -> None:
         _stream()), "causal_conv")
 
 
-def ssm_scan(xbc, proj, dt_col, dt_bias, a_log, d_skip, state, y, step, H, P, N, G, segments: bool = False) -> None:
-    """`segments`: long portions are cut into runs that are walked side by side and joined (another rounding, which
-    depends on the portion's length alone)."""
+def _host_counts(step):
+    """The requests' token counts as a C array (made once per step), or None where the host does not know them."""
+    counts = step.host.get("counts") if step.static_max_len is None else None
+    if not counts or len(counts) != step.n_seqs:
+        return None
+    if "host_counts" not in step.plans:
+        step.plans["host_counts"] = host.ints(counts)
+    return step.plans["host_counts"]
+
+
+def ssm_scan(xbc, proj, dt_col, dt_bias, a_log, d_skip, state, y, step, H, P, N, G, segments: int = 0) -> None:
+    """`segments`: portions of at least so many tokens (True: all of more than one segment) are cut into runs that are walked
+    side by side and joined (another rounding)."""
     _cuda(xbc, proj, state, y)
     lib = library.load()
-    n_segments, scratch = 1, None
-    counts = step.host.get("counts") if segments and step.static_max_len is None else None
-    if counts:
-        run = int(lib.cuca_ssm_segment())
-        if max(counts) > run and lib.cuca_ssm_segments_allowed(P, N) and xbc.shape[1] % 4 == 0:
-            n_segments = -(-max(counts) // run)
-            scratch = torch.empty(n_segments * step.n_seqs * H * (P * N + 1), dtype=torch.float32, device=y.device)
+    scratch, at = None, None
+    counts = _host_counts(step) if segments and lib.cuca_ssm_segments_allowed(P, N) and xbc.shape[1] % 4 == 0 \
+        and (xbc.data_ptr() | state.data_ptr() | y.data_ptr()) % 16 == 0 else None
+    if counts is not None:
+        at = ctypes.addressof(counts)
+        cells = int(lib.cuca_ssm_cells(at, step.n_seqs, int(segments)))
+        if cells:
+            scratch = torch.empty(cells * H * (P * N + 1), dtype=torch.float32, device=y.device)
     library.check(lib.cuca_ssm_scan(
         _p(xbc), _p(proj), proj.stride(0), int(dt_col), _p(dt_bias), _p(a_log), _p(d_skip), _p(state), _p(y),
-        _p(step.req_row0), _p(step.req_count), _p(step.slots), step.n_seqs, H, P, N, G, n_segments, _p(scratch), _stream()),
-        "ssm_scan")
+        _p(step.req_row0), _p(step.req_count), _p(step.slots), step.n_seqs, H, P, N, G, int(segments) if scratch is not None else 0,
+        at, _p(scratch), _stream()), "ssm_scan")
 
 
 def gated_group_norm(y, z, weight, out, parts, eps) -> None:

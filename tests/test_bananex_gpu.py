@@ -448,6 +448,45 @@ def test_latent_attention_on_tensor_cores(layer):
     assert int(rt.err.item()) == 0
 
 
+@pytest.mark.parametrize("counts,cut", [([1] * 40 + [1985] + [1] * 23, [40]), ([600] * 66, list(range(64))),
+                                        ([513, 1, 1537, 512, 40, 700], [0, 2, 5]), ([1, 1100, 1100], [1, 2])])
+def test_state_scan_in_segments_beside_other_requests(rt32, counts, cut):
+    """Scratch is for the segments there are, whatever else the step brings; whole walks and cut ones have the bits that they have
+    alone. Of more portions than one launch holds, the first are cut."""
+    from cuca_b200.kernels import library, ops
+    dev, H, G, P, N = rt32.device, 4, 1, 64, 128
+    run = int(library.load().cuca_ssm_segment())
+    g = torch.Generator(device=dev).manual_seed(len(counts))
+    rows, slots = sum(counts), list(range(len(counts)))[::-1]
+    xbc = torch.randn(rows, H * P + 2 * G * N, device=dev, generator=g)
+    proj = torch.randn(rows, H, device=dev, generator=g) - 2.0
+    bias, a_log, skip = (torch.randn(H, device=dev, generator=g) for _ in range(3))
+    state = torch.randn(len(counts), H, P, N, device=dev, generator=g)
+
+    def scan(which, segments):
+        first = [sum(counts[:q]) for q in which]
+        at = torch.cat([torch.arange(f, f + counts[q], device=dev) for f, q in zip(first, which)])
+        x, pr, st, y = xbc[at], proj[at], state.clone(), torch.full((len(at), H * P), 7.0, device=dev)
+        step = _step(dev, [(0, counts[q]) for q in which], [slots[q] for q in which])
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        ops.ssm_scan(x, pr, 0, bias, a_log, skip, st, y, step, H, P, N, G, segments=segments)
+        return y, st, torch.cuda.max_memory_allocated() - before
+    everyone = list(range(len(counts)))
+    y, st, scratch = scan(everyone, True)
+    plain_y, plain, none = scan(everyone, 0)
+    cells = sum(-(-counts[q] // run) for q in cut)
+    assert none == 0 and scratch <= cells * H * (P * N + 1) * 4 + 512
+    r = 0
+    for q, n in enumerate(counts):
+        same = torch.equal(y[r:r + n], plain_y[r:r + n]) and torch.equal(st[slots[q]], plain[slots[q]])
+        assert same == (q not in cut), q
+        if q in cut[:3]:
+            alone_y, alone, _ = scan([q], True)
+            assert torch.equal(y[r:r + n], alone_y) and torch.equal(st[slots[q]], alone[slots[q]])
+        r += n
+
+
 @pytest.mark.parametrize("layer,tokens", [
     (bu.latent(heads=16, dim=8, rot_dim=64, vdim=8, kv_rank=512, window=130, scale=1.0), 8),  # two halves of the columns
     (bu.latent(heads=16, dim=16, rot_dim=0, vdim=8, kv_rank=64, window=None, scale=1.0), 8),  # one chunk of values
