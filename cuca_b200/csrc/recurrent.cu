@@ -638,6 +638,22 @@ CUCA_API int cuca_ssm_cells(const int* counts, int n_seqs, int cut_from) {
   return cut.first[cut.n];
 }
 
+// From how many tokens on a step's portions are better off cut, 0: none. Segments pay where a whole walk leaves an SM one block
+// at most or little more, which it keeps waiting for one step after the other; blocks that share an SM fill each other's waits,
+// and then the join is all that segments bring. Measured, us (whole, cut): 64 heads of 64 x 128 (128 blocks a request) 1,024 tokens
+// 172, 200, 2,048 340, 304, four requests of 2,048 864, 1,010; 80 heads 2,048 494, 389; 128 heads 493, 524. 24 heads of 64 x 64,
+// 600 tokens 81, 103, 1,024 136, 114, 2,048 269, 136, eight requests of 1,100 246, 327; 64 heads of 64 x 16, 600 tokens 84, 80,
+// 1,024 140, 90, eight requests of 1,100 234, 307.
+CUCA_API int cuca_ssm_cut_from(const int* counts, int n_seqs, int H, int P, int N) {
+  if (!cuca_ssm_segments_allowed(P, N)) return 0;
+  const int from = N > 64 ? 3 * SSM_SEGMENT : 2 * SSM_SEGMENT;
+  long long n = 0;
+  for (int q = 0; q < n_seqs; ++q) n += counts[q] >= from;
+  const int columns = with_split(N, [](auto split) { return (int)decltype(split)::PB; });
+  const long long blocks = n * H * ((P + columns - 1) / columns);
+  return n > 0 && n <= SSM_MAX_CUT && 4 * blocks <= 5ll * cuca_device_sms() ? from : 0;
+}
+
 // cut_from > 0: portions of at least so many tokens and more than cuca_ssm_segment() (the first 64 of them) have their segments
 // walked side by side (another rounding). counts: the requests' tokens, as in req_count, on the host; scratch: cuca_ssm_cells
 // times H (P N + 1) floats, 16-byte aligned.

@@ -88,6 +88,7 @@ _SIGNATURES = {
     "cuca_causal_conv": [_P, _I, _I, _P, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "cuca_ssm_scan": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P],
     "cuca_ssm_cells": [_P, _I, _I],
+    "cuca_ssm_cut_from": [_P, _I, _I, _I, _I],
     "cuca_ssm_segment": [],
     "cuca_ssm_segments_allowed": [_I, _I],
     "cuca_gated_group_norm": [_P, _P, _I, _P, _I, _P, _I, _I, _I, _I, _F, _P],

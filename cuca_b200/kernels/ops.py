@@ -955,6 +955,14 @@ def _host_counts(step):
     return step.plans["host_counts"]
 
 
+def ssm_cut_from(step, H: int, P: int, N: int) -> int:
+    """From how many tokens on `ssm_scan` is better off with this step's portions in segments (0: with none)."""
+    counts = _host_counts(step)
+    if counts is None:
+        return 0
+    return int(library.load().cuca_ssm_cut_from(ctypes.addressof(counts), step.n_seqs, H, P, N))
+
+
 def ssm_scan(xbc, proj, dt_col, dt_bias, a_log, d_skip, state, y, step, H, P, N, G, segments: int = 0) -> None:
     """`segments`: portions of at least so many tokens (True: all of more than one segment) are cut into runs that are walked
     side by side and joined (another rounding)."""

@@ -114,8 +114,9 @@ class Mamba2(Mixer):
         xbc = rt.empty(rows, self.channels, dtype=torch.float32)
         ops.causal_conv(proj, self.inner, self.conv_w, self.conv_b, cache.state["conv"], xbc, step)
         y = rt.empty(rows, self.inner, dtype=torch.float32)
+        cut_from = ops.ssm_cut_from(step, self.heads, self.vdim, self.n_state) if rt.dtype == torch.bfloat16 else 0
         ops.ssm_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.a_log, self.d, cache.state["ssm"], y,
-                     step, self.heads, self.vdim, self.n_state, self.groups, segments=rt.dtype == torch.bfloat16)
+                     step, self.heads, self.vdim, self.n_state, self.groups, segments=cut_from)
         out = rt.empty(rows, self.inner)
         ops.gated_group_norm(y, proj, self.norm_w, out, self.norm_groups, self.eps)
         rt.stream(stream).add_linear(out, self.w_o)

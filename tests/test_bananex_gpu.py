@@ -487,6 +487,18 @@ def test_state_scan_in_segments_beside_other_requests(rt32, counts, cut):
         r += n
 
 
+def test_state_scan_is_cut_where_it_leaves_the_gpu_empty(rt32):
+    """One long portion, alone or beside single tokens; not short ones, not many, not sizes that take no segments."""
+    from cuca_b200.kernels import ops
+    dev = rt32.device
+
+    def cut_from(counts, H=64, P=64, N=128):
+        return ops.ssm_cut_from(_step(dev, [(0, n) for n in counts], list(range(len(counts)))), H, P, N)
+    assert cut_from([2048]) == 1536 and cut_from([1985] + [1] * 63) == 1536 and cut_from([1535]) == 0 and cut_from([2048] * 4) == 0
+    assert cut_from([1024], 24, 64, 64) == 1024 and cut_from([1023], 24, 64, 64) == 0
+    assert cut_from([2048], 4, 66, 128) == 0 and cut_from([2048], 4, 64, 130) == 0 and cut_from([1]) == 0
+
+
 @pytest.mark.parametrize("layer,tokens", [
     (bu.latent(heads=16, dim=8, rot_dim=64, vdim=8, kv_rank=512, window=130, scale=1.0), 8),  # two halves of the columns
     (bu.latent(heads=16, dim=16, rot_dim=0, vdim=8, kv_rank=64, window=None, scale=1.0), 8),  # one chunk of values
