@@ -1130,13 +1130,16 @@ CUCA_API void cuca_gemm_pair_mode(int mode) { allow_pair = mode; }
 // tokens as rows from few tokens on: its column pieces take all of K each and add nothing up. Measured, us (weights as rows,
 // tokens as rows): K = 2,048, N = 2,048, 32 tokens 18.5, 16.4; 64 tokens 25.6, 16.4; 128 tokens 38.0, 16.4; 256 tokens 67.6,
 // 16.4; N = 20,480, 32 tokens 31.6, 30.7; 64 tokens 33.8, 30.7. K = 4,096, N = 6,144, 32 tokens 24.6, 26.6; 64 tokens 28.6,
-// 26.6; 90 tokens 34.8, 26.7. K = 8,192, N = 2,048, 64 tokens 30.7, 38.9; 90 tokens 43.0, 38.9; 256 tokens 71.7, 38.9.
-// K = 14,336 into the stream, 128 tokens 45.1, 69.7; 256 tokens 63.5, 55.3. Up to 32 tokens they differ by a few us either way.
-static bool swapped(int M, int K, int epilogue, bool rows_of_16_bytes) {
+// 26.6; 90 tokens 34.8, 26.7. K = 8,192, 65 tokens into the stream, N = 1,024 43.1, 31.9; 2,048 32.2, 32.8; 4,096 27.3, 33.7 (tiles
+// that slices of K fill the GPU with in fours and threes); 6,144 32.1, 35.6; 8,192 36.6, 35.6; 256 tokens, N = 2,048 71.7, 38.9.
+// K = 14,336 into the stream, N = 4,096, 128 tokens 45.1, 69.7; 256 tokens 63.5, 55.3; N = 1,024, 256 tokens 84.5, 103;
+// N = 11,008, 160 tokens 86.2, 93.8. Up to 32 tokens they differ by a few us either way.
+static bool swapped(int M, int N, int K, int epilogue, bool rows_of_16_bytes) {
   if (epilogue == EPI_SWIGLU) return M <= SWAP_MAX_TOKENS_SWIGLU;
   if (epilogue == EPI_PARTIAL || !rows_of_16_bytes) return M <= SWAP_MAX_TOKENS;
-  if (K > 8192) return M <= (epilogue == EPI_RESIDUAL ? 128 : SWAP_MAX_TOKENS);
-  return M <= (K > 2048 ? 64 : 32);
+  if (K > 8192) return M <= (epilogue == EPI_RESIDUAL && N >= 2048 && N <= 8192 ? 128 : SWAP_MAX_TOKENS);
+  if (K <= 2048) return M <= 32;
+  return M <= (K <= 5632 || N <= 2048 || N >= 8192 ? 64 : 128);
 }
 
 // out = epilogue(A[M,K] W[N,K]^T), bf16 operands. workspace/counters: scratch for tiles split along K
@@ -1179,7 +1182,7 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
   }
   const int out_bytes = out_dtype == CUCA_F32 ? 4 : 2;
   const bool rows_of_16_bytes = ((uintptr_t)out & 15) == 0 && ((size_t)ldo * out_bytes) % 16 == 0;
-  const bool swap = swapped(M, K, epilogue, rows_of_16_bytes);
+  const bool swap = swapped(M, N, K, epilogue, rows_of_16_bytes);
   const int bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
   const uint64_t w_rows = (uint64_t)N * (dual ? 2 : 1);
   CUtensorMap tmA, tmB, tmO;
@@ -1271,7 +1274,8 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
   // SMs but no time, while K slices added up by the last to arrive cost 40 us more than their share of K. Measured, us
   // (slices, pieces): K = 2,048, 256 tokens, N = 2,048 53, 16.4; N = 256 63, 16.4; 1,000 tokens, N = 256 55, 16.4; K = 8,192, N =
   // 2,048, 256 tokens 58, 38.9; into the stream, K = 4,096, N = 1,024 109, 23.6. At K = 14,336 pieces gain nothing. Cutting the
-  // last round of many tiles this way gains nothing either and is not done.
+  // last round of many tiles this way gains nothing either and is not done. SwiGLU's tiles are not cut, only left whole, up to
+  // K = 4,096 (2 x 2,048 rows, 128 tokens, K = 2,048 42.9, 24.0; 4,096 45.7, 35.6; 8,192 51.8, 59.3).
   bool pieced = false;
   if (tall) {
     // whole tiles in turn, nothing split
@@ -1287,7 +1291,7 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
       grid = pieces;
     }
   }
-  if (pieced || tall || (!swap && p.tiles < sms && p.ksteps <= 128)) {
+  if (pieced || tall || (!swap && p.tiles < sms && p.ksteps <= (dual ? 64 : 128))) {
     // nothing is split along K
   } else if (epilogue == EPI_PARTIAL) {
     CUCA_REQUIRE(swap && out_dtype == CUCA_F32 && bias == nullptr && n_slices_out != nullptr,
@@ -1308,10 +1312,13 @@ static int gemm_tc_impl(const void* A, const void* W, const void* bias, void* ou
     // If a whole number of CTAs per tile fills most of the GPU, every CTA gets one even K slice of one tile (one
     // accumulator drain each); else the K steps are dealt out evenly across tile borders.
     const int per_tile = sms / p.tiles;
-    if (swap && bn > 16 && 20 * p.tiles >= 8 * sms && p.tiles < sms) {
-      // Tiles for 40 % of the SMs and more over 17 to 64 tokens: one whole tile per CTA. What the last to arrive has to add grows
-      // with the tokens (measured in a chain of launches, us, K shared out and whole: SwiGLU of 2 x 11,008 x 4,096, 86 tiles, 24
-      // tokens 38.1, 34.5; 64 tokens 51.8, 39.7; 2 x 8,192 x 2,048, 64 tiles, 18.8, 17.7 and 25.5, 23.0; up to 16 tokens equal).
+    if (swap && bn > 16 && 5 * p.tiles >= 2 * sms && p.tiles < sms && p.ksteps <= (per_tile == 1 ? 176 : 32)) {
+      // Tiles for two fifths of the SMs and more over 17 tokens and more: one whole tile per CTA. What the last to arrive has to
+      // add grows with the tokens, and with the tiles where K is dealt out across their borders; two even slices of a long K
+      // (tiles for up to half of the SMs) gain more than that. Measured in a chain of launches, us, K shared out and whole: SwiGLU
+      // of 2 x 11,008 x 4,096, 86 tiles, 24 tokens 38.8, 33.1; 64 tokens 52.5, 38.3; 2 x 8,192, 64 tiles, 24 tokens, K = 2,048 19.6, 17.9,
+      // 4,096 28.2, 29.8; stored, N = 11,008, 17 tokens, K = 4,096 23.4, 20.5, 11,008 46.6, 46.2, 14,336 57.1, 60.2; N = 8,192, K = 2,048
+      // 13.3, 12.2, 5,632 22.5, 25.0, 14,336 43.4, 55.7; up to 16 tokens equal.
       grid = p.tiles;
     } else if (per_tile >= 1 && (long long)per_tile * p.tiles * 4 >= 3LL * sms && p.ksteps >= 2 * per_tile) {
       size_t need = (size_t)p.tiles * per_tile * ncols * TILE_A * sizeof(float);

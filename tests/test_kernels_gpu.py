@@ -938,6 +938,15 @@ def test_rope_store_from_partial_sums(dev):
         assert torch.allclose(vpool[page, :, off].float(), heads[nh + nkv:], atol=3e-2, rtol=3e-2)
 
 
+# what of N and K decides too: 65 to 128 tokens behind K = 5,632 (N above 2,048, below 8,192), more of them behind 8,192 (N from
+# 2,048 to 8,192), whole tiles for two fifths of the SMs (K up to 2,048 and 11,264), SwiGLU's (K up to 4,096)
+@pytest.mark.parametrize("M,N,K", [(65, 2112, 5640), (128, 8192, 5696), (160, 2040, 8200), (129, 2112, 8200), (40, 8192, 2048),
+                                   (40, 8192, 2056), (17, 9728, 2056), (100, 200, 4096), (100, 200, 4104)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+def test_gemm_tcgen05_where_its_form_changes_with_n_and_k(dev, M, N, K, epilogue):
+    test_gemm_tcgen05_where_its_form_changes(dev, M, N, K, epilogue)
+
+
 @pytest.mark.parametrize("d,n_slices", [(128, 3), (64, 1), (8, 5), (72, 4)])
 @pytest.mark.parametrize("with_bias", [False, True])
 def test_rope_store_partial_sixteen_bytes_at_a_time(dev, d, n_slices, with_bias):
