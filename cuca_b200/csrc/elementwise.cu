@@ -907,7 +907,8 @@ __global__ void rope_store_partial_kernel(const float* __restrict__ partial, int
 // The same where whole heads are rotated and rows come in 16-byte pieces: a thread has four columns of each half of a head, so
 // that a block holds eight heads of 128 of a row, and asks for its slices before it looks up where they go. Bound by the
 // round trips of one block (lookups, slices); with a block of 64 threads a head and one value a load, 203 rows of 48 heads
-// of 128 in three slices took 12.2 us, this way 4.4.
+// of 128 in three slices took 12.2 us, this way 4.4. AHEAD: slices whose loads are in flight at once.
+template <int AHEAD>
 __global__ void __launch_bounds__(128)
 rope_store_partial_vec_kernel(const float* __restrict__ partial, int n_slices, size_t slice_stride,
                               const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ q_out,
@@ -931,10 +932,10 @@ rope_store_partial_vec_kernel(const float* __restrict__ partial, int n_slices, s
       b[i] = __bfloat162float(bias[(size_t)head * d + half + o + i]);
     }
   }
-  for (int k0 = 0; k0 < n_slices; k0 += 4) {  // four slices' loads in flight at once, added in slice order
-    float4 x[4], y[4];
+  for (int k0 = 0; k0 < n_slices; k0 += AHEAD) {  // added in slice order
+    float4 x[AHEAD], y[AHEAD];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < AHEAD; ++u) {
       x[u] = y[u] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (k0 + u < n_slices) {
         x[u] = __ldcg(reinterpret_cast<const float4*>(src + (k0 + u) * slice_stride));
@@ -942,7 +943,7 @@ rope_store_partial_vec_kernel(const float* __restrict__ partial, int n_slices, s
       }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < AHEAD; ++u) {
       a[0] += x[u].x; a[1] += x[u].y; a[2] += x[u].z; a[3] += x[u].w;
       b[0] += y[u].x; b[1] += y[u].y; b[2] += y[u].z; b[3] += y[u].w;
     }
@@ -995,7 +996,8 @@ CUCA_API int cuca_rope_store_partial(const float* partial, int n_slices, size_t 
   if (rot == d && d % 8 == 0 && slice_stride % 4 == 0 &&
       (((uintptr_t)partial | (uintptr_t)cos_t | (uintptr_t)sin_t | (uintptr_t)q_out | (uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0) {
     const int blocks = ((nh + 2 * nkv) * (d / 8) + 127) / 128;
-    cuca_launch(rope_store_partial_vec_kernel, dim3(n_rows, blocks), dim3(128), 0, stream, true, partial, n_slices, slice_stride,
+    auto kernel = n_slices > 4 ? rope_store_partial_vec_kernel<8> : rope_store_partial_vec_kernel<4>;
+    cuca_launch(kernel, dim3(n_rows, blocks), dim3(128), 0, stream, true, partial, n_slices, slice_stride,
                 (const __nv_bfloat16*)bias, (__nv_bfloat16*)q_out, positions, seq_of_row, tables, table_stride, cos_t, sin_t,
                 table_rows, (__nv_bfloat16*)kpool, (__nv_bfloat16*)vpool, n_blocks, bs, nh, nkv, d, err);
     CUCA_CHECK_LAUNCH("rope_store_partial");

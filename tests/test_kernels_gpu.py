@@ -1025,6 +1025,12 @@ def test_attention_prefill_tcgen05(dev, nh, nkv, bs, window, d, two_tiles_per_ct
         assert torch.allclose(got, want, atol=2e-2, rtol=2e-2), (r, s, pos, float((got - want).abs().max()))
 
 
+@pytest.mark.parametrize("n_slices", [6, 8, 13])
+def test_rope_store_partial_of_many_slices(dev, n_slices):
+    """More than four slices: eight at a time."""
+    test_rope_store_partial_sixteen_bytes_at_a_time(dev, 128, n_slices, True)
+
+
 @pytest.mark.parametrize("d", [128, 64])
 @pytest.mark.parametrize("two_tiles_per_cta", [False, True])
 def test_attention_prefill_tcgen05_two_heads_a_cta(dev, d, two_tiles_per_cta):
