@@ -361,12 +361,13 @@ class AttentionPlan:
         self.static = step.static_max_len is not None
         if self.static:
             self.n_decode, self.max_len = step.n_rows, step.static_max_len
-            self.n_portions = 0
+            self.n_portions = self.portion_keys = 0
         else:
             starts = step.host["starts"]
             single = [s + 1 for c, s in zip(counts, starts) if c == 1]
             self.n_decode, self.max_len = len(single), max(single, default=1)
             self.n_portions = len(counts) - self.n_decode
+            self.portion_keys = max((s + c for c, s in zip(counts, starts) if c > 1), default=0)  # the most that one sees
         self.identity = self.n_portions == 0  # every row is a single token: decode rows are 0..rows-1
         self._counts = counts
         self._decode_rows = None
@@ -1053,6 +1054,10 @@ def latent_attention(qk, out, cache, step, H, rank, Dk, scale, window, err, sink
                 int(window or 0), sink, splits, _p(acc), _p(ml), _p(err), _stream()), "latent_attention_mma")
         if plan.n_portions:
             tokens = latent_attention_tc_tokens(H, rank, Dk, scale)
+            # the tcgen05 form moves 16 bytes at a time, and its start costs more than it saves where rows are narrow and no portion
+            # sees more than a tile of keys (8 heads, 64 values, 2 tokens 5.2 us against 6.8; 16 heads, 192 values 7.7, 8.5)
+            if (qk.data_ptr() | out.data_ptr() | pool.data_ptr()) % 16 or (Dk <= 192 and plan.portion_keys <= 64):
+                tokens = 0
             row0, nrows, n = plan.tiles(tokens or LATENT_TILE_ROWS)
             if tokens:
                 library.check(lib.cuca_latent_attention_tc(

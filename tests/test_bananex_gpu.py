@@ -514,6 +514,32 @@ def test_latent_attention_in_groups_of_tokens_and_heads(layer, tokens):
     test_latent_attention_on_tensor_cores(layer)
 
 
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("portions", [[(0, 40), (5, 2)], [(0, 70), (30, 34), (0, 64)]])
+def test_latent_attention_of_operands_off_16_bytes_and_of_few_keys(off, portions):
+    """Where the tcgen05 form does not take the addresses, or is not worth its start, the other tensor-core form runs. Against the
+    plain kernel; queries and weights are bfloat16 numbers (2^-9), the values of a row at most their maximum."""
+    from cuca_b200.cache.device import CacheView
+    from cuca_b200.kernels import ops
+    dev, H, rank, rot, bs = torch.device("cuda:0"), 8, 64, 64, 16
+    Dk, n = rank + rot, sum(c for _, c in portions)
+    g = torch.Generator(device=dev).manual_seed(n)
+    step = _step(dev, portions, list(range(len(portions))))
+    pool = torch.randn(32, 1, bs, Dk, device=dev, generator=g).to(torch.bfloat16)
+    tables = torch.randperm(32, device=dev, generator=g).to(torch.int32)[:len(portions) * 8].view(-1, 8).contiguous()
+    qk = torch.empty(n * H * Dk + off, device=dev)[off:].view(n, H, Dk).normal_(generator=g)
+    cache, err, got = CacheView(pool, None, tables, bs, 0, None, step.slots), torch.zeros(1, dtype=torch.int32, device=dev), []
+    for tensor_cores in (True, False):
+        out = torch.full((n * H * rank + off,), 9.0, device=dev)[off:].view(n, H, rank)
+        ops.USE_MMA_LATENT = tensor_cores
+        try:
+            ops.latent_attention(qk, out, cache, step, H, rank, Dk, 0.1, None, err)
+        finally:
+            ops.USE_MMA_LATENT = True
+        got.append(out)
+    assert int(err.item()) == 0 and (got[0] - got[1]).abs().max() < 2e-2 * got[1].abs().max()
+
+
 def test_dense_feed_forward_and_loop_entry_alone(rt32):
     from cuca_b200.parts.base import PartSpec
     from cuca_b200.parts.mlp import DenseActivation
