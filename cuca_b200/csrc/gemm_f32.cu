@@ -558,11 +558,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   if (p.slices > 1) cluster_sync_all();
   else __syncthreads();
   const int items = *abort_flag ? 0 : OUTS * min(NT, p.M - m0);
-  bool lossy = false;
-  if (C::P == 3) {
-    if (p.slices == 1) lossy = *any_lossy;
-    else lossy = __any_sync(0xffffffffu, ld_cluster_u32(smem_u32(any_lossy), lane % p.slices, 0));
-  }
+  uint32_t some_lossy = 0;  // (a CTA a lane)
+  if (C::P == 3) some_lossy = p.slices == 1 ? *any_lossy : ld_cluster_u32(smem_u32(any_lossy), lane % p.slices, 0);
   // a row's marks in all of K
   auto marks_of = [&](const uint32_t* at) {
     uint32_t word = *at;
@@ -581,29 +578,33 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       v = sums[0];
       if (dual) u = sums[16];
     } else if (live) {
-      bool started = false;
-      for (int s = 0; s < p.slices; ++s) {
-        const int have = (s + 1) * blocks / p.slices - s * blocks / p.slices;
-        for (int b0 = 0; b0 < have; b0 += 4) {
-          float x[4], y[4];
+      // eight blocks' sums in flight at once, whichever CTA holds them: one CTA's after the other took a round trip each
+      int s = 0, from = 0, to = blocks / p.slices;
+#pragma unroll 1
+      for (int b0 = 0; b0 < blocks; b0 += 8) {
+        float x[8], y[8];
 #pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const uint32_t at = (uint32_t)((min(b0 + b, have - 1) * NT + m) * ROWS + row) * 4;
-            x[b] = ld_cluster(smem_u32(smem), s, at);
-            if (dual) y[b] = ld_cluster(smem_u32(smem), s, at + 64);
+        for (int b = 0; b < 8; ++b) {
+          if (b0 + b >= blocks) break;
+          if (b0 + b == to) {
+            from = to;
+            ++s;
+            to = (s + 1) * blocks / p.slices;
           }
+          const uint32_t at = (uint32_t)(((b0 + b - from) * NT + m) * ROWS + row) * 4;
+          x[b] = ld_cluster(smem_u32(smem), s, at);
+          if (dual) y[b] = ld_cluster(smem_u32(smem), s, at + 64);
+        }
 #pragma unroll
-          for (int b = 0; b < 4; ++b)
-            if (b0 + b < have) {
-              v = started ? v + x[b] : x[b];
-              if (dual) u = started ? u + y[b] : y[b];
-              started = true;
-            }
+        for (int b = 0; b < 8; ++b) {
+          if (b0 + b >= blocks) break;
+          v = b0 + b > 0 ? v + x[b] : x[b];
+          if (dual) u = b0 + b > 0 ? u + y[b] : y[b];
         }
       }
     }
     uint32_t token = 0, weight = 0, up_weight = 0;
-    if (lossy && live) {
+    if (__any_sync(0xffffffffu, some_lossy) && live) {
       token = marks_of(&token_marks[m]);
       weight = marks_of(&row_marks[row]);
       if (dual) up_weight = marks_of(&row_marks[row + 16]);
