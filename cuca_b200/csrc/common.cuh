@@ -42,7 +42,9 @@ extern "C" const char* cuca_last_error();
 // Programmatic dependent launch: a kernel launched with the attribute may start while its predecessor in
 // the stream still runs. pdl_trigger() lets the successor's CTAs become resident early; pdl_wait() blocks
 // until the predecessor has completed and its writes are visible. Every kernel calls pdl_wait() in every CTA
-// before it reads or writes anything an earlier kernel touches (both are no-ops without the attribute).
+// before it reads or writes anything an earlier kernel touches (both are no-ops without the attribute). The contractions
+// alone ask for their weights before it: those must not be the output of the kernel launched just before (nor of one still
+// running then), as gemm_tc, gemm_partial and, up to 16 tokens, gemm_simt say.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -43,6 +43,7 @@ constexpr int ROWS = TILE_A;          // weight rows of a tile
 constexpr int ROW_BYTES = CHUNK * 2;  // one row of one part in shared memory: one swizzle span
 constexpr int MAX_CLUSTER = 8;
 constexpr int PRE_TOKENS = 32;        // tiles of so many tokens and more take the tokens' parts from memory
+constexpr int FEW_TOKENS = 16;        // up to here 16-byte copies of the weights start before the kernel ahead is done
 constexpr int SPLIT_RUN = 2048;       // elements of a row that one block of `split_kernel` takes
 
 template <typename TI> struct Parts { static constexpr int N = 3; };
@@ -318,8 +319,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   const uint32_t tmem = *tmem_slot;
 
   if (warp == C::LOAD_WARP) {
-    // ---- weights into the ring; they are no earlier kernel's output, so no predecessor is waited for
+    // ---- weights into the ring. Over few tokens no predecessor is waited for: there the weights must not be its output. Beyond,
+    // where a launch's time is not that of the weights' first copies, and in the form through registers, they may be.
     if (VEC && lane == 0) {
+      if (p.M > FEW_TOKENS) pdl_wait();
       const uint64_t once = l2_evict_first();
       for (int c = first, i = 0; c < last; ++c, ++i) {
         const int s = i % C::RAWS;
@@ -447,6 +450,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const TI* w_row = (const TI*)p.W + (size_t)(dual && (lane & 16) ? p.N + w_n : w_n) * p.K;
     const uint32_t a_at = tmem + ((uint32_t)(quarter * 32) << 16) + C::A_AT + half * 16;
     Marks marks;
+    if (!VEC) pdl_wait();
     for (int c = first + set, n = set; c < last; c += C::SETS, n += C::SETS) {
       const int st = n % C::STAGES, raw = n % C::RAWS;
       uint32_t w[C::P][16];
@@ -744,7 +748,7 @@ int go(const GemmParams& p, void* scratch, int form_tokens, int form_slices, cud
 
 // Most tokens for which cuca_gemm_f32 needs no scratch. Beyond, for each token so many 16-bit values, the whole 16-byte aligned:
 // its parts, three of 32-bit operands and one of 16-bit ones, each K rounded up to a multiple of 8, and its marks.
-CUCA_API int cuca_gemm_f32_few_tokens() { return 16; }
+CUCA_API int cuca_gemm_f32_few_tokens() { return FEW_TOKENS; }
 CUCA_API int cuca_gemm_f32_scratch_per_token(int in_dtype, int K) {
   return (in_dtype == CUCA_F32 ? 3 : 1) * scratch_ld(K) + (K + SPLIT_RUN - 1) / SPLIT_RUN;
 }

@@ -160,8 +160,9 @@ _gemm_few: list = []  # most tokens that `gemm_simt` takes without scratch
 
 def gemm_simt(a, w, out, epilogue=EPI_STORE, bias=None, err=None, form=(0, 0)) -> None:
     """out = epilogue(a @ w.T) with 32-bit accuracy; a: [M, K] (row stride >= K), w: [N or 2N, K], both 32-bit or both
-    16-bit, of any size and alignment. A row's result is the same bits whatever M is. `form`: tokens of a tile and CTAs that
-    share its K (tests; 0: the library's choice)."""
+    16-bit, of any size and alignment. A row's result is the same bits whatever M is. Up to 16 rows a 32-bit `w` must not be the
+    output of the launch just before: it is read ahead. `form`: tokens of a tile and CTAs that share its K (tests; 0: the
+    library's choice)."""
     _cuda(a, w, out)
     lib = library.load()
     M, K = a.shape
@@ -265,7 +266,8 @@ def gemm_tc_supported(a, w) -> bool:
 
 
 def gemm_tc(a, w, out, epilogue=EPI_STORE, bias=None, err=None, max_splits=16) -> None:
-    """out = epilogue(a @ w.T) on the tcgen05 tensor cores; bf16 operands, K and the row stride multiples of 8."""
+    """out = epilogue(a @ w.T) on the tcgen05 tensor cores; bf16 operands, K and the row stride multiples of 8. `w` must not be
+    the output of the launch just before: it is read ahead."""
     _cuda(a, w, out)
     lib = library.load()
     M, K = a.shape
@@ -339,7 +341,7 @@ def gemm_pair_mode(mode: int) -> None:
 
 def gemm(a, w, out, epilogue=EPI_STORE, bias=None, err=None) -> None:
     """out = epilogue(a @ w.T), on the kernel that fits dtype and shape: `gemm_tc` for bfloat16 (rows of 16-byte
-    multiples), `gemm_simt` for the 32-bit path and for shapes the former refuses."""
+    multiples), `gemm_simt` for the 32-bit path and for shapes the former refuses. `w` as in those."""
     if a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16) \
             and gemm_tc_supported(a, w):
         gemm_tc(a, w, out, epilogue, bias, err)
@@ -801,7 +803,7 @@ _SLICES_WRITTEN_AT = ctypes.addressof(_slices_written)
 
 
 def gemm_partial(a, w, err=None, max_slices=16) -> PartialSums:
-    """a @ w.T for few rows (`partial_max_tokens`), as partial sums over K slices (see `PartialSums`)."""
+    """a @ w.T for few rows (`partial_max_tokens`), as partial sums over K slices (see `PartialSums`); `w` as in `gemm_tc`."""
     _cuda(a, w)
     lib = library.load()
     M, K = a.shape

@@ -132,6 +132,23 @@ def test_gemm_f32_every_form_gives_the_same_bits(dev, M, N, K, epilogue):
             assert torch.equal(out.isnan(), y.isnan()) and torch.equal(out.isinf() & (out > 0), y.isinf() & (y > 0)), (tokens, slices)
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 200, 512), (70, 600, 2048), (700, 300, 1024), (3, 2048, 1022), (40, 300, 1022)])
+def test_gemm_f32_with_the_output_before_as_weights(dev, M, N, K):
+    """Beyond 16 tokens, and through registers, weights that the launch just before wrote are read after it is done."""
+    from cuca_b200.kernels import ops
+    g = torch.Generator(device=dev).manual_seed(M + K)
+    a, u, v = (torch.randn(*s, device=dev, generator=g) for s in ((M, K), (N, 4096), (K, 4096)))
+    w, out, want = torch.zeros(N, K, device=dev), torch.empty(M, N, device=dev), torch.empty(M, N, device=dev)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        w.zero_()
+        ops.gemm_simt(u, v, w, 0)
+        ops.gemm_simt(a, w, out, 0)
+        torch.cuda.synchronize()
+        ops.gemm_simt(a, w, want, 0)
+        assert torch.equal(out, want) and bool(want.any())
+
+
 @pytest.mark.parametrize("K", [4, 64, 300, 1030, 2048])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gemm_f32_is_exact_where_32_bits_are(dev, K, dtype):
