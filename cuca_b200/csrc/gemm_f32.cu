@@ -23,7 +23,8 @@
 // warps over few tokens, or by a kernel of its own before (`split_kernel`) from 17 tokens on, since every block of weight rows
 // reads them; eight or four warps add the chunks' sums up. Few tiles: a cluster of up to eight CTAs shares a tile's K, each
 // keeps its blocks' sums, and all add them in order out of each other's shared memory. Operands that take no copies
-// (16-bit ones, K or a row stride not a multiple of 4, an address off 16 bytes) come through registers with the same results.
+// (16-bit ones, K or a row stride not a multiple of 4, an address off 16 bytes) come element by element with the same results:
+// 4,096 x 4,090, us, multiply-adds and this: 2,048 tokens 32-bit 2,398, 799, 16-bit 2,018, 1,153; 16 tokens 244, 37 and 240, 38.
 //
 // Epilogues: store (optional bias), add into the 32-bit residual stream, or SwiGLU over a stacked [gate; up] weight (rows
 // 0..N-1 gate, N..2N-1 up).
@@ -112,6 +113,10 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
       ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
       "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid) {
+  const int n = valid ? 4 : 0;  // 0: nothing is read and the 4 bytes become zeros
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -446,12 +451,32 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const int l = quarter * 32 + lane;
     const int raw_row = dual ? quarter * 16 + (lane & 15) + (lane & 16) * 4 : l;  // 16 gate rows and their 16 up rows take turns
     const uint32_t raw_at = (half * 2 + (raw_row >> 6)) * (C::RAW / 4) + (raw_row & 63) * 128;
-    const int w_n = min(dual ? n0 + quarter * 16 + (lane & 15) : n0 + l, p.N - 1);
-    const TI* w_row = (const TI*)p.W + (size_t)(dual && (lane & 16) ? p.N + w_n : w_n) * p.K;
+    // Operands that take no 16-byte copies: an element of each of 32 rows a lane, neighbours side by side, into this warp's own part
+    // of the ring's memory, from where a lane reads its row: 32-bit ones by copies of 4 bytes a chunk ahead, 16-bit ones through
+    // registers. (A lane that reads its row from memory asks for 32 lines an instruction, 4 us a chunk.)
+    constexpr int PITCH = 36, BUFFERS = sizeof(TI) == 4 ? 2 : 1;
+    TI* mine = reinterpret_cast<TI*>(smem) + cw * BUFFERS * 32 * PITCH;
+    static_assert(C::A_WARPS * BUFFERS * 32 * PITCH * 4 <= C::RAWS * C::RAW, "the warps' parts of the ring's memory");
+    TI held[VEC || BUFFERS == 2 ? 1 : 32];
+    auto fetch = [&](int c, int buffer) {
+      const int k = c * CHUNK + half * 32 + lane;
+      const bool there = k < p.K;
+#pragma unroll
+      for (int r = 0; r < 32 && c < last; ++r) {  // (behind the last chunk nothing: the sums are put where it would land)
+        const int n = min(dual ? n0 + quarter * 16 + (r & 15) : n0 + quarter * 32 + r, p.N - 1);
+        const TI* src = (const TI*)p.W + (there ? (size_t)(dual && (r & 16) ? p.N + n : n) * p.K + k : 0);
+        if constexpr (BUFFERS == 2) cp_async4(mine + (buffer * 32 + r) * PITCH + lane, src, there);
+        else held[r] = there ? __ldg(src) : TI(0.f);
+      }
+      if (BUFFERS == 2) asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     const uint32_t a_at = tmem + ((uint32_t)(quarter * 32) << 16) + C::A_AT + half * 16;
     Marks marks;
-    if (!VEC) pdl_wait();
-    for (int c = first + set, n = set; c < last; c += C::SETS, n += C::SETS) {
+    if constexpr (!VEC) {
+      pdl_wait();
+      fetch(first + set, 0);
+    }
+    for (int c = first + set, n = set, buffer = 0; c < last; c += C::SETS, n += C::SETS, buffer ^= BUFFERS - 1) {
       const int st = n % C::STAGES, raw = n % C::RAWS;
       uint32_t w[C::P][16];
       if constexpr (VEC) {
@@ -467,11 +492,20 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(&raw_empty[raw]);
       } else {
+        if constexpr (BUFFERS == 2) {
+          fetch(c + C::SETS, buffer ^ 1);
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+          __syncwarp();
+        } else {
+#pragma unroll
+          for (int r = 0; r < 32; ++r) mine[r * PITCH + lane] = held[r];
+          __syncwarp();
+          fetch(c + C::SETS, 0);
+        }
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const int k = c * CHUNK + half * 32 + 4 * q;
           uint2 x[C::P];
-          split(x, load4<false>(w_row + k, p.K - k), marks);
+          split(x, *reinterpret_cast<const decltype(load4<false>((const TI*)p.W, 0))*>(mine + (buffer * 32 + lane) * PITCH + 4 * q), marks);
 #pragma unroll
           for (int t = 0; t < C::P; ++t) w[t][2 * q] = x[t].x, w[t][2 * q + 1] = x[t].y;
         }
@@ -485,6 +519,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[st]);
     }
+    if (!VEC && BUFFERS == 2) asm volatile("cp.async.wait_all;" ::: "memory");
     if (C::P == 3) note(&row_marks[l], marks.word());
   } else {
     // ---- sums: thread = weight row, COLS tokens
