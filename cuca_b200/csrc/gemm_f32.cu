@@ -736,29 +736,32 @@ bool holds(int K, int slices) {
   return slices == 1 || (slices > 1 && slices <= std::min(MAX_CLUSTER, blocks) && (blocks + slices - 1) / slices <= Form<TI, NT>::BLOCKS_HELD);
 }
 
-// The form with the least estimated time: rounds of CTAs times a CTA's chunks, whose cost in us (`chunk_us`) was measured as
-// the slope over K; 4 us a launch, one more for a cluster's two barriers and reads, 3 for the tokens' split. Measured, us:
-// K = 8,192, 2,048 rows, 4 tokens: 1, 4, 8 CTAs a tile 88, 37, 50 (128 CTAs in clusters of eight do not fit at once).
+// The form with the least estimated time: rounds of CTAs times a CTA's chunks, whose cost in us (`chunk_us`) was measured as the
+// slope over K, and a third more where narrow tiles of tokens read the same weights side by side; 3.5 us a launch, for a cluster
+// 1.3 more and 0.15 for every block's sums that are read across it, 3 for the tokens' split. Measured, us: K = 8,192, 2,048 rows, one
+// token: 1, 4, 6, 8 CTAs a tile 86, 30, 27, 41 (128 CTAs in clusters of eight do not fit at once); 24 tokens, tiles of 16 by 4 CTAs
+// 37.2, of 32 by 6 30.5; K = 2,048, 64 tokens, tiles of 16 by 2 21.3, of 32 by 4 16.1, of 64 by 5 19.5.
 struct Choice { int nt, slices; double cost; };
 template <typename TI, int NT, bool VEC>
 void consider(Choice& best, int M, int N, int K, bool dual, double chunk_us) {
   const int outs = dual ? ROWS / 2 : ROWS, blocks = (K + CHUNK * BLOCK - 1) / (CHUNK * BLOCK);
   const long long tiles = (long long)((M + NT - 1) / NT) * ((N + outs - 1) / outs);
+  if (NT <= 32 && M > NT) chunk_us *= 1.3;
   for (int s = 1; s <= MAX_CLUSTER; ++s) {
     const int per = (blocks + s - 1) / s;
     if (!holds<TI, NT>(K, s) || (s > 1 && (per == (blocks + s - 2) / (s - 1) || tiles * (s - 1) >= cuca_device_sms()))) continue;
     const int held = s > 1 ? clusters_held<TI, NT, VEC>(s) : cuca_device_sms();
-    const double cost = (double)((tiles + held - 1) / held) * (per * BLOCK * chunk_us + (s > 1 ? 5. : 4.)) + (Form<TI, NT>::PRE ? 3. : 0.);
+    const double cost = (double)((tiles + held - 1) / held) * (per * BLOCK * chunk_us + (s > 1 ? 4.8 + 0.15 * blocks : 3.5)) + (Form<TI, NT>::PRE ? 3. : 0.);
     if (cost < best.cost) best = {NT, s, cost};
   }
 }
 template <typename TI, bool VEC>
 Choice choose(int M, int N, int K, bool dual) {
   Choice best = {0, 1, 1e30};
-  consider<TI, 16, VEC>(best, M, N, K, dual, 0.52);
-  if (M > 16) consider<TI, 32, VEC>(best, M, N, K, dual, 0.68);
-  if (M > 32) consider<TI, 64, VEC>(best, M, N, K, dual, 0.76);
-  if (M > 64) consider<TI, 96, VEC>(best, M, N, K, dual, 1.1);
+  consider<TI, 16, VEC>(best, M, N, K, dual, 0.64);
+  if (M > 16) consider<TI, 32, VEC>(best, M, N, K, dual, 0.7);
+  if (M > 32) consider<TI, 64, VEC>(best, M, N, K, dual, 0.92);
+  if (M > 64) consider<TI, 96, VEC>(best, M, N, K, dual, 1.13);
   return best;
 }
 
