@@ -1055,6 +1055,55 @@ def test_attention_prefill_tcgen05_two_heads_a_cta(dev, d, two_tiles_per_cta):
     test_attention_prefill_tcgen05(dev, 32, 8, 16, 150, d, two_tiles_per_cta)
 
 
+@pytest.mark.parametrize("nh,nkv,bs,window", [(20, 10, 8, None), (24, 2, 32, None), (32, 16, 64, 40)])
+@pytest.mark.parametrize("d", [128, 64])
+@pytest.mark.parametrize("two_tiles_per_cta", [False, True])
+def test_attention_prefill_tcgen05_two_heads_a_cta_of_all_pages(dev, nh, nkv, bs, window, d, two_tiles_per_cta):
+    """The same over pages of 8, 32 and 64 keys, groups of exactly two and of twelve heads, with and without a window."""
+    test_attention_prefill_tcgen05(dev, nh, nkv, bs, window, d, two_tiles_per_cta)
+
+
+@pytest.mark.parametrize("options", [{}, {"softcap": 20.0, "sink": True, "sinks": True}, {"sink": True, "window": 150},
+                                     {"window": 70, "keep_first": 3, "softcap": 5.0}, {"slopes": True}, {"gate": True, "window": 130},
+                                     {"key_scale": True}])
+@pytest.mark.parametrize("nh,nkv,bs", [(20, 10, 8), (24, 6, 64)])
+@pytest.mark.parametrize("d", [128, 64])
+def test_attention_prefill_tcgen05_one_or_two_heads_a_cta_are_the_same_bits(dev, options, nh, nkv, bs, d):
+    """All tiles in one launch, more of them than SMs with their heads, go two heads a CTA, a launch for each tile one head."""
+    from cuca_b200.kernels import ops
+    lens, starts = [5, 200, 390, 131, 420], [0, 33, 129, 129, 0]
+    _, _, kpool, vpool, tables = _paged_setup(dev, torch.bfloat16, lens, nh, nkv, d, bs, n_blocks=sum(-(-n // bs) for n in lens) + 3, seed=nh + bs)
+    g = torch.Generator(device=dev).manual_seed(d)
+    rows, seqs, tiles = [], [], []
+    for s, (n, st) in enumerate(zip(lens, starts)):
+        tiles += [(len(rows) + off, min(128, n - st - off)) for off in range(0, n - st, 128)]
+        rows += list(range(st, n))
+        seqs += [s] * (n - st)
+    assert len(tiles) * nh > ops.sm_count()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)  # noqa: E731
+    row0, count, positions, seq = i32([t[0] for t in tiles]), i32([t[1] for t in tiles]), i32(rows), i32(seqs)
+    q = torch.randn(len(rows), nh * d, device=dev, generator=g).bfloat16()
+    o = dict(options)
+    window = o.pop("window", None)
+    if o.pop("sinks", False):
+        o["sink_values"] = torch.randn(nh, device=dev, generator=g)
+    if o.get("slopes"):
+        o["slopes"] = torch.rand(nh, device=dev, generator=g)
+    if o.get("gate"):
+        o["gate"] = torch.randn(len(rows), nh * d, device=dev, generator=g).bfloat16()
+    if o.get("key_scale"):
+        vpool, o["key_scale"] = kpool, torch.rand(kpool.shape[:3], device=dev, generator=g) + 0.5
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+
+    def launch(out, first, n):
+        ops.attention_prefill_tc(q, out, kpool, vpool, positions, seq, tables, row0[first:], count[first:], n, nh, nkv, d, 0.3, window, err, **o)
+    two, one = torch.zeros(len(rows), nh * d, device=dev, dtype=torch.bfloat16), torch.zeros(len(rows), nh * d, device=dev, dtype=torch.bfloat16)
+    launch(two, 0, len(tiles))
+    for i in range(len(tiles)):
+        launch(one, i, 1)
+    assert int(err.item()) == 0 and bool(two.any(1).all()) and torch.equal(two, one)
+
+
 @pytest.mark.parametrize("E", [1024, 2048, 4096, 8192, 9000])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_rmsnorm_is_the_same_bits_wherever_it_reads_its_weights(dev, E, dtype):
