@@ -1,6 +1,8 @@
 """Bananex on the GPU against the plain implementation (`plain_bananex.py`): every mechanism alone, whole and cut,
 then whole models through the replayer in the four work splits, pages and slots used again, long decoding past
 every window, and greedy generation through the entry point and its scheduler."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -468,6 +470,7 @@ def test_state_scan_in_segments_beside_other_requests(rt32, counts, cut):
         at = torch.cat([torch.arange(f, f + counts[q], device=dev) for f, q in zip(first, which)])
         x, pr, st, y = xbc[at], proj[at], state.clone(), torch.full((len(at), H * P), 7.0, device=dev)
         step = _step(dev, [(0, counts[q]) for q in which], [slots[q] for q in which])
+        gc.collect()  # (what earlier tests left in cycles must not be freed in between)
         before = torch.cuda.memory_allocated()
         torch.cuda.reset_peak_memory_stats()
         ops.ssm_scan(x, pr, 0, bias, a_log, skip, st, y, step, H, P, N, G, segments=segments)
