@@ -16,7 +16,7 @@
 // one warp issues contractions, whatever is ready first; eight warps own the rows, two threads a row. A tile takes 4,150
 // clocks: 1,550 of scores and 520 of P V on the tensor pipe, and with two tiles' memory a tile's copies (2,500) start when the
 // P V two tiles before is done. A CTA's start, 288 KB of 32-bit queries, is 15 us of some 40. 2,048 tokens, 16 heads, 512 + 64,
-// window 1,024: 140 us (391 TFLOP/s); 16 tokens of a head a group on mma.sync 521.
+// window 1,024: 152 us (361 TFLOP/s); 16 tokens of a head a group on mma.sync 526.
 #include "tcgen05.cuh"
 #include <math.h>
 
@@ -85,14 +85,6 @@ __device__ __forceinline__ bool soft_vote(int quarter, bool ok) {
       "{\n.reg .pred p, q;\nsetp.ne.b32 p, %2, 0;\nbar.red.and.pred q, %1, 64, p;\nselp.u32 %0, 1, 0, q;\n}\n"
       : "=r"(both) : "r"(4 + quarter), "r"((uint32_t)ok) : "memory");
   return both != 0;
-}
-__device__ __forceinline__ void tmem_st16_raw(uint32_t taddr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -371,7 +363,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const Params
         sum2[e & 1] = __fadd2_rn(sum2[e & 1], p2);
         pw[e] = pack_bf16(p2.x, p2.y);
       }
-      tmem_st16_raw(s_at + half * 16, pw);
+      tmem_st16(s_at + half * 16, pw);
       l = l * corr + (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
       m = m_new;
       // the P V before this one has finished before O is rescaled (its phase is awaited every time, so that the barrier never
