@@ -960,10 +960,12 @@ def _host_counts(step):
 
 def ssm_cut_from(step, H: int, P: int, N: int) -> int:
     """From how many tokens on `ssm_scan` is better off with this step's portions in segments (0: with none)."""
-    counts = _host_counts(step)
-    if counts is None:
-        return 0
-    return int(library.load().cuca_ssm_cut_from(ctypes.addressof(counts), step.n_seqs, H, P, N))
+    key = ("ssm_cut_from", H, P, N)  # (the same for every layer of a step)
+    if key not in step.plans:
+        counts = _host_counts(step)
+        step.plans[key] = 0 if counts is None else int(
+            library.load().cuca_ssm_cut_from(ctypes.addressof(counts), step.n_seqs, H, P, N))
+    return step.plans[key]
 
 
 def ssm_scan(xbc, proj, dt_col, dt_bias, a_log, d_skip, state, y, step, H, P, N, G, segments: int = 0) -> None:
