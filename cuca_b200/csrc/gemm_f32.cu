@@ -13,8 +13,8 @@
 // value has no parts) or a tiny one, and where values below 2^-110 that lost something in their parts (the converters note whose
 // rows have any) may matter beside it: see `settled`.
 // Error against 64 bits, relative 2-norm, normal values (multiply-adds in runs of 64 in brackets): K = 1 2.6e-8 (2.5e-8), 16
-// 3.6e-8 (7.4e-8), 2,048 9.8e-8 (1.8e-7), 8,192 1.3e-7 (2.5e-7); values of one sign, K = 64 7.9e-8 (1.2e-7), 256 8.1e-8
-// (7.0e-8), 2,048 8.2e-8 (8.1e-8), 8,192 1.0e-7 (1.5e-7). With one accumulator for all products and a unit in the last place given
+// 3.5e-8 (7.3e-8), 2,048 9.8e-8 (1.8e-7), 8,192 1.3e-7 (2.5e-7); values of one sign, where what is cut off adds up, K = 64
+// 9.0e-8 (1.2e-7), 256 9.1e-8 (7.3e-8), 2,048 9.3e-8 (9.2e-8), 8,192 1.2e-7 (1.8e-7). With one accumulator for all products and a unit in the last place given
 // back to every chunk for what is cut off, sums that are exact came out wrong (1 x 1) and K = 1 had 6.5e-8.
 //
 // The weights are the 128-row operand, the tokens the columns. A CTA (one an SM): the copy engine streams weight chunks
@@ -24,7 +24,7 @@
 // reads them; eight or four warps add the chunks' sums up. Few tiles: a cluster of up to eight CTAs shares a tile's K, each
 // keeps its blocks' sums, and all add them in order out of each other's shared memory. Operands that take no copies
 // (16-bit ones, K or a row stride not a multiple of 4, an address off 16 bytes) come element by element with the same results:
-// 4,096 x 4,090, us, multiply-adds and this: 2,048 tokens 32-bit 2,398, 799, 16-bit 2,018, 1,153; 16 tokens 244, 37 and 240, 38.
+// 4,096 x 4,090, us, multiply-adds and this: 2,048 tokens 32-bit 2,398, 650, 16-bit 2,018, 960; 16 tokens 244, 37 and 240, 38.
 //
 // Epilogues: store (optional bias), add into the 32-bit residual stream, or SwiGLU over a stacked [gate; up] weight (rows
 // 0..N-1 gate, N..2N-1 up).
