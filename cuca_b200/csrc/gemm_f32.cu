@@ -31,6 +31,7 @@
 #include "tcgen05.cuh"
 #include "f32x2.cuh"
 #include <algorithm>
+#include <type_traits>
 
 #define EPI_STORE 0
 #define EPI_RESIDUAL 1
@@ -63,10 +64,14 @@ struct GemmParams {
   int slices;   // CTAs of a cluster that share a tile's K
 };
 
+struct Marks;
+struct MarksByTwo;
+
 template <typename TI, int NT>
 struct Form {
   static constexpr int P = Parts<TI>::N;
   static constexpr bool PRE = NT >= PRE_TOKENS;  // the tokens' parts come from memory, else from converters of this kernel
+  using RowMarks = std::conditional_t<PRE, Marks, MarksByTwo>;
   // warps: sums, weight converters (eight a set; two sets take chunks in turn), the tokens' (converters, or one that copies),
   // the ring's loader, contractions
   static constexpr int EPI_WARPS = PRE ? 8 : 4;
@@ -129,7 +134,23 @@ constexpr uint32_t LOSSY = 1, LARGE = 2;
 struct Marks {
   uint32_t lost = 0;  // the third parts' bits, of which bfloat16 holds the upper half
   float most = 0.f;
+  __device__ __forceinline__ void see(float4 v, uint2) {
+    most = fmaxf(most, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+  }
   __device__ __forceinline__ uint32_t word() const { return (lost << 16 ? LOSSY : 0) | (most >= 1.09951163e12f ? LARGE : 0); }
+};
+// The same, the largest of the first parts, two a step: where the converters set the pace (tiles of 16 tokens: 2,048 x 8,192, a CTA a
+// tile, 86 -> 83 us; in tiles of 96, which have no registers for it, 320 -> 326).
+struct MarksByTwo {
+  uint32_t lost = 0;
+  __nv_bfloat162 most = __floats2bfloat162_rn(0.f, 0.f);
+  __device__ __forceinline__ void see(float4, uint2 part) {
+    most = __hmax2(most, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&part.x)));
+    most = __hmax2(most, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&part.y)));
+  }
+  __device__ __forceinline__ uint32_t word() const {
+    return (lost << 16 ? LOSSY : 0) | (__bfloat162float(__hmax(most.x, most.y)) >= 1.09951163e12f ? LARGE : 0);
+  }
 };
 // Whether a total stands. Finite, and not so small (2^-100) that products of small parts may have been lost; and where a row lost
 // something of its values, they met none of 2^40 or more and the total is no less than 2^-50, beside which K times 2^-93 is nothing.
@@ -209,17 +230,20 @@ __device__ __forceinline__ uint32_t upper_halves(float a, float b) {
   return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 // four elements' parts
-__device__ __forceinline__ void split(uint2 (&w)[3], float4 v, Marks& marks) {
-  marks.most = fmaxf(marks.most, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+template <typename M>
+__device__ __forceinline__ void split(uint2 (&w)[3], float4 v, M& marks) {
+  const float4 whole = v;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
     w[t].x = take_part(v.x, v.y);
     w[t].y = take_part(v.z, v.w);
   }
+  marks.see(whole, w[0]);
   marks.lost |= __float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w);
   w[2] = make_uint2(upper_halves(v.x, v.y), upper_halves(v.z, v.w));
 }
-__device__ __forceinline__ void split(uint2 (&w)[1], uint2 v, Marks&) { w[0] = v; }
+template <typename M>
+__device__ __forceinline__ void split(uint2 (&w)[1], uint2 v, M&) { w[0] = v; }
 __device__ __forceinline__ void clear(float4& v) { v = make_float4(0.f, 0.f, 0.f, 0.f); }
 __device__ __forceinline__ void clear(uint2& v) { v = make_uint2(0, 0); }
 
@@ -410,7 +434,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
       for (int i = 0; i < C::PASSES; ++i) held[i] = load(i, first);
       const uint32_t at0 = r0 * ROW_BYTES + ((kq / 8 ^ (r0 & 7)) << 4) + (kq & 4) * 2;
-      Marks marks[C::PASSES];
+      typename C::RowMarks marks[C::PASSES];
       for (int c = first, n = 0; c < last; ++c, ++n) {
         const int st = n % C::STAGES;
         if (VEC && (c + 1) * CHUNK > p.K && c * CHUNK + kq >= p.K) {
@@ -463,7 +487,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       if (BUFFERS == 2) asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const uint32_t a_at = tmem + ((uint32_t)(quarter * 32) << 16) + C::A_AT + half * 16;
-    Marks marks;
+    typename C::RowMarks marks;
     if constexpr (!VEC) {
       pdl_wait();
       fetch(first + set, 0);
